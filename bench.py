@@ -4,12 +4,12 @@
 crates/pir/src/pir_wrapper.rs:493-615) on B200s.
 
 Workload (one GPU): 2^22 entries of 2560 B, laid out by get_database_shape
-(256 full shards of 768 MiB, secondary group of order 2048).  As many distinct
+(256 full shards of 512 MiB as stored, secondary group of order 2048).  As many distinct
 shards as fit in HBM are preprocessed on the GPU from seeded uniform payloads
 and logical shard k is served by distinct shard k mod D, as the reference's
 --preprocessed-db-count does (pir_wrapper.rs:578).  A step is one query
 answered, one query per launch sequence (the plain path): decode, scan of all
-256 shards (206 GB), epilogue, secondary database build + key-switch chain,
+256 shards (137 GB), epilogue, secondary database build + key-switch chain,
 reply.  Every answer is decrypted by the client and compared with the stored
 entry.  The scan runs on the tensor engine (8-bit limb products on tcgen05)
 unless --engine cuda selects the CUDA-core engine; both give the same replies.
@@ -199,6 +199,14 @@ def int8_tensor_peak(torch, dev, n=8192, seconds=1.5):
     return out
 
 
+def stored_shard_bytes(dp, l1, device=0):
+    """Bytes of one preprocessed shard as a fleet stores it (one pass of the scan reads them once)."""
+    probe = dp.Fleet.general(dp.LOG2_N, l1, 8, 1, device=device)
+    n = probe.slab_bytes
+    probe.close()
+    return n
+
+
 def profiled_traffic(name, algo_bytes):
     """dram bytes per launch from a committed ncu summary (profiles/<name>):
     its measured ratio of dram bytes to algorithmic bytes (the captured launch
@@ -324,7 +332,7 @@ def serve_mix(args, local_rank, rates, seconds):
     t0 = time.time()
     for e in sizes:
         l1, l2, shards = dp.get_database_shape(e)
-        slab = dp.required_memory_general(11, l1) * 32
+        slab = stored_shard_bytes(dp, l1, local_rank)
         free, _ = torch.cuda.mem_get_info()
         d = shards if e < (1 << 22) else max(1, min(shards, int((free - (40 << 30)) // slab)))
         f = dp.Fleet(e, d, device=local_rank)
@@ -469,7 +477,7 @@ def workload_config(entries, l1, l2, shards, world):
         "query_bytes": 2 * 2048 * 50 // 8 + (2 if l1 == 2048 else 1) * 2048 * 34 // 8 +
                        (2 if l2 == 2048 else 1) * 2048 * 34 // 8,
         "reply_bytes": 22272,
-        "l2": "inputs larger than L2 (each step streams every shard slab: 206 GB at 2^22)",
+        "l2": "inputs larger than L2 (each step streams every shard slab: 137 GB at 2^22)",
         "parallelism": f"replica x{world}" if world > 1 else "single process"}
 
 
@@ -579,7 +587,7 @@ def batched_leg(dp, torch, dev, entries, engine, sizes, groups, check_every=8):
     sample of every group size."""
     l1, l2, shards = dp.get_database_shape(entries)
     per = 8 * l1
-    slab_bytes = dp.required_memory_general(11, l1) * 32
+    slab_bytes = stored_shard_bytes(dp, l1)
     t0 = time.time()
     fleet = dp.Fleet(entries, shards)
     if engine == "tensor":
@@ -788,7 +796,7 @@ def main():
     dev = torch.device("cuda", local_rank)
     l1, l2, shards = dp.get_database_shape(args.entries)
     per_shard_entries = 8 * l1
-    slab_bytes = dp.required_memory_general(11, l1) * 32
+    slab_bytes = stored_shard_bytes(dp, l1, local_rank)
     free, _ = torch.cuda.mem_get_info()
     sizes = [int(x) for x in args.batched.split(",") if x.strip()]
     # workspaces: two buffer slots, each with the scan output and the

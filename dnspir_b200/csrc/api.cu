@@ -225,6 +225,48 @@ int get_ctx(int device, DeviceCtx** out) {
   return DNSPIR_OK;
 }
 
+// Constants of the two-array scan (ScanConsts) from the a-parts in NTT form:
+// gk_a0, gk_a1 - 2^26 gk_a0, and the inverses of qry_a of both sets and halves,
+// in (sign, e) slot order.  na[set] = 3 when one of the set's slots is zero.
+static int build_scan_consts(const uint32_t* consts_dev, int log2n, uint32_t** out, uint32_t* na) {
+  const uint32_t n = 1u << log2n, two_n = 2 * n;
+  std::vector<uint32_t> c((size_t)12 * n), s((size_t)12 * n);
+  CK(cudaMemcpy(c.data(), consts_dev, c.size() * 4, cudaMemcpyDeviceToHost));
+  std::vector<uint32_t> pos(n);  // (sign, e) position -> bit-reversed slot position
+  uint32_t p5 = 1;
+  for (uint32_t e = 0; e < n / 2; e++) {
+    pos[e] = brv_host((p5 - 1) / 2, log2n);
+    pos[n / 2 + e] = brv_host((two_n - p5 - 1) / 2, log2n);
+    p5 = (uint32_t)(((uint64_t)p5 * 5) % two_n);
+  }
+  na[0] = na[1] = 2;
+  for (uint32_t pi = 0; pi < 2; pi++) {
+    const uint64_t p = pi ? P2 : P1, c26 = (1ull << LOG2_B) % p;
+    auto at = [&](int poly, uint32_t u) -> uint64_t { return c[((size_t)poly * 2 + pi) * n + pos[u]]; };
+    for (uint32_t u = 0; u < n; u++) {
+      s[(size_t)pi * n + u] = (uint32_t)at(0, u);
+      s[(size_t)(2 + pi) * n + u] = (uint32_t)((at(1, u) + p - at(0, u) * c26 % p) % p);
+    }
+    for (int poly = 2; poly < 6; poly++) {  // polynomial 2 + 2 set + half
+      // all inverses of the row with one exponentiation (products, then back)
+      std::vector<uint64_t> run(n + 1, 1);
+      for (uint32_t u = 0; u < n; u++) {
+        if (at(poly, u) == 0) na[(poly - 2) / 2] = 3;
+        run[u + 1] = run[u] * (at(poly, u) ? at(poly, u) : 1) % p;
+      }
+      uint64_t inv = invmod(run[n], p);
+      for (uint32_t u = n; u-- > 0;) {
+        const uint64_t v = at(poly, u);
+        s[(size_t)(2 * poly + pi) * n + u] = v ? (uint32_t)(inv * run[u] % p) : 0;
+        inv = inv * (v ? v : 1) % p;
+      }
+    }
+  }
+  CK(cudaMalloc(out, s.size() * 4));
+  CK(cudaMemcpy(*out, s.data(), s.size() * 4, cudaMemcpyHostToDevice));
+  return DNSPIR_OK;
+}
+
 // a-parts and the sigma_5 position map for ring dimension 2^log2n
 // a-parts in NTT form for the a-parts now in effect (rebuilt after
 // dnspir_set_a_parts; earlier buffers are kept, a kernel queued before the
@@ -245,7 +287,13 @@ static int ctx_a_parts(DeviceCtx* c, int log2n, uint64_t* version) {
   CK(cudaGetLastError());
   CK(cudaDeviceSynchronize());
   CK(cudaFree(dz));
+  uint32_t* ds = nullptr;
+  uint32_t na[2];
+  CKR(build_scan_consts(dc, log2n, &ds, na));
   if (c->consts[log2n]) c->retired.push_back(c->consts[log2n]);
+  if (c->scan[log2n]) c->retired.push_back(c->scan[log2n]);
+  c->scan[log2n] = ds;
+  c->scan_na[log2n][0] = na[0], c->scan_na[log2n][1] = na[1];
   c->consts[log2n] = dc;
   c->consts_ver[log2n] = ver;
   return DNSPIR_OK;
@@ -310,6 +358,16 @@ ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds) {
   return cc;
 }
 
+ScanConsts scan_consts(DeviceCtx* c, int log2n, int used_seeds) {
+  const size_t n2 = (size_t)2 << log2n;
+  ScanConsts sc;
+  sc.gka0 = c->scan[log2n];
+  sc.kappa = c->scan[log2n] + n2;
+  sc.qinv = c->scan[log2n] + (2 + 2 * used_seeds) * n2;
+  return sc;
+}
+uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds) { return c->scan_na[log2n][used_seeds]; }
+
 int check_group(uint32_t log2n, uint32_t l) {
   if (log2n < 3 || log2n > LOG2_N_MAX) return fail(DNSPIR_ERR_BAD_SHAPE, "log2_n must be in [3, 11]");
   const uint32_t n = 1u << log2n;
@@ -361,7 +419,7 @@ struct dnspir_db {
   cudaStream_t st = nullptr;
   cudaEvent_t noalloc_done = nullptr;  // recorded on the caller's stream after each no-allocation call
   uint32_t* slab = nullptr;
-  DBuf a_zq, a_ms, qz, qlane, part, out, slab_ptr;
+  DBuf a_zq, a_ms, qz, qlane, qv, sum, out;
   EncodeWs ws;
   std::mutex mu;
   ~dnspir_db() {
@@ -397,6 +455,7 @@ int db_noalloc_begin(dnspir_db* db, DbView* out) {
   out->slab = db->slab;
   out->T = db->ctx->T;
   out->maps = slot_maps(db->ctx, db->g.log2n);
+  out->sc = scan_consts(db->ctx, db->g.log2n, db->used_seeds);
   return DNSPIR_OK;
 }
 int db_noalloc_end(dnspir_db* db, cudaStream_t st) {
@@ -501,7 +560,7 @@ int dnspir_db_create(int device, uint32_t log2_n, uint32_t group_order, int used
   std::unique_ptr<dnspir_db> d(new dnspir_db());
   d->device = device;
   d->ctx = c;
-  d->g = make_group(log2_n, group_order);
+  d->g = make_group(log2_n, group_order, scan_arrays(c, log2_n, used_seeds));
   d->used_seeds = used_seeds;
   CK(cudaStreamCreateWithFlags(&d->st, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&d->noalloc_done, cudaEventDisableTiming));
@@ -527,12 +586,22 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
     CK(cudaMemcpyAsync(db->ws.in16.p, entries, want * 2, cudaMemcpyHostToDevice, db->st));
     src = db->ws.in16.as<uint16_t>();
   }
-  uint32_t* slabs[1] = {db->slab};
   db->ready = false;
   // a no-allocation call queued on another stream may still read the slab
   CK(cudaStreamWaitEvent(db->st, db->noalloc_done, 0));
   uint64_t ver = 0;
   CKR(ctx_consts(db->ctx, db->g.log2n, &ver));
+  const uint32_t na = scan_arrays(db->ctx, db->g.log2n, db->used_seeds);
+  if (na != db->g.na || !db->slab) {
+    // a-parts installed since the shard was made need the other slab layout
+    CK(cudaStreamSynchronize(db->st));
+    CK(cudaEventSynchronize(db->noalloc_done));
+    if (db->slab) CK(cudaFree(db->slab));
+    db->slab = nullptr;
+    db->g.na = na;
+    CK(cudaMalloc(&db->slab, slab_words(db->g) * 4));
+  }
+  uint32_t* slabs[1] = {db->slab};
   CKR(preprocess_shards(db->ctx, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
                         db->a_ms.as<uint32_t>(), db->ws, db->st));
   db->ap_ver = ver;
@@ -568,17 +637,19 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
   }
   if (!reduced(z.data(), z.size())) return fail(DNSPIR_ERR_BAD_ARG, "ring element coefficients must be below q");
   DeviceGuard dg(db->device);
-  const int R = scan_chunks(g, 1);
   CKR(db->qz.ensure(z.size() * 8));
   CKR(db->qlane.ensure(z.size() * 2 * 4));
-  CKR(db->part.ensure((size_t)g.H * R * 2 * n * SIMD * 4));
+  CKR(db->qv.ensure((size_t)SIMD * 4 * SCAN_VECS * n * 4));
+  CKR(db->sum.ensure(scan_lanes_sum_words(g) * 4));
   CKR(db->out.ensure((size_t)SIMD * n * 8));
   CK(cudaMemcpyAsync(db->qz.p, z.data(), z.size() * 8, cudaMemcpyHostToDevice, db->st));
   launch_ring_to_ntt(db->qz.as<uint64_t>(), SIMD * 4, db->qlane.as<uint32_t>(), nullptr, g.log2n, db->ctx->T, db->st);
-  launch_scan_lanes(db->slab, db->qlane.as<uint32_t>(), db->part.as<uint32_t>(), g, R, slot_maps(db->ctx, g.log2n),
-                    db->st);
-  launch_epilogue_zq(db->part.as<uint32_t>(), g.H * R, db->out.as<uint64_t>(), g, slot_maps(db->ctx, g.log2n),
-                     db->ctx->T, db->st);
+  const SlotMaps maps = slot_maps(db->ctx, g.log2n);
+  launch_scan_vectors(db->qlane.as<uint32_t>(), 8 * n, 0, 2, SIMD, SIMD, db->qv.as<uint32_t>(), g,
+                      scan_consts(db->ctx, g.log2n, db->used_seeds), maps, db->st);
+  if (launch_scan_lanes(db->slab, db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g, db->st))
+    return fail(DNSPIR_ERR_CUDA, "cannot clear the scan's sums");
+  launch_epilogue_zq(db->sum.as<uint32_t>(), db->out.as<uint64_t>(), g, maps, db->ctx->T, db->st);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(out_b, db->out.p, (size_t)SIMD * n * 8, cudaMemcpyDeviceToHost, db->st));
   CK(cudaStreamSynchronize(db->st));

@@ -340,12 +340,14 @@ __device__ __forceinline__ void primary_body(const ChainArgs& a, int h, int lane
       }
     }
     __syncthreads();
-    // key digits of row i in the scan layout: position u (natural slot k with
-    // 2k+1 = g[u]) holds G_i[idx(5^(L-1-i) g[u])]
+    // row i in the scan layout: position u (natural slot k with 2k+1 = g[u])
+    // holds the values at slot idx(5^(L-1-i) g[u]) -- the new state over the
+    // entries and the high digit, or both digits beside the entries (slab_off)
+    const bool two = a.g.na == 2;
     for (int u = threadIdx.x; u < N; u += CT) {
       const uint32_t jb = brv(gidx(ci * __ldg(a.maps.g + u), mask), logn);
-      slab[slab_off(a.g, p, h, i, 1, u) + lane] = TC[jb];
-      slab[slab_off(a.g, p, h, i, 2, u) + lane] = D[jb];
+      slab[slab_off(a.g, p, h, i, two ? 0 : 1, u) + lane] = two ? A[jb] : TC[jb];
+      slab[slab_off(a.g, p, h, i, two ? 1 : 2, u) + lane] = D[jb];
     }
     // TC and D are rewritten only after the next step's first barrier
     ci = (ci * a.inv5) & mask;

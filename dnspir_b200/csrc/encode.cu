@@ -24,8 +24,9 @@
 
 namespace dnspir {
 
-Group make_group(int log2n, uint32_t l) {
+Group make_group(int log2n, uint32_t l, uint32_t na) {
   Group g;
+  g.na = na;
   g.log2n = log2n;
   g.n = 1u << log2n;
   g.l = l;

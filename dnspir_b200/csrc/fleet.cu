@@ -104,24 +104,24 @@ int fleet_drain(dnspir_fleet* f) {
 // Scan of the decoded queries in s.qnat (kernel batch Bk) into s.fin.
 int launch_scan(dnspir_fleet* f, QSlot& s, int nb, int Bk) {
   const Group& g1 = f->g1;
-  const size_t qv = QV_WORDS_PER_QUERY * g1.n;
+  launch_scan_vectors(s.qnat.as<uint32_t>(), QV_WORDS_PER_QUERY * g1.n, 2, 0, nb, Bk, s.qv.as<uint32_t>(), g1,
+                      scan_consts(f->ctx, g1.log2n, 0), slot_maps(f->ctx, g1.log2n), f->st);
+  f->launches += 1;
   if (f->engine == DNSPIR_ENGINE_TENSOR) {
     int nb_pad = 0;
     const TScanShape& shape = tensor_shape(f, nb, &nb_pad);
     if (nb_pad != Bk) return fail(DNSPIR_ERR_BAD_ARG, "tensor scan batch mismatch");
-    if (launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, s.qnat.as<uint32_t>(), qv, nb, Bk, f->qb.as<uint8_t>(),
-                     s.fin.as<uint32_t>(), f->err_word.as<uint32_t>(), g1, slot_maps(f->ctx, g1.log2n), shape, f->st,
-                     f->limits, f->tmaps.p))
+    if (launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, s.qv.as<uint32_t>(), nb, Bk, f->qb.as<uint8_t>(),
+                     s.fin.as<uint32_t>(), f->err_word.as<uint32_t>(), f->last.as<uint32_t>(),
+                     f->distinct_dev.as<int>(), g1, shape, f->st, f->limits, f->tmaps.p))
       return fail(DNSPIR_ERR_BAD_ARG, "tensor scan shape does not fit");
     f->launches += 2;  // query operand + scan
     return DNSPIR_OK;
   }
-  if (Bk > nb)  // unused query positions of the kernel batch compute on zeros
-    CK(cudaMemsetAsync(s.qnat.as<uint32_t>() + (size_t)nb * qv, 0, (size_t)(Bk - nb) * qv * 4, f->st));
   auto it = f->tuned_cc.find(nb);
   const int per_block = it == f->tuned_cc.end() ? 0 : std::min(it->second, Bk);
-  if (launch_scan_batch(f->slabs_dev.as<uint32_t*>(), f->S, s.qnat.as<uint32_t>(), qv, Bk, per_block,
-                        s.fin.as<uint32_t>(), g1, slot_maps(f->ctx, g1.log2n), f->st))
+  if (launch_scan_batch(f->slabs_dev.as<uint32_t*>(), f->S, s.qv.as<uint32_t>(), Bk, per_block, s.fin.as<uint32_t>(),
+                        g1, f->st))
     return fail(DNSPIR_ERR_BAD_ARG, "unsupported scan batch");
   f->launches += 1;
   return DNSPIR_OK;
@@ -171,6 +171,7 @@ int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbyte
   const size_t n = f->g1.n;
   CKR(s.qnat.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
   CKR(s.qbrv.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
+  CKR(s.qv.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
   CKR(s.fin.ensure((size_t)Bk * f->S * 2 * n * SIMD * 4));
   CKR(s.sec_in.ensure((size_t)f->g2.l * CTXT_PARTS * nb * n * 2));
   CKR(s.qdesc.ensure((size_t)nb * sizeof(QDesc)));
@@ -254,6 +255,24 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
 
 namespace {
 
+// The distinct shards' slabs, their pointers and tensor maps.
+int allocate_slabs(dnspir_fleet* f) {
+  const size_t words = slab_words(f->g1);
+  for (uint32_t d = 0; d < f->D; d++) CK(cudaMalloc(&f->slabs[d], words * 4));
+  std::vector<uint32_t*> ptrs(f->S);
+  for (uint32_t s = 0; s < f->S; s++) ptrs[s] = f->slabs[s % f->D];
+  CKR(f->slabs_dev.ensure(f->S * sizeof(uint32_t*)));
+  CK(cudaMemcpy(f->slabs_dev.p, ptrs.data(), f->S * sizeof(uint32_t*), cudaMemcpyHostToDevice));
+  if (tensor_layout_supported(f->g1)) {
+    // the slabs stay where they are: their tensor maps are made once
+    CKR(f->tmaps.ensure(tscan_slab_map_bytes((int)f->S)));
+    std::vector<uint8_t*> hp(f->S);
+    for (uint32_t s = 0; s < f->S; s++) hp[s] = reinterpret_cast<uint8_t*>(ptrs[s]);
+    if (tscan_slab_maps(hp.data(), (int)f->S, f->g1, f->tmaps.p) != 0) f->tmaps.release();
+  }
+  return DNSPIR_OK;
+}
+
 // One group through both phases with timing events: primary on f->st,
 // secondary on f->sec after the primary.  Query bytes and descriptors (or
 // decoded vectors) must already be queued on f->st.
@@ -296,7 +315,7 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   f->ap_ver = ap_ver;
   f->device = device;
   f->ctx = c;
-  f->g1 = make_group(log2_n, primary_order);
+  f->g1 = make_group(log2_n, primary_order, scan_arrays(c, log2_n, 0));
   f->g2 = make_group(log2_n, secondary_order);
   f->S = num_shards;
   f->D = num_distinct;
@@ -332,25 +351,11 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   }
   f->slabs.assign(num_distinct, nullptr);
   f->ready.assign(num_distinct, false);
-  const size_t words = slab_words(f->g1);
-  for (uint32_t d = 0; d < num_distinct; d++) CK(cudaMalloc(&f->slabs[d], words * 4));
-  std::vector<uint32_t*> ptrs(num_shards);
   std::vector<int> dist(num_shards);
-  for (uint32_t s = 0; s < num_shards; s++) {
-    ptrs[s] = f->slabs[s % num_distinct];
-    dist[s] = (int)(s % num_distinct);
-  }
-  CKR(f->slabs_dev.ensure(num_shards * sizeof(uint32_t*)));
+  for (uint32_t s = 0; s < num_shards; s++) dist[s] = (int)(s % num_distinct);
   CKR(f->distinct_dev.ensure(num_shards * sizeof(int)));
-  CK(cudaMemcpy(f->slabs_dev.p, ptrs.data(), num_shards * sizeof(uint32_t*), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(f->distinct_dev.p, dist.data(), num_shards * sizeof(int), cudaMemcpyHostToDevice));
-  if (tensor_layout_supported(f->g1)) {
-    // the slabs stay where they are: their tensor maps are made once
-    CKR(f->tmaps.ensure(tscan_slab_map_bytes((int)num_shards)));
-    std::vector<uint8_t*> hp(num_shards);
-    for (uint32_t s = 0; s < num_shards; s++) hp[s] = reinterpret_cast<uint8_t*>(ptrs[s]);
-    if (tscan_slab_maps(hp.data(), (int)num_shards, f->g1, f->tmaps.p) != 0) f->tmaps.release();
-  }
+  CKR(allocate_slabs(f.get()));
   CKR(f->a_zq.ensure((size_t)num_distinct * SIMD * f->g1.n * 8));
   CKR(f->a_ms.ensure((size_t)num_distinct * SIMD * f->g1.n * 4));
   *out = f.release();
@@ -419,11 +424,11 @@ int dnspir_fleet_tune(dnspir_fleet* f, uint32_t batch, double* ms_per_shape, int
     max_pad = std::max(max_pad, (nb + q - 1) / q * q);
   }
   // zero queries: the scan's time does not depend on the values
-  DBuf qnat, out, qb;
-  CKR(qnat.ensure((size_t)max_pad * QV_WORDS_PER_QUERY * n * 4));
+  DBuf qv, out, qb;
+  CKR(qv.ensure((size_t)max_pad * QV_WORDS_PER_QUERY * n * 4));
   CKR(out.ensure((size_t)nb * f->S * 2 * n * SIMD * 4));
   CKR(qb.ensure(tscan_query_bytes(g1, max_pad)));
-  CK(cudaMemsetAsync(qnat.p, 0, (size_t)max_pad * QV_WORDS_PER_QUERY * n * 4, f->st));
+  CK(cudaMemsetAsync(qv.p, 0, (size_t)max_pad * QV_WORDS_PER_QUERY * n * 4, f->st));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -439,9 +444,9 @@ int dnspir_fleet_tune(dnspir_fleet* f, uint32_t batch, double* ms_per_shape, int
       float t = 0, tot = 0;
       for (int r = 0; r < 3 && ok; r++) {
         cudaEventRecord(e0, f->st);
-        ok = launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, qnat.as<uint32_t>(), QV_WORDS_PER_QUERY * n, nb, pad,
-                          qb.as<uint8_t>(), out.as<uint32_t>(), f->err_word.as<uint32_t>(), g1,
-                          slot_maps(f->ctx, g1.log2n), sh[i], f->st, TScanLimits(), f->tmaps.p) == 0;
+        ok = launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, qv.as<uint32_t>(), nb, pad, qb.as<uint8_t>(),
+                          out.as<uint32_t>(), f->err_word.as<uint32_t>(), f->last.as<uint32_t>(),
+                          f->distinct_dev.as<int>(), g1, sh[i], f->st, TScanLimits(), f->tmaps.p) == 0;
         cudaEventRecord(e1, f->st);
         if (ok && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) {
           if (r > 0) tot += t;  // the first run warms up
@@ -600,12 +605,12 @@ int dnspir_fleet_tune_cuda_cores(dnspir_fleet* f, uint32_t batch, double* ms_per
   CKR(fleet_ready(f));
   DeviceGuard dg(f->device);
   const Group& g1 = f->g1;
-  const size_t n = g1.n, qv = QV_WORDS_PER_QUERY * n;
+  const size_t n = g1.n;
   const int B = (int)batch;
-  DBuf qnat, out;
-  CKR(qnat.ensure((size_t)B * qv * 4));
+  DBuf qv, out;
+  CKR(qv.ensure((size_t)B * QV_WORDS_PER_QUERY * n * 4));
   CKR(out.ensure((size_t)B * f->S * 2 * n * SIMD * 4));
-  CK(cudaMemsetAsync(qnat.p, 0, (size_t)B * qv * 4, f->st));
+  CK(cudaMemsetAsync(qv.p, 0, (size_t)B * QV_WORDS_PER_QUERY * n * 4, f->st));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -619,8 +624,8 @@ int dnspir_fleet_tune_cuda_cores(dnspir_fleet* f, uint32_t batch, double* ms_per
       bool ok = true;
       for (int r = 0; r < 3 && ok; r++) {
         cudaEventRecord(e0, f->st);
-        ok = launch_scan_batch(f->slabs_dev.as<uint32_t*>(), f->S, qnat.as<uint32_t>(), qv, B, tiles[i],
-                               out.as<uint32_t>(), g1, slot_maps(f->ctx, g1.log2n), f->st) == 0;
+        ok = launch_scan_batch(f->slabs_dev.as<uint32_t*>(), f->S, qv.as<uint32_t>(), B, tiles[i], out.as<uint32_t>(),
+                               g1, f->st) == 0;
         cudaEventRecord(e1, f->st);
         if (ok && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) {
           if (r > 0) tot += t;
@@ -748,7 +753,19 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
     if (ver != f->ap_ver)
       for (uint32_t d = 0; d < f->D; d++) f->ready[d] = false;
     f->ap_ver = ver;
+    const uint32_t na = scan_arrays(f->ctx, f->g1.log2n, 0);
+    if (na != f->g1.na || !f->slabs[f->D - 1]) {
+      // these a-parts need the other slab layout (slab_off): new slabs
+      CK(cudaStreamSynchronize(f->st));
+      for (uint32_t*& p : f->slabs) {
+        if (p) CK(cudaFree(p));
+        p = nullptr;
+      }
+      f->g1.na = na;
+      CKR(allocate_slabs(f));
+    }
   }
+  if (f->engine == DNSPIR_ENGINE_TENSOR && f->g1.na == 2) CKR(f->last.ensure(f->D * last_rows_words(f->g1) * 4));
   const size_t per = (size_t)SIMD * f->g1.l * f->g1.n;
   const uint32_t batch = 16;
   for (uint32_t b0 = 0; b0 < count; b0 += batch) {
@@ -772,8 +789,11 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
         CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cc, src + (size_t)c0 * per,
                               f->a_zq.as<uint64_t>() + (size_t)(first + b0 + c0) * SIMD * f->g1.n,
                               f->a_ms.as<uint32_t>() + (size_t)(first + b0 + c0) * SIMD * f->g1.n, f->ws, f->st));
-        for (uint32_t i = 0; i < cc; i++)
-          launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[first + b0 + c0 + i]), f->g1, f->st);
+        for (uint32_t i = 0; i < cc; i++) {
+          const size_t d = first + b0 + c0 + i;
+          launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d]), f->g1, f->st);
+          if (f->g1.na == 2) launch_last_rows(tmp[i], f->last.as<uint32_t>() + d * last_rows_words(f->g1), f->g1, f->st);
+        }
       }
       CK(cudaStreamSynchronize(f->st));
       f->tmp_lane.release();

@@ -11,7 +11,7 @@ namespace dnspir {
 
 // Buffers of one group of queries in flight.
 struct QSlot {
-  DBuf qbytes, qdesc, qnat, qbrv, fin, sec_in, reply_dev;
+  DBuf qbytes, qdesc, qnat, qbrv, qv, fin, sec_in, reply_dev;
   HBuf qpin, dpin, rpin;  // host staging: query bytes, descriptors, reply bytes
   cudaEvent_t prim_done = nullptr, sec_done = nullptr;
   cudaEvent_t sec_tail = nullptr;  // the secondary phase has reached its last chunk
@@ -32,7 +32,8 @@ struct QSlot {
   }
 };
 
-const size_t QV_WORDS_PER_QUERY = 6 * 2;  // decoded slots x factors, times N
+const size_t QV_WORDS_PER_QUERY = 6 * 2;  // decoded slots x factors, times N; as many for the scan's query vectors
+static_assert(QV_WORDS_PER_QUERY == 2 * SCAN_VECS * 2, "halves x vectors x factors");
 
 }  // namespace dnspir
 
@@ -46,6 +47,7 @@ struct dnspir_fleet {
   std::vector<bool> ready;
   uint64_t ap_ver = 0;  // a-parts version every ready shard was preprocessed under
   dnspir::DBuf slabs_dev, distinct_dev, a_zq, a_ms;
+  dnspir::DBuf last;  // tensor engine: each distinct shard's chain state after its last row (launch_last_rows)
   dnspir::DBuf tmaps;  // tensor maps of the slabs (CTA-pair tensor-map scan); empty when unavailable
   dnspir::EncodeWs ws;
   dnspir::QSlot slot[2];

@@ -37,6 +37,8 @@ struct DeviceCtx {
   uint32_t* consts[LOG2_N_MAX + 1] = {};  // a-parts in NTT form: [6][2][N], bit-reversed positions
   uint64_t consts_ver[LOG2_N_MAX + 1] = {};  // a-parts version they were built from
   std::vector<uint32_t*> retired;            // a-part buffers replaced by dnspir_set_a_parts
+  uint32_t* scan[LOG2_N_MAX + 1] = {};       // scan constants: gka0, kappa, then qinv of each a-part set (ScanConsts)
+  uint32_t scan_na[LOG2_N_MAX + 1][2] = {};  // arrays per slab row of each a-part set: 2, or 3 when qry_a has a zero slot
   uint32_t* galb[LOG2_N_MAX + 1] = {};
   uint32_t* gtab[LOG2_N_MAX + 1] = {};  // scan slot order: position -> odd residue
   uint32_t* uof[LOG2_N_MAX + 1] = {};   // natural slot -> position
@@ -120,6 +122,9 @@ void a_parts_host(int log2n, uint64_t* out, uint64_t* version);
 uint64_t a_parts_version(int log2n);
 SlotMaps slot_maps(DeviceCtx* c, int log2n);
 ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds);
+ScanConsts scan_consts(DeviceCtx* c, int log2n, int used_seeds);
+// Arrays per slab row of shards preprocessed under the context's a-parts (slab_off).
+uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds);
 int check_group(uint32_t log2n, uint32_t l);
 bool reduced(const uint64_t* v, size_t n);
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,

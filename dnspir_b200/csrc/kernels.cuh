@@ -22,8 +22,9 @@ struct Group {
   uint32_t L;   // loop_len: l if l < N else N/2
   uint32_t H;   // halves: 2 if l == N (requires_conj) else 1
   uint32_t qbp; // query_base_power = N / 2 / L
+  uint32_t na;  // stored arrays per slab row: 2 or 3 (slab_off)
 };
-Group make_group(int log2n, uint32_t l);
+Group make_group(int log2n, uint32_t l, uint32_t na = 3);
 
 // Output slots of the scan are ordered by (sign, e): position u = sign * N/2 + e
 // holds the slot k with 2k + 1 = (sign ? -1 : 1) 5^e mod 2N.  g[u] is that odd
@@ -33,12 +34,45 @@ struct SlotMaps {
   const uint32_t* uof;
 };
 
-// Scan-layout offset (in u32 words) of array a (0 = entries E, 1/2 = key digits
-// G0/G1) of row i, half h, factor p, output position u, lane 0 inside one shard slab.
+// Scan-layout offset (in u32 words) of array a of row i, half h, factor p,
+// output position u, lane 0 inside one shard slab.  What the arrays hold:
+//   na = 2: 0 the chain state a_(i+1) after row i, 1 the high key digit G1
+//   na = 3: 0 the entries E, 1 / 2 the key digits G0 / G1
+// The reference scans three arrays (base_pir.rs:1085-1247).  They are tied by
+// the chain that made them: with t_i = sigma_5(a_i) and G0 = t - 2^26 G1,
+//     a_(i+1) = t_i gk_a0 + G1_i (gk_a1 - 2^26 gk_a0) + E_i qry_a   (mod p),
+// so where qry_a is invertible at every slot, E_i follows from a_(i+1), a_i
+// and G1_i, and t_i[j] = a_i[5 j] is array 0 of the row before at the slot the
+// same output reads there.  A scan of two arrays against query vectors that
+// carry the relation (launch_scan_vectors) is the same residue, with two
+// thirds of the bytes and products.  na = 3 is kept for a-parts with a zero
+// among qry_a's slots (about one set in 5500 at N = 2048).
 __host__ __device__ __forceinline__ size_t slab_off(const Group& g, int p, int h, uint32_t i, int a, uint32_t k) {
-  return (((((size_t)p * g.H + h) * g.L + i) * 3 + a) * g.n + k) * SIMD;
+  return (((((size_t)p * g.H + h) * g.L + i) * g.na + a) * g.n + k) * SIMD;
 }
-__host__ __device__ __forceinline__ size_t slab_words(const Group& g) { return (size_t)2 * g.H * g.L * 3 * g.n * SIMD; }
+__host__ __device__ __forceinline__ size_t slab_words(const Group& g) {
+  return (size_t)2 * g.H * g.L * g.na * g.n * SIMD;
+}
+
+// Constants of the two-array scan for one a-part set, (sign, e) slot order:
+// gk_a0, gk_a1 - 2^26 gk_a0 and the inverses of qry_a of each half.
+struct ScanConsts {
+  const uint32_t* gka0;   // [p][N]
+  const uint32_t* kappa;  // [p][N]
+  const uint32_t* qinv;   // [half][p][N]
+};
+// Query vectors of the scan, [q][half][v][factor][N] in (sign, e) order (12 N
+// words a query): na = 2: v = 0, 1 multiply the stored arrays, v = 2 the state
+// after the last row once more; na = 3: v = the query, gk0, gk1.  src: decoded
+// vectors [slot][factor][N] in natural order, q_stride words apart, at slots
+// s_q (conjugate half: s_q + 1), s_gk, s_gk + 1.  Queries nb .. nb_pad - 1 are
+// written as zeros.
+constexpr int SCAN_VECS = 3;
+__host__ __device__ __forceinline__ size_t scan_vec_off(uint32_t n, int h, int v, int p) {
+  return ((size_t)(h * SCAN_VECS + v) * 2 + p) * n;
+}
+void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk, int nb, int nb_pad, uint32_t* qv,
+                         const Group& g, const ScanConsts& sc, const SlotMaps& maps, cudaStream_t st);
 
 // ---- DB encoding (set_transformed_entries, base_pir.rs:662-772)
 // in: coefficients [t < l_in][lane < nl][n < N] (< t); A: [t][lane][x] (q1, transform
@@ -81,12 +115,11 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
 // ---- primary scan (main_pir_loop, base_pir.rs:1085-1247)
 // B queries (a power of two up to 256) in one launch over all shards, each
 // block serving per_block of them (1, 2, 4, 8 or 16; 0: min(B, 16)), the other
-// groups of per_block on grid.y.  qnat: per query [slot][p][N] natural order
-// (slots 0 gk0, 1 gk1, 2 pq, 3 pqc), q_stride words apart.  out:
+// groups of per_block on grid.y.  qv: launch_scan_vectors of B queries.  out:
 // [b][s][p][u][lane] reduced mod p.
 int scan_batch_supported(int B);
-int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qnat, size_t q_stride, int B,
-                      int per_block, uint32_t* out, const Group& g, const SlotMaps& maps, cudaStream_t st);
+int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qv, int B, int per_block, uint32_t* out,
+                      const Group& g, cudaStream_t st);
 // ---- primary scan on the tensor cores (tscan.cu): 8-bit limbs, kind::i8
 // Tensor layout: the slab indexed by query slot, bytes in 128 x 128 blocks
 // [p][sign][m-tile][k-chunk] (same size as the lane layout).  Needs loop_len
@@ -109,29 +142,34 @@ struct TScanLimits {
   uint64_t wait_ns = 0;
   int withhold = -1;
 };
-// nb queries (decoded, qnat) padded to nb_pad (a multiple of shape.nq / 4);
-// qb: tscan_query_bytes of workspace; out as launch_scan_batch; err: one
-// device word set to 1 when a bounded wait gave up.  Returns -1 for a shape
-// that does not fit.
+// nb queries (qv: launch_scan_vectors) padded to nb_pad (a multiple of
+// shape.nq / 4); qb: tscan_query_bytes of workspace; out as
+// launch_scan_batch; err: one device word set to 1 when a bounded wait gave
+// up.  last: the distinct shards' states after the last row
+// (launch_last_rows), distinct_of the distinct shard of each shard (na = 2).
+// Returns -1 for a shape that does not fit.
 // slab_maps: tscan_slab_maps of the shards (device), required by the
 // tensor-map pair shapes (persistent 3), which are refused (-1) without it.
-int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qnat, size_t q_stride, int nb, int nb_pad,
-                 uint8_t* qb, uint32_t* out, uint32_t* err, const Group& g, const SlotMaps& maps,
+int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int nb, int nb_pad, uint8_t* qb,
+                 uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
                  const TScanShape& shape, cudaStream_t st, const TScanLimits& lim = TScanLimits(),
                  const void* slab_maps = nullptr);
+// The chain state after the last row of a lane-layout shard, [p][u][half][lane] (na = 2).
+size_t last_rows_words(const Group& g);
+void launch_last_rows(const uint32_t* lane_slab, uint32_t* last, const Group& g, cudaStream_t st);
 // Tensor maps of the shards' tensor-layout slabs (host pointers; one map of
 // tscan_slab_map_bytes(1) bytes per shard) written to dev_maps; -1 when the
 // driver cannot encode them.
 size_t tscan_slab_map_bytes(int nshards);
 int tscan_slab_maps(uint8_t* const* host_slabs, int nshards, const Group& g, void* dev_maps);
-// Per-lane queries (perform_pir_split): qlane [(lane*4 + v)*2 + p][N] natural order;
-// part: [chunk][p][u][lane], chunks = H * R.
-int scan_chunks(const Group& g, int nshards);
-// Loads the kernels of launch_scan_lanes and launch_epilogue_zq on the current
-// device (0, or -1 on a CUDA error).
+// Per-lane queries (perform_pir_split): qv = launch_scan_vectors of 8 queries,
+// one per lane.  sum: scan_lanes_sum_words of workspace.  -1 on a CUDA error.
+constexpr int SCAN_MAX_CHUNKS = 16;  // row chunks per half
+size_t scan_lanes_sum_words(const Group& g);
+int launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st);
+// Loads the kernels of launch_scan_vectors, launch_scan_lanes and
+// launch_epilogue_zq on the current device (0, or -1 on a CUDA error).
 int preload_pir_split_kernels();
-void launch_scan_lanes(const uint32_t* slab, const uint32_t* qlane, uint32_t* part, const Group& g, int R,
-                       const SlotMaps& maps, cudaStream_t st);
 // Primary epilogue for nq queries: scan output -> b (iNTT, CRT), mod-switch,
 // combine with the shard's a-part, three base-1025 digits -> secondary
 // entries.  Queries are grouped in chunks of `chunk`; chunk c starts at
@@ -140,8 +178,8 @@ void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uin
                              uint16_t* sec_in, int chunk, const Group& g, const SlotMaps& maps, const NttTables& T,
                              cudaStream_t st);
 // Epilogue returning b as Z_q coefficients [lane][n] (shard-level perform_pir_split).
-void launch_epilogue_zq(const uint32_t* part, int chunks, uint64_t* out, const Group& g, const SlotMaps& maps,
-                        const NttTables& T, cudaStream_t st);
+void launch_epilogue_zq(const uint32_t* sum, uint64_t* out, const Group& g, const SlotMaps& maps, const NttTables& T,
+                        cudaStream_t st);
 
 // ---- wire codec (pir_wrapper.rs:84-158, 370-408)
 // Decodes one query's polynomials: poly_off/poly_bits per polynomial (npoly),
@@ -181,6 +219,7 @@ struct DbView {
   const uint32_t* slab;
   NttTables T;
   SlotMaps maps;
+  ScanConsts sc;
 };
 
 // Payload helpers for synthetic databases (dns/bucket.rs:289-303 packing).

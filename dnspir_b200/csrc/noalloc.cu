@@ -24,7 +24,6 @@
 // for that event before they touch the slab.
 // Nothing in the region has to start at zero: each call writes every byte of
 // it that it later reads.
-#include <cstdio>
 #include <mutex>
 #include <string>
 
@@ -37,10 +36,13 @@ namespace dnspir {
 constexpr size_t NOALLOC_ZQ_BYTES = (size_t)SIMD * 4 * N_MAX * 8;
 // their NTTs in both factors:                                        512 KiB
 constexpr size_t NOALLOC_NTT_BYTES = (size_t)SIMD * 4 * 2 * N_MAX * 4;
-// scan partial sums: 2 halves x at most 16 row chunks x 2 factors x N x 8 lanes: 4 MiB
-constexpr int NOALLOC_MAX_CHUNKS = 16;
-constexpr size_t NOALLOC_PART_BYTES = (size_t)2 * NOALLOC_MAX_CHUNKS * 2 * N_MAX * SIMD * 4;
-constexpr size_t NOALLOC_SCRATCH_BYTES = NOALLOC_ZQ_BYTES + NOALLOC_NTT_BYTES + NOALLOC_PART_BYTES;
+// query vectors of the scan, 8 lanes x 2 halves x 3 x 2 factors x N:  768 KiB
+constexpr size_t NOALLOC_QV_BYTES = (size_t)SIMD * 4 * SCAN_VECS * N_MAX * 4;
+// the scan's sums, 2 factors x N x 8 lanes                          128 KiB
+constexpr size_t NOALLOC_SUM_BYTES = (size_t)2 * N_MAX * SIMD * 4;
+constexpr size_t NOALLOC_SCRATCH_BYTES = (size_t)5 << 20;  // the region's documented size
+static_assert(NOALLOC_ZQ_BYTES + NOALLOC_NTT_BYTES + NOALLOC_QV_BYTES + NOALLOC_SUM_BYTES <= NOALLOC_SCRATCH_BYTES,
+              "the scratch region holds every intermediate");
 
 // What the entry point needs from a shard (defined in api.cu): begin locks
 // the shard and fills the view (unlocked again on failure); end records the
@@ -123,18 +125,6 @@ static int noalloc_queue(const DbView& v, const uint64_t* qry_b, const uint64_t*
     return DNSPIR_ERR_BAD_SHAPE;
   }
   const size_t n = g.n;
-  int chunks = scan_chunks(g, 1);
-  if (chunks > NOALLOC_MAX_CHUNKS) chunks = NOALLOC_MAX_CHUNKS;
-  const size_t zq_bytes = (size_t)SIMD * 4 * n * 8;
-  const size_t ntt_bytes = (size_t)SIMD * 4 * 2 * n * 4;
-  const size_t part_bytes = (size_t)g.H * chunks * 2 * n * SIMD * 4;
-  if (zq_bytes > NOALLOC_ZQ_BYTES || ntt_bytes > NOALLOC_NTT_BYTES || part_bytes > NOALLOC_PART_BYTES) {
-    char msg[200];
-    snprintf(msg, sizeof(msg), "shard needs %zu bytes of scratch; the static no-allocation region holds %zu",
-             zq_bytes + ntt_bytes + part_bytes, NOALLOC_SCRATCH_BYTES);
-    set_last_error(msg);
-    return DNSPIR_ERR_BAD_SIZE;
-  }
   int prev = -1;
   cudaError_t e = cudaGetDevice(&prev);
   if (e == cudaSuccess && prev != v.device) e = cudaSetDevice(v.device);
@@ -149,7 +139,8 @@ static int noalloc_queue(const DbView& v, const uint64_t* qry_b, const uint64_t*
   if (rc == DNSPIR_OK) {
     uint64_t* zq = (uint64_t*)scratch;
     uint32_t* ntt = (uint32_t*)(scratch + NOALLOC_ZQ_BYTES);
-    uint32_t* part = (uint32_t*)(scratch + NOALLOC_ZQ_BYTES + NOALLOC_NTT_BYTES);
+    uint32_t* qv = (uint32_t*)(scratch + NOALLOC_ZQ_BYTES + NOALLOC_NTT_BYTES);
+    uint32_t* sum = (uint32_t*)(scratch + NOALLOC_ZQ_BYTES + NOALLOC_NTT_BYTES + NOALLOC_QV_BYTES);
     // gather: lane k's polynomials land at slots 4k + {0: qry, 1: qry_conj, 2: gk0, 3: gk1}
     const size_t row = n * 8, pitch = 4 * row;
     e = cudaMemcpy2DAsync(zq, pitch, qry_b, row, row, SIMD, cudaMemcpyDeviceToDevice, st);
@@ -160,8 +151,8 @@ static int noalloc_queue(const DbView& v, const uint64_t* qry_b, const uint64_t*
       e = cudaMemcpy2DAsync((char*)zq + 2 * row, pitch, gk_b, 2 * row, 2 * row, SIMD, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) {
       launch_ring_to_ntt(zq, SIMD * 4, ntt, nullptr, g.log2n, v.T, st);
-      launch_scan_lanes(v.slab, ntt, part, g, chunks, v.maps, st);
-      launch_epilogue_zq(part, g.H * chunks, out_b, g, v.maps, v.T, st);
+      launch_scan_vectors(ntt, 8 * n, 0, 2, SIMD, SIMD, qv, g, v.sc, v.maps, st);
+      if (launch_scan_lanes(v.slab, qv, sum, g, st) == 0) launch_epilogue_zq(sum, out_b, g, v.maps, v.T, st);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

@@ -12,11 +12,17 @@
 // staged in shared memory for all B queries.  Every row is stored permuted so
 // that the data for output u sits at position u (slab_off), so a block streams
 // its rows contiguously.  Products of canonical residues are below 2^52, so one
-// 64-bit accumulator per (lane, query) absorbs a half (3 * L <= 3072 products)
-// without reduction; it is reduced once between halves and once at the end.
+// 64-bit accumulator per (lane, query) absorbs a half (at most 3 L <= 3072
+// products) without reduction; it is reduced once between halves and once at
+// the end.  Two arrays a row instead of the reference's three (slab_off): at
+// 2^22 entries a pass reads 137 GB instead of 206 (a query of a stream of
+// one-query passes on the tensor engine 29.0 -> 20.1 ms; 16 queries at 2^20 on
+// this engine 43.1 -> 25.8 ms).
 // One block per (shard, factor, sign, tile) item, consecutive blocks sharing a
 // shard; blocks retire after their item so that the higher-priority secondary
 // stream can take SMs while a scan is running.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "ntt2048.cuh"
 
@@ -25,15 +31,65 @@ namespace {
 
 constexpr int SCAN_NT = 256;
 
+// Query vectors (launch_scan_vectors).  With C = gk0 - gk_a0 r and r = q / qry_a
+// per half, the recurrence's contribution of row i at slot j,
+//     t_i gk0 + G1_i (gk1 - 2^26 gk0) + E_i q,
+// becomes, with E_i = (a_(i+1) - t_i gk_a0 - G1_i kappa) / qry_a,
+//     t_i C + G1_i (gk1 - 2^26 gk0 - kappa r) + a_(i+1) r,
+// and t_i[j] C[j] = a_i[5 j] C[j] joins row i - 1, whose slot for the same
+// output is 5 j: array 0 of every row but the last meets r[j] + C[5^-1 j].
+// The last row's state has no following t, so its C term is taken back (v = 2).
+// In (sign, e) order 5^-1 is e - 1.  One thread per slot, factor and query.
+__global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_stride, int s_q, int s_gk, int nb,
+                                    uint32_t* __restrict__ qv, Group g, ScanConsts sc,
+                                    const uint32_t* __restrict__ gtab) {
+  const uint32_t N = g.n, half = N / 2;
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= N) return;
+  const int p = blockIdx.y, q = blockIdx.z;
+  uint32_t* o = qv + (size_t)q * 2 * SCAN_VECS * 2 * N;
+  if (q >= nb) {
+    for (int h = 0; h < (int)g.H; h++)
+      for (int v = 0; v < SCAN_VECS; v++) o[scan_vec_off(N, h, v, p) + u] = 0;
+    return;
+  }
+  src += (size_t)q * q_stride;
+  auto at = [&](int slot, uint32_t x) {
+    return __ldg(src + ((size_t)slot * 2 + p) * N + ((__ldg(gtab + x) - 1) >> 1));
+  };
+  const uint32_t pr = prime_of(p);
+  const uint64_t mu = barrett_mu(pr);
+  const uint32_t gk0 = at(s_gk, u), gk1 = at(s_gk + 1, u);
+  if (g.na == 3) {
+    for (int h = 0; h < (int)g.H; h++) {
+      o[scan_vec_off(N, h, 0, p) + u] = at(s_q + h, u);
+      o[scan_vec_off(N, h, 1, p) + u] = gk0;
+      o[scan_vec_off(N, h, 2, p) + u] = gk1;
+    }
+    return;
+  }
+  const uint32_t um = (u & (half - 1)) ? u - 1 : u + half - 1;  // 5^-1 of this slot
+  const uint32_t gk0m = at(s_gk, um);
+  const uint32_t ga = __ldg(sc.gka0 + (size_t)p * N + um), ka = __ldg(sc.kappa + (size_t)p * N + u);
+  const uint32_t g1 = sub_mod(gk1, mul_mod(gk0, 1u << LOG2_B, pr, mu), pr);
+  for (int h = 0; h < (int)g.H; h++) {
+    const uint32_t* inv = sc.qinv + (size_t)(h * 2 + p) * N;
+    const uint32_t r = mul_mod(at(s_q + h, u), __ldg(inv + u), pr, mu);
+    const uint32_t rm = mul_mod(at(s_q + h, um), __ldg(inv + um), pr, mu);
+    const uint32_t cm = sub_mod(gk0m, mul_mod(ga, rm, pr, mu), pr);
+    o[scan_vec_off(N, h, 0, p) + u] = add_mod(r, cm, pr);
+    o[scan_vec_off(N, h, 1, p) + u] = sub_mod(g1, mul_mod(ka, r, pr, mu), pr);
+    o[scan_vec_off(N, h, 2, p) + u] = cm ? pr - cm : 0;
+  }
+}
+
 struct ScanArgs {
   Group g;
   uint32_t* const* slabs;
   int nshards;
-  const uint32_t* qnat;  // per query [slot][p][N] natural order
-  size_t q_stride;       // words between queries
-  const uint32_t* gtab;  // (sign, e) position -> odd residue
-  uint32_t* out;         // [b][s][p][u][lane], reduced mod p
-  int rows;              // rows per window chunk
+  const uint32_t* qv;  // query vectors, 12 N words a query
+  uint32_t* out;       // [b][s][p][u][lane], reduced mod p
+  int rows;            // rows per window chunk
 };
 
 __device__ __forceinline__ void ld_lanes(const uint32_t* p, uint32_t* v, int lpt) {
@@ -54,18 +110,18 @@ __device__ __forceinline__ void ld_lanes(const uint32_t* p, uint32_t* v, int lpt
 // kernel is latency-bound at one block of 8 warps); the other shapes would
 // spill under that bound and keep the compiler's own register choice (a
 // minimum of 0 blocks leaves it as with no minimum)
-template <int B, int LPT>
+template <int B, int LPT, int NA>
 __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(ScanArgs a) {
   constexpr int LG = SIMD / LPT;     // lane groups per slot
   constexpr int TS = SCAN_NT / LG;   // slots per tile
-  extern __shared__ uint32_t win[];  // [3][B][W]: x fastest, so a warp's slots hit distinct banks
+  extern __shared__ uint32_t win[];  // [NA][B][W]: x fastest, so a warp's slots hit distinct banks
   const Group& g = a.g;
   const uint32_t N = g.n, half = N / 2, L = g.L;
   const uint32_t R = (uint32_t)a.rows;
   const uint32_t W = TS + R - 1;
   const uint32_t tiles = (half + TS - 1) / TS;
   const int slot = threadIdx.x / LG, lg = threadIdx.x % LG;
-  const size_t arr = (size_t)N * SIMD, row_stride = 3 * arr;
+  const size_t arr = (size_t)N * SIMD, row_stride = NA * arr;
   // item = ((s * 2 + p) * 2 + sgn) * tiles + tile
   const uint32_t item = blockIdx.x;
   // grid.y: which group of B queries of the kernel batch this block serves
@@ -81,46 +137,56 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
   const uint32_t pr = prime_of(p);
   const uint64_t mu = barrett_mu(pr);
   const uint32_t* slab = a.slabs[s];
+  const size_t qs = (size_t)2 * SCAN_VECS * 2 * N;
   uint64_t acc[LPT][B];
 #pragma unroll
   for (int l = 0; l < LPT; l++)
 #pragma unroll
     for (int b = 0; b < B; b++) acc[l][b] = 0;
   for (uint32_t h = 0; h < g.H; h++) {
-    // decoded slots: 0 gk0, 1 gk1, 2 pq, 3 pqc -> window vectors (query of this half, gk0, gk1)
-    const int vslot[3] = {2 + (int)h, 0, 1};
     for (uint32_t i0 = 0; i0 < L; i0 += R) {
       const uint32_t i1 = min(L, i0 + R);
       const uint32_t Wr = TS + (i1 - i0) - 1;
       const uint32_t w0 = (e0 + L - i1) % half;
-      for (uint32_t idx = threadIdx.x; idx < 3 * Wr * B; idx += SCAN_NT) {
+      for (uint32_t idx = threadIdx.x; idx < NA * Wr * B; idx += SCAN_NT) {
         const uint32_t x = idx % Wr, b = (idx / Wr) % B, v = idx / (B * Wr);
-        const uint32_t uu = sgn * half + (w0 + x) % half;
-        const uint32_t kk = (__ldg(a.gtab + uu) - 1) >> 1;
-        win[(v * B + b) * W + x] = __ldg(a.qnat + (qbase + b) * a.q_stride + ((size_t)vslot[v] * 2 + p) * N + kk);
+        win[(v * B + b) * W + x] =
+            __ldg(a.qv + (qbase + b) * qs + scan_vec_off(N, h, v, p) + sgn * half + (w0 + x) % half);
       }
       __syncthreads();
       if (active) {
         const uint32_t* row = slab + slab_off(g, p, h, i0, 0, u) + lg * LPT;
         uint32_t x = slot + (i1 - 1 - i0);
-#pragma unroll 2
+#pragma unroll(NA == 2 ? 3 : 2)
         for (uint32_t i = i0; i < i1; i++) {
-          uint32_t ev[LPT], av[LPT], bv[LPT];
-          ld_lanes(row, ev, LPT);
-          ld_lanes(row + arr, av, LPT);
-          ld_lanes(row + 2 * arr, bv, LPT);
+          uint32_t ev[NA][LPT];
+#pragma unroll
+          for (int v = 0; v < NA; v++) ld_lanes(row + v * arr, ev[v], LPT);
 #pragma unroll
           for (int b = 0; b < B; b++) {
-            const uint32_t q = win[b * W + x], g0 = win[(B + b) * W + x], g1 = win[(2 * B + b) * W + x];
+            uint32_t q[NA];
+#pragma unroll
+            for (int v = 0; v < NA; v++) q[v] = win[(v * B + b) * W + x];
 #pragma unroll
             for (int l = 0; l < LPT; l++)
-              acc[l][b] += (uint64_t)ev[l] * q + (uint64_t)av[l] * g0 + (uint64_t)bv[l] * g1;
+#pragma unroll
+              for (int v = 0; v < NA; v++) acc[l][b] += (uint64_t)ev[v][l] * q[v];
           }
           row += row_stride;
           x--;
         }
       }
       __syncthreads();
+    }
+    if (NA == 2 && active) {  // the last row's state once more
+      uint32_t xv[LPT];
+      ld_lanes(slab + slab_off(g, p, h, L - 1, 0, u) + lg * LPT, xv, LPT);
+#pragma unroll
+      for (int b = 0; b < B; b++) {
+        const uint32_t c = __ldg(a.qv + (qbase + b) * qs + scan_vec_off(N, h, 2, p) + u);
+#pragma unroll
+        for (int l = 0; l < LPT; l++) acc[l][b] += (uint64_t)xv[l] * c;
+      }
     }
     if (h + 1 < g.H) {
 #pragma unroll
@@ -139,40 +205,80 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
   }
 }
 
-// Per-lane queries (perform_pir_split): qlane[(lane*4 + v)*2 + p][N] natural
-// order, v = qry, qry_conj, gk0, gk1.  Partials [chunk][p][u][lane].
-__global__ void scan_lanes_kernel(const uint32_t* __restrict__ slab, const uint32_t* __restrict__ qlane,
-                                  uint32_t* __restrict__ part, Group g, int R, const uint32_t* __restrict__ pow5,
-                                  const uint32_t* __restrict__ gtab, uint32_t inv5) {
-  const uint32_t N = g.n, mask = 2 * N - 1;
-  const int HR = g.H * R;
-  const int p = blockIdx.z / HR;
-  const int ch = blockIdx.z % HR;
-  const int h = ch / R, rc = ch % R;
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= N) return;
-  const uint32_t rows = (g.L + R - 1) / R;
-  const uint32_t i0 = rc * rows;
-  const uint32_t i1 = min(g.L, i0 + rows);
-  const uint32_t gu = gtab[u];
-  uint64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (i0 < i1) {
-    uint32_t c = pow5[g.L - 1 - i0];
-    for (uint32_t i = i0; i < i1; i++) {
-      const uint32_t j = ((c * gu) & mask) >> 1;
-      const uint32_t* row = slab + slab_off(g, p, h, i, 0, u);
-      for (int l = 0; l < SIMD; l++) {
-        const uint32_t qv = qlane[(((size_t)l * 4 + h) * 2 + p) * N + j];
-        const uint32_t gv0 = qlane[(((size_t)l * 4 + 2) * 2 + p) * N + j];
-        const uint32_t gv1 = qlane[(((size_t)l * 4 + 3) * 2 + p) * N + j];
-        acc[l] += (uint64_t)row[l] * qv + (uint64_t)row[N * SIMD + l] * gv0 + (uint64_t)row[2 * N * SIMD + l] * gv1;
-      }
-      c = (c * inv5) & mask;
-    }
+// Per-lane queries (perform_pir_split): qv holds lane l's vectors as query l.
+// One block: blockDim.x consecutive slots of one sign, factor and half over
+// one chunk of rows; the lanes' query entries its rows need are one window in
+// shared memory, [vector][lane quad][x][4 lanes], so a thread reads its 8 lanes'
+// entries as 16-byte vectors without bank conflicts.  Bound by the slab's bytes;
+// with the sums kept per slot instead of per chunk the epilogue reads one word
+// where it added up 256 (3.0 ms of a 3.5 ms call at N = 2048; the whole
+// set_db + get_a + split call 14.9 -> 11.6 ms);
+// the chunks' residues (at most 2 SCAN_MAX_CHUNKS = 32 of them, below 2^31 in
+// all) add up in `sum` [p][u][lane], zeroed before the launch.
+constexpr int LANES_NT = 256;
+__global__ void __launch_bounds__(LANES_NT) scan_lanes_kernel(const uint32_t* __restrict__ slab,
+                                                              const uint32_t* __restrict__ qv,
+                                                              uint32_t* __restrict__ sum, Group g, int R) {
+  extern __shared__ __align__(16) uint32_t win[];
+  const uint32_t N = g.n, half = N / 2, L = g.L;
+  const int na = (int)g.na;
+  const int TS = blockDim.x;
+  const uint32_t tiles = half / TS;
+  const uint32_t e0 = (blockIdx.x % tiles) * TS, sgn = blockIdx.x / tiles;
+  const int h = blockIdx.y / R, rc = blockIdx.y % R, p = blockIdx.z;
+  const uint32_t rows = (L + R - 1) / R;
+  const uint32_t i0 = rc * rows, i1 = min(L, i0 + rows);
+  if (i0 >= i1) return;
+  const uint32_t W = TS + rows - 1, Wr = TS + (i1 - i0) - 1;
+  const uint32_t w0 = (e0 + L - i1) % half;
+  const size_t qs = (size_t)2 * SCAN_VECS * 2 * N;
+  for (uint32_t idx = threadIdx.x; idx < (uint32_t)na * SIMD * Wr; idx += TS) {
+    const uint32_t x = idx % Wr, vl = idx / Wr, l = vl % SIMD, v = vl / SIMD;
+    win[((v * 2 + l / 4) * W + x) * 4 + l % 4] =
+        __ldg(qv + l * qs + scan_vec_off(N, h, v, p) + sgn * half + (w0 + x) % half);
   }
+  __syncthreads();
+  const uint32_t u = sgn * half + e0 + threadIdx.x;
   const uint32_t pr = prime_of(p);
+  uint64_t acc[SIMD] = {};
+  const size_t arr = (size_t)N * SIMD;
+  const uint32_t* row = slab + slab_off(g, p, h, i0, 0, u);
+  uint32_t x = threadIdx.x + (i1 - 1 - i0);
+  if (na == 2) {
+#pragma unroll 4
+    for (uint32_t i = i0; i < i1; i++, x--, row += 2 * arr) {
+      uint32_t xv[SIMD], gv[SIMD];
+      ld_lanes(row, xv, SIMD);
+      ld_lanes(row + arr, gv, SIMD);
+#pragma unroll
+      for (int d = 0; d < 2; d++) {
+        const uint4 a = *reinterpret_cast<const uint4*>(win + (d * W + x) * 4);
+        const uint4 b = *reinterpret_cast<const uint4*>(win + ((2 + d) * W + x) * 4);
+        acc[4 * d] += (uint64_t)xv[4 * d] * a.x + (uint64_t)gv[4 * d] * b.x;
+        acc[4 * d + 1] += (uint64_t)xv[4 * d + 1] * a.y + (uint64_t)gv[4 * d + 1] * b.y;
+        acc[4 * d + 2] += (uint64_t)xv[4 * d + 2] * a.z + (uint64_t)gv[4 * d + 2] * b.z;
+        acc[4 * d + 3] += (uint64_t)xv[4 * d + 3] * a.w + (uint64_t)gv[4 * d + 3] * b.w;
+      }
+    }
+    if (i1 == L) {  // the last row's state once more
+      uint32_t xv[SIMD];
+      ld_lanes(slab + slab_off(g, p, h, L - 1, 0, u), xv, SIMD);
+#pragma unroll
+      for (int l = 0; l < SIMD; l++)
+        acc[l] += (uint64_t)xv[l] * __ldg(qv + l * qs + scan_vec_off(N, h, 2, p) + u);
+    }
+  } else {
+    for (uint32_t i = i0; i < i1; i++, x--, row += 3 * arr)
+      for (int v = 0; v < 3; v++) {
+        uint32_t xv[SIMD];
+        ld_lanes(row + v * arr, xv, SIMD);
+#pragma unroll
+        for (int l = 0; l < SIMD; l++) acc[l] += (uint64_t)xv[l] * win[((v * 2 + l / 4) * W + x) * 4 + l % 4];
+      }
+  }
+#pragma unroll
   for (int l = 0; l < SIMD; l++)
-    part[(((size_t)ch * 2 + p) * N + u) * SIMD + l] = reduce64(acc[l], pr, barrett_mu(pr));
+    atomicAdd(sum + ((size_t)p * N + u) * SIMD + l, reduce64(acc[l], pr, barrett_mu(pr)));
 }
 
 // grid: x = shard, y = lane pair, z = query.  b = the query's scan output ->
@@ -283,54 +389,64 @@ __global__ void __launch_bounds__(EPI_NT, 3) primary_epilogue2k_kernel(
   }
 }
 
-__global__ void epilogue_zq_kernel(const uint32_t* __restrict__ part, int chunks, uint64_t* __restrict__ out,
-                                   Group g, const uint32_t* __restrict__ uof, NttTables T, CrtConst crtc) {
-  extern __shared__ uint32_t sm[];
-  const int l0 = blockIdx.x * 2;
-  const int logn = g.log2n;
+// One lane per block: sums of scan_lanes_kernel (below 2^31) -> iNTT -> CRT.
+constexpr int ZQ_NT = 512;
+__global__ void __launch_bounds__(ZQ_NT) epilogue_zq_kernel(const uint32_t* __restrict__ sum,
+                                                            uint64_t* __restrict__ out, Group g,
+                                                            const uint32_t* __restrict__ uof, NttTables T,
+                                                            CrtConst crtc) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const int l = blockIdx.x, logn = g.log2n;
   const uint32_t N = g.n;
-  for (uint32_t x = threadIdx.x; x < 4 * N; x += blockDim.x) {
-    const uint32_t poly = x >> logn, k = x & (N - 1);
-    const int p = poly >> 1, ll = poly & 1;
-    const uint32_t u = __ldg(uof + k);
-    uint64_t sum = 0;
-    for (int c = 0; c < chunks; c++) sum += part[(((size_t)c * 2 + p) * N + u) * SIMD + l0 + ll];
-    const uint32_t pr = prime_of(p);
-    sm[(poly << logn) + brv(k, logn)] = reduce64(sum, pr, barrett_mu(pr));
+  const bool full = logn == LOG2_N_MAX;
+  const uint32_t PW = full ? n2k::PS : N;  // words between the two factors' polynomials
+  for (uint32_t x = threadIdx.x; x < 2 * N; x += ZQ_NT) {
+    const uint32_t p = x >> logn, xx = x & (N - 1);  // position xx holds natural slot brv(xx)
+    const uint32_t v = __ldg(sum + ((size_t)p * N + __ldg(uof + brv(xx, logn))) * SIMD + l);
+    sm[p * PW + (full ? n2k::phys(xx) : xx)] = ntt_detail::canon(v, prime_of(p));
   }
   __syncthreads();
-  ntt_inv_smem2(sm, logn, 2, 2, T);
-  for (uint32_t x = threadIdx.x; x < 2 * N; x += blockDim.x) {
-    const uint32_t ll = x >> logn, n = x & (N - 1);
-    out[(size_t)(l0 + ll) * N + n] = crt(sm[(ll << logn) + n], sm[((2 + ll) << logn) + n], crtc);
+  if (full)
+    n2k::inv<ZQ_NT>(sm, 1, 1, T);
+  else
+    ntt_inv_smem2(sm, logn, 1, 1, T);
+  for (uint32_t n = threadIdx.x; n < N; n += ZQ_NT) {
+    const uint32_t o = full ? n2k::phys(n) : n;
+    out[(size_t)l * N + n] = crt(sm[o], sm[PW + o], crtc);
   }
 }
 
-template <int B, int LPT>
-void launch_batch(const ScanArgs& a, int groups, cudaStream_t st) {
+template <int B, int LPT, int NA>
+void launch_batch_na(const ScanArgs& a, int groups, cudaStream_t st) {
   constexpr int TS = SCAN_NT / (SIMD / LPT);
-  const size_t smem = (size_t)3 * (TS + a.rows - 1) * B * 4;
-  set_smem(scan_batch_kernel<B, LPT>, smem);
+  const size_t smem = (size_t)NA * (TS + a.rows - 1) * B * 4;
+  set_smem(scan_batch_kernel<B, LPT, NA>, smem);
   const uint32_t tiles = (a.g.n / 2 + TS - 1) / TS;
   const uint32_t items = (uint32_t)a.nshards * 4 * tiles;
-  scan_batch_kernel<B, LPT><<<dim3(items, groups), SCAN_NT, smem, st>>>(a);
+  scan_batch_kernel<B, LPT, NA><<<dim3(items, groups), SCAN_NT, smem, st>>>(a);
+}
+template <int B, int LPT>
+void launch_batch(const ScanArgs& a, int groups, cudaStream_t st) {
+  if (a.g.na == 2)
+    launch_batch_na<B, LPT, 2>(a, groups, st);
+  else
+    launch_batch_na<B, LPT, 3>(a, groups, st);
 }
 
 }  // namespace
 
 CrtConst host_crt_const();
-const uint32_t* device_pow5(int log2n, bool inverse);
 
-static uint32_t inv5_of(uint32_t two_n) {
-  for (uint32_t x = 1; x < two_n; x += 2)
-    if ((5 * x) % two_n == 1) return x;
-  return 1;
+void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk, int nb, int nb_pad, uint32_t* qv,
+                         const Group& g, const ScanConsts& sc, const SlotMaps& maps, cudaStream_t st) {
+  const unsigned nt = g.n < 256 ? g.n : 256;
+  scan_vectors_kernel<<<dim3(g.n / nt, 2, nb_pad), nt, 0, st>>>(src, q_stride, s_q, s_gk, nb, qv, g, sc, maps.g);
 }
 
 int scan_batch_supported(int B) { return B >= 1 && B <= 256 && (B & (B - 1)) == 0; }
 
-int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qnat, size_t q_stride, int B,
-                      int per_block, uint32_t* out, const Group& g, const SlotMaps& maps, cudaStream_t st) {
+int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qv, int B, int per_block, uint32_t* out,
+                      const Group& g, cudaStream_t st) {
   if (!scan_batch_supported(B)) return -1;
   if (per_block <= 0) per_block = B < 16 ? B : 16;
   if (per_block > B || B % per_block) return -1;
@@ -339,9 +455,7 @@ int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* q
   a.g = g;
   a.slabs = slabs_dev;
   a.nshards = nshards;
-  a.qnat = qnat;
-  a.q_stride = q_stride;
-  a.gtab = maps.g;
+  a.qv = qv;
   a.out = out;
   a.rows = (int)(g.L < 256 ? g.L : 256);
   switch (per_block) {
@@ -355,23 +469,16 @@ int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* q
   return 0;
 }
 
-int scan_chunks(const Group& g, int nshards) {
-  // enough independent (slot, row chunk) threads to keep every SM streaming
-  const double target = 1.5e6;
-  const double per_chunk = (double)nshards * 2 * g.n * g.H;
-  int R = (int)((target + per_chunk - 1) / per_chunk);
-  if (R < 1) R = 1;
-  const int rmax = (int)(g.L / 8 > 0 ? g.L / 8 : 1);
-  if (R > rmax) R = rmax;
-  return R;
-}
+size_t scan_lanes_sum_words(const Group& g) { return (size_t)2 * g.n * SIMD; }
 
-void launch_scan_lanes(const uint32_t* slab, const uint32_t* qlane, uint32_t* part, const Group& g, int R,
-                       const SlotMaps& maps, cudaStream_t st) {
-  const int nt = 128;
-  dim3 grid((g.n + nt - 1) / nt, 1, 2 * g.H * R);
-  scan_lanes_kernel<<<grid, nt, 0, st>>>(slab, qlane, part, g, R, device_pow5(g.log2n, false), maps.g,
-                                         inv5_of(2 * g.n));
+int launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st) {
+  if (cudaMemsetAsync(sum, 0, scan_lanes_sum_words(g) * 4, st) != cudaSuccess) return -1;
+  const int nt = g.n / 2 < (uint32_t)LANES_NT ? (int)(g.n / 2) : LANES_NT;
+  const int R = (int)std::max<uint32_t>(1, std::min<uint32_t>(SCAN_MAX_CHUNKS, g.L / 8));
+  const uint32_t rows = (g.L + R - 1) / R;
+  const size_t smem = (size_t)g.na * SIMD * (nt + rows - 1) * 4;
+  scan_lanes_kernel<<<dim3(2 * (g.n / 2 / nt), g.H * R, 2), nt, smem, st>>>(slab, qv, sum, g, R);
+  return 0;
 }
 
 void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
@@ -398,7 +505,8 @@ int preload_pir_split_kernels() {
   // the runtime loads kernels lazily, at their first launch; this loads the
   // single-shard scan kernels now (cudaFuncGetAttributes forces the load)
   cudaFuncAttributes a;
-  if (cudaFuncGetAttributes(&a, (const void*)scan_lanes_kernel) != cudaSuccess ||
+  if (cudaFuncGetAttributes(&a, (const void*)scan_vectors_kernel) != cudaSuccess ||
+      cudaFuncGetAttributes(&a, (const void*)scan_lanes_kernel) != cudaSuccess ||
       cudaFuncGetAttributes(&a, (const void*)epilogue_zq_kernel) != cudaSuccess) {
     cudaGetLastError();
     return -1;
@@ -406,11 +514,10 @@ int preload_pir_split_kernels() {
   return 0;
 }
 
-void launch_epilogue_zq(const uint32_t* part, int chunks, uint64_t* out, const Group& g, const SlotMaps& maps,
-                        const NttTables& T, cudaStream_t st) {
-  const size_t smem = (size_t)4 * g.n * 4;
-  set_smem(epilogue_zq_kernel, smem);
-  epilogue_zq_kernel<<<SIMD / 2, 256, smem, st>>>(part, chunks, out, g, maps.uof, T, host_crt_const());
+void launch_epilogue_zq(const uint32_t* sum, uint64_t* out, const Group& g, const SlotMaps& maps, const NttTables& T,
+                        cudaStream_t st) {
+  const size_t smem = (size_t)2 * (g.log2n == LOG2_N_MAX ? n2k::PS : (int)g.n) * 4;
+  epilogue_zq_kernel<<<SIMD, ZQ_NT, smem, st>>>(sum, out, g, maps.uof, T, host_crt_const());
 }
 
 }  // namespace dnspir

@@ -7,11 +7,15 @@
 // slab by d instead of i turns the scan, per (shard, factor p, sign), into a
 // product of integer matrices
 //     out[(e, lane), b] = sum_{K = (h, a, d)} A[(e, lane), K] * V[K, b]
-// with A the slab (E, G0, G1 of each half h) and V the B queries (the query of
-// half h, gk0, gk1 at slot (sign, d)).  Both factors are below 2^32 and split
-// into four 8-bit limbs (the bytes of the word): tcgen05.mma kind::i8 forms the
-// 16 limb products with u8 x u8 -> s32 accumulation, at most
-// K * 255^2 <= 6144 * 65025 < 2^31 per entry, so no partial sum overflows;
+// with A the slab's na arrays of each half h and V the B queries' vectors at
+// slot (sign, d) (slab_off, launch_scan_vectors).  With the reference's three
+// arrays K = 6144 at N = 2048; the two-array form has K = 4096 and adds, in the
+// epilogue, one product per half: the state after the last row (`last`), which
+// sits on the matrix's diagonal, times v = 2 of the query vectors.  Both factors
+// are below 2^32 and split into four 8-bit limbs (the bytes of the word):
+// tcgen05.mma kind::i8 forms the 16 limb products with u8 x u8 -> s32
+// accumulation, at most K * 255^2 <= 6144 * 65025 < 2^31 per entry, so no
+// partial sum overflows;
 // the epilogue recombines sum_{k,j} D_kj * (2^(8(k+j)) mod p) < 2^59 in 64 bits
 // and reduces it mod p.  The result is the same residue as the CUDA-core scan.
 //
@@ -19,7 +23,7 @@
 // block is 128 rows x 128 bytes in the 128-byte-swizzled K-major form the MMA
 // reads (16-byte unit c of row r stored at unit c ^ (r mod 8)).  Row r of
 // m-tile mt is limb r mod 4 of lane (r / 4) mod 8 of slot e = 4 mt + r / 32;
-// byte kb of K-chunk kc is K index kk = 128 kc + kb = (h * 3 + a) * L + d.
+// byte kb of K-chunk kc is K index kk = 128 kc + kb = (h * na + a) * L + d.
 // The query operand has the same form: [p][sign][kc][n = 4 b + j][128 bytes].
 //
 // One CTA of 128 threads per (shard, p, sign, m-tiles, query group): thread 0
@@ -194,6 +198,10 @@ struct TScanArgs {
   uint64_t wait_ns;   // limit of every pipeline wait
   uint32_t withhold;  // test hook: CTA 0's producer stops before this chunk (~0u: never)
   const CUtensorMap* tmaps;  // per shard: the slab as rows of 128 bytes (tensor-map pair kernel)
+  const uint32_t* qv;        // the queries' vectors, 12 N words each
+  const uint32_t* last;      // two-array slabs: [distinct shard][p][u][half][lane]; null otherwise
+  const int* distinct_of;
+  uint32_t H;
 };
 
 // c_w = 2^(8w) mod p (< 2^26) for w = k .. k + 3: the weights of limb product
@@ -223,9 +231,28 @@ __device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr
                                               int c_lo = 0, int c_hi = NQ) {
   constexpr int CW = NQ >= 64 ? 64 : 16;  // columns per TMEM load
   const uint32_t N = 2 * a.half;
+  // the states after the last row at this slot and lane, and the vectors they
+  // meet: lane k keeps query 4 q4 + k's sum, so it adds that query's products
+  uint32_t x0 = 0, x1 = 0;
+  if (a.last) {
+    const uint32_t* x = a.last + ((((size_t)a.distinct_of[s] * 2 + p) * N + u) * a.H) * SIMD + l8;
+    x0 = __ldg(x);
+    if (a.H == 2) x1 = __ldg(x + SIMD);
+  }
+  const size_t qs = (size_t)2 * SCAN_VECS * 2 * N;
+  const uint32_t* vc = a.qv + scan_vec_off(N, 0, 2, p) + u;
+  const size_t vh = scan_vec_off(N, 1, 2, p) - scan_vec_off(N, 0, 2, p);
 #pragma unroll 1
   for (int c0 = c_lo; c0 < c_hi; c0 += CW) {
-    uint32_t v[CW];
+    uint32_t v[CW], v0[CW / 16] = {}, v1[CW / 16] = {};
+    if (a.last) {
+#pragma unroll
+      for (int q4 = 0; q4 < CW / 16; q4++) {
+        const uint32_t bq = min(grp * (NQ / 4) + (c0 / 16 + q4) * 4 + k, a.nvalid - 1);
+        v0[q4] = __ldg(vc + bq * qs);
+        if (a.H == 2) v1[q4] = __ldg(vc + bq * qs + vh);
+      }
+    }
     if constexpr (CW == 64)
       tmem_ld64(taddr + c0, v);
     else
@@ -241,7 +268,8 @@ __device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr
         x += __shfl_xor_sync(0xffffffffu, x, 2);
         tot[qq] = x;
       }
-      const uint64_t mine = k == 0 ? tot[0] : k == 1 ? tot[1] : k == 2 ? tot[2] : tot[3];
+      const uint64_t mine = (k == 0 ? tot[0] : k == 1 ? tot[1] : k == 2 ? tot[2] : tot[3]) +
+                            (uint64_t)x0 * v0[q4] + (uint64_t)x1 * v1[q4];
       const uint32_t bq = grp * (NQ / 4) + (c0 / 16 + q4) * 4 + k;
       if (bq < a.nvalid) a.out[((((size_t)bq * a.nshards + s) * 2 + p) * N + u) * SIMD + l8] = reduce64(mine, pr, mu);
     }
@@ -924,7 +952,7 @@ __global__ void retile_kernel(const uint32_t* __restrict__ src, uint8_t* __restr
   const uint32_t u = sgn * half + e;
   const uint32_t kk0 = kc * 128 + c * 16;  // 16 consecutive K indices of one (h, a)
   const uint32_t ha = kk0 / half, d0 = kk0 % half;
-  const uint32_t h = ha / 3, a = ha % 3;
+  const uint32_t h = ha / g.na, a = ha % g.na;
   uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int x = 0; x < 16; x++) {
@@ -937,11 +965,19 @@ __global__ void retile_kernel(const uint32_t* __restrict__ src, uint8_t* __restr
   *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// The chain state after the last row of a two-array lane slab: row L - 1 of
+// array 0, [p][u][half][lane].  One thread per word.
+__global__ void last_rows_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ last, Group g) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 2 * g.n * g.H * SIMD) return;
+  const uint32_t lane = i % SIMD, h = (i / SIMD) % g.H, u = (i / (SIMD * g.H)) % g.n, p = i / (SIMD * g.H * g.n);
+  last[i] = src[slab_off(g, (int)p, (int)h, g.L - 1, 0, u) + lane];
+}
+
 // Query operand: one thread per (p, sign, query, 16-byte K unit); writes the
 // four limb rows 4b + j.  Queries b >= nb are zero.
-__global__ void tquery_kernel(const uint32_t* __restrict__ qnat, size_t q_stride, uint32_t nb, uint32_t nb_pad,
-                              uint8_t* __restrict__ qb, Group g, const uint32_t* __restrict__ gtab,
-                              uint32_t kc_total) {
+__global__ void tquery_kernel(const uint32_t* __restrict__ qv, uint32_t nb, uint32_t nb_pad, uint8_t* __restrict__ qb,
+                              Group g, uint32_t kc_total) {
   const uint32_t half = g.n / 2, N = g.n;
   const uint32_t units = kc_total * 8;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -953,19 +989,21 @@ __global__ void tquery_kernel(const uint32_t* __restrict__ qnat, size_t q_stride
   const int p = (int)(ps >> 1);
   const uint32_t kk0 = cu * 16;
   const uint32_t ha = kk0 / half, d0 = kk0 % half;
-  const uint32_t h = ha / 3, a = ha % 3;
-  const uint32_t slot = a == 0 ? 2 + h : a - 1;  // decoded slots: 0 gk0, 1 gk1, 2 pq, 3 pqc
+  const uint32_t h = ha / g.na, a = ha % g.na;
   uint32_t w[4][4];
 #pragma unroll
   for (int j = 0; j < 4; j++)
 #pragma unroll
     for (int q = 0; q < 4; q++) w[j][q] = 0;
   if (b < nb) {
-    const uint32_t* src = qnat + (size_t)b * q_stride + ((size_t)slot * 2 + p) * N;
+    const uint4* src = reinterpret_cast<const uint4*>(qv + (size_t)b * 2 * SCAN_VECS * 2 * N +
+                                                      scan_vec_off(N, h, a, p) + sgn * half + d0);
+    uint4 in[4];
+#pragma unroll
+    for (int x = 0; x < 4; x++) in[x] = __ldg(src + x);
 #pragma unroll
     for (int x = 0; x < 16; x++) {
-      const uint32_t k = (__ldg(gtab + sgn * half + d0 + x) - 1) >> 1;
-      const uint32_t v = __ldg(src + k);
+      const uint32_t v = (x & 3) == 0 ? in[x >> 2].x : (x & 3) == 1 ? in[x >> 2].y : (x & 3) == 2 ? in[x >> 2].z : in[x >> 2].w;
 #pragma unroll
       for (int j = 0; j < 4; j++) w[j][x >> 2] |= ((v >> (8 * j)) & 0xFFu) << (8 * (x & 3));
     }
@@ -1105,7 +1143,13 @@ int tensor_layout_supported(const Group& g) { return g.log2n >= 8 && g.L == g.n 
 
 void tensor_dims(const Group& g, uint32_t* mt_total, uint32_t* kc_total) {
   *mt_total = (g.n / 2) * SIMD * 4 / 128;
-  *kc_total = 3 * g.H * (g.n / 2) / 128;
+  *kc_total = g.na * g.H * (g.n / 2) / 128;
+}
+
+size_t last_rows_words(const Group& g) { return (size_t)2 * g.n * g.H * SIMD; }
+
+void launch_last_rows(const uint32_t* lane_slab, uint32_t* last, const Group& g, cudaStream_t st) {
+  last_rows_kernel<<<(unsigned)((last_rows_words(g) + 255) / 256), 256, 0, st>>>(lane_slab, last, g);
 }
 
 void launch_retile(const uint32_t* lane_slab, uint8_t* tensor_slab, const Group& g, cudaStream_t st) {
@@ -1161,8 +1205,8 @@ int tscan_slab_maps(uint8_t* const* host_slabs, int nshards, const Group& g, voi
 
 size_t tscan_slab_map_bytes(int nshards) { return (size_t)nshards * sizeof(CUtensorMap); }
 
-int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qnat, size_t q_stride, int nb, int nb_pad,
-                 uint8_t* qb, uint32_t* out, uint32_t* err, const Group& g, const SlotMaps& maps,
+int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int nb, int nb_pad, uint8_t* qb,
+                 uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
                  const TScanShape& shape, cudaStream_t st, const TScanLimits& lim, const void* slab_maps) {
   uint32_t mt, kc;
   tensor_dims(g, &mt, &kc);
@@ -1170,7 +1214,7 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qnat, s
   if (nb_pad % qpc || nb_pad < qpc || mt % shape.mtpc) return -1;
   {
     const size_t threads = (size_t)4 * nb_pad * kc * 8;
-    tquery_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(qnat, q_stride, nb, nb_pad, qb, g, maps.g, kc);
+    tquery_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(qv, nb, nb_pad, qb, g, kc);
   }
   TScanArgs a;
   a.slabs = slabs_dev;
@@ -1188,6 +1232,10 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qnat, s
   a.wait_ns = lim.wait_ns ? lim.wait_ns : WAIT_NS;
   a.withhold = lim.withhold < 0 ? ~0u : (uint32_t)lim.withhold;
   a.tmaps = static_cast<const CUtensorMap*>(slab_maps);
+  a.qv = qv;
+  a.last = g.na == 2 ? last : nullptr;
+  a.distinct_of = distinct_of;
+  a.H = g.H;
   const int stg = shape.stages;
   if (shape.persistent == 2) {
     switch (shape.nq * 10 + shape.mtpc) {

@@ -48,7 +48,8 @@ int dnspir_get_database_shape(uint64_t num_entries, uint32_t* primary_order, uin
                               uint32_t* num_shards);
 /* choose_index_group_secondary (pir_wrapper.rs:166-175) */
 int dnspir_choose_secondary_order(uint32_t num_shards, uint32_t* secondary_order);
-/* PIRDatabase::required_memory_general (base_pir.rs:369-371), in 32-byte elements */
+/* PIRDatabase::required_memory_general (base_pir.rs:369-371), in 32-byte elements: the
+ * reference's three arrays a row; a fleet stores two (dnspir_fleet_slab_bytes) */
 uint64_t dnspir_required_memory_general(uint32_t log2_n, uint32_t group_order);
 /* byte length of a query (prepare_query_general output, pir_wrapper.rs:304-316) and of a reply (:401-408) */
 uint64_t dnspir_query_bytes(uint32_t primary_order, uint32_t secondary_order);
