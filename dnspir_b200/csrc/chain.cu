@@ -25,6 +25,7 @@
 // (position q <-> slot brv(q)); the constants are stored the same way.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "kernels.cuh"
@@ -361,8 +362,8 @@ __device__ __forceinline__ void primary_body(const ChainArgs& a, int h, int lane
 // Secondary chain: LN of the three parts of one query's secondary ciphertext
 // at half h in one block (factor p = rank in the cluster), parts part0 ..
 // part0 + LN - 1 (the library launches LN = 1: the block then needs 88 KiB and
-// shares an SM with a scan block, so the chains of a few queries overlap the
-// next scan; larger chunks use secondary_dual_kernel below).  The key constants gk_a0,
+// shares an SM with a scan block; the register-transform chains and
+// secondary_dual_kernel below take the other cases).  The key constants gk_a0,
 // gk_a1, qry_a, gk_b0, gk_b1, qry_b (Montgomery form) and the sigma_5
 // destinations of a thread's positions live in its registers.  Each step's
 // pointwise stage writes the next step's sigma_5-permuted a and b straight
@@ -427,7 +428,8 @@ __device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q,
   for (uint32_t i = 0; i < a.g.L; i++) {
     const int cur = (int)(i & 1) * N, nxt = N - cur;
     // entries of row i (the three parts' lanes are adjacent), consumed at the end of the step
-    const uint32_t* Ei = a.E + ((((size_t)p * a.g.H + h) * a.g.L + i) * a.nl + (size_t)q * CTXT_PARTS + part0) * N;
+    const uint32_t* Ei =
+        a.E + ((((size_t)p * a.g.H + h) * a.g.L + a.g.L - 1 - i) * a.nl + (size_t)q * CTXT_PARTS + part0) * N;
     uint32_t e[LN][PER];
 #pragma unroll
     for (int t = 0; t < LN; t++)
@@ -661,7 +663,8 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
     uint32_t e[2][PER];
 #pragma unroll
     for (int p = 0; p < 2; p++) {
-      const uint32_t* Ei = a.E + ((((size_t)p * a.g.H + h) * a.g.L + i) * a.nl + (size_t)q * CTXT_PARTS + part) * N;
+      const uint32_t* Ei =
+          a.E + ((((size_t)p * a.g.H + h) * a.g.L + a.g.L - 1 - i) * a.nl + (size_t)q * CTXT_PARTS + part) * N;
 #pragma unroll
       for (int c = 0; c < PER; c++) {
         const int pos = threadIdx.x + c * CT;
@@ -715,172 +718,279 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
   }
 }
 
-// ---- N = 2048: one block per part and half carrying both factors, on the
-// register transforms of ntt2048.cuh.  The block's two 256-thread halves
-// work one RNS factor each: half f holds factor f's polynomials in every pass,
-// and thread t of a half owns positions 8t .. 8t + 7 of its factor in the
-// first inverse pass, the last forward pass and the pointwise stage, so those
-// run from registers.  The halves meet once a step: between the last inverse
-// pass and the first forward pass each takes the other's values at its
-// positions for the CRT high digit (the one block-wide barrier); every other
-// barrier is a named barrier of one half.  The inverse work space D is double
-// buffered by step parity, so a half may run a step ahead of the other's reads
-// of its last inverse pass.  The state a, b stays in natural position order:
-// instead of scattering the next step's sigma_5(a), sigma_5(b) (which needs a
-// second buffer of each), every step gathers them at its own positions through
-// the inverse of galb.  Shared memory, padded polynomials of n2k::PS words:
-// A[2] (a; also the forward transform's work space), B[2] (b), D[2][2]; then
-// the six key constants (Montgomery form) of every position, [j][factor]
-// [quad half][thread] as 16-byte vectors, each thread reading only its own.
-constexpr int SEC2K_KC_WORDS = 6 * 2 * 2 * 256 * 4;
-constexpr int SEC2K_WORDS = 8 * n2k::PS + SEC2K_KC_WORDS;
+// ---- N = 2048, register transforms (ntt2048.cuh): one block carries PARTS of
+// the three parts of one query's secondary ciphertext at half h.  A group of
+// 256 threads works one part in BOTH factors: thread t owns positions 8t .. 8t
+// + 7 of each factor in the first inverse pass, the last forward pass and the
+// pointwise stage, and words t + 256 k between the last inverse and the first
+// forward pass, where the CRT high digit needs both factors -- so those run
+// from registers, the digit needs no exchange, and the groups meet no barrier
+// but their own.  The key constants are the same for the three parts and are
+// kept once per block.
+//
+// With r = qry_b / qry_a per slot (both of the secondary query's half) the b
+// part is carried as b^ = b - r a, which drops the entries from its recurrence:
+//     a' = t ka0 + n1 ka1 + E qa
+//     b^' = sigma_5(b^) + t (C + sigma_5(r)) + n1 V
+// (t = sigma_5(a), n1 = NTT(d1), ka1 = gk_a1 - 2^26 gk_a0, C = gk_b0 - gk_a0 r,
+// V = gk_b1 - 2^26 gk_b0 - ka1 r): five products and five constants a position
+// instead of six; b = b^ + r a once at the end.  Needs every slot of qry_a
+// invertible (launch_secondary_chain).
+//
+// Measured (1024 steps, 64 queries): 10.6 ms for the chunk against 16.6 for one
+// part per block of 512 threads with one factor per half (three waves of
+// blocks, 5.5 us a step); a single query 4.6 ms against 5.8 as two-block
+// clusters.  Three parts keep the heavy FMA pipe 73 % and the L1 / shared-memory
+// pipe 83 % busy; the twiddle loads are a third of the latter.
+//
+// Bounds: a is canonical, b^ below 2p.  The forward transform ends below 2^31
+// (ntt.cuh) and n1 is used as it is: t ka0 + n1 ka1 + E qa < 34 p^2, so its
+// Montgomery reduction is below 34 p^2 / 2^32 + p < 2p, and b^' stays below 2p
+// + 33 p^2 / 2^32 + p < 4p before one subtraction of 2p (p < 2^26).
+//
+// Shared memory: per part A[2], B[2] (padded polynomials; A is also the
+// transforms' work space), then the five constants (Montgomery form) as
+// [j][factor][quad half][thread] 16-byte vectors.
+constexpr int SEC2K_KC = 5;
+constexpr int sec2k_words(int parts) { return parts * 4 * n2k::PS + SEC2K_KC * 2 * 2 * 256 * 4; }
 
-__device__ __forceinline__ void half_sync() {
-  asm volatile("bar.sync %0, 256;" ::"r"(1 + (threadIdx.x >> 8)) : "memory");
+// T R^-1 mod p, below T / 2^32 + p (T < 2^62)
+__device__ __forceinline__ uint32_t mont_lazy(uint64_t T, uint32_t p, uint32_t pinv) {
+  return (uint32_t)((T + (uint64_t)((uint32_t)T * pinv) * p) >> 32);
 }
 
-__global__ void __launch_bounds__(CT, 1) secondary_chain2k_kernel(ChainArgs a) {
+__device__ __forceinline__ double u32_to_double_biased(uint32_t x) {  // 2^52 + x, exactly
+  return __hiloint2double(0x43300000, (int)x);
+}
+
+// high_digit() plus p for each factor's forward transform, from inverse
+// outputs c1 (mod q1) and c2 (mod q2): the conversions to and from double are
+// additions of 2^52 folded into exact fused multiply-adds (x1 P2 and x2 P1 are
+// below 2^51), and floor is the rounding mode of the last addition.
+__device__ __forceinline__ int32_t high_digit_both(uint32_t c1, uint32_t c2, const ChainPrime& A, const ChainPrime& B) {
+  using ntt_detail::red;
+  const uint32_t x1 = red(shoup_lazy(c1, A.k1, A.k1q, P1), P1);
+  const uint32_t x2 = red(shoup_lazy(c2, B.k2, B.k2q, P2), P2);
+  constexpr double Q = (double)QQ, HALF_Q = (double)(QQ / 2), BIAS = 4503599627370496.0;  // 2^52
+  double v = fma(u32_to_double_biased(x1), (double)P2, -BIAS * (double)P2) +
+             fma(u32_to_double_biased(x2), (double)P1, -BIAS * (double)P1);
+  v = v >= Q ? v - Q : v;
+  v = v > HALF_Q ? v - Q : v;
+  // 1.5 2^52 + floor(v / 2^26 + 1/2): its low word is the digit
+  return __double2loint(__dadd_rd(fma(v, 1.0 / (double)(1u << LOG2_B), 0.5), 1.5 * BIAS));
+}
+
+// One radix-8 pass over both factors' polynomials x, x + PS of a 256-thread group.
+template <int M, bool INV>
+__device__ __forceinline__ void pass8_both(uint32_t* x, int t, const NttTables& T) {
+  using Gm = n2k::Geo8<M>;
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const uint32_t p = prime_of(f);
+    const n2k::Tw8 tw = n2k::load_tw8(INV ? T.iw2[f] : T.fw2[f], M, Gm::blk(t));
+    uint32_t* y = x + f * n2k::PS + Gm::base(t);
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = y[k * Gm::STR];
+    if (INV)
+      n2k::inv8_bf(v, tw, p);
+    else
+      n2k::fwd8_bf(v, tw, p);
+#pragma unroll
+    for (int k = 0; k < 8; k++) y[k * Gm::STR] = v[k];
+  }
+}
+
+template <int PARTS>
+__global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(ChainArgs a, ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
   using namespace n2k;
-  static_assert(CT == 512 && N_MAX == N, "two quads per thread of one factor");
-  const int h = blockIdx.x % a.g.H, part = blockIdx.x / a.g.H, q = blockIdx.y;
-  uint32_t* const A = sm;
-  uint32_t* const B = sm + 2 * PS;
-  uint32_t* const D = sm + 4 * PS;  // [parity][factor]
-  const int tid = threadIdx.x;
-  const int f = tid >> 8, t = tid & 255;  // factor of this half, thread within the half
-  const int qb = (int)phys(8 * t);       // positions 8t .. 8t + 7 sit in one padded row: qb .. qb + 7
-  const ChainPrime cp = f ? a.cp[1] : a.cp[0];
-  const uint32_t p = cp.p;
-  // sigma_5 sources of the positions (galb inverted through D), a = b = 0
-  for (int b = tid; b < N; b += CT) D[__ldg(a.galb + b)] = b;
-  for (int b = tid; b < 4 * PS; b += CT) sm[b] = 0;
+  constexpr int NT = 256 * PARTS;
+  const int h = blockIdx.x % a.g.H, q = blockIdx.y;
+  const int pt = threadIdx.x >> 8, t = threadIdx.x & 255;
+  const int part = PARTS == 3 ? pt : (int)(blockIdx.x / a.g.H);
+  uint32_t* const A = sm + pt * 4 * PS;
+  uint32_t* const B = A + 2 * PS;
+  uint4* const KC = reinterpret_cast<uint4*>(sm + PARTS * 4 * PS);
+  const int qb = (int)phys(8 * t);  // positions 8t .. 8t + 7 sit in one padded row: qb .. qb + 7
+  auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + pt) : "memory"); };
+  // sigma_5 sources of the positions (galb inverted through the constants' space)
+  uint32_t* const inv = sm + PARTS * 4 * PS;
+  for (int b = threadIdx.x; b < N; b += NT) inv[__ldg(a.galb + b)] = b;
+  for (int b = threadIdx.x; b < PARTS * 4 * PS; b += NT) sm[b] = 0;  // a = b^ = 0
   __syncthreads();
   uint32_t src[4];  // two 16-bit padded positions per word (PS < 2^16)
 #pragma unroll
-  for (int m = 0; m < 4; m++) src[m] = phys(D[8 * t + 2 * m]) | (phys(D[8 * t + 2 * m + 1]) << 16);
+  for (int m = 0; m < 4; m++) src[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
   const uint32_t* qq = a.qv + (size_t)q * a.qv_stride;
-  uint4* const KC = reinterpret_cast<uint4*>(sm + 8 * PS);  // [j][factor][quad half][t]
+  // r at a position of factor f
+  auto ratio = [&](int f, uint32_t pos) {
+    const uint32_t pr = prime_of(f);
+    return mul_mod(__ldg(qq + ((size_t)(4 + h) * 2 + f) * N + pos),
+                   __ldg(sc.qinv + (size_t)(h * 2 + f) * N + __ldg(a.maps.uof + brv11(pos))), pr, barrett_mu(pr));
+  };
+  // the constants of position quads, dealt over the whole block: item = (factor, quad)
+  {
+    constexpr int ITEMS = 2 * N / 4, PER = (ITEMS + NT - 1) / NT;
+    uint32_t from[PER][4];
 #pragma unroll
-  for (int h4 = 0; h4 < 2; h4++) {
-    uint32_t kc[6][4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-      const size_t o = (size_t)f * N + 8 * t + 4 * h4 + m;
-      kc[0][m] = mont_reduce((uint64_t)a.gka[o] * cp.r2, cp.p, cp.pinv);
-      kc[1][m] = mont_reduce((uint64_t)a.gka[2 * (size_t)N + o] * cp.r2, cp.p, cp.pinv);
-      kc[2][m] = mont_reduce((uint64_t)a.qa[(size_t)h * 2 * N + o] * cp.r2, cp.p, cp.pinv);
-      kc[3][m] = mont_reduce((uint64_t)qq[o] * cp.r2, cp.p, cp.pinv);
-      kc[4][m] = mont_reduce((uint64_t)qq[2 * (size_t)N + o] * cp.r2, cp.p, cp.pinv);
-      kc[5][m] = mont_reduce((uint64_t)qq[(size_t)(4 + h) * 2 * N + o] * cp.r2, cp.p, cp.pinv);
-      // with t = sigma_5(a): NTT(d0) gk0 + NTT(d1) gk1 = t gk0 + NTT(d1) (gk1 - 2^26 gk0),
-      // and likewise for the b-part keys, so the pointwise stage needs no d0
-      kc[1][m] = sub_mod(kc[1][m], mont_reduce((uint64_t)kc[0][m] * cp.c26, cp.p, cp.pinv), cp.p);
-      kc[4][m] = sub_mod(kc[4][m], mont_reduce((uint64_t)kc[3][m] * cp.c26, cp.p, cp.pinv), cp.p);
-    }
-#pragma unroll
-    for (int j = 0; j < 6; j++)
-      KC[((j * 2 + f) * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
-  }
-  __syncthreads();  // the table in D is overwritten by the first step
-  const size_t lane = (size_t)q * CTXT_PARTS + part;
-  const uint4* Erow = reinterpret_cast<const uint4*>(a.E + (((size_t)f * a.g.H + h) * a.g.L * a.nl + lane) * N);
-  const size_t erow_stride = (size_t)a.nl * N / 4;  // uint4 per row i
-  for (uint32_t i = 0; i < a.g.L; i++) {
-    uint32_t* const Dc = D + (i & 1) * 2 * PS;
-    // sigma_5(a) (the inverse transform's input and the kept t) and sigma_5(b)
-    uint32_t ta[8], tb[8];
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      const uint32_t sp = m & 1 ? src[m >> 1] >> 16 : src[m >> 1] & 0xFFFFu;
-      ta[m] = A[f * PS + sp], tb[m] = B[f * PS + sp];
-    }
-    // inverse stages 0-1 from registers, two quads
-#pragma unroll
-    for (int h4 = 0; h4 < 2; h4++) {
-      const Tw4 w = load_tw4(a.T.iw2[f], 2 * t + h4);
-      uint4 v = make_uint4(ta[4 * h4], ta[4 * h4 + 1], ta[4 * h4 + 2], ta[4 * h4 + 3]);
-      gs(v.x, v.y, w.b0, w.b0q, p);
-      gs(v.z, v.w, w.b1, w.b1q, p);
-      gs(v.x, v.z, w.a, w.aq, p);
-      gs(v.y, v.w, w.a, w.aq, p);
-      *reinterpret_cast<uint4*>(Dc + f * PS + qb + 4 * h4) = v;
-    }
-    half_sync();
-    pass8<CT, 64, true, 1>(Dc, 1, 1, a.T, (void*)nullptr);
-    pass8<CT, 8, true, 1>(Dc, 1, 1, a.T, (void*)nullptr);
-    {
-      // last inverse pass (unscaled: N^-1 sits in the CRT constants), the
-      // other factor's values at the same positions, high digit, first
-      // forward pass; group g = t, words g + 256 k
-      const int base = (int)phys(t);
-      constexpr int STR = Geo8<1>::STR;
-      uint32_t v[8];
-      uint32_t* y = Dc + f * PS + base;
-#pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = y[k * STR];
-      inv8_bf(v, load_tw8(a.T.iw2[f], 1, 0), p);
-#pragma unroll
-      for (int k = 0; k < 8; k++) y[k * STR] = v[k];
-      __syncthreads();
-      const uint32_t* z = Dc + (1 - f) * PS + base;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t o = z[k * STR];
-        const int32_t hd = f == 0 ? high_digit(v[k], o, a.cp[0], a.cp[1]) : high_digit(o, v[k], a.cp[0], a.cp[1]);
-        v[k] = hd < 0 ? (uint32_t)(hd + (int32_t)p) : (uint32_t)hd;
-      }
-      fwd8_bf(v, load_tw8(a.T.fw2[f], 1, 0), p);
-      uint32_t* w = A + f * PS + base;
-#pragma unroll
-      for (int k = 0; k < 8; k++) w[k * STR] = v[k];
-      half_sync();
-    }
-    // entries of row i at the positions, consumed by the pointwise stage
-    // (loaded here: the two forward passes cover their latency)
-    const uint4 e0 = __ldg(Erow + i * erow_stride + 2 * t), e1 = __ldg(Erow + i * erow_stride + 2 * t + 1);
-    pass8<CT, 8, false, 1>(A, 1, 1, a.T, (void*)nullptr);
-    pass8<CT, 64, false, 1>(A, 1, 1, a.T, (void*)nullptr);
-    // forward stages 9-10 and the pointwise stage at the two quads
-#pragma unroll
-    for (int h4 = 0; h4 < 2; h4++) {
-      const Tw4 w = load_tw4(a.T.fw2[f], 2 * t + h4);
-      uint4 v = *reinterpret_cast<const uint4*>(A + f * PS + qb + 4 * h4);
-      ct(v.x, v.z, w.a, w.aq, p);
-      ct(v.y, v.w, w.a, w.aq, p);
-      ct(v.x, v.y, w.b0, w.b0q, p);
-      ct(v.z, v.w, w.b1, w.b1q, p);
-      const uint32_t n1s[4] = {canon(v.x, p), canon(v.y, p), canon(v.z, p), canon(v.w, p)};
-      const uint4 e = h4 ? e1 : e0;
-      const uint32_t es[4] = {e.x, e.y, e.z, e.w};
-      uint32_t kc[6][4];
-#pragma unroll
-      for (int j = 0; j < 6; j++) {
-        const uint4 c = KC[((j * 2 + f) * 2 + h4) * 256 + t];
-        kc[j][0] = c.x, kc[j][1] = c.y, kc[j][2] = c.z, kc[j][3] = c.w;
-      }
-      uint32_t an[4], bn[4];
+    for (int c = 0; c < PER; c++)
 #pragma unroll
       for (int m = 0; m < 4; m++) {
-        const int j = 4 * h4 + m;
-        const uint32_t n1 = n1s[m], tt = ta[j];
-        an[m] = mont_reduce((uint64_t)tt * kc[0][m] + (uint64_t)n1 * kc[1][m] + (uint64_t)es[m] * kc[2][m], p,
-                            cp.pinv);
-        bn[m] = mont_reduce(((uint64_t)tb[j] << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1 * kc[4][m] +
-                                (uint64_t)es[m] * kc[5][m],
-                            p, cp.pinv);
+        const int it = threadIdx.x + c * NT;
+        from[c][m] = it < ITEMS ? inv[4 * (it & (N / 4 - 1)) + m] : 0;
       }
-      *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = make_uint4(an[0], an[1], an[2], an[3]);
-      *reinterpret_cast<uint4*>(B + f * PS + qb + 4 * h4) = make_uint4(bn[0], bn[1], bn[2], bn[3]);
+    __syncthreads();  // the table is overwritten by the constants
+#pragma unroll
+    for (int c = 0; c < PER; c++) {
+      const int it = threadIdx.x + c * NT;
+      if (it < ITEMS) {
+        const int f = it / (N / 4), quad = it & (N / 4 - 1);
+        const ChainPrime cp = f ? a.cp[1] : a.cp[0];
+        const uint64_t mu = barrett_mu(cp.p);
+        uint32_t kc[SEC2K_KC][4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const uint32_t pos = 4 * quad + m;
+          const size_t o = (size_t)f * N + pos;
+          const uint32_t ga0 = __ldg(a.gka + o), c26 = (1u << LOG2_B) % cp.p;
+          const uint32_t ka1 = sub_mod(__ldg(a.gka + 2 * (size_t)N + o), mul_mod(ga0, c26, cp.p, mu), cp.p);
+          const uint32_t gb0 = __ldg(qq + o), gb1 = __ldg(qq + 2 * (size_t)N + o);
+          const uint32_t r = ratio(f, pos), r5 = ratio(f, from[c][m]);
+          const uint32_t C = sub_mod(gb0, mul_mod(ga0, r, cp.p, mu), cp.p);
+          const uint32_t V = sub_mod(sub_mod(gb1, mul_mod(gb0, c26, cp.p, mu), cp.p), mul_mod(ka1, r, cp.p, mu), cp.p);
+          const uint32_t k[SEC2K_KC] = {ga0, ka1, __ldg(a.qa + (size_t)h * 2 * N + o), add_mod(C, r5, cp.p), V};
+#pragma unroll
+          for (int j = 0; j < SEC2K_KC; j++) kc[j][m] = mont_reduce((uint64_t)k[j] * cp.r2, cp.p, cp.pinv);
+        }
+#pragma unroll
+        for (int j = 0; j < SEC2K_KC; j++)
+          KC[((j * 2 + f) * 2 + (quad & 1)) * 256 + (quad >> 1)] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
+      }
     }
-    half_sync();
+  }
+  __syncthreads();
+  const size_t lane = (size_t)q * CTXT_PARTS + part;
+  const uint4* Erow = reinterpret_cast<const uint4*>(a.E + ((size_t)h * a.g.L * a.nl + lane) * N) + 2 * t;
+  const size_t erow_stride = (size_t)a.nl * N / 4;             // uint4 per row
+  const size_t efac = (size_t)a.g.H * a.g.L * a.nl * (N / 4);  // uint4 per factor
+  for (uint32_t i = 0; i < a.g.L; i++) {
+    // t = sigma_5(a), kept for the pointwise stage
+    uint32_t ta[2][8];
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int m = 0; m < 8; m++) ta[f][m] = A[f * PS + (m & 1 ? src[m >> 1] >> 16 : src[m >> 1] & 0xFFFFu)];
+    group_sync();
+    // inverse stages 0-1 from registers, two quads a factor
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      const uint32_t p = prime_of(f);
+#pragma unroll
+      for (int h4 = 0; h4 < 2; h4++) {
+        const Tw4 w = load_tw4(a.T.iw2[f], 2 * t + h4);
+        uint4 v = make_uint4(ta[f][4 * h4], ta[f][4 * h4 + 1], ta[f][4 * h4 + 2], ta[f][4 * h4 + 3]);
+        gs(v.x, v.y, w.b0, w.b0q, p);
+        gs(v.z, v.w, w.b1, w.b1q, p);
+        gs(v.x, v.z, w.a, w.aq, p);
+        gs(v.y, v.w, w.a, w.aq, p);
+        *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = v;
+      }
+    }
+    group_sync();
+    pass8_both<64, true>(A, t, a.T);
+    group_sync();
+    pass8_both<8, true>(A, t, a.T);
+    group_sync();
+    {
+      // last inverse pass (unscaled: N^-1 sits in the CRT constants), high
+      // digit, first forward pass; words t + 256 k
+      uint32_t* const y = A + phys(t);
+      constexpr int STR = Geo8<1>::STR;
+      uint32_t v[2][8];
+#pragma unroll
+      for (int f = 0; f < 2; f++) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[f][k] = y[f * PS + k * STR];
+        inv8_bf(v[f], load_tw8(a.T.iw2[f], 1, 0), prime_of(f));
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int32_t hd = high_digit_both(v[0][k], v[1][k], a.cp[0], a.cp[1]);
+        v[0][k] = (uint32_t)(hd + (int32_t)P1), v[1][k] = (uint32_t)(hd + (int32_t)P2);
+      }
+#pragma unroll
+      for (int f = 0; f < 2; f++) {
+        fwd8_bf(v[f], load_tw8(a.T.fw2[f], 1, 0), prime_of(f));
+#pragma unroll
+        for (int k = 0; k < 8; k++) y[f * PS + k * STR] = v[f][k];
+      }
+    }
+    group_sync();
+    pass8_both<8, false>(A, t, a.T);
+    group_sync();
+    // entries of row i, consumed by the pointwise stage
+    uint4 e[2][2];
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int h4 = 0; h4 < 2; h4++) e[f][h4] = __ldg(Erow + f * efac + (a.g.L - 1 - i) * erow_stride + h4);
+    pass8_both<64, false>(A, t, a.T);
+    group_sync();
+    // forward stages 9-10 and the pointwise stage at the two quads
+    uint4 bn[2][2];
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      const uint32_t p = prime_of(f), pinv = f ? a.cp[1].pinv : a.cp[0].pinv;
+#pragma unroll
+      for (int h4 = 0; h4 < 2; h4++) {
+        const Tw4 w = load_tw4(a.T.fw2[f], 2 * t + h4);
+        uint4 v = *reinterpret_cast<const uint4*>(A + f * PS + qb + 4 * h4);
+        ct(v.x, v.z, w.a, w.aq, p);
+        ct(v.y, v.w, w.a, w.aq, p);
+        ct(v.x, v.y, w.b0, w.b0q, p);
+        ct(v.z, v.w, w.b1, w.b1q, p);
+        const uint32_t n1[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t es[4] = {e[f][h4].x, e[f][h4].y, e[f][h4].z, e[f][h4].w};
+        uint32_t kc[SEC2K_KC][4], an[4], b4[4];
+#pragma unroll
+        for (int j = 0; j < SEC2K_KC; j++) {
+          const uint4 c = KC[((j * 2 + f) * 2 + h4) * 256 + t];
+          kc[j][0] = c.x, kc[j][1] = c.y, kc[j][2] = c.z, kc[j][3] = c.w;
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const int j = 4 * h4 + m;
+          const uint32_t tt = ta[f][j];
+          const uint32_t tb = B[f * PS + (j & 1 ? src[j >> 1] >> 16 : src[j >> 1] & 0xFFFFu)];
+          an[m] = red(mont_lazy((uint64_t)tt * kc[0][m] + (uint64_t)n1[m] * kc[1][m] + (uint64_t)es[m] * kc[2][m], p,
+                                pinv),
+                      p);
+          b4[m] = red(mont_lazy(((uint64_t)tb << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m], p, pinv),
+                      2 * p);
+        }
+        *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = make_uint4(an[0], an[1], an[2], an[3]);
+        bn[f][h4] = make_uint4(b4[0], b4[1], b4[2], b4[3]);
+      }
+    }
+    group_sync();  // every gather of b^ is done
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int h4 = 0; h4 < 2; h4++) *reinterpret_cast<uint4*>(B + f * PS + qb + 4 * h4) = bn[f][h4];
   }
   uint32_t* o = a.out + ((((size_t)q * a.g.H + h) * CTXT_PARTS + part) * 2) * 2 * N;
 #pragma unroll
-  for (int h4 = 0; h4 < 2; h4++) {
-    reinterpret_cast<uint4*>(o + (size_t)f * N)[2 * t + h4] = *reinterpret_cast<const uint4*>(A + f * PS + qb + 4 * h4);
-    reinterpret_cast<uint4*>(o + 2 * (size_t)N + (size_t)f * N)[2 * t + h4] =
-        *reinterpret_cast<const uint4*>(B + f * PS + qb + 4 * h4);
+  for (int f = 0; f < 2; f++) {
+    const uint32_t p = prime_of(f);
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const uint32_t av = A[f * PS + qb + m];
+      const uint32_t br = red(B[f * PS + qb + m], p);
+      o[(size_t)f * N + 8 * t + m] = av;
+      o[2 * (size_t)N + (size_t)f * N + 8 * t + m] =
+          add_mod(br, mul_mod(av, ratio(f, 8 * t + m), p, barrett_mu(p)), p);
+    }
   }
 }
 
@@ -1010,27 +1120,34 @@ void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq,
   primary_finalize_kernel<<<grid, 256, smem, st>>>(a_out, a_zq, a_ms, g, T, host_crt_const());
 }
 
+int secondary_chain_wave(const Group& g, int sms) {
+  return std::max(1, g.log2n == LOG2_N_MAX ? sms / (int)g.H : 2 * sms / (2 * CTXT_PARTS * (int)g.H));
+}
+
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st,
-                            bool clustered) {
+                            const Group& g, const ChainConsts& cc, const ScanConsts* sc, const NttTables& T,
+                            cudaStream_t st, bool clustered) {
   ChainArgs a = chain_args(g, cc, T);
   a.E = E;
   a.qv = qv;
   a.qv_stride = qv_stride;
   a.nl = nq * CTXT_PARTS;
   a.out = out;
-  // one part and factor per block in 2-block clusters (88 KiB, 64 registers;
-  // for a few queries: the chains run on many SMs, and a block fits beside a
-  // scan block) while the chunk needs at most one block per SM; beyond that one
-  // block per part carrying both factors (no cluster barrier, twice the work
-  // per barrier): at N = 2048 the register-transform kernel, else the generic one.
-  // `clustered` asks for the cluster form at any chunk size (it shares SMs with
-  // a running scan; the pipeline tuner picks it per group size when faster)
+  // N = 2048: one part per block while every part finds an SM of its own (4.5
+  // us a step), beyond that the three parts of a query and half per block
+  // (10.4 us a step for three parts: 2.3 times the time, three times the work,
+  // the constants kept once).  Other lengths, or a-parts with a zero query
+  // slot: one part and factor per block in 2-block clusters while the chunk
+  // needs at most one block per SM, then one block per part carrying both
+  // factors.  `clustered` asks for the cluster form at any chunk size (88 KiB,
+  // 64 registers: it shares SMs with a running scan; the pipeline tuner picks it
+  // per group size when faster).
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool full = g.log2n == LOG2_N_MAX;
-  if (clustered || (long)nq * CTXT_PARTS * g.H * 2 <= sms) {
+  const bool reg = full && sc;
+  if (clustered || (!reg && (long)nq * CTXT_PARTS * g.H * 2 <= sms)) {
     const size_t smem = chain_smem(g, 1);
     const dim3 grid(2, CTXT_PARTS * g.H, nq);
     if (full) {
@@ -1040,10 +1157,14 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
       set_smem(secondary_chain_kernel<1, 0>, smem);
       secondary_chain_kernel<1, 0><<<grid, CT, smem, st>>>(a);
     }
-  } else if (full) {
-    const size_t smem = (size_t)SEC2K_WORDS * 4;
-    set_smem(secondary_chain2k_kernel, smem);
-    secondary_chain2k_kernel<<<dim3(CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
+  } else if (reg && (long)nq * CTXT_PARTS * g.H <= sms) {
+    const size_t smem = (size_t)sec2k_words(1) * 4;
+    set_smem(secondary_chain2k_kernel<1>, smem);
+    secondary_chain2k_kernel<1><<<dim3(CTXT_PARTS * g.H, nq), 256, smem, st>>>(a, *sc);
+  } else if (reg) {
+    const size_t smem = (size_t)sec2k_words(CTXT_PARTS) * 4;
+    set_smem(secondary_chain2k_kernel<CTXT_PARTS>, smem);
+    secondary_chain2k_kernel<CTXT_PARTS><<<dim3(g.H, nq), 256 * CTXT_PARTS, smem, st>>>(a, *sc);
   } else {
     const size_t smem = (size_t)SEC_DUAL_WORDS * g.n * 4;
     set_smem(secondary_dual_kernel<0>, smem);

@@ -103,8 +103,11 @@ __global__ void encode_rows_kernel(const uint32_t* __restrict__ A, uint32_t* __r
 // One block: column r of half h for up to 8 lanes.
 constexpr int LIFT_LANES_CHAIN = 4;
 
-__global__ void encode_lift_kernel(const uint32_t* __restrict__ Ahat, uint32_t* __restrict__ out, Group g, int nl,
-                                   int frame, uint32_t scale, const uint32_t* __restrict__ pow5inv,
+// In the chain layout factor 0 of the output may lie on Ahat itself (row r of
+// half h is where it was read from, and a block reads all of its rows before it
+// writes any), so neither pointer is __restrict__ and the loads are plain.
+__global__ void encode_lift_kernel(const uint32_t* Ahat, uint32_t* out, Group g, int nl, int frame, uint32_t scale,
+                                   const uint32_t* __restrict__ pow5inv,
                                    const uint32_t* __restrict__ gtab, NttTables T) {
   extern __shared__ uint32_t sm[];
   const uint32_t r = blockIdx.x, h = blockIdx.y;
@@ -145,7 +148,8 @@ __global__ void encode_lift_kernel(const uint32_t* __restrict__ Ahat, uint32_t* 
       out[slab_off(g, p, h, c, 0, u) + kk] = sm[((p * nlg + kk) << logn) + brv(k, logn)];
     }
   } else {
-    // chain layout, bit-reversed positions, E_c[j] = E^_r[idx(5^-r (2j+1))]
+    // chain layout (row r of it is chain step c), bit-reversed positions,
+    // E_c[j] = E^_r[idx(5^-r (2j+1))]
     const uint32_t mask = 2 * N - 1;
     for (uint32_t b = threadIdx.x; b < 2 * (uint32_t)nlg * N; b += blockDim.x) {
       const uint32_t p = b / (nlg * N);
@@ -153,7 +157,7 @@ __global__ void encode_lift_kernel(const uint32_t* __restrict__ Ahat, uint32_t* 
       const uint32_t kk = rem >> logn, pos = rem & (N - 1);
       const uint32_t j = brv(pos, logn);
       const uint32_t src = gidx(pow5inv[r] * (2 * j + 1), mask);
-      out[((((size_t)p * g.H + h) * g.L + c) * nl + lane0 + kk) * N + pos] =
+      out[((((size_t)p * g.H + h) * g.L + r) * nl + lane0 + kk) * N + pos] =
           sm[((p * nlg + kk) << logn) + brv(src, logn)];
     }
   }
@@ -246,9 +250,9 @@ struct LiftFin {
   }
 };
 
-// One block: column r of half h for up to LIFT_LANES_CHAIN lanes, chain layout.
-__global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* __restrict__ Ahat,
-                                                             uint32_t* __restrict__ out, Group g, int nl,
+// One block: column r of half h for up to LIFT_LANES_CHAIN lanes, chain layout
+// (factor 0 of the output may lie on Ahat, as in encode_lift_kernel).
+__global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* Ahat, uint32_t* out, Group g, int nl,
                                                              uint32_t scale, uint32_t scale_q,
                                                              const uint32_t* __restrict__ pow5inv, NttTables T) {
   extern __shared__ __align__(16) uint32_t sm[];
@@ -258,14 +262,13 @@ __global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* __r
   const int nlg = min(LIFT_LANES_CHAIN, nl - lane0);
   for (int b = threadIdx.x; b < nlg * (N / 4); b += NT2K) {
     const int kk = b >> 9, q = b & (N / 4 - 1);
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(Ahat + (((size_t)h * g.L + r) * nl + lane0 + kk) * N) + q);
+    const uint4 v = reinterpret_cast<const uint4*>(Ahat + (((size_t)h * g.L + r) * nl + lane0 + kk) * N)[q];
     *reinterpret_cast<uint4*>(sm + kk * PS + phys(4 * q)) = v;
   }
   __syncthreads();
   inv<NT2K>(sm, nlg, 0, T, LiftFin{nlg, scale, scale_q});
   fwd<NT2K>(sm, nlg, nlg, T);
-  // E_c[j] = E^_r[idx(5^-r (2j+1))] at bit-reversed position brv(j)
-  const uint32_t c = g.L - 1 - r;
+  // E_c[j] = E^_r[idx(5^-r (2j+1))] at bit-reversed position brv(j), c = L - 1 - r
   const uint32_t pw = __ldg(pow5inv + r);
   constexpr uint32_t mask = 2 * N - 1;
   for (int q = threadIdx.x; q < N / 4; q += NT2K) {
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* __r
     for (int pk = 0; pk < 2 * nlg; pk++) {
       const int pp = pk >= nlg, kk = pk - pp * nlg;
       const uint32_t* s = sm + pk * PS;
-      reinterpret_cast<uint4*>(out + ((((size_t)pp * g.H + h) * g.L + c) * nl + lane0 + kk) * N)[q] =
+      reinterpret_cast<uint4*>(out + ((((size_t)pp * g.H + h) * g.L + r) * nl + lane0 + kk) * N)[q] =
           make_uint4(s[idx[0]], s[idx[1]], s[idx[2]], s[idx[3]]);
     }
   }

@@ -5,8 +5,8 @@
 // Queries are answered in groups of up to `batch`: one pass of the scan over
 // every shard serves the whole group (the slab is read once per group), then
 // the secondary databases are encoded and evaluated in chunks of one wave of
-// chain clusters (two one-part blocks per SM: 2 SMs / (6 H) queries, capped by
-// a memory budget).  Two scan
+// chain blocks (secondary_chain_wave: SMs / H queries at N = 2048, capped by a
+// memory budget).  Two scan
 // engines: CUDA cores over the lane layout (groups of a power of two up to 256) and
 // the tensor cores over the tensor layout (groups up to 256, tile shape per
 // group size from a table or from dnspir_fleet_tune).  Two buffer slots
@@ -33,7 +33,7 @@ dnspir_fleet::~dnspir_fleet() {
 
 namespace {
 
-const size_t SEC_BUDGET = (size_t)6 << 30;  // secondary workspace of one chunk
+const size_t SEC_BUDGET = (size_t)8 << 30;  // secondary workspace of one chunk
 const int TENSOR_MAX_BATCH = 256;
 
 #define NOT_SERVING(f) \
@@ -186,11 +186,10 @@ int fleet_secondary_workspace(dnspir_fleet* f, int nb) {
   const size_t n = g2.n;
   const int cmax = std::min(nb, f->sec_chunk);
   const int nlmax = CTXT_PARTS * cmax;
-  // the encoder's column transforms (A) are dead before the lift writes secE:
-  // A lives at the start of secE's buffer
-  const size_t a_bytes = (size_t)g2.l * nlmax * n * 4, e_bytes = (size_t)2 * g2.H * g2.L * nlmax * n * 4;
-  CKR(f->ws.Ahat.ensure((size_t)g2.H * g2.L * nlmax * n * 4));
-  CKR(f->secE.ensure(std::max(a_bytes, e_bytes)));
+  // the entries of both factors; factor 0's rows first hold the orbit values
+  // that the lift works in place, factor 1's the column transforms they are
+  // made from (l = H L of them)
+  CKR(f->secE.ensure((size_t)2 * g2.H * g2.L * nlmax * n * 4));
   CKR(f->chain_out.ensure((size_t)cmax * g2.H * CTXT_PARTS * 2 * 2 * n * 4));
   return DNSPIR_OK;
 }
@@ -226,6 +225,8 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
   f->launches += 1;
   const SlotMaps maps = slot_maps(f->ctx, g2.log2n);
   const ChainConsts cc = chain_consts(f->ctx, g2.log2n, 1);
+  const ScanConsts sc = scan_consts(f->ctx, g2.log2n, 1);
+  const bool two = scan_arrays(f->ctx, g2.log2n, 1) == 2;
   const auto tc = f->tuned_chain.find(nb);
   const bool clustered = tc != f->tuned_chain.end() && tc->second;
   for (int c0 = 0; c0 < nb; c0 += f->sec_chunk) {
@@ -235,11 +236,14 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     // instead of the whole phase (it then shares the SMs the last chunk leaves idle)
     if (c0 + f->sec_chunk >= nb && s.sec_tail) CK(cudaEventRecord(s.sec_tail, st));
     const uint16_t* in = s.sec_in.as<uint16_t>() + (size_t)c0 * CTXT_PARTS * l_in * n;
-    launch_encode_cols(in, f->secE.as<uint32_t>(), g2, l_in, nl, f->ctx->T, st);
-    launch_encode_rows(f->secE.as<uint32_t>(), f->ws.Ahat.as<uint32_t>(), g2, l_in, nl, f->ctx->T, st);
-    launch_encode_lift(f->ws.Ahat.as<uint32_t>(), f->secE.as<uint32_t>(), g2, nl, 1, maps, f->ctx->T, st);
+    uint32_t* const E = f->secE.as<uint32_t>();
+    uint32_t* const A = E + (size_t)g2.H * g2.L * nl * n;
+    launch_encode_cols(in, A, g2, l_in, nl, f->ctx->T, st);
+    launch_encode_rows(A, E, g2, l_in, nl, f->ctx->T, st);
+    launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
-                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), g2, cc, f->ctx->T, st, clustered);
+                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), g2, cc, two ? &sc : nullptr,
+                           f->ctx->T, st, clustered);
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);
@@ -320,13 +324,12 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   f->S = num_shards;
   f->D = num_distinct;
   {
-    // one wave of secondary chain clusters (one-part blocks, two per SM:
-    // 2 x 3 x H blocks per query)
+    // one wave of secondary chain blocks
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const Group& g2 = f->g2;
-    const size_t per_query = ((size_t)2 * g2.H * g2.L + (size_t)g2.H * g2.L) * CTXT_PARTS * g2.n * 4;
-    const int wave = std::max(1, 2 * sms / (2 * CTXT_PARTS * (int)g2.H));
+    const size_t per_query = (size_t)2 * g2.H * g2.L * CTXT_PARTS * g2.n * 4;
+    const int wave = secondary_chain_wave(g2, sms);
     f->sec_chunk = (int)std::max<size_t>(1, std::min<size_t>(wave, SEC_BUDGET / per_query));
   }
   CK(cudaStreamCreateWithFlags(&f->own, cudaStreamNonBlocking));

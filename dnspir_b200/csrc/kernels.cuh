@@ -83,7 +83,8 @@ void launch_encode_cols(const uint16_t* in, uint32_t* A, const Group& g, uint32_
 void launch_encode_rows(const uint32_t* A, uint32_t* Ahat, const Group& g, uint32_t l_in, int nl, const NttTables& T,
                         cudaStream_t st);
 // Ahat -> transformed entries.  frame 0: scan layout in `slab` (nl == 8);
-// frame 1: chain layout out[((p*H + h)*L + c)*nl + lane][pos] in bit-reversed slot order.
+// frame 1: chain layout out[((p*H + h)*L + r)*nl + lane][pos] in bit-reversed slot order,
+// row r for chain step L - 1 - r; out may be Ahat itself (its rows become factor 0).
 void launch_encode_lift(const uint32_t* Ahat, uint32_t* out, const Group& g, int nl, int frame, const SlotMaps& maps,
                         const NttTables& T, cudaStream_t st);
 
@@ -108,9 +109,13 @@ void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq,
 // launch_encode_lift(frame 1) with nl = 3 * nq lanes; qv: per query decoded
 // vectors [q][slot][p][pos] (bit-reversed), slots 0 gk0, 1 gk1, 2 pq, 3 pqc, 4 sq, 5 sqc.
 // out: [q][h][part][a/b][p][pos].
+// sc: scan_consts of the secondary's a-part set, or null when one of its query
+// slots is zero.
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st,
-                            bool clustered = false);
+                            const Group& g, const ChainConsts& cc, const ScanConsts* sc, const NttTables& T,
+                            cudaStream_t st, bool clustered = false);
+// Queries whose chains fill the SMs once.
+int secondary_chain_wave(const Group& g, int sms);
 
 // ---- primary scan (main_pir_loop, base_pir.rs:1085-1247)
 // B queries (a power of two up to 256) in one launch over all shards, each

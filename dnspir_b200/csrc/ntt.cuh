@@ -43,7 +43,9 @@ namespace ntt_detail {
 __device__ __forceinline__ uint32_t lazy_mul(uint32_t x, uint32_t w, uint32_t wq, uint32_t p) {
   return x * w - __umulhi(x, wq) * p;  // in [0, 2p) for any x < 2^32
 }
-__device__ __forceinline__ uint32_t red(uint32_t x, uint32_t m) { return x >= m ? x - m : x; }
+// x - m where x >= m, else x: the wrapped difference is the larger one when
+// x < m, so min(x - m, x) as one add-and-min instruction
+__device__ __forceinline__ uint32_t red(uint32_t x, uint32_t m) { return __viaddmin_u32(x, 0u - m, x); }
 // x mod p for any x < 2^32, p in {q1, q2}: the Shoup product x * 1 (companion
 // floor(2^32 / p)) lands in [0, 2p), one conditional subtraction finishes
 __device__ __forceinline__ uint32_t canon(uint32_t x, uint32_t p) {

@@ -127,3 +127,54 @@ def test_split_matches_oracle_over_shapes(log2n, l, seeds):
     gk = gen.integers(0, orc.Q, size=(8, 2, n), dtype=np.int64)
     assert np.array_equal(db.perform_pir_split(qb, qc, gk).astype(np.int64), ref.perform_pir_split(qb, qc, gk))
     db.close()
+
+
+def _wire_fleet(l2, shards=2):
+    l1 = 1024
+    data = np.random.default_rng(l2).integers(0, orc.T, size=(1, 8 * l1, 2048), dtype=np.uint16)
+    fleet = dp.Fleet.general(11, l1, l2, shards, 1)
+    fleet.set_engine(dp.ENGINE_TENSOR)
+    fleet.set_shards(0, data)
+    return fleet, data
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("l2,groups", [(2048, (24, 25, 75)), (1024, (49, 50)), (16, (50,))])
+def test_chain_forms_give_the_same_replies(l2, groups):
+    # one part per block up to one block per SM, three parts per block beyond
+    # it, a second chunk beyond one wave
+    fleet, _ = _wire_fleet(l2)
+    rng = orc.Rng(bytes([l2 % 251]) * 32)
+    queries = [orc.prepare_query(rng, (97 * k) % 8192, k % 2, 1024, l2)[0] for k in range(max(groups))]
+    single = fleet.process_queries(queries)
+    for nb in groups:
+        fleet.set_batch(nb)
+        assert fleet.process_queries(queries[:nb]) == single[:nb]
+    fleet.close()
+
+
+@pytest.mark.gpu
+def test_secondary_a_parts_with_zero_slots():
+    # the chains whose b part carries the entries serve a-parts without inverses
+    l2 = 16
+    parts = dp.get_a_parts(11).copy()
+    parts[4] = 0  # SecondSet query
+    try:
+        dp.set_a_parts(11, parts)
+        orc.set_aparts(11, parts)
+        fleet, data = _wire_fleet(l2)
+        ref = orc.Database(11, 1024)
+        ref.set_db(data[0])
+        rng = orc.Rng(bytes(range(32)))
+        queries = [orc.prepare_query(rng, 31 * k, k % 2, 1024, l2)[0] for k in range(60)]
+        want = [orc.process_query([ref, ref], q, l2) for q in queries[:3]]
+        for batch in (1, 60):
+            fleet.set_batch(batch)
+            got = fleet.process_queries(queries)
+            assert got[:3] == want
+            assert batch == 1 or got == first
+            first = got
+        fleet.close()
+    finally:
+        dp.set_a_parts(11, None)
+        orc.set_aparts(11, None)
