@@ -192,6 +192,11 @@ static int build_tables(DeviceCtx& c) {
       c.T.ninvq[pi][lg] = (uint32_t)(((u128)ni << 32) / p);
     }
   }
+  for (int pi = 0; pi < 2; pi++)
+    for (int k = 0; k < 8; k++) {
+      c.T.fw7[pi][k] = make_uint2(h[(0 + pi) * n + k], h[(2 + pi) * n + k]);
+      c.T.iw7[pi][k] = make_uint2(h[(4 + pi) * n + k], h[(6 + pi) * n + k]);
+    }
   CK(cudaMalloc(&c.tables, h.size() * 4));
   CK(cudaMemcpy(c.tables, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
   for (int pi = 0; pi < 2; pi++) {
@@ -358,12 +363,13 @@ ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds) {
   return cc;
 }
 
-ScanConsts scan_consts(DeviceCtx* c, int log2n, int used_seeds) {
-  const size_t n2 = (size_t)2 << log2n;
+ScanConsts scan_consts(DeviceCtx* c, const Group& g, int used_seeds) {
+  const size_t n2 = (size_t)2 << g.log2n;
   ScanConsts sc;
-  sc.gka0 = c->scan[log2n];
-  sc.kappa = c->scan[log2n] + n2;
-  sc.qinv = c->scan[log2n] + (2 + 2 * used_seeds) * n2;
+  sc.gka0 = c->scan[g.log2n];
+  sc.kappa = c->scan[g.log2n] + n2;
+  sc.qinv = c->scan[g.log2n] + (2 + 2 * used_seeds) * n2;
+  for (int p = 0; p < 2; p++) chain_state_scale(g, p, &sc.xscale[p], &sc.xinv[p]);
   return sc;
 }
 uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds) { return c->scan_na[log2n][used_seeds]; }
@@ -377,27 +383,64 @@ int check_group(uint32_t log2n, uint32_t l) {
   return DNSPIR_OK;
 }
 
-// Encodes `count` shards' entries (device u16, one shard after another) into
-// their slabs, runs the preprocessing chain and the a-part finalisation.
+const size_t ROWS_BUDGET = (size_t)13 << 28;  // chain layout of the shards in flight (3.25 GiB)
+
+uint32_t preprocess_batch(const Group& g) {
+  if (!chain_rows_supported(g)) return 16;
+  return (uint32_t)std::max<size_t>(1, ROWS_BUDGET / (2 * chain_rows_words(g) * 4));
+}
+
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
-                             const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws,
-                             cudaStream_t st) {
+                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, cudaStream_t st,
+                      uint32_t* last) {
   const size_t per_shard = (size_t)SIMD * g.l * g.n;
+  const SlotMaps maps = slot_maps(c, g.log2n);
+  const ChainConsts cc = chain_consts(c, g.log2n, used_seeds);
+  const size_t a_out_words = (size_t)g.H * SIMD * 2 * g.n;
+  CKR(ws.a_out.ensure(count * a_out_words * 4));
+  uint32_t* const a_out = ws.a_out.as<uint32_t>();
+  if (chain_rows_supported(g)) {
+    const size_t words = chain_rows_words(g), stride = 2 * words;
+    CKR(ws.rows.ensure(count * stride * 4));
+    for (int s = 0; s < count; s++) {
+      // the columns' transforms use the digits' space, the orbit values factor 0's rows
+      uint32_t *rows = ws.rows.as<uint32_t>() + s * stride, *digits = rows + words;
+      launch_encode_cols(entries_dev + s * per_shard, digits, g, g.l, SIMD, c->T, st);
+      launch_encode_rows(digits, rows, g, g.l, SIMD, c->T, st);
+      launch_encode_lift(rows, rows, g, SIMD, 1, maps, c->T, st);
+    }
+    uint32_t* const rows = ws.rows.as<uint32_t>();
+    launch_primary_chain_rows(rows, rows + words, stride, count, a_out, g, cc, c->T, st);
+    launch_primary_finalize(a_out, count, a_zq, a_ms, g, c->T, st);
+    if (last) {
+      launch_order_rows(rows, count * stride, maps, st);
+      for (int s = 0; s < count; s++) {
+        launch_retile_rows(rows + s * stride, rows + s * stride + words, reinterpret_cast<uint8_t*>(slabs_host[s]), g, st);
+        launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(c, g, used_seeds), maps, st);
+      }
+    } else {
+      for (int s = 0; s < count; s++)
+        launch_lane_rows(rows + s * stride, rows + s * stride + words, slabs_host[s], g, maps, st);
+    }
+    CK(cudaGetLastError());
+    return DNSPIR_OK;
+  }
   CKR(ws.A.ensure((size_t)g.l * SIMD * g.n * 4));
   CKR(ws.Ahat.ensure((size_t)g.H * g.L * SIMD * g.n * 4));
-  CKR(ws.a_out.ensure((size_t)count * g.H * SIMD * 2 * g.n * 4));
   CKR(ws.slab_ptrs.ensure((size_t)count * sizeof(uint32_t*)));
   for (int s = 0; s < count; s++) {
     launch_encode_cols(entries_dev + s * per_shard, ws.A.as<uint32_t>(), g, g.l, SIMD, c->T, st);
     launch_encode_rows(ws.A.as<uint32_t>(), ws.Ahat.as<uint32_t>(), g, g.l, SIMD, c->T, st);
-    launch_encode_lift(ws.Ahat.as<uint32_t>(), slabs_host[s], g, SIMD, 0, slot_maps(c, g.log2n), c->T, st);
+    launch_encode_lift(ws.Ahat.as<uint32_t>(), slabs_host[s], g, SIMD, 0, maps, c->T, st);
   }
   CK(cudaMemcpyAsync(ws.slab_ptrs.p, slabs_host, (size_t)count * sizeof(uint32_t*), cudaMemcpyHostToDevice, st));
-  launch_primary_chain(ws.slab_ptrs.as<uint32_t*>(), count, ws.a_out.as<uint32_t>(), g,
-                       chain_consts(c, g.log2n, used_seeds), c->T, st);
-  launch_primary_finalize(ws.a_out.as<uint32_t>(), count, a_zq, a_ms, g, c->T, st);
+  launch_primary_chain(ws.slab_ptrs.as<uint32_t*>(), count, a_out, g, cc, c->T, st);
+  launch_primary_finalize(a_out, count, a_zq, a_ms, g, c->T, st);
+  if (last && g.na == 2)
+    for (int s = 0; s < count; s++)
+      launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(c, g, used_seeds), maps, st);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(st));
+  CK(cudaStreamSynchronize(st));  // slabs_host is the caller's
   return DNSPIR_OK;
 }
 
@@ -455,7 +498,7 @@ int db_noalloc_begin(dnspir_db* db, DbView* out) {
   out->slab = db->slab;
   out->T = db->ctx->T;
   out->maps = slot_maps(db->ctx, db->g.log2n);
-  out->sc = scan_consts(db->ctx, db->g.log2n, db->used_seeds);
+  out->sc = scan_consts(db->ctx, db->g, db->used_seeds);
   return DNSPIR_OK;
 }
 int db_noalloc_end(dnspir_db* db, cudaStream_t st) {
@@ -604,6 +647,7 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   uint32_t* slabs[1] = {db->slab};
   CKR(preprocess_shards(db->ctx, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
                         db->a_ms.as<uint32_t>(), db->ws, db->st));
+  CK(cudaStreamSynchronize(db->st));
   db->ap_ver = ver;
   db->ready = true;
   return DNSPIR_OK;
@@ -646,7 +690,7 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
   launch_ring_to_ntt(db->qz.as<uint64_t>(), SIMD * 4, db->qlane.as<uint32_t>(), nullptr, g.log2n, db->ctx->T, db->st);
   const SlotMaps maps = slot_maps(db->ctx, g.log2n);
   launch_scan_vectors(db->qlane.as<uint32_t>(), 8 * n, 0, 2, SIMD, SIMD, db->qv.as<uint32_t>(), g,
-                      scan_consts(db->ctx, g.log2n, db->used_seeds), maps, db->st);
+                      scan_consts(db->ctx, g, db->used_seeds), maps, db->st);
   if (launch_scan_lanes(db->slab, db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g, db->st))
     return fail(DNSPIR_ERR_CUDA, "cannot clear the scan's sums");
   launch_epilogue_zq(db->sum.as<uint32_t>(), db->out.as<uint64_t>(), g, maps, db->ctx->T, db->st);

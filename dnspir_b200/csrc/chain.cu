@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "ntt2048.cuh"
@@ -59,6 +60,7 @@ struct ChainPrime {
   uint32_t c26;          // 2^26 R mod p
   uint32_t k1, k1q;      // q2^-1 N^-1 mod q1 with its Shoup companion (CRT, factor 1)
   uint32_t k2, k2q;      // q1^-1 N^-1 mod q2 (CRT, factor 2)
+  uint32_t k, kinv;      // this factor's CRT constant (k1 or k2) and its inverse (N times the other factor)
 };
 
 // radix-4 / radix-2 transforms of one length-2^logn vector by CT threads, with
@@ -737,6 +739,10 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
 // instead of six; b = b^ + r a once at the end.  Needs every slot of qry_a
 // invertible (launch_secondary_chain).
 //
+// The state is carried as k a, k the factor's CRT constant: a global scale that
+// the constants absorb (ka1 and qa times k, C + sigma_5(r) over k), so that the
+// inverse transform's outputs are the CRT terms and the digit needs no products.
+//
 // Measured (1024 steps, 64 queries): 10.6 ms for the chunk against 16.6 for one
 // part per block of 512 threads with one factor per half (three waves of
 // blocks, 5.5 us a step); a single query 4.6 ms against 5.8 as two-block
@@ -752,7 +758,7 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
 // transforms' work space), then the five constants (Montgomery form) as
 // [j][factor][quad half][thread] 16-byte vectors.
 constexpr int SEC2K_KC = 5;
-constexpr int sec2k_words(int parts) { return parts * 4 * n2k::PS + SEC2K_KC * 2 * 2 * 256 * 4; }
+constexpr int SEC2K_WORDS = CTXT_PARTS * 4 * n2k::PS + SEC2K_KC * 2 * 2 * 256 * 4;
 
 // T R^-1 mod p, below T / 2^32 + p (T < 2^62)
 __device__ __forceinline__ uint32_t mont_lazy(uint64_t T, uint32_t p, uint32_t pinv) {
@@ -763,14 +769,12 @@ __device__ __forceinline__ double u32_to_double_biased(uint32_t x) {  // 2^52 + 
   return __hiloint2double(0x43300000, (int)x);
 }
 
-// high_digit() plus p for each factor's forward transform, from inverse
-// outputs c1 (mod q1) and c2 (mod q2): the conversions to and from double are
-// additions of 2^52 folded into exact fused multiply-adds (x1 P2 and x2 P1 are
-// below 2^51), and floor is the rounding mode of the last addition.
-__device__ __forceinline__ int32_t high_digit_both(uint32_t c1, uint32_t c2, const ChainPrime& A, const ChainPrime& B) {
-  using ntt_detail::red;
-  const uint32_t x1 = red(shoup_lazy(c1, A.k1, A.k1q, P1), P1);
-  const uint32_t x2 = red(shoup_lazy(c2, B.k2, B.k2q, P2), P2);
+// high_digit() from inverse outputs that carry the CRT constants (below 2p):
+// the conversions to and from double are additions of 2^52 folded into exact
+// fused multiply-adds (x1 P2 and x2 P1 are below 2^51), and floor is the
+// rounding mode of the last addition.
+__device__ __forceinline__ int32_t high_digit_scaled(uint32_t c1, uint32_t c2) {
+  const uint32_t x1 = ntt_detail::red(c1, P1), x2 = ntt_detail::red(c2, P2);
   constexpr double Q = (double)QQ, HALF_Q = (double)(QQ / 2), BIAS = 4503599627370496.0;  // 2^52
   double v = fma(u32_to_double_biased(x1), (double)P2, -BIAS * (double)P2) +
              fma(u32_to_double_biased(x2), (double)P1, -BIAS * (double)P1);
@@ -801,34 +805,143 @@ __device__ __forceinline__ void pass8_both(uint32_t* x, int t, const NttTables& 
   }
 }
 
-template <int PARTS>
-__global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(ChainArgs a, ScanConsts sc) {
+// Padded words that sigma_5 brings to positions 8t .. 8t + 7, two per register (PS < 2^16).
+struct Sources {
+  uint32_t w[4];
+  __device__ __forceinline__ uint32_t at(int m) const { return m & 1 ? w[m >> 1] >> 16 : w[m >> 1] & 0xFFFFu; }
+};
+
+// Transforms of one step on a group's work space x (x, x + PS: the factors):
+// from ta = sigma_5(a) at positions 8t .. 8t + 7 to the high digit's forward
+// transform after stage 8.  `between` runs before the last pass (loads whose
+// latency it covers).  Starts and ends with a barrier of the group.
+template <class Sync, class Between>
+__device__ __forceinline__ void step_transforms(uint32_t* x, const uint32_t (&ta)[2][8], int t, int qb,
+                                                const ChainArgs& a, const Sync& group_sync, const Between& between) {
+  using namespace n2k;
+  group_sync();
+  // inverse stages 0-1 from registers, two quads a factor
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const uint32_t p = prime_of(f);
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++) {
+      const Tw4 w = load_tw4(a.T.iw2[f], 2 * t + h4);
+      uint4 v = make_uint4(ta[f][4 * h4], ta[f][4 * h4 + 1], ta[f][4 * h4 + 2], ta[f][4 * h4 + 3]);
+      gs(v.x, v.y, w.b0, w.b0q, p);
+      gs(v.z, v.w, w.b1, w.b1q, p);
+      gs(v.x, v.z, w.a, w.aq, p);
+      gs(v.y, v.w, w.a, w.aq, p);
+      *reinterpret_cast<uint4*>(x + f * PS + qb + 4 * h4) = v;
+    }
+  }
+  group_sync();
+  pass8_both<64, true>(x, t, a.T);
+  group_sync();
+  pass8_both<8, true>(x, t, a.T);
+  group_sync();
+  {
+    // last inverse pass, high digit, first forward pass; words t + 256 k
+    uint32_t* const y = x + phys(t);
+    constexpr int STR = Geo8<1>::STR;
+    uint32_t v[2][8];
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[f][k] = y[f * PS + k * STR];
+      inv8_bf(v[f], param_tw8(a.T.iw7[f]), prime_of(f));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int32_t hd = high_digit_scaled(v[0][k], v[1][k]);
+      v[0][k] = (uint32_t)(hd + (int32_t)P1), v[1][k] = (uint32_t)(hd + (int32_t)P2);
+    }
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      fwd8_bf(v[f], param_tw8(a.T.fw7[f]), prime_of(f));
+#pragma unroll
+      for (int k = 0; k < 8; k++) y[f * PS + k * STR] = v[f][k];
+    }
+  }
+  group_sync();
+  pass8_both<8, false>(x, t, a.T);
+  group_sync();
+  between();
+  pass8_both<64, false>(x, t, a.T);
+  group_sync();
+}
+
+// Forward stages 9-10 at quad h4 of positions 8t .. 8t + 7: values below 2^31.
+__device__ __forceinline__ uint4 last_stages(const uint32_t* x, int f, int h4, int t, int qb, const NttTables& T) {
+  const uint32_t p = prime_of(f);
+  const n2k::Tw4 w = n2k::load_tw4(T.fw2[f], 2 * t + h4);
+  uint4 v = *reinterpret_cast<const uint4*>(x + f * n2k::PS + qb + 4 * h4);
+  n2k::ct(v.x, v.z, w.a, w.aq, p);
+  n2k::ct(v.y, v.w, w.a, w.aq, p);
+  n2k::ct(v.x, v.y, w.b0, w.b0q, p);
+  n2k::ct(v.z, v.w, w.b1, w.b1q, p);
+  return v;
+}
+
+// r = qry_b / qry_a of half h of query q at a position of factor f
+__device__ __forceinline__ uint32_t query_ratio(const ChainArgs& a, const ScanConsts& sc, int h, int q, int f,
+                                                uint32_t pos) {
+  const uint32_t p = prime_of(f);
+  return mul_mod(__ldg(a.qv + (size_t)q * a.qv_stride + ((size_t)(4 + h) * 2 + f) * N_MAX + pos),
+                 __ldg(sc.qinv + (size_t)(h * 2 + f) * N_MAX + __ldg(a.maps.uof + n2k::brv11(pos))), p, barrett_mu(p));
+}
+
+// ka0, k ka1, k qa (Montgomery form) at a position of factor f
+__device__ __forceinline__ void state_constants(const ChainArgs& a, int h, int f, uint32_t pos, uint32_t* k) {
+  const ChainPrime cp = f ? a.cp[1] : a.cp[0];
+  const uint64_t mu = barrett_mu(cp.p);
+  const size_t o = (size_t)f * N_MAX + pos;
+  const uint32_t ga0 = __ldg(a.gka + o);
+  const uint32_t ka1 =
+      sub_mod(__ldg(a.gka + 2 * (size_t)N_MAX + o), mul_mod(ga0, (1u << LOG2_B) % cp.p, cp.p, mu), cp.p);
+  const uint32_t c[3] = {ga0, mul_mod(ka1, cp.k, cp.p, mu),
+                         mul_mod(__ldg(a.qa + (size_t)h * 2 * N_MAX + o), cp.k, cp.p, mu)};
+#pragma unroll
+  for (int j = 0; j < 3; j++) k[j] = mont_reduce((uint64_t)c[j] * cp.r2, cp.p, cp.pinv);
+}
+
+// the same, then (C + sigma_5(r)) / k and V; from: the position sigma_5 brings here
+__device__ __forceinline__ void secondary_constants(const ChainArgs& a, const ScanConsts& sc, int h, int q, int f,
+                                                    uint32_t pos, uint32_t from, uint32_t* k) {
+  state_constants(a, h, f, pos, k);
+  const ChainPrime cp = f ? a.cp[1] : a.cp[0];
+  const uint64_t mu = barrett_mu(cp.p);
+  const size_t o = (size_t)f * N_MAX + pos;
+  const uint32_t* qq = a.qv + (size_t)q * a.qv_stride;
+  const uint32_t c26 = (1u << LOG2_B) % cp.p, ga0 = __ldg(a.gka + o);
+  const uint32_t ka1 = sub_mod(__ldg(a.gka + 2 * (size_t)N_MAX + o), mul_mod(ga0, c26, cp.p, mu), cp.p);
+  const uint32_t gb0 = __ldg(qq + o), gb1 = __ldg(qq + 2 * (size_t)N_MAX + o);
+  const uint32_t r = query_ratio(a, sc, h, q, f, pos), r5 = query_ratio(a, sc, h, q, f, from);
+  const uint32_t C = sub_mod(gb0, mul_mod(ga0, r, cp.p, mu), cp.p);
+  const uint32_t V = sub_mod(sub_mod(gb1, mul_mod(gb0, c26, cp.p, mu), cp.p), mul_mod(ka1, r, cp.p, mu), cp.p);
+  k[3] = mont_reduce((uint64_t)mul_mod(add_mod(C, r5, cp.p), cp.kinv, cp.p, mu) * cp.r2, cp.p, cp.pinv);
+  k[4] = mont_reduce((uint64_t)V * cp.r2, cp.p, cp.pinv);
+}
+
+__global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(ChainArgs a, ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
   using namespace n2k;
-  constexpr int NT = 256 * PARTS;
-  const int h = blockIdx.x % a.g.H, q = blockIdx.y;
-  const int pt = threadIdx.x >> 8, t = threadIdx.x & 255;
-  const int part = PARTS == 3 ? pt : (int)(blockIdx.x / a.g.H);
-  uint32_t* const A = sm + pt * 4 * PS;
+  constexpr int PARTS = CTXT_PARTS, NT = 256 * PARTS;
+  const int h = blockIdx.x, q = blockIdx.y;
+  const int part = threadIdx.x >> 8, t = threadIdx.x & 255;
+  uint32_t* const A = sm + part * 4 * PS;
   uint32_t* const B = A + 2 * PS;
   uint4* const KC = reinterpret_cast<uint4*>(sm + PARTS * 4 * PS);
   const int qb = (int)phys(8 * t);  // positions 8t .. 8t + 7 sit in one padded row: qb .. qb + 7
-  auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + pt) : "memory"); };
+  auto group_sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + part) : "memory"); };
   // sigma_5 sources of the positions (galb inverted through the constants' space)
   uint32_t* const inv = sm + PARTS * 4 * PS;
   for (int b = threadIdx.x; b < N; b += NT) inv[__ldg(a.galb + b)] = b;
   for (int b = threadIdx.x; b < PARTS * 4 * PS; b += NT) sm[b] = 0;  // a = b^ = 0
   __syncthreads();
-  uint32_t src[4];  // two 16-bit padded positions per word (PS < 2^16)
+  Sources src;
 #pragma unroll
-  for (int m = 0; m < 4; m++) src[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
-  const uint32_t* qq = a.qv + (size_t)q * a.qv_stride;
-  // r at a position of factor f
-  auto ratio = [&](int f, uint32_t pos) {
-    const uint32_t pr = prime_of(f);
-    return mul_mod(__ldg(qq + ((size_t)(4 + h) * 2 + f) * N + pos),
-                   __ldg(sc.qinv + (size_t)(h * 2 + f) * N + __ldg(a.maps.uof + brv11(pos))), pr, barrett_mu(pr));
-  };
+  for (int m = 0; m < 4; m++) src.w[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
   // the constants of position quads, dealt over the whole block: item = (factor, quad)
   {
     constexpr int ITEMS = 2 * N / 4, PER = (ITEMS + NT - 1) / NT;
@@ -846,22 +959,13 @@ __global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(Chain
       const int it = threadIdx.x + c * NT;
       if (it < ITEMS) {
         const int f = it / (N / 4), quad = it & (N / 4 - 1);
-        const ChainPrime cp = f ? a.cp[1] : a.cp[0];
-        const uint64_t mu = barrett_mu(cp.p);
         uint32_t kc[SEC2K_KC][4];
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-          const uint32_t pos = 4 * quad + m;
-          const size_t o = (size_t)f * N + pos;
-          const uint32_t ga0 = __ldg(a.gka + o), c26 = (1u << LOG2_B) % cp.p;
-          const uint32_t ka1 = sub_mod(__ldg(a.gka + 2 * (size_t)N + o), mul_mod(ga0, c26, cp.p, mu), cp.p);
-          const uint32_t gb0 = __ldg(qq + o), gb1 = __ldg(qq + 2 * (size_t)N + o);
-          const uint32_t r = ratio(f, pos), r5 = ratio(f, from[c][m]);
-          const uint32_t C = sub_mod(gb0, mul_mod(ga0, r, cp.p, mu), cp.p);
-          const uint32_t V = sub_mod(sub_mod(gb1, mul_mod(gb0, c26, cp.p, mu), cp.p), mul_mod(ka1, r, cp.p, mu), cp.p);
-          const uint32_t k[SEC2K_KC] = {ga0, ka1, __ldg(a.qa + (size_t)h * 2 * N + o), add_mod(C, r5, cp.p), V};
+          uint32_t k[SEC2K_KC];
+          secondary_constants(a, sc, h, q, f, 4 * quad + m, from[c][m], k);
 #pragma unroll
-          for (int j = 0; j < SEC2K_KC; j++) kc[j][m] = mont_reduce((uint64_t)k[j] * cp.r2, cp.p, cp.pinv);
+          for (int j = 0; j < SEC2K_KC; j++) kc[j][m] = k[j];
         }
 #pragma unroll
         for (int j = 0; j < SEC2K_KC; j++)
@@ -880,63 +984,14 @@ __global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(Chain
 #pragma unroll
     for (int f = 0; f < 2; f++)
 #pragma unroll
-      for (int m = 0; m < 8; m++) ta[f][m] = A[f * PS + (m & 1 ? src[m >> 1] >> 16 : src[m >> 1] & 0xFFFFu)];
-    group_sync();
-    // inverse stages 0-1 from registers, two quads a factor
+      for (int m = 0; m < 8; m++) ta[f][m] = A[f * PS + src.at(m)];
+    uint4 e[2][2];  // entries of the step
+    step_transforms(A, ta, t, qb, a, group_sync, [&] {
 #pragma unroll
-    for (int f = 0; f < 2; f++) {
-      const uint32_t p = prime_of(f);
+      for (int f = 0; f < 2; f++)
 #pragma unroll
-      for (int h4 = 0; h4 < 2; h4++) {
-        const Tw4 w = load_tw4(a.T.iw2[f], 2 * t + h4);
-        uint4 v = make_uint4(ta[f][4 * h4], ta[f][4 * h4 + 1], ta[f][4 * h4 + 2], ta[f][4 * h4 + 3]);
-        gs(v.x, v.y, w.b0, w.b0q, p);
-        gs(v.z, v.w, w.b1, w.b1q, p);
-        gs(v.x, v.z, w.a, w.aq, p);
-        gs(v.y, v.w, w.a, w.aq, p);
-        *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = v;
-      }
-    }
-    group_sync();
-    pass8_both<64, true>(A, t, a.T);
-    group_sync();
-    pass8_both<8, true>(A, t, a.T);
-    group_sync();
-    {
-      // last inverse pass (unscaled: N^-1 sits in the CRT constants), high
-      // digit, first forward pass; words t + 256 k
-      uint32_t* const y = A + phys(t);
-      constexpr int STR = Geo8<1>::STR;
-      uint32_t v[2][8];
-#pragma unroll
-      for (int f = 0; f < 2; f++) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) v[f][k] = y[f * PS + k * STR];
-        inv8_bf(v[f], load_tw8(a.T.iw2[f], 1, 0), prime_of(f));
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int32_t hd = high_digit_both(v[0][k], v[1][k], a.cp[0], a.cp[1]);
-        v[0][k] = (uint32_t)(hd + (int32_t)P1), v[1][k] = (uint32_t)(hd + (int32_t)P2);
-      }
-#pragma unroll
-      for (int f = 0; f < 2; f++) {
-        fwd8_bf(v[f], load_tw8(a.T.fw2[f], 1, 0), prime_of(f));
-#pragma unroll
-        for (int k = 0; k < 8; k++) y[f * PS + k * STR] = v[f][k];
-      }
-    }
-    group_sync();
-    pass8_both<8, false>(A, t, a.T);
-    group_sync();
-    // entries of row i, consumed by the pointwise stage
-    uint4 e[2][2];
-#pragma unroll
-    for (int f = 0; f < 2; f++)
-#pragma unroll
-      for (int h4 = 0; h4 < 2; h4++) e[f][h4] = __ldg(Erow + f * efac + (a.g.L - 1 - i) * erow_stride + h4);
-    pass8_both<64, false>(A, t, a.T);
-    group_sync();
+        for (int h4 = 0; h4 < 2; h4++) e[f][h4] = __ldg(Erow + f * efac + (a.g.L - 1 - i) * erow_stride + h4);
+    });
     // forward stages 9-10 and the pointwise stage at the two quads
     uint4 bn[2][2];
 #pragma unroll
@@ -944,12 +999,7 @@ __global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(Chain
       const uint32_t p = prime_of(f), pinv = f ? a.cp[1].pinv : a.cp[0].pinv;
 #pragma unroll
       for (int h4 = 0; h4 < 2; h4++) {
-        const Tw4 w = load_tw4(a.T.fw2[f], 2 * t + h4);
-        uint4 v = *reinterpret_cast<const uint4*>(A + f * PS + qb + 4 * h4);
-        ct(v.x, v.z, w.a, w.aq, p);
-        ct(v.y, v.w, w.a, w.aq, p);
-        ct(v.x, v.y, w.b0, w.b0q, p);
-        ct(v.z, v.w, w.b1, w.b1q, p);
+        const uint4 v = last_stages(A, f, h4, t, qb, a.T);
         const uint32_t n1[4] = {v.x, v.y, v.z, v.w};
         const uint32_t es[4] = {e[f][h4].x, e[f][h4].y, e[f][h4].z, e[f][h4].w};
         uint32_t kc[SEC2K_KC][4], an[4], b4[4];
@@ -961,8 +1011,7 @@ __global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(Chain
 #pragma unroll
         for (int m = 0; m < 4; m++) {
           const int j = 4 * h4 + m;
-          const uint32_t tt = ta[f][j];
-          const uint32_t tb = B[f * PS + (j & 1 ? src[j >> 1] >> 16 : src[j >> 1] & 0xFFFFu)];
+          const uint32_t tt = ta[f][j], tb = B[f * PS + src.at(j)];
           an[m] = red(mont_lazy((uint64_t)tt * kc[0][m] + (uint64_t)n1[m] * kc[1][m] + (uint64_t)es[m] * kc[2][m], p,
                                 pinv),
                       p);
@@ -985,12 +1034,355 @@ __global__ void __launch_bounds__(256 * PARTS, 1) secondary_chain2k_kernel(Chain
     const uint32_t p = prime_of(f);
 #pragma unroll
     for (int m = 0; m < 8; m++) {
-      const uint32_t av = A[f * PS + qb + m];
+      const uint32_t av = mul_mod(A[f * PS + qb + m], f ? a.cp[1].kinv : a.cp[0].kinv, p, barrett_mu(p));
       const uint32_t br = red(B[f * PS + qb + m], p);
       o[(size_t)f * N + 8 * t + m] = av;
       o[2 * (size_t)N + (size_t)f * N + 8 * t + m] =
-          add_mod(br, mul_mod(av, ratio(f, 8 * t + m), p, barrett_mu(p)), p);
+          add_mod(br, mul_mod(av, query_ratio(a, sc, h, q, f, 8 * t + m), p, barrett_mu(p)), p);
     }
+  }
+}
+
+// Preprocessing chain at N = 2048 with two stored arrays: one chain (shard,
+// half, lane) per block of 256 threads on the same step, without a b part.
+// Rows of the chain layout, E on input, take the state k a' in their place; the
+// canonical high digits' transforms go to `digits`, the same layout.  Three
+// blocks fit an SM (67 KiB, 80 registers), so up to one wave of 444 chains runs
+// at once.  Against two-block clusters with one factor per block (radix-4
+// passes, uncoalesced stores): 9.9 -> PRIM2K ms for 64 chains of 1024 steps.
+constexpr int PRIM2K_KC = 3;
+constexpr int PRIM2K_WORDS = 2 * n2k::PS + PRIM2K_KC * 2 * 2 * 256 * 4;
+
+__global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits,
+                                                                 size_t shard_words) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  using namespace n2k;
+  const int t = threadIdx.x, h = blockIdx.x % a.g.H, lane = blockIdx.x / a.g.H, s = blockIdx.y;
+  uint32_t* const A = sm;
+  uint4* const KC = reinterpret_cast<uint4*>(sm + 2 * PS);
+  uint32_t* const inv = sm + 2 * PS;
+  const int qb = (int)phys(8 * t);
+  for (int b = t; b < N; b += 256) inv[__ldg(a.galb + b)] = b;
+  for (int b = t; b < 2 * PS; b += 256) A[b] = 0;
+  __syncthreads();
+  Sources src;
+#pragma unroll
+  for (int m = 0; m < 4; m++) src.w[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
+  __syncthreads();  // the table is overwritten by the constants, each thread reading only its own
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++) {
+      uint32_t kc[PRIM2K_KC][4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        uint32_t k[PRIM2K_KC];
+        state_constants(a, h, f, 8 * t + 4 * h4 + m, k);
+#pragma unroll
+        for (int j = 0; j < PRIM2K_KC; j++) kc[j][m] = k[j];
+      }
+#pragma unroll
+      for (int j = 0; j < PRIM2K_KC; j++)
+        KC[((j * 2 + f) * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
+    }
+  }
+  const size_t first = (size_t)s * shard_words + ((size_t)h * a.g.L * SIMD + lane) * N + 8 * t;
+  const size_t row_stride = (size_t)SIMD * N, efac = (size_t)a.g.H * a.g.L * row_stride;
+  for (uint32_t i = 0; i < a.g.L; i++) {
+    const size_t row = first + (a.g.L - 1 - i) * row_stride;
+    uint32_t ta[2][8];
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int m = 0; m < 8; m++) ta[f][m] = A[f * PS + src.at(m)];
+    uint4 e[2][2];  // entries of the step (plain loads: the row is rewritten below)
+    step_transforms(A, ta, t, qb, a, [] { __syncthreads(); }, [&] {
+#pragma unroll
+      for (int f = 0; f < 2; f++)
+#pragma unroll
+        for (int h4 = 0; h4 < 2; h4++) e[f][h4] = *reinterpret_cast<const uint4*>(rows + row + f * efac + 4 * h4);
+    });
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      const uint32_t p = prime_of(f), pinv = f ? a.cp[1].pinv : a.cp[0].pinv;
+#pragma unroll
+      for (int h4 = 0; h4 < 2; h4++) {
+        const uint4 v = last_stages(A, f, h4, t, qb, a.T);
+        const uint32_t n1[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t es[4] = {e[f][h4].x, e[f][h4].y, e[f][h4].z, e[f][h4].w};
+        const uint4 k0 = KC[(f * 2 + h4) * 256 + t], k1 = KC[((2 + f) * 2 + h4) * 256 + t],
+                    k2 = KC[((4 + f) * 2 + h4) * 256 + t];
+        const uint32_t kc[PRIM2K_KC][4] = {
+            {k0.x, k0.y, k0.z, k0.w}, {k1.x, k1.y, k1.z, k1.w}, {k2.x, k2.y, k2.z, k2.w}};
+        uint32_t an[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+          an[m] = red(mont_lazy((uint64_t)ta[f][4 * h4 + m] * kc[0][m] + (uint64_t)n1[m] * kc[1][m] +
+                                    (uint64_t)es[m] * kc[2][m],
+                                p, pinv),
+                      p);
+        const uint4 x = make_uint4(an[0], an[1], an[2], an[3]);
+        *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = x;
+        *reinterpret_cast<uint4*>(rows + row + f * efac + 4 * h4) = x;
+        *reinterpret_cast<uint4*>(digits + row + f * efac + 4 * h4) =
+            make_uint4(canon(n1[0], p), canon(n1[1], p), canon(n1[2], p), canon(n1[3], p));
+      }
+    }
+    __syncthreads();
+  }
+  uint32_t* o = a.a_out + (((size_t)s * a.g.H + h) * SIMD + lane) * 2 * N;
+#pragma unroll
+  for (int f = 0; f < 2; f++)
+#pragma unroll
+    for (int m = 0; m < 8; m++)
+      o[(size_t)f * N + 8 * t + m] = mul_mod(A[f * PS + qb + m], f ? a.cp[1].kinv : a.cp[0].kinv, prime_of(f),
+                                             barrett_mu(prime_of(f)));
+}
+
+// ---- The same two chains when they are few: 512 threads per chain, each
+// 256-thread half one factor, which halves a step's serial work per thread (a
+// chain alone on its SM waits on latency, not on a pipe).  The halves exchange
+// their inverse outputs through X, double-buffered by step parity, with the
+// one block-wide barrier of a step; every other barrier is a half's own, so a
+// half may run ahead of the other's reads.  F: the half's factor, so that
+// primes and shared twiddles are constants of its code.
+constexpr int WIDE_NT = 512;
+constexpr int wide_words(int kc) {  // A[2], B[2] (secondary), X[2][2], constants
+  return (kc > 3 ? 4 : 2) * n2k::PS + 4 * N_MAX + kc * 2 * 2 * 256 * 4;
+}
+
+template <int F, bool SEC>
+__device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm, int h, int q,
+                                           int unit, uint32_t* rows, uint32_t* digits) {
+  using namespace n2k;
+  constexpr int NKC = SEC ? SEC2K_KC : PRIM2K_KC;
+  constexpr uint32_t p = F ? P2 : P1;
+  const int t = threadIdx.x & 255;
+  uint32_t* const A = sm + F * PS;
+  uint32_t* const B = sm + (2 + F) * PS;
+  uint32_t* const X = sm + (SEC ? 4 : 2) * PS;  // [parity][factor][k][t]
+  uint4* const KC = reinterpret_cast<uint4*>(X + 4 * N) + F * NKC * 2 * 256;  // [j][quad half][t]
+  auto half_sync = [] { asm volatile("bar.sync %0, 256;" ::"n"(1 + F) : "memory"); };
+  auto full_sync = [] { asm volatile("bar.sync 3, 512;" ::: "memory"); };
+  const int qb = (int)phys(8 * t);
+  // sigma_5 sources (galb inverted through X), a = b^ = 0, constants
+  for (int b = threadIdx.x; b < N; b += WIDE_NT) X[__ldg(a.galb + b)] = b;
+#pragma unroll
+  for (int h4 = 0; h4 < 2; h4++) {
+    *reinterpret_cast<uint4*>(A + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
+    if (SEC) *reinterpret_cast<uint4*>(B + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
+  }
+  full_sync();
+  Sources src;
+#pragma unroll
+  for (int m = 0; m < 4; m++) src.w[m] = phys(X[8 * t + 2 * m]) | (phys(X[8 * t + 2 * m + 1]) << 16);
+#pragma unroll
+  for (int h4 = 0; h4 < 2; h4++) {
+    uint32_t kc[NKC][4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      uint32_t k[NKC];
+      if constexpr (SEC)
+        secondary_constants(a, sc, h, q, F, 8 * t + 4 * h4 + m, X[8 * t + 4 * h4 + m], k);
+      else
+        state_constants(a, h, F, 8 * t + 4 * h4 + m, k);
+#pragma unroll
+      for (int j = 0; j < NKC; j++) kc[j][m] = k[j];
+    }
+#pragma unroll
+    for (int j = 0; j < NKC; j++) KC[(j * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
+  }
+  full_sync();  // X is free
+  const size_t lanes = SEC ? (size_t)a.nl : SIMD;
+  const size_t first = (((size_t)F * a.g.H + h) * a.g.L * lanes + unit) * N + 8 * t;
+  const Tw4 iw0 = load_tw4(a.T.iw2[F], 2 * t), iw1 = load_tw4(a.T.iw2[F], 2 * t + 1);
+  const Tw4 fw0 = load_tw4(a.T.fw2[F], 2 * t), fw1 = load_tw4(a.T.fw2[F], 2 * t + 1);
+  constexpr uint32_t pinv = neg_inv32(p);
+  auto radix8 = [&](auto m, bool inverse) {
+    constexpr int M = decltype(m)::value;
+    using Gm = Geo8<M>;
+    uint32_t* y = A + Gm::base(t);
+    uint32_t v[8];
+    const Tw8 tw = load_tw8(inverse ? a.T.iw2[F] : a.T.fw2[F], M, Gm::blk(t));
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = y[k * Gm::STR];
+    if (inverse)
+      inv8_bf(v, tw, p);
+    else
+      fwd8_bf(v, tw, p);
+#pragma unroll
+    for (int k = 0; k < 8; k++) y[k * Gm::STR] = v[k];
+  };
+  for (uint32_t i = 0; i < a.g.L; i++) {
+    const size_t row = first + (size_t)(a.g.L - 1 - i) * lanes * N;
+    uint32_t ta[8], tb[8];
+#pragma unroll
+    for (int m = 0; m < 8; m++) ta[m] = A[src.at(m)];
+    if (SEC) {
+#pragma unroll
+      for (int m = 0; m < 8; m++) tb[m] = B[src.at(m)];
+    }
+    uint4 e[2];  // entries of the step
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++)
+      e[h4] = SEC ? __ldg(reinterpret_cast<const uint4*>(a.E + row) + h4)
+                  : *(reinterpret_cast<const uint4*>(rows + row) + h4);
+    half_sync();
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++) {
+      const Tw4& w = h4 ? iw1 : iw0;
+      uint4 v = make_uint4(ta[4 * h4], ta[4 * h4 + 1], ta[4 * h4 + 2], ta[4 * h4 + 3]);
+      gs(v.x, v.y, w.b0, w.b0q, p);
+      gs(v.z, v.w, w.b1, w.b1q, p);
+      gs(v.x, v.z, w.a, w.aq, p);
+      gs(v.y, v.w, w.a, w.aq, p);
+      *reinterpret_cast<uint4*>(A + qb + 4 * h4) = v;
+    }
+    half_sync();
+    radix8(std::integral_constant<int, 64>(), true);
+    half_sync();
+    radix8(std::integral_constant<int, 8>(), true);
+    half_sync();
+    {
+      uint32_t* const y = A + phys(t);
+      constexpr int STR = Geo8<1>::STR;
+      uint32_t* const Xc = X + (i & 1) * 2 * N + t;
+      uint32_t v[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] = y[k * STR];
+      inv8_bf(v, param_tw8(a.T.iw7[F]), p);
+#pragma unroll
+      for (int k = 0; k < 8; k++) Xc[F * N + 256 * k] = v[k];
+      full_sync();
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const uint32_t o = Xc[(1 - F) * N + 256 * k];
+        v[k] = (uint32_t)((F ? high_digit_scaled(o, v[k]) : high_digit_scaled(v[k], o)) + (int32_t)p);
+      }
+      fwd8_bf(v, param_tw8(a.T.fw7[F]), p);
+#pragma unroll
+      for (int k = 0; k < 8; k++) y[k * STR] = v[k];
+    }
+    half_sync();
+    radix8(std::integral_constant<int, 8>(), false);
+    half_sync();
+    radix8(std::integral_constant<int, 64>(), false);
+    half_sync();
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++) {
+      const Tw4& w = h4 ? fw1 : fw0;
+      uint4 v = *reinterpret_cast<const uint4*>(A + qb + 4 * h4);
+      ct(v.x, v.z, w.a, w.aq, p);
+      ct(v.y, v.w, w.a, w.aq, p);
+      ct(v.x, v.y, w.b0, w.b0q, p);
+      ct(v.z, v.w, w.b1, w.b1q, p);
+      const uint32_t n1[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t es[4] = {e[h4].x, e[h4].y, e[h4].z, e[h4].w};
+      uint32_t kc[NKC][4], an[4], bn[4];
+#pragma unroll
+      for (int j = 0; j < NKC; j++) {
+        const uint4 c = KC[(j * 2 + h4) * 256 + t];
+        kc[j][0] = c.x, kc[j][1] = c.y, kc[j][2] = c.z, kc[j][3] = c.w;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const uint32_t tt = ta[4 * h4 + m];
+        an[m] = red(mont_lazy((uint64_t)tt * kc[0][m] + (uint64_t)n1[m] * kc[1][m] + (uint64_t)es[m] * kc[2][m], p, pinv),
+                    p);
+        if constexpr (SEC)
+          bn[m] = red(mont_lazy(((uint64_t)tb[4 * h4 + m] << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m],
+                                p, pinv),
+                      2 * p);
+      }
+      const uint4 x = make_uint4(an[0], an[1], an[2], an[3]);
+      *reinterpret_cast<uint4*>(A + qb + 4 * h4) = x;
+      if constexpr (SEC) {
+        *reinterpret_cast<uint4*>(B + qb + 4 * h4) = make_uint4(bn[0], bn[1], bn[2], bn[3]);
+      } else {
+        *(reinterpret_cast<uint4*>(rows + row) + h4) = x;
+        *(reinterpret_cast<uint4*>(digits + row) + h4) =
+            make_uint4(canon(n1[0], p), canon(n1[1], p), canon(n1[2], p), canon(n1[3], p));
+      }
+    }
+    half_sync();
+  }
+  constexpr uint64_t mu = barrett_mu(p);
+  const uint32_t kinv = a.cp[F].kinv;
+#pragma unroll
+  for (int m = 0; m < 8; m++) {
+    const uint32_t av = mul_mod(A[qb + m], kinv, p, mu), pos = 8 * t + m;
+    if constexpr (SEC) {
+      uint32_t* o = a.out + (((size_t)q * a.g.H + h) * CTXT_PARTS + (unit - q * CTXT_PARTS)) * 4 * N + F * N + pos;
+      o[0] = av;
+      o[2 * N] = add_mod(red(B[qb + m], p), mul_mod(av, query_ratio(a, sc, h, q, F, pos), p, mu), p);
+    } else {
+      a.a_out[((size_t)h * SIMD + unit) * 2 * N + F * N + pos] = av;
+    }
+  }
+}
+
+// grid: x = part * H + half, y = query
+__global__ void __launch_bounds__(WIDE_NT, 1) secondary_chain_wide_kernel(ChainArgs a, ScanConsts sc) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const int h = blockIdx.x % a.g.H, q = blockIdx.y, unit = q * CTXT_PARTS + blockIdx.x / a.g.H;
+  if (threadIdx.x < 256)
+    wide_chain<0, true>(a, sc, sm, h, q, unit, nullptr, nullptr);
+  else
+    wide_chain<1, true>(a, sc, sm, h, q, unit, nullptr, nullptr);
+}
+
+// grid: x = lane * H + half, y = shard
+__global__ void __launch_bounds__(WIDE_NT, 1) primary_chain_wide_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits,
+                                                                        size_t shard_words) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const int h = blockIdx.x % a.g.H, s = blockIdx.y, lane = blockIdx.x / a.g.H;
+  rows += s * shard_words, digits += s * shard_words;
+  a.a_out += (size_t)s * a.g.H * SIMD * 2 * N_MAX;
+  if (threadIdx.x < 256)
+    wide_chain<0, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+  else
+    wide_chain<1, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+}
+
+// Rows of the chain layout (bit-reversed positions) to (sign, e) order, in
+// place; one block per row.
+__global__ void __launch_bounds__(256) order_rows_kernel(uint32_t* rows, const uint32_t* __restrict__ gtab) {
+  __shared__ uint4 sm[N_MAX / 4];
+  uint4* const row = reinterpret_cast<uint4*>(rows + (size_t)blockIdx.x * N_MAX);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(sm);
+#pragma unroll
+  for (int c = 0; c < 2; c++) sm[threadIdx.x + 256 * c] = row[threadIdx.x + 256 * c];
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const int q = threadIdx.x + 256 * c;
+    const uint4 g = __ldg(reinterpret_cast<const uint4*>(gtab) + q);
+    row[q] = make_uint4(w[n2k::brv11((g.x - 1) >> 1)], w[n2k::brv11((g.y - 1) >> 1)], w[n2k::brv11((g.z - 1) >> 1)],
+                        w[n2k::brv11((g.w - 1) >> 1)]);
+  }
+}
+
+// Chain-layout rows of the 8 lanes (states and digits) to a shard's lane
+// layout; one block per (factor, half, row) and array.  Position u = (sign, e)
+// of row r holds slot (sign, e + r) (slab_off: row i = L - 1 - r).
+constexpr int LANE_PAD = N_MAX + 4;
+__global__ void __launch_bounds__(512) lane_rows_kernel(const uint32_t* __restrict__ rows,
+                                                        const uint32_t* __restrict__ digits,
+                                                        uint32_t* __restrict__ slab, Group g,
+                                                        const uint32_t* __restrict__ gtab) {
+  extern __shared__ __align__(16) uint32_t sm[];  // [8][LANE_PAD]
+  const uint32_t r = blockIdx.x % g.L, ph = blockIdx.x / g.L, h = ph % g.H, p = ph / g.H;
+  const int arr = blockIdx.y;
+  const uint4* src = reinterpret_cast<const uint4*>((arr ? digits : rows) + (size_t)blockIdx.x * SIMD * N_MAX);
+  for (int q = threadIdx.x; q < SIMD * N_MAX / 4; q += 512)
+    *reinterpret_cast<uint4*>(sm + (q >> 9) * LANE_PAD + 4 * (q & 511)) = __ldg(src + q);
+  __syncthreads();
+  uint32_t* const dst = slab + slab_off(g, (int)p, (int)h, g.L - 1 - r, arr, 0);
+  for (int x = threadIdx.x; x < 2 * N_MAX; x += 512) {
+    const uint32_t u = x >> 1, l0 = (x & 1) * 4;
+    const uint32_t us = (u & (N_MAX / 2)) | ((u + r) & (N_MAX / 2 - 1));
+    const uint32_t* w = sm + l0 * LANE_PAD + n2k::brv11((__ldg(gtab + us) - 1) >> 1);
+    reinterpret_cast<uint4*>(dst)[x] = make_uint4(w[0], w[LANE_PAD], w[2 * LANE_PAD], w[3 * LANE_PAD]);
   }
 }
 
@@ -1085,6 +1477,8 @@ static ChainArgs chain_args(const Group& g, const ChainConsts& cc, const NttTabl
     c.k1q = (uint32_t)(((uint64_t)c.k1 << 32) / P1);
     c.k2 = (uint32_t)((uint64_t)crtc.q1inv2 * ninv2 % P2);
     c.k2q = (uint32_t)(((uint64_t)c.k2 << 32) / P2);
+    c.k = p ? c.k2 : c.k1;
+    c.kinv = (uint32_t)(n * (p ? P1 : P2) % c.p);
   }
   return a;
 }
@@ -1104,13 +1498,47 @@ void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_o
   a.cinv_first = pow_mod2n(a.inv5, g.L - 1, mask);
   const size_t smem = chain_smem(g, 0);
   dim3 grid(2, SIMD * g.H, nshards);
-  if (g.log2n == LOG2_N_MAX) {
-    set_smem(primary_chain_kernel<LOG2_N_MAX>, smem);
-    primary_chain_kernel<LOG2_N_MAX><<<grid, CT, smem, st>>>(a);
-  } else {
-    set_smem(primary_chain_kernel<0>, smem);
-    primary_chain_kernel<0><<<grid, CT, smem, st>>>(a);
+  set_smem(primary_chain_kernel<0>, smem);
+  primary_chain_kernel<0><<<grid, CT, smem, st>>>(a);
+}
+
+int chain_rows_supported(const Group& g) { return g.log2n == LOG2_N_MAX && g.na == 2; }
+
+size_t chain_rows_words(const Group& g) { return (size_t)2 * g.H * g.L * SIMD * g.n; }
+
+void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
+                               const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st) {
+  ChainArgs a = chain_args(g, cc, T);
+  a.a_out = a_out;
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (SIMD * (long)g.H * nshards <= sms) {  // every chain has an SM of its own
+    const size_t smem = (size_t)wide_words(PRIM2K_KC) * 4;
+    set_smem(primary_chain_wide_kernel, smem);
+    primary_chain_wide_kernel<<<dim3(SIMD * g.H, nshards), WIDE_NT, smem, st>>>(a, rows, digits, shard_words);
+    return;
   }
+  const size_t smem = (size_t)PRIM2K_WORDS * 4;
+  set_smem(primary_chain2k_kernel, smem);
+  primary_chain2k_kernel<<<dim3(SIMD * g.H, nshards), 256, smem, st>>>(a, rows, digits, shard_words);
+}
+
+void launch_order_rows(uint32_t* rows, size_t words, const SlotMaps& maps, cudaStream_t st) {
+  order_rows_kernel<<<(unsigned)(words / N_MAX), 256, 0, st>>>(rows, maps.g);
+}
+
+void launch_lane_rows(const uint32_t* rows, const uint32_t* digits, uint32_t* slab, const Group& g,
+                      const SlotMaps& maps, cudaStream_t st) {
+  const size_t smem = (size_t)SIMD * LANE_PAD * 4;
+  set_smem(lane_rows_kernel, smem);
+  lane_rows_kernel<<<dim3(2 * g.H * g.L, 2), 512, smem, st>>>(rows, digits, slab, g, maps.g);
+}
+
+void chain_state_scale(const Group& g, int p, uint32_t* scale, uint32_t* inverse) {
+  const uint32_t pr = p ? P2 : P1;
+  *inverse = chain_rows_supported(g) ? (uint32_t)((uint64_t)g.n * (p ? P1 : P2) % pr) : 1;
+  *scale = (uint32_t)pw(*inverse, pr - 2, pr);
 }
 
 void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq, uint32_t* a_ms, const Group& g,
@@ -1158,13 +1586,13 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
       secondary_chain_kernel<1, 0><<<grid, CT, smem, st>>>(a);
     }
   } else if (reg && (long)nq * CTXT_PARTS * g.H <= sms) {
-    const size_t smem = (size_t)sec2k_words(1) * 4;
-    set_smem(secondary_chain2k_kernel<1>, smem);
-    secondary_chain2k_kernel<1><<<dim3(CTXT_PARTS * g.H, nq), 256, smem, st>>>(a, *sc);
+    const size_t smem = (size_t)wide_words(SEC2K_KC) * 4;
+    set_smem(secondary_chain_wide_kernel, smem);
+    secondary_chain_wide_kernel<<<dim3(CTXT_PARTS * g.H, nq), WIDE_NT, smem, st>>>(a, *sc);
   } else if (reg) {
-    const size_t smem = (size_t)sec2k_words(CTXT_PARTS) * 4;
-    set_smem(secondary_chain2k_kernel<CTXT_PARTS>, smem);
-    secondary_chain2k_kernel<CTXT_PARTS><<<dim3(g.H, nq), 256 * CTXT_PARTS, smem, st>>>(a, *sc);
+    const size_t smem = (size_t)SEC2K_WORDS * 4;
+    set_smem(secondary_chain2k_kernel, smem);
+    secondary_chain2k_kernel<<<dim3(g.H, nq), 256 * CTXT_PARTS, smem, st>>>(a, *sc);
   } else {
     const size_t smem = (size_t)SEC_DUAL_WORDS * g.n * 4;
     set_smem(secondary_dual_kernel<0>, smem);

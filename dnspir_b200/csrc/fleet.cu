@@ -105,7 +105,7 @@ int fleet_drain(dnspir_fleet* f) {
 int launch_scan(dnspir_fleet* f, QSlot& s, int nb, int Bk) {
   const Group& g1 = f->g1;
   launch_scan_vectors(s.qnat.as<uint32_t>(), QV_WORDS_PER_QUERY * g1.n, 2, 0, nb, Bk, s.qv.as<uint32_t>(), g1,
-                      scan_consts(f->ctx, g1.log2n, 0), slot_maps(f->ctx, g1.log2n), f->st);
+                      scan_consts(f->ctx, g1, 0), slot_maps(f->ctx, g1.log2n), f->st);
   f->launches += 1;
   if (f->engine == DNSPIR_ENGINE_TENSOR) {
     int nb_pad = 0;
@@ -225,7 +225,7 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
   f->launches += 1;
   const SlotMaps maps = slot_maps(f->ctx, g2.log2n);
   const ChainConsts cc = chain_consts(f->ctx, g2.log2n, 1);
-  const ScanConsts sc = scan_consts(f->ctx, g2.log2n, 1);
+  const ScanConsts sc = scan_consts(f->ctx, g2, 1);
   const bool two = scan_arrays(f->ctx, g2.log2n, 1) == 2;
   const auto tc = f->tuned_chain.find(nb);
   const bool clustered = tc != f->tuned_chain.end() && tc->second;
@@ -769,44 +769,41 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
     }
   }
   if (f->engine == DNSPIR_ENGINE_TENSOR && f->g1.na == 2) CKR(f->last.ensure(f->D * last_rows_words(f->g1) * 4));
-  const size_t per = (size_t)SIMD * f->g1.l * f->g1.n;
-  const uint32_t batch = 16;
+  const size_t per = (size_t)SIMD * f->g1.l * f->g1.n, n8 = (size_t)SIMD * f->g1.n;
+  const bool tensor = f->engine == DNSPIR_ENGINE_TENSOR, rows = chain_rows_supported(f->g1);
+  const size_t words = slab_words(f->g1), last_words = last_rows_words(f->g1);
+  // without chain rows the tensor engine preprocesses into lane-layout scratch
+  // and re-tiles from there, four shards at a time
+  const uint32_t batch = tensor && !rows ? 4 : preprocess_batch(f->g1);
+  for (uint32_t i = 0; i < count; i++) f->ready[first + i] = false;
   for (uint32_t b0 = 0; b0 < count; b0 += batch) {
-    const uint32_t cnt = count - b0 < batch ? count - b0 : batch;
+    const uint32_t cnt = std::min(count - b0, batch), d0 = first + b0;
     const uint16_t* src = entries + (size_t)b0 * per;
     if (!entries_on_device) {
       CKR(f->ws.in16.ensure((size_t)cnt * per * 2));
       CK(cudaMemcpyAsync(f->ws.in16.p, src, (size_t)cnt * per * 2, cudaMemcpyHostToDevice, f->st));
       src = f->ws.in16.as<uint16_t>();
     }
-    for (uint32_t i = 0; i < cnt; i++) f->ready[first + b0 + i] = false;
-    if (f->engine == DNSPIR_ENGINE_TENSOR) {
-      // preprocess into lane-layout scratch, then re-tile into the fleet slab
-      const uint32_t tb = 4;
-      const size_t words = slab_words(f->g1);
-      CKR(f->tmp_lane.ensure((size_t)std::min(cnt, tb) * words * 4));
-      for (uint32_t c0 = 0; c0 < cnt; c0 += tb) {
-        const uint32_t cc = std::min(tb, cnt - c0);
-        std::vector<uint32_t*> tmp(cc);
-        for (uint32_t i = 0; i < cc; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
-        CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cc, src + (size_t)c0 * per,
-                              f->a_zq.as<uint64_t>() + (size_t)(first + b0 + c0) * SIMD * f->g1.n,
-                              f->a_ms.as<uint32_t>() + (size_t)(first + b0 + c0) * SIMD * f->g1.n, f->ws, f->st));
-        for (uint32_t i = 0; i < cc; i++) {
-          const size_t d = first + b0 + c0 + i;
-          launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d]), f->g1, f->st);
-          if (f->g1.na == 2) launch_last_rows(tmp[i], f->last.as<uint32_t>() + d * last_rows_words(f->g1), f->g1, f->st);
-        }
-      }
-      CK(cudaStreamSynchronize(f->st));
-      f->tmp_lane.release();
+    uint64_t* const a_zq = f->a_zq.as<uint64_t>() + d0 * n8;
+    uint32_t* const a_ms = f->a_ms.as<uint32_t>() + d0 * n8;
+    uint32_t* const last = tensor && f->g1.na == 2 ? f->last.as<uint32_t>() + d0 * last_words : nullptr;
+    if (tensor && !rows) {
+      CKR(f->tmp_lane.ensure((size_t)cnt * words * 4));
+      std::vector<uint32_t*> tmp(cnt);
+      for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
+      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws, f->st, last));
+      for (uint32_t i = 0; i < cnt; i++)
+        launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d0 + i]), f->g1, f->st);
     } else {
-      CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[first + b0], (int)cnt, src,
-                            f->a_zq.as<uint64_t>() + (size_t)(first + b0) * SIMD * f->g1.n,
-                            f->a_ms.as<uint32_t>() + (size_t)(first + b0) * SIMD * f->g1.n, f->ws, f->st));
+      CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws, f->st, last));
     }
-    for (uint32_t i = 0; i < cnt; i++) f->ready[first + b0 + i] = true;
   }
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(f->st));
+  for (uint32_t i = 0; i < count; i++) f->ready[first + i] = true;
+  // the scratch of a bulk load goes back; an update of a few shards keeps its own
+  f->tmp_lane.release();
+  if (count > batch) f->ws.rows.release();
   return DNSPIR_OK;
 }
 

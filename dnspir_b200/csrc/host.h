@@ -98,6 +98,7 @@ struct HBuf {
 // Device buffers shared by set_db and the secondary phase.
 struct EncodeWs {
   DBuf A, Ahat, in16, a_out, slab_ptrs;
+  DBuf rows;  // chain layout of the shards in flight: entries, then states | digits (chain_rows_supported)
 };
 
 struct DeviceGuard {
@@ -122,12 +123,19 @@ void a_parts_host(int log2n, uint64_t* out, uint64_t* version);
 uint64_t a_parts_version(int log2n);
 SlotMaps slot_maps(DeviceCtx* c, int log2n);
 ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds);
-ScanConsts scan_consts(DeviceCtx* c, int log2n, int used_seeds);
+ScanConsts scan_consts(DeviceCtx* c, const Group& g, int used_seeds);
 // Arrays per slab row of shards preprocessed under the context's a-parts (slab_off).
 uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds);
 int check_group(uint32_t log2n, uint32_t l);
 bool reduced(const uint64_t* v, size_t n);
+// Encodes `count` shards' entries (device u16, one shard after another), runs
+// the preprocessing chains and the a-part finalisation, and writes the slabs:
+// lane layout, or tensor layout with `last` rows when last is given (tensor
+// engine, chain_rows_supported).  Queued on st; the caller synchronises.
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
-                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, cudaStream_t st);
+                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, cudaStream_t st,
+                      uint32_t* last = nullptr);
+// Shards that one call of preprocess_shards may carry.
+uint32_t preprocess_batch(const Group& g);
 
 }  // namespace dnspir

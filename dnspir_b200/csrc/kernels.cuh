@@ -60,6 +60,7 @@ struct ScanConsts {
   const uint32_t* gka0;   // [p][N]
   const uint32_t* kappa;  // [p][N]
   const uint32_t* qinv;   // [half][p][N]
+  uint32_t xscale[2], xinv[2];  // scale of the stored states per factor (chain_state_scale) and its inverse
 };
 // Query vectors of the scan, [q][half][v][factor][N] in (sign, e) order (12 N
 // words a query): na = 2: v = 0, 1 multiply the stored arrays, v = 2 the state
@@ -99,6 +100,23 @@ struct ChainConsts {
 // writes G0/G1 into the slabs and a_out[s][h][lane][p][pos].
 void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_out, const Group& g,
                           const ChainConsts& cc, const NttTables& T, cudaStream_t st);
+// The same at N = 2048 with two stored arrays (chain_rows_supported): shard s's
+// rows (launch_encode_lift, frame 1, nl = 8) lie at rows + s * shard_words and
+// take the states, times the factor's CRT constant, in place; the high digits
+// go to digits + s * shard_words, the same layout [p][half][r][lane][pos] with
+// row r for chain step L - 1 - r (chain_rows_words a shard).
+int chain_rows_supported(const Group& g);
+size_t chain_rows_words(const Group& g);
+void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
+                               const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st);
+// Rows of `words` words in all: bit-reversed positions -> (sign, e) order, in place.
+void launch_order_rows(uint32_t* rows, size_t words, const SlotMaps& maps, cudaStream_t st);
+// One shard's rows and digits (bit-reversed positions) -> its lane-layout slab.
+void launch_lane_rows(const uint32_t* rows, const uint32_t* digits, uint32_t* slab, const Group& g,
+                      const SlotMaps& maps, cudaStream_t st);
+// Scale that the stored states carry mod factor p, and its inverse (1 where the
+// generic chain stores them).
+void chain_state_scale(const Group& g, int p, uint32_t* scale, uint32_t* inverse);
 // Sums the halves of a_out, returns reply_a as Z_q coefficients (u64) and the
 // 17-bit mod-switched a-part (u32) per shard: [s][lane][n].
 void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq, uint32_t* a_ms, const Group& g,
@@ -138,6 +156,9 @@ struct TScanShape {
 int tensor_layout_supported(const Group& g);
 void tensor_dims(const Group& g, uint32_t* mt_total, uint32_t* kc_total);
 void launch_retile(const uint32_t* lane_slab, uint8_t* tensor_slab, const Group& g, cudaStream_t st);
+// The same from one shard's rows and digits in (sign, e) order (launch_order_rows).
+void launch_retile_rows(const uint32_t* rows, const uint32_t* digits, uint8_t* tensor_slab, const Group& g,
+                        cudaStream_t st);
 const TScanShape* tscan_shapes(int* count);
 size_t tscan_query_bytes(const Group& g, int nb_pad);
 // Limits of the tensor scan's pipeline waits: wait_ns (0: the default, 2 s)
@@ -159,9 +180,11 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
                  uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
                  const TScanShape& shape, cudaStream_t st, const TScanLimits& lim = TScanLimits(),
                  const void* slab_maps = nullptr);
-// The chain state after the last row of a lane-layout shard, [p][u][half][lane] (na = 2).
+// A shard's chain state after its last row, [p][u][half][lane] (na = 2), from
+// its a_out (launch_primary_chain).
 size_t last_rows_words(const Group& g);
-void launch_last_rows(const uint32_t* lane_slab, uint32_t* last, const Group& g, cudaStream_t st);
+void launch_last_rows(const uint32_t* a_out, uint32_t* last, const Group& g, const ScanConsts& sc, const SlotMaps& maps,
+                      cudaStream_t st);
 // Tensor maps of the shards' tensor-layout slabs (host pointers; one map of
 // tscan_slab_map_bytes(1) bytes per shard) written to dev_maps; -1 when the
 // driver cannot encode them.

@@ -26,6 +26,10 @@ struct NttTables {
   const uint2* iw2[2];
   uint32_t ninv[2][LOG2_N_MAX + 1];   // n^-1 mod p for n = 2^i
   uint32_t ninvq[2][LOG2_N_MAX + 1];
+  // entries 1 .. 7 of the tables, (w, companion): the twiddles of the pass that
+  // every thread shares, read from the kernel's parameters instead of loaded
+  uint2 fw7[2][8];
+  uint2 iw7[2][8];
 };
 
 __device__ __forceinline__ uint32_t brv(uint32_t i, int logn) { return logn ? (__brev(i) >> (32 - logn)) : 0; }

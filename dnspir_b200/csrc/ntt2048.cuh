@@ -71,6 +71,16 @@ __device__ __forceinline__ Tw8 load_tw8(const uint2* __restrict__ tw2, int M, in
   t.c[2] = c1.x, t.cq[2] = c1.y, t.c[3] = c1.z, t.cq[3] = c1.w;
   return t;
 }
+// The same for M = 1 (entries 1 .. 7, shared by all groups) from the kernel's
+// parameters: no loads, and the products take them as constant operands.
+__device__ __forceinline__ Tw8 param_tw8(const uint2 (&w)[8]) {
+  Tw8 t;
+  t.a = w[1].x, t.aq = w[1].y;
+  t.b[0] = w[2].x, t.bq[0] = w[2].y, t.b[1] = w[3].x, t.bq[1] = w[3].y;
+  t.c[0] = w[4].x, t.cq[0] = w[4].y, t.c[1] = w[5].x, t.cq[1] = w[5].y;
+  t.c[2] = w[6].x, t.cq[2] = w[6].y, t.c[3] = w[7].x, t.cq[3] = w[7].y;
+  return t;
+}
 // The three twiddles of the radix-4 pass on quad g: tw[512 + g] and the pair
 // tw[1024 + 2g], tw[1024 + 2g + 1].
 struct Tw4 {
@@ -150,7 +160,7 @@ __device__ __forceinline__ void pass8(uint32_t* x, int cnt0, int cnt1, const Ntt
       const int lo = pi ? cnt0 : 0, hi = pi ? cnt0 + cnt1 : cnt0;
       if (lo >= hi) continue;
       const uint32_t p = prime_of(pi);
-      const Tw8 t = load_tw8(INV ? T.iw2[pi] : T.fw2[pi], M, blk);
+      const Tw8 t = M == 1 ? param_tw8(INV ? T.iw7[pi] : T.fw7[pi]) : load_tw8(INV ? T.iw2[pi] : T.fw2[pi], M, blk);
       // polynomials are dealt to the PPI thread groups by their global index
       // (poly mod PPI), so one polynomial per factor still spreads over all
       // groups

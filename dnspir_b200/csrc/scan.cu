@@ -39,7 +39,8 @@ constexpr int SCAN_NT = 256;
 // and t_i[j] C[j] = a_i[5 j] C[j] joins row i - 1, whose slot for the same
 // output is 5 j: array 0 of every row but the last meets r[j] + C[5^-1 j].
 // The last row's state has no following t, so its C term is taken back (v = 2).
-// In (sign, e) order 5^-1 is e - 1.  One thread per slot, factor and query.
+// In (sign, e) order 5^-1 is e - 1.  States stored with a scale (ScanConsts xinv)
+// meet vectors divided by it.  One thread per slot, factor and query.
 __global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_stride, int s_q, int s_gk, int nb,
                                     uint32_t* __restrict__ qv, Group g, ScanConsts sc,
                                     const uint32_t* __restrict__ gtab) {
@@ -77,9 +78,9 @@ __global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_s
     const uint32_t r = mul_mod(at(s_q + h, u), __ldg(inv + u), pr, mu);
     const uint32_t rm = mul_mod(at(s_q + h, um), __ldg(inv + um), pr, mu);
     const uint32_t cm = sub_mod(gk0m, mul_mod(ga, rm, pr, mu), pr);
-    o[scan_vec_off(N, h, 0, p) + u] = add_mod(r, cm, pr);
+    o[scan_vec_off(N, h, 0, p) + u] = mul_mod(add_mod(r, cm, pr), sc.xinv[p], pr, mu);
     o[scan_vec_off(N, h, 1, p) + u] = sub_mod(g1, mul_mod(ka, r, pr, mu), pr);
-    o[scan_vec_off(N, h, 2, p) + u] = cm ? pr - cm : 0;
+    o[scan_vec_off(N, h, 2, p) + u] = cm ? pr - mul_mod(cm, sc.xinv[p], pr, mu) : 0;
   }
 }
 

@@ -965,13 +965,73 @@ __global__ void retile_kernel(const uint32_t* __restrict__ src, uint8_t* __restr
   *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// The chain state after the last row of a two-array lane slab: row L - 1 of
-// array 0, [p][u][half][lane].  One thread per word.
-__global__ void last_rows_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ last, Group g) {
+// The tensor layout from one shard's rows in (sign, e) order ([p][half][r][lane]
+// [u], states and digits; row r = L - 1 - i).  One block: 16 slots e (four
+// m-tiles) of one factor and sign against one K-chunk (128 slots d of one half
+// and array).  Output (e, d) is word d of row r = (d - e) mod L, so the block
+// reads 64-byte pieces of 143 rows, turns them in shared memory and writes whole
+// 128-byte limb rows.  Bound by HBM: 2 x slab bytes (and the pieces' overlap)
+// once a preprocessing; from the lane layout, whose reads are 4-byte words, a
+// full shard took 1.1 ms.
+constexpr int RT_E = 16, RT_PAD = 132;
+__global__ void __launch_bounds__(256) retile_rows_kernel(const uint32_t* __restrict__ rows,
+                                                          const uint32_t* __restrict__ digits,
+                                                          uint8_t* __restrict__ dst, Group g, uint32_t mt_total,
+                                                          uint32_t kc_total) {
+  extern __shared__ __align__(16) uint32_t sm[];  // [16 e][8 lanes][RT_PAD]
+  const uint32_t half = g.n / 2, L = g.L;  // powers of two
+  const uint32_t e0 = blockIdx.x * RT_E, kc = blockIdx.y;
+  const uint32_t sgn = blockIdx.z & 1;
+  const int p = blockIdx.z >> 1;
+  const uint32_t d0 = (kc * 128) & (half - 1), ha = (kc * 128 - d0) / half;
+  const uint32_t h = ha / 2;
+  const uint32_t* src = (ha & 1 ? digits : rows) + ((size_t)p * g.H + h) * L * SIMD * g.n + sgn * half;
+  // k fastest (the 16 words of a piece), then lane, then row
+#pragma unroll 8
+  for (uint32_t x = threadIdx.x; x < (128 + RT_E - 1) * SIMD * RT_E; x += 256) {
+    const uint32_t k = x % RT_E, lane = x / RT_E % SIMD, rr = x / (RT_E * SIMD);
+    const int dd = (int)(rr + k) - (RT_E - 1);  // d - d0; row r = (d0 + rr - 15 - e0) mod L
+    if (dd >= 0 && dd < 128) {
+      const uint32_t r = (d0 + rr + 2 * L - (RT_E - 1) - e0) & (L - 1);
+      sm[(k * SIMD + lane) * RT_PAD + dd] = __ldg(src + ((size_t)r * SIMD + lane) * g.n + d0 + dd);
+    }
+  }
+  __syncthreads();
+  // one thread per (e, lane, 16-byte unit): 16 words -> their four limb rows
+  for (uint32_t x = threadIdx.x; x < RT_E * SIMD * 8; x += 256) {
+    const uint32_t c = x & 7, lane = (x >> 3) % SIMD, k = x / (8 * SIMD);
+    const uint4* w = reinterpret_cast<const uint4*>(sm + (k * SIMD + lane) * RT_PAD + 16 * c);
+    uint32_t o[4][4];  // [limb][word]
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint4 v = w[q];
+      const uint32_t lo01 = __byte_perm(v.x, v.y, 0x5140), lo23 = __byte_perm(v.z, v.w, 0x5140);
+      const uint32_t hi01 = __byte_perm(v.x, v.y, 0x7362), hi23 = __byte_perm(v.z, v.w, 0x7362);
+      o[0][q] = __byte_perm(lo01, lo23, 0x5410);
+      o[1][q] = __byte_perm(lo01, lo23, 0x7632);
+      o[2][q] = __byte_perm(hi01, hi23, 0x5410);
+      o[3][q] = __byte_perm(hi01, hi23, 0x7632);
+    }
+    const uint32_t e = e0 + k, mt = e / 4;
+    uint8_t* blk = dst + ((((size_t)p * 2 + sgn) * mt_total + mt) * kc_total + kc) * TBLK;
+#pragma unroll
+    for (int limb = 0; limb < 4; limb++) {
+      const uint32_t r = (e % 4) * 32 + lane * 4 + limb;
+      *reinterpret_cast<uint4*>(blk + r * 128 + ((c ^ (r & 7)) << 4)) =
+          make_uint4(o[limb][0], o[limb][1], o[limb][2], o[limb][3]);
+    }
+  }
+}
+
+// The chain state after the last row, scaled as the stored states are, from
+// a_out [half][lane][p][pos] to [p][u][half][lane].  One thread per word.
+__global__ void last_rows_kernel(const uint32_t* __restrict__ a_out, uint32_t* __restrict__ last, Group g,
+                                 ScanConsts sc, const uint32_t* __restrict__ gtab) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * g.n * g.H * SIMD) return;
   const uint32_t lane = i % SIMD, h = (i / SIMD) % g.H, u = (i / (SIMD * g.H)) % g.n, p = i / (SIMD * g.H * g.n);
-  last[i] = src[slab_off(g, (int)p, (int)h, g.L - 1, 0, u) + lane];
+  const uint32_t pos = brv((__ldg(gtab + u) - 1) >> 1, g.log2n), pr = prime_of((int)p);
+  last[i] = mul_mod(__ldg(a_out + (((size_t)h * SIMD + lane) * 2 + p) * g.n + pos), sc.xscale[p], pr, barrett_mu(pr));
 }
 
 // Query operand: one thread per (p, sign, query, 16-byte K unit); writes the
@@ -1148,8 +1208,18 @@ void tensor_dims(const Group& g, uint32_t* mt_total, uint32_t* kc_total) {
 
 size_t last_rows_words(const Group& g) { return (size_t)2 * g.n * g.H * SIMD; }
 
-void launch_last_rows(const uint32_t* lane_slab, uint32_t* last, const Group& g, cudaStream_t st) {
-  last_rows_kernel<<<(unsigned)((last_rows_words(g) + 255) / 256), 256, 0, st>>>(lane_slab, last, g);
+void launch_last_rows(const uint32_t* a_out, uint32_t* last, const Group& g, const ScanConsts& sc, const SlotMaps& maps,
+                      cudaStream_t st) {
+  last_rows_kernel<<<(unsigned)((last_rows_words(g) + 255) / 256), 256, 0, st>>>(a_out, last, g, sc, maps.g);
+}
+
+void launch_retile_rows(const uint32_t* rows, const uint32_t* digits, uint8_t* tensor_slab, const Group& g,
+                        cudaStream_t st) {
+  uint32_t mt, kc;
+  tensor_dims(g, &mt, &kc);
+  const size_t smem = (size_t)RT_E * SIMD * RT_PAD * 4;
+  set_smem(retile_rows_kernel, smem);
+  retile_rows_kernel<<<dim3(mt * 4 / RT_E, kc, 4), 256, smem, st>>>(rows, digits, tensor_slab, g, mt, kc);
 }
 
 void launch_retile(const uint32_t* lane_slab, uint8_t* tensor_slab, const Group& g, cudaStream_t st) {
