@@ -178,3 +178,19 @@ def test_secondary_a_parts_with_zero_slots():
     finally:
         dp.set_a_parts(11, None)
         orc.set_aparts(11, None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("l2", [8, 16, 32, 64, 128, 256, 512, 1024])
+def test_secondary_orders_match_oracle(l2):
+    # every length of the encoder's subgroup transforms, with zero columns
+    # above the shards' (one shard, or as many as the order takes up to three)
+    shards = min(3, l2 // 8)
+    fleet, data = _wire_fleet(l2, shards)
+    ref = orc.Database(11, 1024)
+    ref.set_db(data[0])
+    rng = orc.Rng(bytes([7, l2 % 256]) * 16)
+    queries = [orc.prepare_query(rng, 1000 + k, k % shards, 1024, l2)[0] for k in range(2)]
+    fleet.set_batch(2)
+    assert fleet.process_queries(queries) == [orc.process_query([ref] * shards, q, l2) for q in queries]
+    fleet.close()
