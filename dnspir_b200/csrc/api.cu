@@ -278,11 +278,12 @@ static int build_scan_consts(const uint32_t* consts_dev, int log2n, uint32_t** o
 // change may still read them)
 static int ctx_a_parts(DeviceCtx* c, int log2n, uint64_t* version) {
   const uint32_t n = 1u << log2n;
-  uint64_t ver = 0;
+  uint64_t ver = a_parts_version(log2n);
+  if (version) *version = ver;
+  if (c->consts[log2n] && c->consts_ver[log2n] == ver) return DNSPIR_OK;
   std::vector<uint64_t> ap(6 * (size_t)n);
   a_parts_host(log2n, ap.data(), &ver);
   if (version) *version = ver;
-  if (c->consts[log2n] && c->consts_ver[log2n] == ver) return DNSPIR_OK;
   uint64_t* dz = nullptr;
   uint32_t* dc = nullptr;
   CK(cudaMalloc(&dz, ap.size() * 8));

@@ -65,12 +65,35 @@ const TScanShape& tensor_shape(dnspir_fleet* f, int nb, int* nb_pad) {
   if (it != f->tuned.end()) {
     idx = it->second;
   } else {
-    // untuned: the narrowest query tile that holds the group, one m-tile,
-    // the one-tile-per-CTA kernel
-    const int want = nb <= 4 ? 16 : nb <= 8 ? 32 : nb <= 16 ? 64 : nb <= 32 ? 128 : nb <= 64 ? 256 : 512;
+    // untuned, by whole calls measured over 4 half-size to 64 full shards (ms at
+    // 64 full shards).  A group alone on the device (a call of one group, or
+    // the serial schedules) takes the narrowest query tile that holds it in a
+    // persistent or CTA-pair form, which keeps more of the slab in flight
+    // (30 queries 10.1 against 10.5 one tile per CTA, 50: 16.8 / 17.3).  Groups
+    // that overlap the last one's secondary phase take one tile per CTA: a
+    // persistent CTA whose SM a chain block holds would start its whole share
+    // late (four groups of 12: 27.1 / 31.5, of 50: 59.9 / 64.8).  65 to 96
+    // queries run as three 32-query tiles (24.7 against 28.8 as one 128-query
+    // tile); beyond, the scan is bound by the tensor pipe either way and the
+    // persistent 64-query tile with two m-tiles is best (four groups of 120:
+    // 114.7 / 125.9).  Up to 8 queries HBM bounds every shape alike.  The pair
+    // kernels need the slabs' tensor maps.
+    const auto so = f->tuned_serial.find(nb);
+    const bool alone = f->one_group || (so != f->tuned_serial.end() && so->second);
+    const bool maps = f->tmaps.p != nullptr;
+    TScanShape want;
+    if (nb <= 4) want = TScanShape{16, 1, 5, 0};
+    else if (nb <= 8) want = TScanShape{32, 1, 5, 0};
+    else if (nb <= 16) want = alone ? TScanShape{64, 2, 4, 1} : TScanShape{64, 1, 4, 0};
+    else if (nb <= 32) want = alone && maps ? TScanShape{128, 2, 4, 3} : TScanShape{128, 2, 2, 0};
+    else if (nb <= 64) want = alone && maps ? TScanShape{256, 1, 6, 3} : TScanShape{256, 1, 2, 0};
+    else if (nb <= 96) want = TScanShape{128, 2, 2, 0};
+    else want = TScanShape{256, 2, 3, 1};
     idx = 0;
     for (int i = count - 1; i >= 0; i--)
-      if (sh[i].nq == want && sh[i].mtpc == 1 && !sh[i].persistent) idx = i;
+      if (sh[i].nq == want.nq && sh[i].mtpc == want.mtpc && sh[i].stages == want.stages &&
+          sh[i].persistent == want.persistent)
+        idx = i;
   }
   const int q = sh[idx].nq / 4;
   *nb_pad = (nb + q - 1) / q * q;
@@ -708,6 +731,7 @@ int dnspir_fleet_scan(dnspir_fleet* f, const uint32_t* qnat_dev, uint32_t nq, ui
   const size_t per_out = (size_t)f->S * 2 * n * SIMD;
   QSlot& s = f->slot[0];
   CKR(slot_acquire(f, s));
+  f->one_group = true;  // no secondary phase beside the scans
   for (uint32_t g0 = 0; g0 < nq; g0 += f->batch) {
     const int nb = (int)std::min<uint32_t>(f->batch, nq - g0);
     const int Bk = fleet_kernel_batch(f, nb);
@@ -839,6 +863,7 @@ int dnspir_fleet_process_queries(dnspir_fleet* f, const uint8_t* const* queries,
   }
   if (!on_device && !ok.empty()) CKR(f->rpin.ensure(ok.size() * RB));
   uint32_t gi = 0;
+  f->one_group = ok.size() <= (size_t)f->batch;
   for (size_t g0 = 0; g0 < ok.size(); g0 += f->batch, gi++) {
     const int nb = (int)std::min<size_t>(f->batch, ok.size() - g0);
     const int Bk = fleet_kernel_batch(f, nb);
@@ -934,6 +959,7 @@ int dnspir_fleet_perform_double_pir(dnspir_fleet* f, const uint64_t* pq, const u
   CK(cudaEventCreateWithFlags(&s.sec_done, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&s.sec_tail, cudaEventDisableTiming));
   for (auto& o : f->slot) CKR(slot_acquire(f, o));
+  f->one_group = true;
   const int Bk = fleet_kernel_batch(f, 1);
   cudaEvent_t* t = nullptr;
   CKR(group_events(f, 0, &t));

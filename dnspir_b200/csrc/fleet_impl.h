@@ -57,6 +57,7 @@ struct dnspir_fleet {
   int sec_chunk = 1;  // queries per secondary launch sequence
   int engine = DNSPIR_ENGINE_CUDA_CORES;
   bool serving = false;                       // attached to a running server
+  bool one_group = false;                     // the call in progress is one group (default tile shape)
   dnspir::DBuf qb, err_word, tmp_lane;        // tensor engine: query operand, wait-error word, preprocessing scratch
   dnspir::TScanLimits limits;                 // tensor engine: wait limit (and the timeout-test hook)
   std::map<int, int> tuned;                   // tensor engine: group size -> tile shape index

@@ -435,6 +435,7 @@ int dnspir_server_start(dnspir_server* sv, int use_graphs) {
       db.f->st = db.st;
       db.f->sec = db.sec;
       db.f->serving = true;
+      db.f->one_group = false;  // a database's groups overlap
     }
   }
   CK(cudaDeviceSynchronize());
