@@ -743,11 +743,10 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
 // the constants absorb (ka1 and qa times k, C + sigma_5(r) over k), so that the
 // inverse transform's outputs are the CRT terms and the digit needs no products.
 //
-// Measured (1024 steps, 64 queries): 10.6 ms for the chunk against 16.6 for one
-// part per block of 512 threads with one factor per half (three waves of
-// blocks, 5.5 us a step); a single query 4.6 ms against 5.8 as two-block
-// clusters.  Three parts keep the heavy FMA pipe 73 % and the L1 / shared-memory
-// pipe 83 % busy; the twiddle loads are a third of the latter.
+// Measured (1024 steps, 64 queries): 10.2 ms for the chunk against 16.6 for one
+// part per block of 512 threads with one factor per half and a wave of blocks
+// per 24 queries.  Three parts keep the heavy FMA pipe 73 % and the L1 /
+// shared-memory pipe 83 % busy; the loaded twiddles are a quarter of the latter.
 //
 // Bounds: a is canonical, b^ below 2p.  The forward transform ends below 2^31
 // (ntt.cuh) and n1 is used as it is: t ka0 + n1 ka1 + E qa < 34 p^2, so its
@@ -1049,7 +1048,8 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
 // canonical high digits' transforms go to `digits`, the same layout.  Three
 // blocks fit an SM (67 KiB, 80 registers), so up to one wave of 444 chains runs
 // at once.  Against two-block clusters with one factor per block (radix-4
-// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (4.2 as one chain per SM, below).
+// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (3.4 when
+// there are fewer, on two SMs each, below).
 constexpr int PRIM2K_KC = 3;
 constexpr int PRIM2K_WORDS = 2 * n2k::PS + PRIM2K_KC * 2 * 2 * 256 * 4;
 
@@ -1139,40 +1139,55 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
                                              barrett_mu(prime_of(f)));
 }
 
-// ---- The same two chains when they are few: 512 threads per chain, each
-// 256-thread half one factor, which halves a step's serial work per thread (a
-// chain alone on its SM waits on latency, not on a pipe).  The halves exchange
-// their inverse outputs through X, double-buffered by step parity, with the
-// one block-wide barrier of a step; every other barrier is a half's own, so a
-// half may run ahead of the other's reads.  F: the half's factor, so that
-// primes and shared twiddles are constants of its code.
-constexpr int WIDE_NT = 512;
-constexpr int wide_words(int kc) {  // A[2], B[2] (secondary), X[2][2], constants
-  return (kc > 3 ? 4 : 2) * n2k::PS + 4 * N_MAX + kc * 2 * 2 * 256 * 4;
+// ---- The same two chains when they are few: 256 threads per factor, so that a
+// step is half as long for a thread.  PAIR: the factors' threads are the two
+// blocks of a cluster, on two SMs while there are two for every chain -- a
+// chain alone on one SM keeps its heavy FMA pipe 60 % busy, so the second SM
+// is what shortens the step (3.4 us against 4.2).  Otherwise they are the two
+// halves of one 512-thread block (up to one chain per SM: 4.2 us a step, 4.7 as
+// two cluster blocks per SM).  The factors send each other their inverse outputs:
+// every thread writes its eight values into the other's inbox (double-buffered
+// by step parity, so that one may run ahead of the other's reads) before the
+// one barrier of a step that both meet.  F: the factor, so that primes and
+// shared twiddles are constants of its code.
+constexpr int few_words(int kc) {  // of one factor: A, B (secondary), inbox[2], constants
+  return (kc > 3 ? 2 : 1) * n2k::PS + 2 * N_MAX + kc * 2 * 256 * 4;
 }
 
-template <int F, bool SEC>
-__device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm, int h, int q,
+template <int F, bool SEC, bool PAIR>
+__device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm, int h, int q,
                                            int unit, uint32_t* rows, uint32_t* digits) {
   using namespace n2k;
   constexpr int NKC = SEC ? SEC2K_KC : PRIM2K_KC;
   constexpr uint32_t p = F ? P2 : P1;
+  constexpr int WORDS = few_words(NKC), XO = (SEC ? 2 : 1) * PS;
   const int t = threadIdx.x & 255;
-  uint32_t* const A = sm + F * PS;
-  uint32_t* const B = sm + (2 + F) * PS;
-  uint32_t* const X = sm + (SEC ? 4 : 2) * PS;  // [parity][factor][k][t]
-  uint4* const KC = reinterpret_cast<uint4*>(X + 4 * N) + F * NKC * 2 * 256;  // [j][quad half][t]
-  auto half_sync = [] { asm volatile("bar.sync %0, 256;" ::"n"(1 + F) : "memory"); };
-  auto full_sync = [] { asm volatile("bar.sync 3, 512;" ::: "memory"); };
+  uint32_t* const A = sm + (PAIR ? 0 : F * WORDS);
+  uint32_t* const B = A + PS;
+  uint32_t* const X = A + XO;  // inbox: [parity][half of 8][t] 16-byte vectors
+  uint4* const KC = reinterpret_cast<uint4*>(X + 2 * N);  // [j][quad half][t]
+  // barrier of this factor's threads, and of both factors'
+  auto sync = [] {
+    if constexpr (PAIR)
+      __syncthreads();
+    else
+      asm volatile("bar.sync %0, 256;" ::"n"(1 + F) : "memory");
+  };
+  auto sync_both = [] {
+    if constexpr (PAIR)
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+      asm volatile("bar.sync 3, 512;" ::: "memory");
+  };
   const int qb = (int)phys(8 * t);
   // sigma_5 sources (galb inverted through X), a = b^ = 0, constants
-  for (int b = threadIdx.x; b < N; b += WIDE_NT) X[__ldg(a.galb + b)] = b;
+  for (int b = t; b < N; b += 256) X[__ldg(a.galb + b)] = b;
 #pragma unroll
   for (int h4 = 0; h4 < 2; h4++) {
     *reinterpret_cast<uint4*>(A + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
     if (SEC) *reinterpret_cast<uint4*>(B + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
   }
-  full_sync();
+  sync();
   Sources src;
 #pragma unroll
   for (int m = 0; m < 4; m++) src.w[m] = phys(X[8 * t + 2 * m]) | (phys(X[8 * t + 2 * m + 1]) << 16);
@@ -1192,7 +1207,10 @@ __device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts&
 #pragma unroll
     for (int j = 0; j < NKC; j++) KC[(j * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
   }
-  full_sync();  // X is free
+  // shared::cluster address of the other factor's inbox
+  uint32_t peer = (uint32_t)__cvta_generic_to_shared(PAIR ? X : sm + (1 - F) * WORDS + XO);
+  if constexpr (PAIR) asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(peer) : "r"(1 - F));
+  sync_both();  // both run and both inboxes are free
   const size_t lanes = SEC ? (size_t)a.nl : SIMD;
   const size_t first = (((size_t)F * a.g.H + h) * a.g.L * lanes + unit) * N + 8 * t;
   const Tw4 iw0 = load_tw4(a.T.iw2[F], 2 * t), iw1 = load_tw4(a.T.iw2[F], 2 * t + 1);
@@ -1227,7 +1245,7 @@ __device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts&
     for (int h4 = 0; h4 < 2; h4++)
       e[h4] = SEC ? __ldg(reinterpret_cast<const uint4*>(a.E + row) + h4)
                   : *(reinterpret_cast<const uint4*>(rows + row) + h4);
-    half_sync();
+    sync();
 #pragma unroll
     for (int h4 = 0; h4 < 2; h4++) {
       const Tw4& w = h4 ? iw1 : iw0;
@@ -1238,36 +1256,44 @@ __device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts&
       gs(v.y, v.w, w.a, w.aq, p);
       *reinterpret_cast<uint4*>(A + qb + 4 * h4) = v;
     }
-    half_sync();
+    sync();
     radix8(std::integral_constant<int, 64>(), true);
-    half_sync();
+    sync();
     radix8(std::integral_constant<int, 8>(), true);
-    half_sync();
+    sync();
     {
       uint32_t* const y = A + phys(t);
       constexpr int STR = Geo8<1>::STR;
-      uint32_t* const Xc = X + (i & 1) * 2 * N + t;
+      const uint32_t xo = ((i & 1) * 512 + t) * 16;  // bytes into X
       uint32_t v[8];
 #pragma unroll
       for (int k = 0; k < 8; k++) v[k] = y[k * STR];
       inv8_bf(v, param_tw8(a.T.iw7[F]), p);
 #pragma unroll
-      for (int k = 0; k < 8; k++) Xc[F * N + 256 * k] = v[k];
-      full_sync();
+      for (int h4 = 0; h4 < 2; h4++)
+        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(peer + xo + h4 * 4096), "r"(v[4 * h4]),
+                     "r"(v[4 * h4 + 1]), "r"(v[4 * h4 + 2]), "r"(v[4 * h4 + 3])
+                     : "memory");
+      sync_both();
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t o = Xc[(1 - F) * N + 256 * k];
-        v[k] = (uint32_t)((F ? high_digit_scaled(o, v[k]) : high_digit_scaled(v[k], o)) + (int32_t)p);
+      for (int h4 = 0; h4 < 2; h4++) {
+        const uint4 x = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(X) + xo + h4 * 4096);
+        const uint32_t o[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          uint32_t& w = v[4 * h4 + m];
+          w = (uint32_t)((F ? high_digit_scaled(o[m], w) : high_digit_scaled(w, o[m])) + (int32_t)p);
+        }
       }
       fwd8_bf(v, param_tw8(a.T.fw7[F]), p);
 #pragma unroll
       for (int k = 0; k < 8; k++) y[k * STR] = v[k];
     }
-    half_sync();
+    sync();
     radix8(std::integral_constant<int, 8>(), false);
-    half_sync();
+    sync();
     radix8(std::integral_constant<int, 64>(), false);
-    half_sync();
+    sync();
 #pragma unroll
     for (int h4 = 0; h4 < 2; h4++) {
       const Tw4& w = h4 ? fw1 : fw0;
@@ -1304,7 +1330,7 @@ __device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts&
             make_uint4(canon(n1[0], p), canon(n1[1], p), canon(n1[2], p), canon(n1[3], p));
       }
     }
-    half_sync();
+    sync();
   }
   constexpr uint64_t mu = barrett_mu(p);
   const uint32_t kinv = a.cp[F].kinv;
@@ -1321,27 +1347,48 @@ __device__ __forceinline__ void wide_chain(const ChainArgs& a, const ScanConsts&
   }
 }
 
-// grid: x = part * H + half, y = query
-__global__ void __launch_bounds__(WIDE_NT, 1) secondary_chain_wide_kernel(ChainArgs a, ScanConsts sc) {
-  extern __shared__ __align__(16) uint32_t sm[];
-  const int h = blockIdx.x % a.g.H, q = blockIdx.y, unit = q * CTXT_PARTS + blockIdx.x / a.g.H;
-  if (threadIdx.x < 256)
-    wide_chain<0, true>(a, sc, sm, h, q, unit, nullptr, nullptr);
+// grid: x = part * H + half (times 2, + factor, as pairs), y = query
+template <bool PAIR>
+__device__ __forceinline__ void few_secondary(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm) {
+  const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, f = PAIR ? blockIdx.x & 1 : threadIdx.x >> 8;
+  const int h = c % a.g.H, q = blockIdx.y, unit = q * CTXT_PARTS + c / a.g.H;
+  if (f == 0)
+    few_chain<0, true, PAIR>(a, sc, sm, h, q, unit, nullptr, nullptr);
   else
-    wide_chain<1, true>(a, sc, sm, h, q, unit, nullptr, nullptr);
+    few_chain<1, true, PAIR>(a, sc, sm, h, q, unit, nullptr, nullptr);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2) secondary_chain_pair_kernel(ChainArgs a,
+                                                                                               ScanConsts sc) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  few_secondary<true>(a, sc, sm);
+}
+__global__ void __launch_bounds__(512, 1) secondary_chain_wide_kernel(ChainArgs a, ScanConsts sc) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  few_secondary<false>(a, sc, sm);
 }
 
-// grid: x = lane * H + half, y = shard
-__global__ void __launch_bounds__(WIDE_NT, 1) primary_chain_wide_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits,
-                                                                        size_t shard_words) {
-  extern __shared__ __align__(16) uint32_t sm[];
-  const int h = blockIdx.x % a.g.H, s = blockIdx.y, lane = blockIdx.x / a.g.H;
+// grid: x = lane * H + half (times 2, + factor, as pairs), y = shard
+template <bool PAIR>
+__device__ __forceinline__ void few_primary(ChainArgs& a, uint32_t* rows, uint32_t* digits, size_t shard_words,
+                                            uint32_t* sm) {
+  const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, f = PAIR ? blockIdx.x & 1 : threadIdx.x >> 8;
+  const int h = c % a.g.H, s = blockIdx.y, lane = c / a.g.H;
   rows += s * shard_words, digits += s * shard_words;
   a.a_out += (size_t)s * a.g.H * SIMD * 2 * N_MAX;
-  if (threadIdx.x < 256)
-    wide_chain<0, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+  if (f == 0)
+    few_chain<0, false, PAIR>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
   else
-    wide_chain<1, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+    few_chain<1, false, PAIR>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
+    primary_chain_pair_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits, size_t shard_words) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  few_primary<true>(a, rows, digits, shard_words, sm);
+}
+__global__ void __launch_bounds__(512, 1)
+    primary_chain_wide_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits, size_t shard_words) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  few_primary<false>(a, rows, digits, shard_words, sm);
 }
 
 // Rows of the chain layout (bit-reversed positions) to (sign, e) order, in
@@ -1455,6 +1502,8 @@ static uint32_t inv5_mod2n(uint32_t two_n) {
   return 1;
 }
 
+constexpr size_t PAIR_SMEM = 116 * 1024;  // more than half an SM's shared memory
+
 static ChainArgs chain_args(const Group& g, const ChainConsts& cc, const NttTables& T) {
   ChainArgs a;
   memset(&a, 0, sizeof(a));
@@ -1513,10 +1562,16 @@ void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_wo
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (SIMD * (long)g.H * nshards <= sms) {  // every chain has an SM of its own
-    const size_t smem = (size_t)wide_words(PRIM2K_KC) * 4;
+  const long chains = SIMD * (long)g.H * nshards;
+  if (2 * chains <= sms) {
+    set_smem(primary_chain_pair_kernel, PAIR_SMEM);
+    primary_chain_pair_kernel<<<dim3(2 * SIMD * g.H, nshards), 256, PAIR_SMEM, st>>>(a, rows, digits, shard_words);
+    return;
+  }
+  if (chains <= sms) {
+    const size_t smem = (size_t)2 * few_words(PRIM2K_KC) * 4;
     set_smem(primary_chain_wide_kernel, smem);
-    primary_chain_wide_kernel<<<dim3(SIMD * g.H, nshards), WIDE_NT, smem, st>>>(a, rows, digits, shard_words);
+    primary_chain_wide_kernel<<<dim3(SIMD * g.H, nshards), 512, smem, st>>>(a, rows, digits, shard_words);
     return;
   }
   const size_t smem = (size_t)PRIM2K_WORDS * 4;
@@ -1561,38 +1616,38 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
   a.qv_stride = qv_stride;
   a.nl = nq * CTXT_PARTS;
   a.out = out;
-  // N = 2048: one part per block while every part finds an SM of its own (4.5
-  // us a step), beyond that the three parts of a query and half per block
-  // (10.4 us a step for three parts: 2.3 times the time, three times the work,
-  // the constants kept once).  Other lengths, or a-parts with a zero query
-  // slot: one part and factor per block in 2-block clusters while the chunk
-  // needs at most one block per SM, then one block per part carrying both
-  // factors.  `clustered` asks for the cluster form at any chunk size (88 KiB,
-  // 64 registers: it shares SMs with a running scan; the pipeline tuner picks it
-  // per group size when faster).
+  // N = 2048 (1024 steps of order 2048): a part's chain on two SMs while there
+  // are two for each (3.5 ms), on one while there is one (4.4), beyond that the
+  // three parts of a query and half per block (10.2: 2.4 times the time of one
+  // part alone, three times the work, the constants kept once).  Other lengths,
+  // or a-parts with a zero query slot: one part and factor per block in
+  // two-block clusters while the chunk needs at most one block per SM, then one
+  // block per part carrying both factors.  `clustered` asks for the cluster
+  // form at any chunk size (its blocks share SMs with a running scan; the
+  // pipeline tuner picks it per group size when faster).
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool full = g.log2n == LOG2_N_MAX;
   const bool reg = full && sc;
-  if (clustered || (!reg && (long)nq * CTXT_PARTS * g.H * 2 <= sms)) {
-    const size_t smem = chain_smem(g, 1);
-    const dim3 grid(2, CTXT_PARTS * g.H, nq);
-    if (full) {
-      set_smem(secondary_chain_kernel<1, LOG2_N_MAX>, smem);
-      secondary_chain_kernel<1, LOG2_N_MAX><<<grid, CT, smem, st>>>(a);
-    } else {
-      set_smem(secondary_chain_kernel<1, 0>, smem);
-      secondary_chain_kernel<1, 0><<<grid, CT, smem, st>>>(a);
-    }
-  } else if (reg && (long)nq * CTXT_PARTS * g.H <= sms) {
-    const size_t smem = (size_t)wide_words(SEC2K_KC) * 4;
+  const long chains = (long)nq * CTXT_PARTS * g.H;
+  if (reg && (clustered || 2 * chains <= sms)) {
+    // PAIR_SMEM keeps the two blocks off one SM (and fits beside a scan block)
+    const size_t smem = clustered && 2 * chains > sms ? (size_t)few_words(SEC2K_KC) * 4 : PAIR_SMEM;
+    set_smem(secondary_chain_pair_kernel, smem);
+    secondary_chain_pair_kernel<<<dim3(2 * CTXT_PARTS * g.H, nq), 256, smem, st>>>(a, *sc);
+  } else if (reg && chains <= sms) {
+    const size_t smem = (size_t)2 * few_words(SEC2K_KC) * 4;
     set_smem(secondary_chain_wide_kernel, smem);
-    secondary_chain_wide_kernel<<<dim3(CTXT_PARTS * g.H, nq), WIDE_NT, smem, st>>>(a, *sc);
+    secondary_chain_wide_kernel<<<dim3(CTXT_PARTS * g.H, nq), 512, smem, st>>>(a, *sc);
   } else if (reg) {
     const size_t smem = (size_t)SEC2K_WORDS * 4;
     set_smem(secondary_chain2k_kernel, smem);
     secondary_chain2k_kernel<<<dim3(g.H, nq), 256 * CTXT_PARTS, smem, st>>>(a, *sc);
+  } else if (clustered || 2 * chains <= sms) {
+    const size_t smem = chain_smem(g, 1);
+    set_smem(secondary_chain_kernel<1, 0>, smem);
+    secondary_chain_kernel<1, 0><<<dim3(2, CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
   } else {
     const size_t smem = (size_t)SEC_DUAL_WORDS * g.n * 4;
     set_smem(secondary_dual_kernel<0>, smem);
