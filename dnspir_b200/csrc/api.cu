@@ -446,9 +446,9 @@ int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* co
 }
 
 bool reduced(const uint64_t* v, size_t n) {
-  for (size_t i = 0; i < n; i++)
-    if (v[i] >= QQ) return false;
-  return true;
+  uint64_t over = 0;  // top bit set by any value of q or more, without a branch per value
+  for (size_t i = 0; i < n; i++) over |= v[i] | (QQ - 1 - v[i]);
+  return over >> 63 == 0;
 }
 
 }  // namespace dnspir
@@ -464,6 +464,7 @@ struct dnspir_db {
   cudaEvent_t noalloc_done = nullptr;  // recorded on the caller's stream after each no-allocation call
   uint32_t* slab = nullptr;
   DBuf a_zq, a_ms, qz, qlane, qv, sum, out;
+  HBuf pin;  // host staging of perform_pir_split: query elements in, reply out
   EncodeWs ws;
   std::mutex mu;
   ~dnspir_db() {
@@ -673,21 +674,24 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
     return fail(DNSPIR_ERR_BAD_SHAPE, "conjugate query must be given exactly when the group requires it");
   const size_t n = g.n;
   // [lane][v][N], v = qry, qry_conj, gk0, gk1
-  std::vector<uint64_t> z((size_t)SIMD * 4 * n, 0);
-  for (int k = 0; k < SIMD; k++) {
-    memcpy(&z[((size_t)k * 4 + 0) * n], qry_b + k * n, n * 8);
-    if (qry_conj_b) memcpy(&z[((size_t)k * 4 + 1) * n], qry_conj_b + k * n, n * 8);
-    memcpy(&z[((size_t)k * 4 + 2) * n], gk_b + (2 * k) * n, n * 8);
-    memcpy(&z[((size_t)k * 4 + 3) * n], gk_b + (2 * k + 1) * n, n * 8);
-  }
-  if (!reduced(z.data(), z.size())) return fail(DNSPIR_ERR_BAD_ARG, "ring element coefficients must be below q");
   DeviceGuard dg(db->device);
-  CKR(db->qz.ensure(z.size() * 8));
-  CKR(db->qlane.ensure(z.size() * 2 * 4));
+  CK(cudaStreamSynchronize(db->st));  // an earlier call that failed may still copy from the staging buffer
+  const size_t words = (size_t)SIMD * 4 * n;
+  CKR(db->pin.ensure(words * 8));
+  uint64_t* const z = db->pin.as<uint64_t>();
+  for (size_t k = 0; k < SIMD; k++) {
+    memcpy(z + (k * 4 + 0) * n, qry_b + k * n, n * 8);
+    if (qry_conj_b) memcpy(z + (k * 4 + 1) * n, qry_conj_b + k * n, n * 8);
+    else memset(z + (k * 4 + 1) * n, 0, n * 8);
+    memcpy(z + (k * 4 + 2) * n, gk_b + 2 * k * n, 2 * n * 8);
+  }
+  if (!reduced(z, words)) return fail(DNSPIR_ERR_BAD_ARG, "ring element coefficients must be below q");
+  CKR(db->qz.ensure(words * 8));
+  CKR(db->qlane.ensure(words * 2 * 4));
   CKR(db->qv.ensure((size_t)SIMD * 4 * SCAN_VECS * n * 4));
   CKR(db->sum.ensure(scan_lanes_sum_words(g) * 4));
   CKR(db->out.ensure((size_t)SIMD * n * 8));
-  CK(cudaMemcpyAsync(db->qz.p, z.data(), z.size() * 8, cudaMemcpyHostToDevice, db->st));
+  CK(cudaMemcpyAsync(db->qz.p, z, words * 8, cudaMemcpyHostToDevice, db->st));
   launch_ring_to_ntt(db->qz.as<uint64_t>(), SIMD * 4, db->qlane.as<uint32_t>(), nullptr, g.log2n, db->ctx->T, db->st);
   const SlotMaps maps = slot_maps(db->ctx, g.log2n);
   launch_scan_vectors(db->qlane.as<uint32_t>(), 8 * n, 0, 2, SIMD, SIMD, db->qv.as<uint32_t>(), g,
@@ -696,8 +700,9 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
     return fail(DNSPIR_ERR_CUDA, "cannot clear the scan's sums");
   launch_epilogue_zq(db->sum.as<uint32_t>(), db->out.as<uint64_t>(), g, maps, db->ctx->T, db->st);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(out_b, db->out.p, (size_t)SIMD * n * 8, cudaMemcpyDeviceToHost, db->st));
+  CK(cudaMemcpyAsync(z, db->out.p, (size_t)SIMD * n * 8, cudaMemcpyDeviceToHost, db->st));
   CK(cudaStreamSynchronize(db->st));
+  memcpy(out_b, z, (size_t)SIMD * n * 8);
   return DNSPIR_OK;
 }
 

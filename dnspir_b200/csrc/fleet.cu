@@ -110,13 +110,16 @@ int slot_acquire(dnspir_fleet* f, QSlot& s) {
 int fleet_drain(dnspir_fleet* f) {
   for (auto& s : f->slot)
     if (s.sec_pending) CK(cudaStreamWaitEvent(f->st, s.sec_done, 0));
+  const bool tensor = f->engine == DNSPIR_ENGINE_TENSOR;
+  if (tensor) {  // the error word comes with the same wait
+    CKR(f->epin.ensure(4));
+    CK(cudaMemcpyAsync(f->epin.p, f->err_word.p, 4, cudaMemcpyDeviceToHost, f->st));
+  }
   CK(cudaStreamSynchronize(f->st));
   CK(cudaStreamSynchronize(f->sec));
   for (auto& s : f->slot) s.sec_pending = false;
-  if (f->engine == DNSPIR_ENGINE_TENSOR) {
-    uint32_t e = 0;
-    CK(cudaMemcpy(&e, f->err_word.p, 4, cudaMemcpyDeviceToHost));
-    if (e) {
+  if (tensor) {
+    if (*f->epin.as<uint32_t>()) {
       CK(cudaMemset(f->err_word.p, 0, 4));
       return fail(DNSPIR_ERR_TIMEOUT, "tensor scan: a pipeline wait gave up");
     }
@@ -218,10 +221,10 @@ int fleet_secondary_workspace(dnspir_fleet* f, int nb) {
 }
 
 int fleet_primary_kernels(dnspir_fleet* f, QSlot& s, int nb, int Bk, const uint32_t* sess_nat,
-                          const uint32_t* sess_brv, cudaEvent_t scan0, cudaEvent_t scan1) {
+                          const uint32_t* sess_brv, cudaEvent_t scan0, cudaEvent_t scan1, bool decode) {
   const Group& g1 = f->g1;
   const size_t qv = QV_WORDS_PER_QUERY * g1.n;
-  if (s.qbytes.p) {
+  if (decode) {
     launch_decode_query(s.qbytes.as<uint8_t>(), s.qdesc.as<QDesc>(), nb, fleet_wire_spec(f), fleet_gk_bytes(f),
                         s.qnat.as<uint32_t>(), s.qbrv.as<uint32_t>(), qv, sess_nat, sess_brv, g1.log2n, f->ctx->T,
                         f->st);
@@ -304,8 +307,8 @@ int allocate_slabs(dnspir_fleet* f) {
 // secondary on f->sec after the primary.  Query bytes and descriptors (or
 // decoded vectors) must already be queued on f->st.
 int run_group(dnspir_fleet* f, QSlot& s, int nb, int Bk, cudaEvent_t* t, uint8_t* reply_dev, size_t reply_stride,
-              uint64_t* reply_zq, uint8_t* host_reply) {
-  CKR(fleet_primary_kernels(f, s, nb, Bk, nullptr, nullptr, t[1], t[2]));
+              uint64_t* reply_zq, uint8_t* host_reply, bool decode = true) {
+  CKR(fleet_primary_kernels(f, s, nb, Bk, nullptr, nullptr, t[1], t[2], decode));
   CK(cudaEventRecord(t[3], f->st));
   CK(cudaEventRecord(s.prim_done, f->st));
   s.prim_recorded = true;
@@ -943,38 +946,39 @@ int dnspir_fleet_perform_double_pir(dnspir_fleet* f, const uint64_t* pq, const u
   if ((f->g2.H == 2) != (sqc != nullptr))
     return fail(DNSPIR_ERR_BAD_SHAPE, "conjugate secondary query must be given exactly when required");
   const size_t n = f->g1.n;
-  std::vector<uint64_t> z(6 * n, 0);
-  memcpy(&z[0], gk, n * 8);
-  memcpy(&z[n], gk + n, n * 8);
-  memcpy(&z[2 * n], pq, n * 8);
-  if (pqc) memcpy(&z[3 * n], pqc, n * 8);
-  memcpy(&z[4 * n], sq, n * 8);
-  if (sqc) memcpy(&z[5 * n], sqc, n * 8);
-  if (!reduced(z.data(), z.size())) return fail(DNSPIR_ERR_BAD_ARG, "ring element coefficients must be below q");
   DeviceGuard dg(f->device);
-  // a private slot without query bytes: the ring elements go straight to the
-  // decoded vectors
-  QSlot s;
-  CK(cudaEventCreateWithFlags(&s.prim_done, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&s.sec_done, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&s.sec_tail, cudaEventDisableTiming));
+  // pinned staging: the six elements in, the six polynomials of the reply out
+  const size_t words = 6 * n;
+  static_assert(CTXT_PARTS * 2 == 6, "as many polynomials out as in");
   for (auto& o : f->slot) CKR(slot_acquire(f, o));
+  CK(cudaStreamSynchronize(f->st));  // an earlier call that failed may still copy from it
+  CKR(f->zpin.ensure(words * 8));
+  uint64_t* const z = f->zpin.as<uint64_t>();
+  const uint64_t* const in[6] = {gk, gk + n, pq, pqc, sq, sqc};
+  for (int i = 0; i < 6; i++) {
+    if (in[i]) memcpy(z + i * n, in[i], n * 8);
+    else memset(z + i * n, 0, n * 8);
+  }
+  if (!reduced(z, words)) return fail(DNSPIR_ERR_BAD_ARG, "ring element coefficients must be below q");
+  // the first slot, without query bytes: the ring elements go straight to the
+  // decoded vectors
+  QSlot& s = f->slot[0];
   f->one_group = true;
   const int Bk = fleet_kernel_batch(f, 1);
   cudaEvent_t* t = nullptr;
   CKR(group_events(f, 0, &t));
   CKR(fleet_slot_workspace(f, s, Bk, 1, 0));
-  CKR(f->qzq.ensure(z.size() * 8));
-  CKR(f->reply_zq.ensure((size_t)CTXT_PARTS * 2 * n * 8));
+  CKR(f->qzq.ensure(words * 8));
+  CKR(f->reply_zq.ensure(words * 8));
   CK(cudaEventRecord(t[0], f->st));
-  CK(cudaMemcpyAsync(f->qzq.p, z.data(), z.size() * 8, cudaMemcpyHostToDevice, f->st));
+  CK(cudaMemcpyAsync(f->qzq.p, z, words * 8, cudaMemcpyHostToDevice, f->st));
   launch_ring_to_ntt(f->qzq.as<uint64_t>(), 6, s.qnat.as<uint32_t>(), s.qbrv.as<uint32_t>(), f->g1.log2n, f->ctx->T,
                      f->st);
-  CKR(run_group(f, s, 1, Bk, t, nullptr, 0, f->reply_zq.as<uint64_t>(), nullptr));
+  CKR(run_group(f, s, 1, Bk, t, nullptr, 0, f->reply_zq.as<uint64_t>(), nullptr, false));
   f->q_group.assign(1, 0);
-  CK(cudaStreamWaitEvent(f->st, s.sec_done, 0));
+  CK(cudaMemcpyAsync(z, f->reply_zq.p, words * 8, cudaMemcpyDeviceToHost, f->sec));
   CKR(fleet_drain(f));
-  CK(cudaMemcpy(out, f->reply_zq.p, (size_t)CTXT_PARTS * 2 * n * 8, cudaMemcpyDeviceToHost));
+  memcpy(out, z, words * 8);
   return DNSPIR_OK;
 }
 

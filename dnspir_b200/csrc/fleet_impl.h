@@ -53,6 +53,7 @@ struct dnspir_fleet {
   dnspir::QSlot slot[2];
   dnspir::DBuf secE, chain_out, qzq, reply_zq;  // used by one stream at a time
   dnspir::HBuf rpin;                            // host staging of the replies of one call
+  dnspir::HBuf zpin, epin;                      // host staging of perform_double_pir's elements, of the error word
   int batch = 1;
   int sec_chunk = 1;  // queries per secondary launch sequence
   int engine = DNSPIR_ENGINE_CUDA_CORES;
@@ -89,9 +90,9 @@ int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbyte
 int fleet_secondary_workspace(dnspir_fleet* f, int nb);
 // Primary kernels of a group on f->st: decode (bytes and descriptors already
 // in s.qbytes / s.qdesc) and scan.  scan0/scan1: optional events around the
-// scan.
+// scan.  decode = false: the decoded vectors are there already.
 int fleet_primary_kernels(dnspir_fleet* f, QSlot& s, int nb, int Bk, const uint32_t* sess_nat,
-                          const uint32_t* sess_brv, cudaEvent_t scan0, cudaEvent_t scan1);
+                          const uint32_t* sess_brv, cudaEvent_t scan0, cudaEvent_t scan1, bool decode = true);
 // Secondary kernels of a group on f->sec: primary epilogue, encode, chains, replies (bytes at
 // reply_dev + q * reply_stride, or Z_q ciphertexts at reply_zq), and the copy
 // of nb reply bytes to host_reply when given.
