@@ -345,16 +345,16 @@ struct LiftFin {
   }
 };
 
-// One block: column r of half h for up to LIFT_LANES_CHAIN lanes, chain layout
+// One block: column r of half h for up to `lpb` lanes, chain layout
 // (factor 0 of the output may lie on Ahat, as in encode_lift_kernel).
 __global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* Ahat, uint32_t* out, Group g, int nl,
-                                                             uint32_t scale, uint32_t scale_q,
+                                                             int lpb, uint32_t scale, uint32_t scale_q,
                                                              const uint32_t* __restrict__ pow5inv, NttTables T) {
   extern __shared__ __align__(16) uint32_t sm[];
   using namespace n2k;
   const uint32_t r = blockIdx.x, h = blockIdx.y;
-  const int lane0 = blockIdx.z * LIFT_LANES_CHAIN;
-  const int nlg = min(LIFT_LANES_CHAIN, nl - lane0);
+  const int lane0 = blockIdx.z * lpb;
+  const int nlg = min(lpb, nl - lane0);
   for (int b = threadIdx.x; b < nlg * (N / 4); b += NT2K) {
     const int kk = b >> 9, q = b & (N / 4 - 1);
     const uint4 v = reinterpret_cast<const uint4*>(Ahat + (((size_t)h * g.L + r) * nl + lane0 + kk) * N)[q];
@@ -435,7 +435,7 @@ void launch_encode_cols(const uint16_t* in, uint32_t* A, const Group& g, uint32_
   const uint32_t total = l_in * nl;
   if (!total) return;
   if (g.log2n == 11) {
-    const int ppc = 4;
+    const int ppc = total <= 592 ? 1 : 4;  // polynomials per block, as above
     const size_t smem = (size_t)ppc * n2k::PS * 4;
     set_smem(encode_cols2k_kernel, smem);
     encode_cols2k_kernel<<<(total + ppc - 1) / ppc, NT2K, smem, st>>>(in, A, total, ppc, T);
@@ -492,11 +492,14 @@ void launch_encode_lift(const uint32_t* Ahat, uint32_t* out, const Group& g, int
     if ((x * (g.l % TPLAIN)) % TPLAIN == 1) linv = x;
   if (g.log2n == 11 && frame == 1) {
     const uint32_t sq = (uint32_t)(((uint64_t)linv << 32) / TPLAIN);
-    const int nlg = nl < LIFT_LANES_CHAIN ? nl : LIFT_LANES_CHAIN;
+    // lanes share a block's twiddles; one lane per block where that many
+    // blocks (three fit an SM) do not fill the SMs once
+    const int lpb = (size_t)g.L * g.H * nl <= 444 ? 1 : LIFT_LANES_CHAIN;
+    const int nlg = nl < lpb ? nl : lpb;
     const size_t smem = (size_t)2 * nlg * n2k::PS * 4;
-    dim3 grid(g.L, g.H, (nl + LIFT_LANES_CHAIN - 1) / LIFT_LANES_CHAIN);
+    dim3 grid(g.L, g.H, (nl + lpb - 1) / lpb);
     set_smem(encode_lift2k_kernel, smem);
-    encode_lift2k_kernel<<<grid, NT2K, smem, st>>>(Ahat, out, g, nl, linv, sq, pow_table(g.log2n, true), T);
+    encode_lift2k_kernel<<<grid, NT2K, smem, st>>>(Ahat, out, g, nl, lpb, linv, sq, pow_table(g.log2n, true), T);
     return;
   }
   // frame 0 writes the 8 lanes of a slot together; frame 1 (chain layout)

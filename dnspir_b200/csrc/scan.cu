@@ -331,7 +331,9 @@ __global__ void primary_epilogue_kernel(const uint32_t* __restrict__ fin, int ns
 // gather per position and factor brings four lanes (half a 32-byte sector; the
 // other half is the neighbouring block's), the eight inverse transforms run
 // together, the CRT uses Shoup companions of its two constants and the 12-bit
-// switch an exact 64-bit rounding (v 2^13 + q < 2^64 for v < q).
+// switch an exact 64-bit rounding (v 2^13 + q < 2^64 for v < q).  LN = 1: one
+// lane per block, for so few shards and queries that the blocks do not fill the
+// SMs (one query of 4 shards: 25 -> 12.6 us).
 constexpr int EPI_NT = 512;
 
 __device__ __forceinline__ uint32_t ms_encode12(uint64_t v) {
@@ -348,33 +350,38 @@ __device__ __forceinline__ uint32_t ms_encode12(uint64_t v) {
   return (uint32_t)r & ((1u << PRIM_B_BITS) - 1);
 }
 
-__global__ void __launch_bounds__(EPI_NT, 3) primary_epilogue2k_kernel(
+template <int LN>
+__global__ void __launch_bounds__(EPI_NT, LN == 4 ? 3 : 0) primary_epilogue2k_kernel(
     const uint32_t* __restrict__ fin, int nshards, const uint32_t* __restrict__ a_ms,
     const int* __restrict__ distinct_of, uint16_t* __restrict__ sec_in, int nq, int chunk,
     const uint32_t* __restrict__ uof, NttTables T, uint32_t k1, uint32_t k1q, uint32_t k2, uint32_t k2q) {
-  extern __shared__ __align__(16) uint32_t sm[];  // [q1 lanes l0 .. l0 + 3][q2 lanes], padded
+  extern __shared__ __align__(16) uint32_t sm[];  // [q1 lanes l0 .. l0 + LN - 1][q2 lanes], padded
   using namespace n2k;
-  const int s = blockIdx.x, l0 = blockIdx.y * 4, b = blockIdx.z;
+  const int s = blockIdx.x, l0 = blockIdx.y * LN, b = blockIdx.z;
   // position x of factor p holds natural slot brv(x)
   for (int x = threadIdx.x; x < 2 * N; x += EPI_NT) {
     const int p = x >> 11, xx = x & (N - 1);
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(
-        fin + ((((size_t)b * nshards + s) * 2 + p) * N + __ldg(uof + brv11(xx))) * SIMD + l0));
-    uint32_t* o = sm + 4 * p * PS + phys(xx);
-    o[0] = v.x, o[PS] = v.y, o[2 * PS] = v.z, o[3 * PS] = v.w;
+    const uint32_t* src = fin + ((((size_t)b * nshards + s) * 2 + p) * N + __ldg(uof + brv11(xx))) * SIMD + l0;
+    uint32_t* o = sm + LN * p * PS + phys(xx);
+    if constexpr (LN == 4) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+      o[0] = v.x, o[PS] = v.y, o[2 * PS] = v.z, o[3 * PS] = v.w;
+    } else {
+      o[0] = __ldg(src);
+    }
   }
   __syncthreads();
-  inv<EPI_NT>(sm, 4, 4, T);
+  inv<EPI_NT>(sm, LN, LN, T);
   const int ds = distinct_of[s];
   // the secondary input of queries [c * chunk, ...) is one [t][lanes_c][N] block
   const int c = b / chunk, bl = b % chunk;
   const size_t lanes_c = (size_t)CTXT_PARTS * min(chunk, nq - c * chunk);
   uint16_t* const base = sec_in + (size_t)c * chunk * CTXT_PARTS * nshards * SIMD * N;
-  for (int x = threadIdx.x; x < 4 * N; x += EPI_NT) {
+  for (int x = threadIdx.x; x < LN * N; x += EPI_NT) {
     const int ll = x >> 11, n = x & (N - 1);
     const uint32_t o = phys(n);
     const uint32_t x1 = shoup_mul(sm[ll * PS + o], k1, k1q, P1);
-    const uint32_t x2 = shoup_mul(sm[(4 + ll) * PS + o], k2, k2q, P2);
+    const uint32_t x2 = shoup_mul(sm[(LN + ll) * PS + o], k2, k2q, P2);
     uint64_t v = (uint64_t)x1 * P2 + (uint64_t)x2 * P1;
     v = v >= QQ ? v - QQ : v;
     const uint32_t aq = __ldg(a_ms + ((size_t)ds * SIMD + l0 + ll) * N + n);
@@ -489,9 +496,14 @@ void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uin
     const CrtConst cc = host_crt_const();
     const uint32_t k1q = (uint32_t)(((uint64_t)cc.q2inv1 << 32) / P1);
     const uint32_t k2q = (uint32_t)(((uint64_t)cc.q1inv2 << 32) / P2);
+    if ((size_t)nshards * SIMD * nq <= 256) {
+      primary_epilogue2k_kernel<1><<<dim3(nshards, SIMD, nq), EPI_NT, (size_t)2 * n2k::PS * 4, st>>>(
+          fin, nshards, a_ms, distinct_of, sec_in, nq, chunk, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
+      return;
+    }
     const size_t smem = (size_t)8 * n2k::PS * 4;
-    set_smem(primary_epilogue2k_kernel, smem);
-    primary_epilogue2k_kernel<<<dim3(nshards, SIMD / 4, nq), EPI_NT, smem, st>>>(
+    set_smem(primary_epilogue2k_kernel<4>, smem);
+    primary_epilogue2k_kernel<4><<<dim3(nshards, SIMD / 4, nq), EPI_NT, smem, st>>>(
         fin, nshards, a_ms, distinct_of, sec_in, nq, chunk, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
     return;
   }
