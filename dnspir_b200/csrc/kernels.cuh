@@ -137,8 +137,8 @@ int secondary_chain_wave(const Group& g, int sms);
 
 // ---- primary scan (main_pir_loop, base_pir.rs:1085-1247)
 // B queries (a power of two up to 256) in one launch over all shards, each
-// block serving per_block of them (1, 2, 4, 8 or 16; 0: min(B, 16)), the other
-// groups of per_block on grid.y.  qv: launch_scan_vectors of B queries.  out:
+// block serving per_block of them (1, 2, 4, 8 or 16; 0: min(B, 8)), the groups
+// of one tile in consecutive blocks.  qv: launch_scan_vectors of B queries.  out:
 // [b][s][p][u][lane] reduced mod p.
 int scan_batch_supported(int B);
 int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qv, int B, int per_block, uint32_t* out,

@@ -91,6 +91,7 @@ struct ScanArgs {
   const uint32_t* qv;  // query vectors, 12 N words a query
   uint32_t* out;       // [b][s][p][u][lane], reduced mod p
   int rows;            // rows per window chunk
+  uint32_t groups;     // groups of B queries
 };
 
 __device__ __forceinline__ void ld_lanes(const uint32_t* p, uint32_t* v, int lpt) {
@@ -107,12 +108,18 @@ __device__ __forceinline__ void ld_lanes(const uint32_t* p, uint32_t* v, int lpt
   }
 }
 
-// 16 queries per block: two blocks per SM (128 registers, 16 warps: the
-// kernel is latency-bound at one block of 8 warps); the other shapes would
-// spill under that bound and keep the compiler's own register choice (a
-// minimum of 0 blocks leaves it as with no minimum)
-template <int B, int LPT, int NA>
-__global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(ScanArgs a) {
+// B queries per block, LPT lanes per thread, MINB blocks per SM (0: as many as
+// the registers give), UN rows unrolled.  One and two queries are bound by HBM
+// and take light threads with many rows in flight (64 full shards: one query 4.65
+// ms, 7.4 TB/s; two 4.8, 5.2 as eight lanes a thread); from four on the wide multiply-adds bound it (four cycles a warp on the heavy
+// FMA pipe: 7.5 ms for 8 queries of 64 full shards), and four lanes a thread
+// halve the shared-memory reads per product against two: 8 queries 9.7 ms as
+// two blocks per SM, 16 19.0 as two such groups against 21.2 as 16 with two lanes;
+// four queries 5.7 at three blocks per SM and four lanes, 8.1 at eight lanes
+// (130 registers; 0.38 / 0.56 at 4 half-size shards).  Tried: a third of the queries on the FP64 pipe, exactly, with
+// 13-bit halves (8 queries 16 ms).
+template <int B, int LPT, int NA, int MINB, int UN>
+__global__ void __launch_bounds__(SCAN_NT, MINB) scan_batch_kernel(ScanArgs a) {
   constexpr int LG = SIMD / LPT;     // lane groups per slot
   constexpr int TS = SCAN_NT / LG;   // slots per tile
   extern __shared__ uint32_t win[];  // [NA][B][W]: x fastest, so a warp's slots hit distinct banks
@@ -123,10 +130,11 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
   const uint32_t tiles = (half + TS - 1) / TS;
   const int slot = threadIdx.x / LG, lg = threadIdx.x % LG;
   const size_t arr = (size_t)N * SIMD, row_stride = NA * arr;
-  // item = ((s * 2 + p) * 2 + sgn) * tiles + tile
-  const uint32_t item = blockIdx.x;
-  // grid.y: which group of B queries of the kernel batch this block serves
-  const size_t qbase = (size_t)blockIdx.y * B;
+  // item = ((s * 2 + p) * 2 + sgn) * tiles + tile; the groups of B queries of one
+  // item are consecutive blocks, so that its rows come from HBM once and from
+  // L2 for the others
+  const uint32_t item = blockIdx.x / a.groups;
+  const size_t qbase = (size_t)(blockIdx.x % a.groups) * B;
   const uint32_t tile = item % tiles;
   const uint32_t sgn = (item / tiles) & 1;
   const int p = (item / (2 * tiles)) & 1;
@@ -158,7 +166,7 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
       if (active) {
         const uint32_t* row = slab + slab_off(g, p, h, i0, 0, u) + lg * LPT;
         uint32_t x = slot + (i1 - 1 - i0);
-#pragma unroll(NA == 2 ? 3 : 2)
+#pragma unroll UN
         for (uint32_t i = i0; i < i1; i++) {
           uint32_t ev[NA][LPT];
 #pragma unroll
@@ -179,21 +187,14 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
       }
       __syncthreads();
     }
-    if (NA == 2 && active) {  // the last row's state once more
-      uint32_t xv[LPT];
-      ld_lanes(slab + slab_off(g, p, h, L - 1, 0, u) + lg * LPT, xv, LPT);
+    uint32_t xv[LPT] = {};  // the last row's state once more
+    if (NA == 2 && active) ld_lanes(slab + slab_off(g, p, h, L - 1, 0, u) + lg * LPT, xv, LPT);
 #pragma unroll
-      for (int b = 0; b < B; b++) {
-        const uint32_t c = __ldg(a.qv + (qbase + b) * qs + scan_vec_off(N, h, 2, p) + u);
+    for (int b = 0; b < B; b++) {
+      uint32_t c = 0;
+      if (NA == 2 && active) c = __ldg(a.qv + (qbase + b) * qs + scan_vec_off(N, h, 2, p) + u);
 #pragma unroll
-        for (int l = 0; l < LPT; l++) acc[l][b] += (uint64_t)xv[l] * c;
-      }
-    }
-    if (h + 1 < g.H) {
-#pragma unroll
-      for (int l = 0; l < LPT; l++)
-#pragma unroll
-        for (int b = 0; b < B; b++) acc[l][b] = reduce64(acc[l][b], pr, mu);
+      for (int l = 0; l < LPT; l++) acc[l][b] = reduce64(acc[l][b] + (uint64_t)xv[l] * c, pr, mu);
     }
   }
   if (active) {
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(SCAN_NT, B == 16 ? 2 : 0) scan_batch_kernel(Sc
     for (int b = 0; b < B; b++) {
       uint32_t* o = a.out + ((((qbase + b) * a.nshards + s) * 2 + p) * N + u) * SIMD + lg * LPT;
 #pragma unroll
-      for (int l = 0; l < LPT; l++) o[l] = reduce64(acc[l][b], pr, mu);
+      for (int l = 0; l < LPT; l++) o[l] = (uint32_t)acc[l][b];
     }
   }
 }
@@ -424,21 +425,21 @@ __global__ void __launch_bounds__(ZQ_NT) epilogue_zq_kernel(const uint32_t* __re
   }
 }
 
-template <int B, int LPT, int NA>
-void launch_batch_na(const ScanArgs& a, int groups, cudaStream_t st) {
+template <int B, int LPT, int NA, int MINB, int UN>
+void launch_batch_na(const ScanArgs& a, cudaStream_t st) {
   constexpr int TS = SCAN_NT / (SIMD / LPT);
   const size_t smem = (size_t)NA * (TS + a.rows - 1) * B * 4;
-  set_smem(scan_batch_kernel<B, LPT, NA>, smem);
+  set_smem(scan_batch_kernel<B, LPT, NA, MINB, UN>, smem);
   const uint32_t tiles = (a.g.n / 2 + TS - 1) / TS;
   const uint32_t items = (uint32_t)a.nshards * 4 * tiles;
-  scan_batch_kernel<B, LPT, NA><<<dim3(items, groups), SCAN_NT, smem, st>>>(a);
+  scan_batch_kernel<B, LPT, NA, MINB, UN><<<items * a.groups, SCAN_NT, smem, st>>>(a);
 }
-template <int B, int LPT>
-void launch_batch(const ScanArgs& a, int groups, cudaStream_t st) {
+template <int B, int LPT, int MINB, int UN>
+void launch_batch(const ScanArgs& a, cudaStream_t st) {
   if (a.g.na == 2)
-    launch_batch_na<B, LPT, 2>(a, groups, st);
+    launch_batch_na<B, LPT, 2, MINB, UN>(a, st);
   else
-    launch_batch_na<B, LPT, 3>(a, groups, st);
+    launch_batch_na<B, LPT, 3, MINB, 1>(a, st);
 }
 
 }  // namespace
@@ -456,7 +457,7 @@ int scan_batch_supported(int B) { return B >= 1 && B <= 256 && (B & (B - 1)) == 
 int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* qv, int B, int per_block, uint32_t* out,
                       const Group& g, cudaStream_t st) {
   if (!scan_batch_supported(B)) return -1;
-  if (per_block <= 0) per_block = B < 16 ? B : 16;
+  if (per_block <= 0) per_block = B < 8 ? B : 8;
   if (per_block > B || B % per_block) return -1;
   const int groups = B / per_block;
   ScanArgs a;
@@ -466,12 +467,26 @@ int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* q
   a.qv = qv;
   a.out = out;
   a.rows = (int)(g.L < 256 ? g.L : 256);
+  a.groups = (uint32_t)groups;
   switch (per_block) {
-    case 1: launch_batch<1, 8>(a, groups, st); break;
-    case 2: launch_batch<2, 8>(a, groups, st); break;
-    case 4: launch_batch<4, 8>(a, groups, st); break;
-    case 8: launch_batch<8, 4>(a, groups, st); break;
-    case 16: launch_batch<16, 2>(a, groups, st); break;
+    case 1: {
+      // rows in flight per thread against threads: few blocks need the depth,
+      // many give it themselves (4 / 11 / 25 half-size and 64 full shards: 4 rows
+      // 0.51 / 0.52 / 0.55 / 4.65 ms, 8 rows 0.37 / 0.39 / 0.48 / 4.85, 12 rows at
+      // three blocks per SM 0.25 / 0.30 / 0.76 / 4.69)
+      int sms = 0, dev = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const size_t blocks = (size_t)nshards * 4 * ((g.n / 2 + 127) / 128) * groups;
+      if (blocks <= (size_t)3 * sms) launch_batch<1, 4, 3, 12>(a, st);
+      else if (blocks <= (size_t)7 * sms) launch_batch<1, 4, 0, 8>(a, st);
+      else launch_batch<1, 4, 0, 4>(a, st);
+      break;
+    }
+    case 2: launch_batch<2, 4, 3, 6>(a, st); break;
+    case 4: launch_batch<4, 4, 3, 6>(a, st); break;
+    case 8: launch_batch<8, 4, 2, 4>(a, st); break;
+    case 16: launch_batch<16, 2, 2, 6>(a, st); break;
     default: return -1;
   }
   return 0;
