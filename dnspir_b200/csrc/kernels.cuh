@@ -180,8 +180,8 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
                  uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
                  const TScanShape& shape, cudaStream_t st, const TScanLimits& lim = TScanLimits(),
                  const void* slab_maps = nullptr);
-// A shard's chain state after its last row, [p][u][half][lane] (na = 2), from
-// its a_out (launch_primary_chain).
+// A shard's chain state after its last row times 2^32, [p][u][half][lane] (na =
+// 2), from its a_out (launch_primary_chain).
 size_t last_rows_words(const Group& g);
 void launch_last_rows(const uint32_t* a_out, uint32_t* last, const Group& g, const ScanConsts& sc, const SlotMaps& maps,
                       cudaStream_t st);

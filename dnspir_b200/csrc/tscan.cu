@@ -204,31 +204,52 @@ struct TScanArgs {
   uint32_t H;
 };
 
-// c_w = 2^(8w) mod p (< 2^26) for w = k .. k + 3: the weights of limb product
-// D_kj (j = 0..3) in the recombination
-__device__ __forceinline__ void limb_weights(uint32_t pr, uint64_t mu, int k, uint32_t (&c)[4]) {
-  const uint32_t w3 = (uint32_t)reduce64(1ull << 24, pr, mu);
-  const uint64_t c32 = reduce64(1ull << 32, pr, mu);
-  const uint64_t c40 = reduce64(c32 << 8, pr, mu);
-  const uint64_t c48 = reduce64(c40 << 8, pr, mu);
-  c[0] = k == 0 ? 1u : k == 1 ? 256u : k == 2 ? 65536u : w3;
-  c[1] = k == 0 ? 256u : k == 1 ? 65536u : k == 2 ? w3 : (uint32_t)c32;
-  c[2] = k == 0 ? 65536u : k == 1 ? w3 : k == 2 ? (uint32_t)c32 : (uint32_t)c40;
-  c[3] = k == 0 ? w3 : k == 1 ? (uint32_t)c32 : k == 2 ? (uint32_t)c40 : (uint32_t)c48;
+// c_w = 2^(8w + 32) mod p (< 2^26) for w = k .. k + 3: the weights of limb
+// product D_kj (j = 0..3) in the recombination, with the 2^32 that its Montgomery
+// reduction takes away
+__device__ __forceinline__ void limb_weights(int p, int k, uint32_t (&c)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int w = 0; w < 7; w++) {
+      // (2^(4 w + 16))^2 = 2^(8 w + 32)
+      constexpr auto weight = [](int e, uint64_t m) {
+        const uint64_t h = (1ull << (4 * e + 16)) % m;
+        return (uint32_t)(h * h % m);
+      };
+      if (w - j >= 0 && w - j < 4 && k == w - j) v = p ? weight(w, P2) : weight(w, P1);
+    }
+    c[j] = v;
+  }
+}
+
+// T 2^-32 mod p in [0, p), T < 2^62: Montgomery, then canon
+template <uint32_t P>
+__device__ __forceinline__ uint32_t mont_canon(uint64_t T) {
+  constexpr uint32_t inv = [] {  // -P^-1 mod 2^32, by Newton's iteration
+    uint32_t x = P;
+    for (int i = 0; i < 5; i++) x *= 2u - P * x;
+    return 0u - x;
+  }();
+  return ntt_detail::canon((uint32_t)((T + (uint64_t)((uint32_t)T * inv) * P) >> 32), P);
 }
 
 // Epilogue of one m-tile: the warp's 32 TMEM lanes (rows (slot, lane, limb k)
 // of output slot u) x NQ columns (query-operand rows 4 b + j of query group
 // grp) starting at TMEM address taddr.  Each query's 16 limb products are
-// recombined with the weights c and reduced mod pr; lanes 4 l8 .. 4 l8 + 3
-// hold the four limbs k of SIMD lane l8, so three of every four lanes sum the
-// others' partial recombinations with shuffles and lane k keeps query
-// 4 q4 + k's sum.  The warp reads columns c_lo .. c_hi - 1 (multiples of the
-// load width), 64 (16 for NQ = 16) per TMEM load.
+// recombined with the weights c and reduced mod p; lanes 4 l8 .. 4 l8 + 3 hold
+// the four limbs k of SIMD lane l8, and four queries' partial recombinations
+// are summed over them by halving: a lane hands two of its four to its
+// neighbour, then one of the two left, and lane k ends with query 4 q4 + k's sum
+// (6 shuffles of 32 bits instead of the 16 of summing all four everywhere).  The
+// sum, below 2^61 plus two products below 2^52, takes one Montgomery step and
+// canon (about 7 instructions; a 64-bit Barrett reduction about 25).  The warp
+// reads columns c_lo .. c_hi - 1 (multiples of the load width), 64 (16 for NQ =
+// 16) per TMEM load.
 template <int NQ>
-__device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr, const uint32_t (&c)[4], uint32_t pr,
-                                              uint64_t mu, uint32_t grp, uint32_t u, int s, int p, int k, int l8,
-                                              int c_lo = 0, int c_hi = NQ) {
+__device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr, const uint32_t (&c)[4], uint32_t grp,
+                                              uint32_t u, int s, int p, int k, int l8, int c_lo = 0, int c_hi = NQ) {
   constexpr int CW = NQ >= 64 ? 64 : 16;  // columns per TMEM load
   const uint32_t N = 2 * a.half;
   // the states after the last row at this slot and lane, and the vectors they
@@ -263,15 +284,17 @@ __device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr
 #pragma unroll
       for (int qq = 0; qq < 4; qq++) {
         const uint32_t* w = v + 16 * q4 + 4 * qq;
-        uint64_t x = (uint64_t)w[0] * c[0] + (uint64_t)w[1] * c[1] + (uint64_t)w[2] * c[2] + (uint64_t)w[3] * c[3];
-        x += __shfl_xor_sync(0xffffffffu, x, 1);
-        x += __shfl_xor_sync(0xffffffffu, x, 2);
-        tot[qq] = x;
+        tot[qq] = (uint64_t)w[0] * c[0] + (uint64_t)w[1] * c[1] + (uint64_t)w[2] * c[2] + (uint64_t)w[3] * c[3];
       }
-      const uint64_t mine = (k == 0 ? tot[0] : k == 1 ? tot[1] : k == 2 ? tot[2] : tot[3]) +
+      // k's high bit keeps queries 2, 3 or 0, 1; its low bit one of the two
+      const bool hi = k & 2, odd = k & 1;
+      uint64_t even2 = (hi ? tot[2] : tot[0]) + __shfl_xor_sync(0xffffffffu, hi ? tot[0] : tot[2], 2);
+      uint64_t odd2 = (hi ? tot[3] : tot[1]) + __shfl_xor_sync(0xffffffffu, hi ? tot[1] : tot[3], 2);
+      const uint64_t mine = (odd ? odd2 : even2) + __shfl_xor_sync(0xffffffffu, odd ? even2 : odd2, 1) +
                             (uint64_t)x0 * v0[q4] + (uint64_t)x1 * v1[q4];
       const uint32_t bq = grp * (NQ / 4) + (c0 / 16 + q4) * 4 + k;
-      if (bq < a.nvalid) a.out[((((size_t)bq * a.nshards + s) * 2 + p) * N + u) * SIMD + l8] = reduce64(mine, pr, mu);
+      const uint32_t y = p ? mont_canon<P2>(mine) : mont_canon<P1>(mine);
+      if (bq < a.nvalid) a.out[((((size_t)bq * a.nshards + s) * 2 + p) * N + u) * SIMD + l8] = y;
     }
   }
 }
@@ -383,13 +406,11 @@ __global__ void __launch_bounds__(TSCAN_NT, 1) tscan_kernel(TScanArgs a) {
   const bool acc_ok = mbar_wait(accb, 0, a.wait_ns);
   tc_fence_after();
   if (acc_ok) {
-    const uint32_t pr = prime_of(p);
-    const uint64_t mu = barrett_mu(pr);
     const int k = lane & 3, l8 = lane >> 2;
     uint32_t c[4];
-    limb_weights(pr, mu, k, c);
+    limb_weights(p, k, c);
     for (int t = 0; t < MTPC; t++)
-      epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * warp) << 16) + t * NQ, c, pr, mu, grp,
+      epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * warp) << 16) + t * NQ, c, grp,
                         sgn * a.half + 4 * (mt0 + t) + warp, s, p, k, l8);
   } else if (threadIdx.x == 0) {
     atomicOr(a.err, 1u);
@@ -586,12 +607,10 @@ __global__ void __launch_bounds__(tscanp_nt<NQ>(), 1) tscanp_kernel(TScanArgs a)
       uint32_t grp, mt0, sgn;
       int p, s;
       tile_of(item, grp, mt0, sgn, p, s);
-      const uint32_t pr = prime_of(p);
-      const uint64_t mu = barrett_mu(pr);
       uint32_t c[4];
-      limb_weights(pr, mu, k, c);
+      limb_weights(p, k, c);
       for (int t = 0; t < MTPC; t++)
-        epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * q) << 16) + buf * ACC + t * NQ, c, pr, mu, grp,
+        epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * q) << 16) + buf * ACC + t * NQ, c, grp,
                           sgn * a.half + 4 * (mt0 + t) + q, s, p, k, l8, c_lo, c_lo + NQ / EW);
       tc_fence_before();
       __syncwarp();
@@ -889,12 +908,10 @@ __global__ void __launch_bounds__(tscanp_nt<NQ>(), 1) tscan2_kernel(const __grid
       uint32_t grp, mt0, sgn;
       int p, s;
       tile_of(item, grp, mt0, sgn, p, s);
-      const uint32_t pr = prime_of(p);
-      const uint64_t mu = barrett_mu(pr);
       uint32_t c[4];
-      limb_weights(pr, mu, k, c);
+      limb_weights(p, k, c);
       for (int t = 0; t < MTPC; t++)
-        epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * q) << 16) + buf * ACC + t * NQ, c, pr, mu, grp,
+        epilogue_tile<NQ>(a, tmem + ((uint32_t)(32 * q) << 16) + buf * ACC + t * NQ, c, grp,
                           sgn * a.half + 4 * (mt0 + rank * MTPC + t) + q, s, p, k, l8, c_lo, c_lo + NQ / EW);
       tc_fence_before();
       __syncwarp();
@@ -971,8 +988,9 @@ __global__ void retile_kernel(const uint32_t* __restrict__ src, uint8_t* __restr
 // and array).  Output (e, d) is word d of row r = (d - e) mod L, so the block
 // reads 64-byte pieces of 143 rows, turns them in shared memory and writes whole
 // 128-byte limb rows.  Bound by HBM: 2 x slab bytes (and the pieces' overlap)
-// once a preprocessing; from the lane layout, whose reads are 4-byte words, a
-// full shard took 1.1 ms.
+// once a preprocessing: 0.15 ms for a half-size shard (268 MB each way), 0.34
+// with loads through registers, 0.57 from the lane layout's 4-byte words (three
+// arrays).
 constexpr int RT_E = 16, RT_PAD = 132;
 __global__ void __launch_bounds__(256) retile_rows_kernel(const uint32_t* __restrict__ rows,
                                                           const uint32_t* __restrict__ digits,
@@ -987,15 +1005,18 @@ __global__ void __launch_bounds__(256) retile_rows_kernel(const uint32_t* __rest
   const uint32_t h = ha / 2;
   const uint32_t* src = (ha & 1 ? digits : rows) + ((size_t)p * g.H + h) * L * SIMD * g.n + sgn * half;
   // k fastest (the 16 words of a piece), then lane, then row
-#pragma unroll 8
   for (uint32_t x = threadIdx.x; x < (128 + RT_E - 1) * SIMD * RT_E; x += 256) {
     const uint32_t k = x % RT_E, lane = x / RT_E % SIMD, rr = x / (RT_E * SIMD);
     const int dd = (int)(rr + k) - (RT_E - 1);  // d - d0; row r = (d0 + rr - 15 - e0) mod L
     if (dd >= 0 && dd < 128) {
       const uint32_t r = (d0 + rr + 2 * L - (RT_E - 1) - e0) & (L - 1);
-      sm[(k * SIMD + lane) * RT_PAD + dd] = __ldg(src + ((size_t)r * SIMD + lane) * g.n + d0 + dd);
+      // straight to shared memory: all of a thread's 72 words are in flight at once
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa(sm + (k * SIMD + lane) * RT_PAD + dd)),
+                   "l"(src + ((size_t)r * SIMD + lane) * g.n + d0 + dd)
+                   : "memory");
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // one thread per (e, lane, 16-byte unit): 16 words -> their four limb rows
   for (uint32_t x = threadIdx.x; x < RT_E * SIMD * 8; x += 256) {
@@ -1023,15 +1044,18 @@ __global__ void __launch_bounds__(256) retile_rows_kernel(const uint32_t* __rest
   }
 }
 
-// The chain state after the last row, scaled as the stored states are, from
-// a_out [half][lane][p][pos] to [p][u][half][lane].  One thread per word.
+// The chain state after the last row, scaled as the stored states are and times
+// 2^32 (the epilogue's Montgomery form), from a_out [half][lane][p][pos] to
+// [p][u][half][lane].  One thread per word.
 __global__ void last_rows_kernel(const uint32_t* __restrict__ a_out, uint32_t* __restrict__ last, Group g,
                                  ScanConsts sc, const uint32_t* __restrict__ gtab) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * g.n * g.H * SIMD) return;
   const uint32_t lane = i % SIMD, h = (i / SIMD) % g.H, u = (i / (SIMD * g.H)) % g.n, p = i / (SIMD * g.H * g.n);
   const uint32_t pos = brv((__ldg(gtab + u) - 1) >> 1, g.log2n), pr = prime_of((int)p);
-  last[i] = mul_mod(__ldg(a_out + (((size_t)h * SIMD + lane) * 2 + p) * g.n + pos), sc.xscale[p], pr, barrett_mu(pr));
+  const uint64_t mu = barrett_mu(pr);
+  const uint32_t x = mul_mod(__ldg(a_out + (((size_t)h * SIMD + lane) * 2 + p) * g.n + pos), sc.xscale[p], pr, mu);
+  last[i] = reduce64((uint64_t)x << 32, pr, mu);
 }
 
 // Query operand: one thread per (p, sign, query, 16-byte K unit); writes the
