@@ -322,62 +322,132 @@ __global__ void __launch_bounds__(RowsSub<LOGL>::NT) encode_rows_sub_kernel(cons
   }
 }
 
-// Ends the inverse transform of the lift: coefficient v (mod q1, unscaled)
-// -> c = centred(v N^-1), y = centred((c l^-1) mod t), written as y mod q1 in
-// place and y mod q2 into polynomial cnt + poly.  (c l^-1) mod t is taken as
-// (u s) mod t with u = c + LIFT_M > 0 and a Shoup quotient for s = l^-1 mod t.
-struct LiftFin {
-  int cnt;
-  uint32_t s, sq;  // l^-1 mod t and floor(s 2^32 / t)
-  __device__ __forceinline__ void operator()(uint32_t* y, int, int, uint32_t (&v)[8], uint32_t p, uint32_t ni,
-                                             uint32_t niq) const {
-    using namespace n2k;
+// The lift at N = 2048, chain layout: one block of 512 threads takes column r of
+// half h for up to `lpb` lanes, each 256-thread half every other lane with
+// barriers of its own (three blocks per SM).  Thread t owns positions 8t .. 8t +
+// 7 where data comes from and goes to global memory, which the first inverse
+// and last forward stages work in registers, and words t + 256 k in the middle:
+// there the last inverse pass, the lift and the first forward pass of both
+// factors meet in registers, and the Galois permutation E_c[j] =
+// E^_r[idx(5^-r (2j+1))] is taken on the lifted coefficients, as a(X^(5^-r)): one
+// exchange of one polynomial at odd strides, free of bank conflicts, instead of
+// a gather of both transforms.  A coefficient v (mod q1, unscaled) becomes y =
+// centred((c l^-1) mod t) with c = centred(v N^-1); (c l^-1) mod t is taken as (u s)
+// mod t with u = c + LIFT_M > 0 and a Shoup quotient for s = l^-1 mod t.  192 lanes of order
+// 2048: 6.1 -> 5.5 ms (heavy FMA pipe 74 % busy) against whole transforms in shared memory.  Factor 0 of the
+// output may lie on Ahat, as in encode_lift_kernel.
+template <int M, bool INV>
+__device__ __forceinline__ void lift_pass(uint32_t* x, int t, const n2k::Tw8& tw, uint32_t p) {
+  using Gm = n2k::Geo8<M>;
+  uint32_t* y = x + Gm::base(t);
+  uint32_t v[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const uint32_t c = red(lazy_mul(v[k], ni, niq, p), p);
-      const uint32_t u = c + (c > P1 / 2 ? LIFT_M - P1 : LIFT_M);
-      uint32_t m = u * s - __umulhi(u, sq) * TPLAIN;  // in [0, 2t)
-      m = m >= TPLAIN ? m - TPLAIN : m;
-      const bool neg = m > TPLAIN / 2;
-      y[k * Geo8<1>::STR] = neg ? m + (P1 - TPLAIN) : m;
-      y[cnt * PS + k * Geo8<1>::STR] = neg ? m + (P2 - TPLAIN) : m;
-    }
-  }
-};
+  for (int k = 0; k < 8; k++) v[k] = y[k * Gm::STR];
+  if (INV)
+    n2k::inv8_bf(v, tw, p);
+  else
+    n2k::fwd8_bf(v, tw, p);
+#pragma unroll
+  for (int k = 0; k < 8; k++) y[k * Gm::STR] = v[k];
+}
 
-// One block: column r of half h for up to `lpb` lanes, chain layout
-// (factor 0 of the output may lie on Ahat, as in encode_lift_kernel).
-__global__ void __launch_bounds__(NT2K) encode_lift2k_kernel(const uint32_t* Ahat, uint32_t* out, Group g, int nl,
-                                                             int lpb, uint32_t scale, uint32_t scale_q,
-                                                             const uint32_t* __restrict__ pow5inv, NttTables T) {
-  extern __shared__ __align__(16) uint32_t sm[];
+__global__ void __launch_bounds__(NT2K, 3) encode_lift2k_kernel(const uint32_t* Ahat, uint32_t* out, Group g, int nl,
+                                                                int lpb, uint32_t scale, uint32_t scale_q,
+                                                                const uint32_t* __restrict__ pow5inv, NttTables T) {
+  extern __shared__ __align__(16) uint32_t sm[];  // per lane: two padded polynomials
   using namespace n2k;
   const uint32_t r = blockIdx.x, h = blockIdx.y;
-  const int lane0 = blockIdx.z * lpb;
-  const int nlg = min(lpb, nl - lane0);
-  for (int b = threadIdx.x; b < nlg * (N / 4); b += NT2K) {
-    const int kk = b >> 9, q = b & (N / 4 - 1);
-    const uint4 v = reinterpret_cast<const uint4*>(Ahat + (((size_t)h * g.L + r) * nl + lane0 + kk) * N)[q];
-    *reinterpret_cast<uint4*>(sm + kk * PS + phys(4 * q)) = v;
-  }
-  __syncthreads();
-  inv<NT2K>(sm, nlg, 0, T, LiftFin{nlg, scale, scale_q});
-  fwd<NT2K>(sm, nlg, nlg, T);
-  // E_c[j] = E^_r[idx(5^-r (2j+1))] at bit-reversed position brv(j), c = L - 1 - r
-  const uint32_t pw = __ldg(pow5inv + r);
-  constexpr uint32_t mask = 2 * N - 1;
-  for (int q = threadIdx.x; q < N / 4; q += NT2K) {
-    uint32_t idx[4];
+  const int lane0 = blockIdx.z * lpb, nlg = min(lpb, nl - lane0);
+  const int t = threadIdx.x & 255, grp = threadIdx.x >> 8, qb = (int)phys(8 * t);
+  constexpr int STR = Geo8<1>::STR;
+  auto sync = [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + grp) : "memory"); };
+  const size_t row = (((size_t)h * g.L + r) * nl + lane0) * N + 8 * t, efac = (size_t)g.H * g.L * nl * N;
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-      const uint32_t j = brv11(4 * q + m);
-      idx[m] = phys(brv11(((pw * (2 * j + 1)) & mask) >> 1));
+  for (int h4 = 0; h4 < 2; h4++) {
+    const Tw4 w = load_tw4(T.iw2[0], 2 * t + h4);
+    for (int l = grp; l < nlg; l += 2) {
+      uint4 v = *reinterpret_cast<const uint4*>(Ahat + row + (size_t)l * N + 4 * h4);
+      gs(v.x, v.y, w.b0, w.b0q, P1);
+      gs(v.z, v.w, w.b1, w.b1q, P1);
+      gs(v.x, v.z, w.a, w.aq, P1);
+      gs(v.y, v.w, w.a, w.aq, P1);
+      *reinterpret_cast<uint4*>(sm + 2 * l * PS + qb + 4 * h4) = v;
     }
-    for (int pk = 0; pk < 2 * nlg; pk++) {
-      const int pp = pk >= nlg, kk = pk - pp * nlg;
-      const uint32_t* s = sm + pk * PS;
-      reinterpret_cast<uint4*>(out + ((((size_t)pp * g.H + h) * g.L + r) * nl + lane0 + kk) * N)[q] =
-          make_uint4(s[idx[0]], s[idx[1]], s[idx[2]], s[idx[3]]);
+  }
+  sync();
+  {
+    const Tw8 tw = load_tw8(T.iw2[0], 64, Geo8<64>::blk(t));
+    for (int l = grp; l < nlg; l += 2) lift_pass<64, true>(sm + 2 * l * PS, t, tw, P1);
+  }
+  sync();
+  {
+    const Tw8 tw = load_tw8(T.iw2[0], 8, Geo8<8>::blk(t));
+    for (int l = grp; l < nlg; l += 2) lift_pass<8, true>(sm + 2 * l * PS, t, tw, P1);
+  }
+  sync();
+  const uint32_t pw = __ldg(pow5inv + r);
+  for (int l = grp; l < nlg; l += 2) {
+    const uint32_t* y = sm + 2 * l * PS + phys(t);
+    int32_t* const x = reinterpret_cast<int32_t*>(sm + (2 * l + 1) * PS);
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = y[k * STR];
+    inv8_bf(v, param_tw8(T.iw7[0]), P1);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const uint32_t c = red(lazy_mul(v[k], T.ninv[0][11], T.ninvq[0][11], P1), P1);
+      const uint32_t u = c + (c > P1 / 2 ? LIFT_M - P1 : LIFT_M);
+      const uint32_t m = red(u * scale - __umulhi(u, scale_q) * TPLAIN, TPLAIN);
+      const int32_t s = m > TPLAIN / 2 ? (int32_t)m - (int32_t)TPLAIN : (int32_t)m;
+      const uint32_t n = pw * (uint32_t)(t + 256 * k);  // X^n -> X^(n pw), X^N = -1
+      x[n & (N - 1)] = n & N ? -s : s;
+    }
+  }
+  sync();
+  // both factors' first forward pass; factor 0 may be stored at once, factor 1
+  // where the coefficients lie after everyone has read them
+  for (int l = grp; l < nlg; l += 2) {
+    const int32_t* x = reinterpret_cast<const int32_t*>(sm + (2 * l + 1) * PS);
+    uint32_t v[8], w[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = (uint32_t)(x[t + 256 * k] + (int32_t)P1), w[k] = v[k] - P1 + P2;
+    fwd8_bf(v, param_tw8(T.fw7[0]), P1);
+    uint32_t* y = sm + 2 * l * PS + phys(t);
+#pragma unroll
+    for (int k = 0; k < 8; k++) y[k * STR] = v[k];
+    sync();
+    fwd8_bf(w, param_tw8(T.fw7[1]), P2);
+#pragma unroll
+    for (int k = 0; k < 8; k++) y[PS + k * STR] = w[k];
+  }
+  sync();
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const Tw8 tw = load_tw8(T.fw2[f], 8, Geo8<8>::blk(t));
+    for (int l = grp; l < nlg; l += 2) lift_pass<8, false>(sm + (2 * l + f) * PS, t, tw, prime_of(f));
+  }
+  sync();
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const Tw8 tw = load_tw8(T.fw2[f], 64, Geo8<64>::blk(t));
+    for (int l = grp; l < nlg; l += 2) lift_pass<64, false>(sm + (2 * l + f) * PS, t, tw, prime_of(f));
+  }
+  sync();
+#pragma unroll
+  for (int f = 0; f < 2; f++) {
+    const uint32_t p = prime_of(f);
+#pragma unroll
+    for (int h4 = 0; h4 < 2; h4++) {
+      const Tw4 w = load_tw4(T.fw2[f], 2 * t + h4);
+      for (int l = grp; l < nlg; l += 2) {
+        uint4 v = *reinterpret_cast<const uint4*>(sm + (2 * l + f) * PS + qb + 4 * h4);
+        ct(v.x, v.z, w.a, w.aq, p);
+        ct(v.y, v.w, w.a, w.aq, p);
+        ct(v.x, v.y, w.b0, w.b0q, p);
+        ct(v.z, v.w, w.b1, w.b1q, p);
+        *reinterpret_cast<uint4*>(out + f * efac + row + (size_t)l * N + 4 * h4) =
+            make_uint4(canon(v.x, p), canon(v.y, p), canon(v.z, p), canon(v.w, p));
+      }
     }
   }
 }
