@@ -1048,7 +1048,7 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
 // canonical high digits' transforms go to `digits`, the same layout.  Three
 // blocks fit an SM (67 KiB, 80 registers), so up to one wave of 444 chains runs
 // at once.  Against two-block clusters with one factor per block (radix-4
-// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (3.4 when
+// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (2.7 when
 // there are fewer, on two SMs each, below).
 constexpr int PRIM2K_KC = 3;
 constexpr int PRIM2K_WORDS = 2 * n2k::PS + PRIM2K_KC * 2 * 2 * 256 * 4;
@@ -1143,9 +1143,8 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // step is half as long for a thread.  PAIR: the factors' threads are the two
 // blocks of a cluster, on two SMs while there are two for every chain -- a
 // chain alone on one SM keeps its heavy FMA pipe 60 % busy, so the second SM
-// is what shortens the step (3.4 us against 4.2).  Otherwise they are the two
-// halves of one 512-thread block (up to one chain per SM: 4.2 us a step, 4.7 as
-// two cluster blocks per SM).  The factors send each other their inverse outputs:
+// is what shortens the step (2.7 us against 3.7).  Otherwise they are the two
+// halves of one 512-thread block (up to one chain per SM).  The factors send each other their inverse outputs:
 // every thread writes its eight values into the other's inbox (double-buffered
 // by step parity, so that one may run ahead of the other's reads) before the
 // one barrier of a step that both meet.  F: the factor, so that primes and
@@ -1216,12 +1215,17 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   const Tw4 iw0 = load_tw4(a.T.iw2[F], 2 * t), iw1 = load_tw4(a.T.iw2[F], 2 * t + 1);
   const Tw4 fw0 = load_tw4(a.T.fw2[F], 2 * t), fw1 = load_tw4(a.T.fw2[F], 2 * t + 1);
   constexpr uint32_t pinv = neg_inv32(p);
-  auto radix8 = [&](auto m, bool inverse) {
+  // a thread's groups are the same in every step: its twiddles stay in registers
+  // (loading them in every pass put their latency behind each barrier: 3.5 ms per
+  // 1024 steps instead of 2.7 as pairs, 4.4 instead of 3.8 as wide blocks, although
+  // those have 128 registers a thread and spill some)
+  const Tw8 i64 = load_tw8(a.T.iw2[F], 64, Geo8<64>::blk(t)), i8 = load_tw8(a.T.iw2[F], 8, Geo8<8>::blk(t));
+  const Tw8 f64 = load_tw8(a.T.fw2[F], 64, Geo8<64>::blk(t)), f8 = load_tw8(a.T.fw2[F], 8, Geo8<8>::blk(t));
+  auto radix8 = [&](auto m, bool inverse, const Tw8& tw) {
     constexpr int M = decltype(m)::value;
     using Gm = Geo8<M>;
     uint32_t* y = A + Gm::base(t);
     uint32_t v[8];
-    const Tw8 tw = load_tw8(inverse ? a.T.iw2[F] : a.T.fw2[F], M, Gm::blk(t));
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] = y[k * Gm::STR];
     if (inverse)
@@ -1257,9 +1261,9 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
       *reinterpret_cast<uint4*>(A + qb + 4 * h4) = v;
     }
     sync();
-    radix8(std::integral_constant<int, 64>(), true);
+    radix8(std::integral_constant<int, 64>(), true, i64);
     sync();
-    radix8(std::integral_constant<int, 8>(), true);
+    radix8(std::integral_constant<int, 8>(), true, i8);
     sync();
     {
       uint32_t* const y = A + phys(t);
@@ -1290,9 +1294,9 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
       for (int k = 0; k < 8; k++) y[k * STR] = v[k];
     }
     sync();
-    radix8(std::integral_constant<int, 8>(), false);
+    radix8(std::integral_constant<int, 8>(), false, f8);
     sync();
-    radix8(std::integral_constant<int, 64>(), false);
+    radix8(std::integral_constant<int, 64>(), false, f64);
     sync();
 #pragma unroll
     for (int h4 = 0; h4 < 2; h4++) {
@@ -1357,7 +1361,7 @@ __device__ __forceinline__ void few_secondary(const ChainArgs& a, const ScanCons
   else
     few_chain<1, true, PAIR>(a, sc, sm, h, q, unit, nullptr, nullptr);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2) secondary_chain_pair_kernel(ChainArgs a,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1) secondary_chain_pair_kernel(ChainArgs a,
                                                                                                ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
   few_secondary<true>(a, sc, sm);
@@ -1380,7 +1384,7 @@ __device__ __forceinline__ void few_primary(ChainArgs& a, uint32_t* rows, uint32
   else
     few_chain<1, false, PAIR>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 2)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     primary_chain_pair_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits, size_t shard_words) {
   extern __shared__ __align__(16) uint32_t sm[];
   few_primary<true>(a, rows, digits, shard_words, sm);
@@ -1617,9 +1621,8 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
   a.nl = nq * CTXT_PARTS;
   a.out = out;
   // N = 2048 (1024 steps of order 2048): a part's chain on two SMs while there
-  // are two for each (3.5 ms), on one while there is one (4.4), beyond that the
-  // three parts of a query and half per block (10.2: 2.4 times the time of one
-  // part alone, three times the work, the constants kept once).  Other lengths,
+  // are two for each (2.7 ms), on one while there is one (3.8), beyond that the
+  // three parts of a query and half per block (10.2, the constants kept once).  Other lengths,
   // or a-parts with a zero query slot: one part and factor per block in
   // two-block clusters while the chunk needs at most one block per SM, then one
   // block per part carrying both factors.  `clustered` asks for the cluster
