@@ -392,8 +392,8 @@ uint32_t preprocess_batch(const Group& g) {
 }
 
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
-                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, cudaStream_t st,
-                      uint32_t* last) {
+                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, uint32_t* err,
+                      cudaStream_t st, uint32_t* last) {
   const size_t per_shard = (size_t)SIMD * g.l * g.n;
   const SlotMaps maps = slot_maps(c, g.log2n);
   const ChainConsts cc = chain_consts(c, g.log2n, used_seeds);
@@ -411,7 +411,7 @@ int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* co
       launch_encode_lift(rows, rows, g, SIMD, 1, maps, c->T, st);
     }
     uint32_t* const rows = ws.rows.as<uint32_t>();
-    launch_primary_chain_rows(rows, rows + words, stride, count, a_out, g, cc, c->T, st);
+    launch_primary_chain_rows(rows, rows + words, stride, count, a_out, err, g, cc, c->T, st);
     launch_primary_finalize(a_out, count, a_zq, a_ms, g, c->T, st);
     if (last) {
       launch_order_rows(rows, count * stride, maps, st);
@@ -464,6 +464,7 @@ struct dnspir_db {
   cudaEvent_t noalloc_done = nullptr;  // recorded on the caller's stream after each no-allocation call
   uint32_t* slab = nullptr;
   DBuf a_zq, a_ms, qz, qlane, qv, sum, out;
+  DBuf err;  // wait-error word of the preprocessing chains
   HBuf pin;  // host staging of perform_pir_split: query elements in, reply out
   EncodeWs ws;
   std::mutex mu;
@@ -613,6 +614,8 @@ int dnspir_db_create(int device, uint32_t log2_n, uint32_t group_order, int used
   // slab takes the memory (module loading is lazy)
   CKR(noalloc_reserve(device));
   CK(cudaMalloc(&d->slab, slab_words(d->g) * 4));
+  CKR(d->err.ensure(4));
+  CK(cudaMemset(d->err.p, 0, 4));
   CKR(d->a_zq.ensure((size_t)SIMD * d->g.n * 8));
   CKR(d->a_ms.ensure((size_t)SIMD * d->g.n * 4));
   *out = d.release();
@@ -648,8 +651,14 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   }
   uint32_t* slabs[1] = {db->slab};
   CKR(preprocess_shards(db->ctx, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
-                        db->a_ms.as<uint32_t>(), db->ws, db->st));
+                        db->a_ms.as<uint32_t>(), db->ws, db->err.as<uint32_t>(), db->st));
+  CKR(db->pin.ensure(4));
+  CK(cudaMemcpyAsync(db->pin.p, db->err.p, 4, cudaMemcpyDeviceToHost, db->st));
   CK(cudaStreamSynchronize(db->st));
+  if (*db->pin.as<uint32_t>()) {
+    CK(cudaMemset(db->err.p, 0, 4));
+    return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
+  }
   db->ap_ver = ver;
   db->ready = true;
   return DNSPIR_OK;

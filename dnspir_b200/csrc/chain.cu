@@ -243,6 +243,7 @@ struct ChainArgs {
   // primary: slabs and a-part output
   uint32_t* const* slabs;
   uint32_t* a_out;
+  uint32_t* err;  // set to 1 when a wait for the peer block gives up
   uint32_t c_first, cinv_first, inv5;
 };
 
@@ -1149,8 +1150,36 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // by step parity, so that one may run ahead of the other's reads) before the
 // one barrier of a step that both meet.  F: the factor, so that primes and
 // shared twiddles are constants of its code.
-constexpr int few_words(int kc) {  // of one factor: A, B (secondary), inbox[2], constants
-  return (kc > 3 ? 2 : 1) * n2k::PS + 2 * N_MAX + kc * 2 * 256 * 4;
+// As pairs the inbox fills by st.async, which counts its bytes on the
+// receiver's mbarrier: no barrier of the cluster and no fence in a step.  A wait
+// is bounded; when it gives up the block raises the error word, stops waiting and
+// runs to its end on what it has.
+constexpr uint64_t PEER_WAIT_NS = 2000000000ull;
+constexpr int few_words(int kc) {  // of one factor: A, B (secondary), inbox[2], constants, two mbarriers
+  return (kc > 3 ? 2 : 1) * n2k::PS + 2 * N_MAX + kc * 2 * 256 * 4 + 4;
+}
+
+// Waits for the phase of `parity` of a barrier that the peer block's copies
+// complete; false after PEER_WAIT_NS.
+__device__ __forceinline__ bool wait_peer(uint32_t bar, uint32_t parity) {
+  auto done = [&] {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
+        "p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  if (done()) return true;
+  uint64_t t0, t1;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (;;) {
+    if (done()) return true;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    if (t1 - t0 > PEER_WAIT_NS) return false;
+  }
 }
 
 template <int F, bool SEC, bool PAIR>
@@ -1209,7 +1238,17 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   // shared::cluster address of the other factor's inbox
   uint32_t peer = (uint32_t)__cvta_generic_to_shared(PAIR ? X : sm + (1 - F) * WORDS + XO);
   if constexpr (PAIR) asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(peer) : "r"(1 - F));
-  sync_both();  // both run and both inboxes are free
+  // PAIR: one mbarrier per parity, behind the constants; its phase i / 2 ends with
+  // the peer's 8 KiB of step i
+  const uint32_t bars = (uint32_t)__cvta_generic_to_shared(KC + NKC * 2 * 256);
+  const uint32_t peer_bars = peer + (bars - (uint32_t)__cvta_generic_to_shared(X));
+  bool alive = true;
+  if (PAIR && t == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tmbarrier.init.shared::cta.b64 [%0 + 8], 1;\n\t"
+                 "fence.mbarrier_init.release.cluster;" ::"r"(bars)
+                 : "memory");
+  }
+  sync_both();  // both run, both inboxes are free and the barriers exist
   const size_t lanes = SEC ? (size_t)a.nl : SIMD;
   const size_t first = (((size_t)F * a.g.H + h) * a.g.L * lanes + unit) * N + 8 * t;
   const Tw4 iw0 = load_tw4(a.T.iw2[F], 2 * t), iw1 = load_tw4(a.T.iw2[F], 2 * t + 1);
@@ -1273,12 +1312,30 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
 #pragma unroll
       for (int k = 0; k < 8; k++) v[k] = y[k * STR];
       inv8_bf(v, param_tw8(a.T.iw7[F]), p);
+      if constexpr (PAIR) {
+        const uint32_t bo = (i & 1) * 8;
 #pragma unroll
-      for (int h4 = 0; h4 < 2; h4++)
-        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(peer + xo + h4 * 4096), "r"(v[4 * h4]),
-                     "r"(v[4 * h4 + 1]), "r"(v[4 * h4 + 2]), "r"(v[4 * h4 + 3])
-                     : "memory");
-      sync_both();
+        for (int h4 = 0; h4 < 2; h4++)
+          asm volatile(
+              "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                  peer + xo + h4 * 4096),
+              "r"(v[4 * h4]), "r"(v[4 * h4 + 1]), "r"(v[4 * h4 + 2]), "r"(v[4 * h4 + 3]), "r"(peer_bars + bo)
+              : "memory");
+        // (copies may land before this: the count may run below zero meanwhile)
+        if (t == 0)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + bo), "r"(256 * 32) : "memory");
+        if (alive && !wait_peer(bars + bo, (i >> 1) & 1)) {
+          alive = false;
+          if (a.err) atomicOr(a.err, 1u);
+        }
+      } else {
+#pragma unroll
+        for (int h4 = 0; h4 < 2; h4++)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(peer + xo + h4 * 4096), "r"(v[4 * h4]),
+                       "r"(v[4 * h4 + 1]), "r"(v[4 * h4 + 2]), "r"(v[4 * h4 + 3])
+                       : "memory");
+        sync_both();
+      }
 #pragma unroll
       for (int h4 = 0; h4 < 2; h4++) {
         const uint4 x = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(X) + xo + h4 * 4096);
@@ -1336,6 +1393,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
     }
     sync();
   }
+  if constexpr (PAIR) sync_both();  // neither block leaves while the peer may still write into it
   constexpr uint64_t mu = barrett_mu(p);
   const uint32_t kinv = a.cp[F].kinv;
 #pragma unroll
@@ -1560,9 +1618,11 @@ int chain_rows_supported(const Group& g) { return g.log2n == LOG2_N_MAX && g.na 
 size_t chain_rows_words(const Group& g) { return (size_t)2 * g.H * g.L * SIMD * g.n; }
 
 void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
-                               const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st) {
+                               uint32_t* err, const Group& g, const ChainConsts& cc, const NttTables& T,
+                               cudaStream_t st) {
   ChainArgs a = chain_args(g, cc, T);
   a.a_out = a_out;
+  a.err = err;
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1612,9 +1672,10 @@ int secondary_chain_wave(const Group& g, int sms) {
 }
 
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            const Group& g, const ChainConsts& cc, const ScanConsts* sc, const NttTables& T,
-                            cudaStream_t st, bool clustered) {
+                            uint32_t* err, const Group& g, const ChainConsts& cc, const ScanConsts* sc,
+                            const NttTables& T, cudaStream_t st, bool clustered) {
   ChainArgs a = chain_args(g, cc, T);
+  a.err = err;
   a.E = E;
   a.qv = qv;
   a.qv_stride = qv_stride;

@@ -110,19 +110,15 @@ int slot_acquire(dnspir_fleet* f, QSlot& s) {
 int fleet_drain(dnspir_fleet* f) {
   for (auto& s : f->slot)
     if (s.sec_pending) CK(cudaStreamWaitEvent(f->st, s.sec_done, 0));
-  const bool tensor = f->engine == DNSPIR_ENGINE_TENSOR;
-  if (tensor) {  // the error word comes with the same wait
-    CKR(f->epin.ensure(4));
-    CK(cudaMemcpyAsync(f->epin.p, f->err_word.p, 4, cudaMemcpyDeviceToHost, f->st));
-  }
+  // the error word comes with the same wait
+  CKR(f->epin.ensure(4));
+  CK(cudaMemcpyAsync(f->epin.p, f->err_word.p, 4, cudaMemcpyDeviceToHost, f->st));
   CK(cudaStreamSynchronize(f->st));
   CK(cudaStreamSynchronize(f->sec));
   for (auto& s : f->slot) s.sec_pending = false;
-  if (tensor) {
-    if (*f->epin.as<uint32_t>()) {
-      CK(cudaMemset(f->err_word.p, 0, 4));
-      return fail(DNSPIR_ERR_TIMEOUT, "tensor scan: a pipeline wait gave up");
-    }
+  if (*f->epin.as<uint32_t>()) {
+    CK(cudaMemset(f->err_word.p, 0, 4));
+    return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
   }
   return DNSPIR_OK;
 }
@@ -268,8 +264,8 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     launch_encode_rows(A, E, g2, l_in, nl, f->ctx->T, st);
     launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
-                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), g2, cc, two ? &sc : nullptr,
-                           f->ctx->T, st, clustered);
+                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), f->err_word.as<uint32_t>(), g2, cc,
+                           two ? &sc : nullptr, f->ctx->T, st, clustered);
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);
@@ -384,6 +380,8 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   for (uint32_t s = 0; s < num_shards; s++) dist[s] = (int)(s % num_distinct);
   CKR(f->distinct_dev.ensure(num_shards * sizeof(int)));
   CK(cudaMemcpy(f->distinct_dev.p, dist.data(), num_shards * sizeof(int), cudaMemcpyHostToDevice));
+  CKR(f->err_word.ensure(4));
+  CK(cudaMemset(f->err_word.p, 0, 4));
   CKR(allocate_slabs(f.get()));
   CKR(f->a_zq.ensure((size_t)num_distinct * SIMD * f->g1.n * 8));
   CKR(f->a_ms.ensure((size_t)num_distinct * SIMD * f->g1.n * 4));
@@ -419,10 +417,6 @@ int dnspir_fleet_set_engine(dnspir_fleet* f, int engine) {
   if (engine == DNSPIR_ENGINE_TENSOR && !tensor_layout_supported(f->g1))
     return fail(DNSPIR_ERR_BAD_SHAPE, "the tensor layout needs loop_len = N/2 and N >= 256");
   DeviceGuard dg(f->device);
-  if (engine == DNSPIR_ENGINE_TENSOR) {
-    CKR(f->err_word.ensure(4));
-    CK(cudaMemset(f->err_word.p, 0, 4));
-  }
   if (engine != f->engine)
     for (uint32_t d = 0; d < f->D; d++) f->ready[d] = false;  // the slab layout changes
   f->engine = engine;
@@ -818,15 +812,16 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
       CKR(f->tmp_lane.ensure((size_t)cnt * words * 4));
       std::vector<uint32_t*> tmp(cnt);
       for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
-      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws, f->st, last));
+      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws, f->err_word.as<uint32_t>(), f->st, last));
       for (uint32_t i = 0; i < cnt; i++)
         launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d0 + i]), f->g1, f->st);
     } else {
-      CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws, f->st, last));
+      CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws,
+                            f->err_word.as<uint32_t>(), f->st, last));
     }
   }
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(f->st));
+  CKR(fleet_drain(f));
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = true;
   // the scratch of a bulk load goes back; an update of a few shards keeps its own
   f->tmp_lane.release();

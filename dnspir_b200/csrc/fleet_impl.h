@@ -59,7 +59,8 @@ struct dnspir_fleet {
   int engine = DNSPIR_ENGINE_CUDA_CORES;
   bool serving = false;                       // attached to a running server
   bool one_group = false;                     // the call in progress is one group (default tile shape)
-  dnspir::DBuf qb, err_word, tmp_lane;        // tensor engine: query operand, wait-error word, preprocessing scratch
+  dnspir::DBuf qb, tmp_lane;                  // tensor engine: query operand, preprocessing scratch
+  dnspir::DBuf err_word;                      // set by a kernel whose bounded wait gave up
   dnspir::TScanLimits limits;                 // tensor engine: wait limit (and the timeout-test hook)
   std::map<int, int> tuned;                   // tensor engine: group size -> tile shape index
   std::map<int, int> tuned_cc;                // CUDA-core engine: group size -> queries per block

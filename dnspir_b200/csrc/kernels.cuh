@@ -104,11 +104,14 @@ void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_o
 // rows (launch_encode_lift, frame 1, nl = 8) lie at rows + s * shard_words and
 // take the states, times the factor's CRT constant, in place; the high digits
 // go to digits + s * shard_words, the same layout [p][half][r][lane][pos] with
-// row r for chain step L - 1 - r (chain_rows_words a shard).
+// row r for chain step L - 1 - r (chain_rows_words a shard).  err: one device word
+// set to 1 when a bounded wait between the blocks of a chain gave up (here and in
+// launch_secondary_chain).
 int chain_rows_supported(const Group& g);
 size_t chain_rows_words(const Group& g);
 void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
-                               const Group& g, const ChainConsts& cc, const NttTables& T, cudaStream_t st);
+                               uint32_t* err, const Group& g, const ChainConsts& cc, const NttTables& T,
+                               cudaStream_t st);
 // Rows of `words` words in all: bit-reversed positions -> (sign, e) order, in place.
 void launch_order_rows(uint32_t* rows, size_t words, const SlotMaps& maps, cudaStream_t st);
 // One shard's rows and digits (bit-reversed positions) -> its lane-layout slab.
@@ -130,8 +133,8 @@ void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq,
 // sc: scan_consts of the secondary's a-part set, or null when one of its query
 // slots is zero.
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            const Group& g, const ChainConsts& cc, const ScanConsts* sc, const NttTables& T,
-                            cudaStream_t st, bool clustered = false);
+                            uint32_t* err, const Group& g, const ChainConsts& cc, const ScanConsts* sc,
+                            const NttTables& T, cudaStream_t st, bool clustered = false);
 // Queries whose chains fill the SMs once.
 int secondary_chain_wave(const Group& g, int sms);
 

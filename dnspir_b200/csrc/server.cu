@@ -264,7 +264,7 @@ void worker_main(dnspir_server* sv) {
         if (e != cudaSuccess) {
           cudaGetLastError();
           status = DNSPIR_ERR_CUDA;
-        } else if (db.f->engine == DNSPIR_ENGINE_TENSOR) {
+        } else {
           uint32_t w = 0;
           if (cudaMemcpy(&w, db.f->err_word.p, 4, cudaMemcpyDeviceToHost) != cudaSuccess || w) {
             cudaMemset(db.f->err_word.p, 0, 4);
