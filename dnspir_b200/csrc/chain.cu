@@ -1155,9 +1155,15 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // is bounded; when it gives up the block raises the error word, stops waiting and
 // runs to its end on what it has.
 constexpr uint64_t PEER_WAIT_NS = 2000000000ull;
-constexpr int few_words(int kc) {  // of one factor: A, B (secondary), inbox[2], constants, two mbarriers
-  return (kc > 3 ? 2 : 1) * n2k::PS + 2 * N_MAX + kc * 2 * 256 * 4 + 4;
+// The states a and b^ are kept apart from the transforms' work space and
+// transposed, position 8 t + m at word 256 m + t: sigma_5 maps a warp's
+// positions of one m to 32 positions whose t differ mod 32, so its gathers have
+// no bank conflict (three-way in the padded order), and the first pass may
+// write its work space without waiting for them.
+constexpr int few_words(int kc) {  // of one factor: work space, a, b^ (secondary), inbox[2], constants, two mbarriers
+  return n2k::PS + (kc > 3 ? 4 : 3) * N_MAX + kc * 2 * 256 * 4 + 4;
 }
+__device__ __forceinline__ uint32_t state_word(uint32_t pos) { return ((pos & 7) << 8) | (pos >> 3); }
 
 // Waits for the phase of `parity` of a barrier that the peer block's copies
 // complete; false after PEER_WAIT_NS.
@@ -1188,10 +1194,11 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   using namespace n2k;
   constexpr int NKC = SEC ? SEC2K_KC : PRIM2K_KC;
   constexpr uint32_t p = F ? P2 : P1;
-  constexpr int WORDS = few_words(NKC), XO = (SEC ? 2 : 1) * PS;
+  constexpr int WORDS = few_words(NKC), XO = PS + (SEC ? 2 : 1) * N;
   const int t = threadIdx.x & 255;
-  uint32_t* const A = sm + (PAIR ? 0 : F * WORDS);
-  uint32_t* const B = A + PS;
+  uint32_t* const A = sm + (PAIR ? 0 : F * WORDS);  // work space
+  uint32_t* const S = A + PS;                       // a
+  uint32_t* const B = S + N;                        // b^
   uint32_t* const X = A + XO;  // inbox: [parity][half of 8][t] 16-byte vectors
   uint4* const KC = reinterpret_cast<uint4*>(X + 2 * N);  // [j][quad half][t]
   // barrier of this factor's threads, and of both factors'
@@ -1209,16 +1216,15 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   };
   const int qb = (int)phys(8 * t);
   // sigma_5 sources (galb inverted through X), a = b^ = 0, constants
-  for (int b = t; b < N; b += 256) X[__ldg(a.galb + b)] = b;
-#pragma unroll
-  for (int h4 = 0; h4 < 2; h4++) {
-    *reinterpret_cast<uint4*>(A + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
-    if (SEC) *reinterpret_cast<uint4*>(B + qb + 4 * h4) = make_uint4(0, 0, 0, 0);
+  for (int b = t; b < N; b += 256) {
+    X[__ldg(a.galb + b)] = b;
+    S[b] = 0;
+    if (SEC) B[b] = 0;
   }
   sync();
   Sources src;
 #pragma unroll
-  for (int m = 0; m < 4; m++) src.w[m] = phys(X[8 * t + 2 * m]) | (phys(X[8 * t + 2 * m + 1]) << 16);
+  for (int m = 0; m < 4; m++) src.w[m] = state_word(X[8 * t + 2 * m]) | (state_word(X[8 * t + 2 * m + 1]) << 16);
 #pragma unroll
   for (int h4 = 0; h4 < 2; h4++) {
     uint32_t kc[NKC][4];
@@ -1278,7 +1284,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
     const size_t row = first + (size_t)(a.g.L - 1 - i) * lanes * N;
     uint32_t ta[8], tb[8];
 #pragma unroll
-    for (int m = 0; m < 8; m++) ta[m] = A[src.at(m)];
+    for (int m = 0; m < 8; m++) ta[m] = S[src.at(m)];
     if (SEC) {
 #pragma unroll
       for (int m = 0; m < 8; m++) tb[m] = B[src.at(m)];
@@ -1288,7 +1294,6 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
     for (int h4 = 0; h4 < 2; h4++)
       e[h4] = SEC ? __ldg(reinterpret_cast<const uint4*>(a.E + row) + h4)
                   : *(reinterpret_cast<const uint4*>(rows + row) + h4);
-    sync();
 #pragma unroll
     for (int h4 = 0; h4 < 2; h4++) {
       const Tw4& w = h4 ? iw1 : iw0;
@@ -1381,12 +1386,13 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
                                 p, pinv),
                       2 * p);
       }
-      const uint4 x = make_uint4(an[0], an[1], an[2], an[3]);
-      *reinterpret_cast<uint4*>(A + qb + 4 * h4) = x;
-      if constexpr (SEC) {
-        *reinterpret_cast<uint4*>(B + qb + 4 * h4) = make_uint4(bn[0], bn[1], bn[2], bn[3]);
-      } else {
-        *(reinterpret_cast<uint4*>(rows + row) + h4) = x;
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        S[256 * (4 * h4 + m) + t] = an[m];
+        if constexpr (SEC) B[256 * (4 * h4 + m) + t] = bn[m];
+      }
+      if constexpr (!SEC) {
+        *(reinterpret_cast<uint4*>(rows + row) + h4) = make_uint4(an[0], an[1], an[2], an[3]);
         *(reinterpret_cast<uint4*>(digits + row) + h4) =
             make_uint4(canon(n1[0], p), canon(n1[1], p), canon(n1[2], p), canon(n1[3], p));
       }
@@ -1398,11 +1404,11 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   const uint32_t kinv = a.cp[F].kinv;
 #pragma unroll
   for (int m = 0; m < 8; m++) {
-    const uint32_t av = mul_mod(A[qb + m], kinv, p, mu), pos = 8 * t + m;
+    const uint32_t av = mul_mod(S[256 * m + t], kinv, p, mu), pos = 8 * t + m;
     if constexpr (SEC) {
       uint32_t* o = a.out + (((size_t)q * a.g.H + h) * CTXT_PARTS + (unit - q * CTXT_PARTS)) * 4 * N + F * N + pos;
       o[0] = av;
-      o[2 * N] = add_mod(red(B[qb + m], p), mul_mod(av, query_ratio(a, sc, h, q, F, pos), p, mu), p);
+      o[2 * N] = add_mod(red(B[256 * m + t], p), mul_mod(av, query_ratio(a, sc, h, q, F, pos), p, mu), p);
     } else {
       a.a_out[((size_t)h * SIMD + unit) * 2 * N + F * N + pos] = av;
     }
