@@ -944,32 +944,25 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
   for (int m = 0; m < 4; m++) src.w[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
   // the constants of position quads, dealt over the whole block: item = (factor, quad)
   {
-    constexpr int ITEMS = 2 * N / 4, PER = (ITEMS + NT - 1) / NT;
-    uint32_t from[PER][4];
+    constexpr int PER = (2 * N + NT - 1) / NT;
+    uint32_t from[PER];
 #pragma unroll
-    for (int c = 0; c < PER; c++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const int it = threadIdx.x + c * NT;
-        from[c][m] = it < ITEMS ? inv[4 * (it & (N / 4 - 1)) + m] : 0;
-      }
+    for (int c = 0; c < PER; c++) from[c] = inv[(threadIdx.x + c * NT) & (N - 1)];
     __syncthreads();  // the table is overwritten by the constants
-#pragma unroll
+    // (not unrolled, as in few_chain)
+#pragma unroll 1
     for (int c = 0; c < PER; c++) {
       const int it = threadIdx.x + c * NT;
-      if (it < ITEMS) {
-        const int f = it / (N / 4), quad = it & (N / 4 - 1);
-        uint32_t kc[SEC2K_KC][4];
+      if (it < 2 * N) {
+        const int f = it / N, pos = it & (N - 1);
+        uint32_t k[SEC2K_KC];
+        uint32_t src_pos = from[0];
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-          uint32_t k[SEC2K_KC];
-          secondary_constants(a, sc, h, q, f, 4 * quad + m, from[c][m], k);
-#pragma unroll
-          for (int j = 0; j < SEC2K_KC; j++) kc[j][m] = k[j];
-        }
+        for (int x = 1; x < PER; x++) src_pos = c == x ? from[x] : src_pos;
+        secondary_constants(a, sc, h, q, f, pos, src_pos, k);
 #pragma unroll
         for (int j = 0; j < SEC2K_KC; j++)
-          KC[((j * 2 + f) * 2 + (quad & 1)) * 256 + (quad >> 1)] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
+          reinterpret_cast<uint32_t*>(KC)[(((j * 2 + f) * 2 + (pos >> 2 & 1)) * 256 + (pos >> 3)) * 4 + (pos & 3)] = k[j];
       }
     }
   }
@@ -1029,10 +1022,10 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
       for (int h4 = 0; h4 < 2; h4++) *reinterpret_cast<uint4*>(B + f * PS + qb + 4 * h4) = bn[f][h4];
   }
   uint32_t* o = a.out + ((((size_t)q * a.g.H + h) * CTXT_PARTS + part) * 2) * 2 * N;
-#pragma unroll
+#pragma unroll 1
   for (int f = 0; f < 2; f++) {
     const uint32_t p = prime_of(f);
-#pragma unroll
+#pragma unroll 1
     for (int m = 0; m < 8; m++) {
       const uint32_t av = mul_mod(A[f * PS + qb + m], f ? a.cp[1].kinv : a.cp[0].kinv, p, barrett_mu(p));
       const uint32_t br = red(B[f * PS + qb + m], p);
@@ -1070,22 +1063,14 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 #pragma unroll
   for (int m = 0; m < 4; m++) src.w[m] = phys(inv[8 * t + 2 * m]) | (phys(inv[8 * t + 2 * m + 1]) << 16);
   __syncthreads();  // the table is overwritten by the constants, each thread reading only its own
+#pragma unroll 1
+  for (int fm = 0; fm < 16; fm++) {  // (not unrolled, as in few_chain)
+    const int f = fm >> 3, m = fm & 7;
+    uint32_t k[PRIM2K_KC];
+    state_constants(a, h, f, 8 * t + m, k);
 #pragma unroll
-  for (int f = 0; f < 2; f++) {
-#pragma unroll
-    for (int h4 = 0; h4 < 2; h4++) {
-      uint32_t kc[PRIM2K_KC][4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        uint32_t k[PRIM2K_KC];
-        state_constants(a, h, f, 8 * t + 4 * h4 + m, k);
-#pragma unroll
-        for (int j = 0; j < PRIM2K_KC; j++) kc[j][m] = k[j];
-      }
-#pragma unroll
-      for (int j = 0; j < PRIM2K_KC; j++)
-        KC[((j * 2 + f) * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
-    }
+    for (int j = 0; j < PRIM2K_KC; j++)
+      reinterpret_cast<uint32_t*>(KC)[(((j * 2 + f) * 2 + (m >> 2)) * 256 + t) * 4 + (m & 3)] = k[j];
   }
   const size_t first = (size_t)s * shard_words + ((size_t)h * a.g.L * SIMD + lane) * N + 8 * t;
   const size_t row_stride = (size_t)SIMD * N, efac = (size_t)a.g.H * a.g.L * row_stride;
@@ -1225,21 +1210,18 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   Sources src;
 #pragma unroll
   for (int m = 0; m < 4; m++) src.w[m] = state_word(X[8 * t + 2 * m]) | (state_word(X[8 * t + 2 * m + 1]) << 16);
+  // (not unrolled: eight copies of this code, run once, cost more to fetch than to
+  // run -- 47 us of set-up instead of 21)
+#pragma unroll 1
+  for (int m = 0; m < 8; m++) {
+    uint32_t k[NKC];
+    if constexpr (SEC)
+      secondary_constants(a, sc, h, q, F, 8 * t + m, X[8 * t + m], k);
+    else
+      state_constants(a, h, F, 8 * t + m, k);
 #pragma unroll
-  for (int h4 = 0; h4 < 2; h4++) {
-    uint32_t kc[NKC][4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-      uint32_t k[NKC];
-      if constexpr (SEC)
-        secondary_constants(a, sc, h, q, F, 8 * t + 4 * h4 + m, X[8 * t + 4 * h4 + m], k);
-      else
-        state_constants(a, h, F, 8 * t + 4 * h4 + m, k);
-#pragma unroll
-      for (int j = 0; j < NKC; j++) kc[j][m] = k[j];
-    }
-#pragma unroll
-    for (int j = 0; j < NKC; j++) KC[(j * 2 + h4) * 256 + t] = make_uint4(kc[j][0], kc[j][1], kc[j][2], kc[j][3]);
+    for (int j = 0; j < NKC; j++)
+      reinterpret_cast<uint32_t*>(KC)[((j * 2 + (m >> 2)) * 256 + t) * 4 + (m & 3)] = k[j];
   }
   // shared::cluster address of the other factor's inbox
   uint32_t peer = (uint32_t)__cvta_generic_to_shared(PAIR ? X : sm + (1 - F) * WORDS + XO);
@@ -1402,7 +1384,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   if constexpr (PAIR) sync_both();  // neither block leaves while the peer may still write into it
   constexpr uint64_t mu = barrett_mu(p);
   const uint32_t kinv = a.cp[F].kinv;
-#pragma unroll
+#pragma unroll 1
   for (int m = 0; m < 8; m++) {
     const uint32_t av = mul_mod(S[256 * m + t], kinv, p, mu), pos = 8 * t + m;
     if constexpr (SEC) {
