@@ -72,7 +72,9 @@ const TScanShape& tensor_shape(dnspir_fleet* f, int nb, int* nb_pad) {
     // (30 queries 10.1 against 10.5 one tile per CTA, 50: 16.8 / 17.3).  Groups
     // that overlap the last one's secondary phase take one tile per CTA: a
     // persistent CTA whose SM a chain block holds would start its whole share
-    // late (four groups of 12: 27.1 / 31.5, of 50: 59.9 / 64.8).  65 to 96
+    // late (four groups of 12: 23.9 / 26.6, of 60: 56.4 / 61.1).  33 to 48
+    // queries have a tile of their own (three groups of 40 at 2^22 138 against
+    // 146 ms in the 64-query tile, one of 37 10.8 / 10.9).  65 to 96
     // queries run as three 32-query tiles (24.7 against 28.8 as one 128-query
     // tile); beyond, the scan is bound by the tensor pipe either way and the
     // persistent 64-query tile with two m-tiles is best (four groups of 120:
@@ -86,6 +88,7 @@ const TScanShape& tensor_shape(dnspir_fleet* f, int nb, int* nb_pad) {
     else if (nb <= 8) want = TScanShape{32, 1, 5, 0};
     else if (nb <= 16) want = alone ? TScanShape{64, 2, 4, 1} : TScanShape{64, 1, 4, 0};
     else if (nb <= 32) want = alone && maps ? TScanShape{128, 2, 4, 3} : TScanShape{128, 2, 2, 0};
+    else if (nb <= 48) want = alone && maps ? TScanShape{192, 1, 7, 3} : TScanShape{192, 1, 2, 0};
     else if (nb <= 64) want = alone && maps ? TScanShape{256, 1, 6, 3} : TScanShape{256, 1, 2, 0};
     else if (nb <= 96) want = TScanShape{128, 2, 2, 0};
     else want = TScanShape{256, 2, 3, 1};

@@ -299,14 +299,21 @@ __device__ __forceinline__ void epilogue_tile(const TScanArgs& a, uint32_t taddr
   }
 }
 
+// TMEM columns to allocate for c columns of accumulators: a power of two, at least 32
+constexpr int tmem_cols(int c) {
+  int n = 32;
+  while (n < c) n *= 2;
+  return n;
+}
+
 template <int NQ, int MTPC>
 __global__ void __launch_bounds__(TSCAN_NT, 1) tscan_kernel(TScanArgs a) {
   constexpr uint32_t A_BYTES = MTPC * TBLK;
   constexpr uint32_t STAGE = A_BYTES + NQ * 128;
-  constexpr uint32_t COLS = (MTPC * NQ) <= 32 ? 32 : (MTPC * NQ);
+  constexpr uint32_t COLS = tmem_cols(MTPC * NQ);
   constexpr int NSPLIT = NQ > 256 ? NQ / 256 : 1;
   constexpr int NMMA = NQ / NSPLIT;
-  static_assert(STAGE % 1024 == 0 && COLS <= 512 && (COLS & (COLS - 1)) == 0, "tile shape");
+  static_assert(STAGE % 1024 == 0 && COLS <= 512, "tile shape");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t S_ = a.stages;
@@ -444,7 +451,7 @@ __global__ void __launch_bounds__(TSCAN_NT, 1) tscan_kernel(TScanArgs a) {
 // in flight before it frees TMEM.
 template <int NQ>
 constexpr int tscanp_ew() {
-  return NQ >= 256 ? 4 : NQ >= 128 ? 2 : 1;
+  return NQ >= 128 ? NQ / 64 : 1;
 }
 template <int NQ>
 constexpr int tscanp_nt() {
@@ -463,9 +470,9 @@ __global__ void __launch_bounds__(tscanp_nt<NQ>(), 1) tscanp_kernel(TScanArgs a)
   // two accumulators when they fit the SM's 512 columns; with one, the MMAs of
   // a tile wait for the previous tile's epilogue, but its chunks still stream in
   constexpr uint32_t BUFS = 2 * ACC <= 512 ? 2 : 1;
-  constexpr uint32_t COLS = BUFS * ACC;
+  constexpr uint32_t COLS = tmem_cols(BUFS * ACC);
   constexpr int EW = tscanp_ew<NQ>();  // epilogue warps per TMEM lane quarter
-  static_assert(STAGE % 1024 == 0 && ACC >= 16 && COLS <= 512 && (COLS & (COLS - 1)) == 0, "tile shape");
+  static_assert(STAGE % 1024 == 0 && ACC >= 16 && COLS <= 512, "tile shape");
   static_assert(NQ % EW == 0 && (EW == 1 || NQ / EW == 64), "columns per epilogue warp");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -736,9 +743,9 @@ __global__ void __launch_bounds__(tscanp_nt<NQ>(), 1) tscan2_kernel(const __grid
   constexpr uint32_t STAGE = A_BYTES + V_BYTES;
   constexpr uint32_t ACC = MTPC * NQ;  // TMEM columns of one accumulator
   constexpr uint32_t BUFS = 2 * ACC <= 512 ? 2 : 1;
-  constexpr uint32_t COLS = BUFS * ACC < 32 ? 32 : BUFS * ACC;
+  constexpr uint32_t COLS = tmem_cols(BUFS * ACC);
   static_assert(NQ >= 32 && NQ <= 256 && NQ % 32 == 0, "pair MMA: N in 32..256, a multiple of 32");
-  static_assert(STAGE % 1024 == 0 && ACC <= 512 && (COLS & (COLS - 1)) == 0, "tile shape");
+  static_assert(STAGE % 1024 == 0 && COLS <= 512, "tile shape");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t S_ = a.stages;
@@ -1111,7 +1118,7 @@ int launch_t(const TScanArgs& a0, int stages, cudaStream_t st) {
   if (smem > 227 * 1024) return -1;
   set_smem(tscan_kernel<NQ, MTPC>, smem);
   // resident CTAs must not ask for more TMEM columns than the SM has
-  constexpr int COLS = (MTPC * NQ) <= 32 ? 32 : (MTPC * NQ);
+  constexpr int COLS = tmem_cols(MTPC * NQ);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tscan_kernel<NQ, MTPC>, TSCAN_NT, smem);
   if (per_sm * COLS > 512) return -1;
@@ -1128,7 +1135,7 @@ int launch_tp(const TScanArgs& a0, int stages, cudaStream_t st) {
   const size_t smem = 1024 + (size_t)stages * STAGE + (2 * stages + 5) * 8 + 16;
   if (smem > 227 * 1024) return -1;
   set_smem(tscanp_kernel<NQ, MTPC>, smem);
-  constexpr int COLS = (2 * MTPC * NQ <= 512 ? 2 : 1) * MTPC * NQ;
+  constexpr int COLS = tmem_cols((2 * MTPC * NQ <= 512 ? 2 : 1) * MTPC * NQ);
   int per_sm = 0, dev = 0, sms = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tscanp_kernel<NQ, MTPC>, tscanp_nt<NQ>(), smem);
   // resident CTAs must not ask for more TMEM columns than the SM has (a CTA
@@ -1275,6 +1282,9 @@ const TScanShape* tscan_shapes(int* count) {
       // (30.1 ms per group at 2^22 against 29.5-30.9 for the one-tile-per-CTA
       // shapes; (64, 1, 8-9) and (128, 1, 6-7) measured 35-37 ms)
       {64, 2, 5, 1},
+      // 48 queries: groups of 33 to 48 would compute on a quarter to half of
+      // zeros in a 64-query tile
+      {192, 1, 2, 0}, {192, 1, 5, 1}, {192, 1, 7, 3},
   };
   *count = (int)(sizeof(shapes) / sizeof(shapes[0]));
   return shapes;
@@ -1346,6 +1356,7 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
       case 641: return launch_t2<64, 1, true>(a, stg, st);
       case 1281: return launch_t2<128, 1, true>(a, stg, st);
       case 1282: return launch_t2<128, 2, true>(a, stg, st);
+      case 1921: return launch_t2<192, 1, true>(a, stg, st);
       case 2561: return launch_t2<256, 1, true>(a, stg, st);
       case 2562: return launch_t2<256, 2, true>(a, stg, st);
       default: return -1;
@@ -1358,6 +1369,7 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
       case 642: return launch_tp<64, 2>(a, stg, st);
       case 1281: return launch_tp<128, 1>(a, stg, st);
       case 1282: return launch_tp<128, 2>(a, stg, st);
+      case 1921: return launch_tp<192, 1>(a, stg, st);
       case 2561: return launch_tp<256, 1>(a, stg, st);
       case 2562: return launch_tp<256, 2>(a, stg, st);
       default: return -1;
@@ -1370,6 +1382,7 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
     case 642: return launch_t<64, 2>(a, stg, st);
     case 1281: return launch_t<128, 1>(a, stg, st);
     case 1282: return launch_t<128, 2>(a, stg, st);
+    case 1921: return launch_t<192, 1>(a, stg, st);
     case 2561: return launch_t<256, 1>(a, stg, st);
     case 2562: return launch_t<256, 2>(a, stg, st);
     case 5121: return launch_t<512, 1>(a, stg, st);
