@@ -198,7 +198,7 @@ int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbyte
   CKR(s.qbrv.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
   CKR(s.qv.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
   CKR(s.fin.ensure((size_t)Bk * f->S * 2 * n * SIMD * 4));
-  CKR(s.sec_in.ensure((size_t)f->g2.l * CTXT_PARTS * nb * n * 2));
+  if (!epilogue_cols_supported(f->g1)) CKR(s.sec_in.ensure((size_t)f->g2.l * CTXT_PARTS * nb * n * 2));
   CKR(s.qdesc.ensure((size_t)nb * sizeof(QDesc)));
   CKR(s.dpin.ensure((size_t)nb * sizeof(QDesc)));
   if (qbytes) CKR(s.qbytes.ensure(qbytes));
@@ -245,9 +245,13 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
   // the primary epilogue (scan output -> secondary entries) runs here, on the
   // secondary stream, so that the next group's scan does not wait for it; it
   // reads and writes only this slot's buffers
-  launch_primary_epilogue(s.fin.as<uint32_t>(), nb, f->S, f->a_ms.as<uint32_t>(), f->distinct_dev.as<int>(),
-                          s.sec_in.as<uint16_t>(), f->sec_chunk, f->g1, slot_maps(f->ctx, f->g1.log2n), f->ctx->T, st);
-  f->launches += 1;
+  const bool fused = epilogue_cols_supported(f->g1);
+  if (!fused) {
+    launch_primary_epilogue(s.fin.as<uint32_t>(), nb, f->S, f->a_ms.as<uint32_t>(), f->distinct_dev.as<int>(),
+                            s.sec_in.as<uint16_t>(), f->sec_chunk, f->g1, slot_maps(f->ctx, f->g1.log2n), f->ctx->T,
+                            st);
+    f->launches += 1;
+  }
   const SlotMaps maps = slot_maps(f->ctx, g2.log2n);
   const ChainConsts cc = chain_consts(f->ctx, g2.log2n, 1);
   const ScanConsts sc = scan_consts(f->ctx, g2, 1);
@@ -260,10 +264,13 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     // the last chunk's start: a later group's primary phase may wait for this
     // instead of the whole phase (it then shares the SMs the last chunk leaves idle)
     if (c0 + f->sec_chunk >= nb && s.sec_tail) CK(cudaEventRecord(s.sec_tail, st));
-    const uint16_t* in = s.sec_in.as<uint16_t>() + (size_t)c0 * CTXT_PARTS * l_in * n;
     uint32_t* const E = f->secE.as<uint32_t>();
     uint32_t* const A = E + (size_t)g2.H * g2.L * nl * n;
-    launch_encode_cols(in, A, g2, l_in, nl, f->ctx->T, st);
+    if (fused)
+      launch_epilogue_cols(s.fin.as<uint32_t>() + (size_t)c0 * f->S * 2 * n * SIMD, nc, f->S, f->a_ms.as<uint32_t>(),
+                           f->distinct_dev.as<int>(), A, slot_maps(f->ctx, f->g1.log2n), f->ctx->T, st);
+    else
+      launch_encode_cols(s.sec_in.as<uint16_t>() + (size_t)c0 * CTXT_PARTS * l_in * n, A, g2, l_in, nl, f->ctx->T, st);
     launch_encode_rows(A, E, g2, l_in, nl, f->ctx->T, st);
     launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
@@ -272,7 +279,7 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);
-    f->launches += 5;  // encoder columns, rows, lift; chains; replies
+    f->launches += 5;  // encoder columns (with the epilogue), rows, lift; chains; replies
   }
   if (host_reply)
     CK(cudaMemcpyAsync(host_reply, reply_dev, (size_t)nb * dnspir_reply_bytes(), cudaMemcpyDeviceToHost, st));

@@ -208,6 +208,11 @@ int preload_pir_split_kernels();
 void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
                              uint16_t* sec_in, int chunk, const Group& g, const SlotMaps& maps, const NttTables& T,
                              cudaStream_t st);
+// The same for one chunk of nq queries at N = 2048, ending in the encoder's
+// column transforms A [t][lane][x] (launch_encode_cols' output) instead of entries.
+int epilogue_cols_supported(const Group& g);
+void launch_epilogue_cols(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
+                          uint32_t* A, const SlotMaps& maps, const NttTables& T, cudaStream_t st);
 // Epilogue returning b as Z_q coefficients [lane][n] (shard-level perform_pir_split).
 void launch_epilogue_zq(const uint32_t* sum, uint64_t* out, const Group& g, const SlotMaps& maps, const NttTables& T,
                         cudaStream_t st);

@@ -327,14 +327,19 @@ __global__ void primary_epilogue_kernel(const uint32_t* __restrict__ fin, int ns
   }
 }
 
-// ---- N = 2048: the same epilogue on the register transforms of
-// ntt2048.cuh.  Grid: x = shard, y = four lanes, z = query.  One 16-byte
-// gather per position and factor brings four lanes (half a 32-byte sector; the
-// other half is the neighbouring block's), the eight inverse transforms run
-// together, the CRT uses Shoup companions of its two constants and the 12-bit
-// switch an exact 64-bit rounding (v 2^13 + q < 2^64 for v < q).  LN = 1: one
-// lane per block, for so few shards and queries that the blocks do not fill the
-// SMs (one query of 4 shards: 25 -> 12.6 us).
+// ---- N = 2048: the same epilogue on the register transforms of ntt2048.cuh,
+// with the encoder's column transforms (encode.cu) in the same block: the three
+// digits of a coefficient stay in shared memory as one word, and each digit's
+// polynomial is transformed from there into A [t][lane][x].  Grid: x = shard, y =
+// LN lanes, z = query of the chunk.  One 16-byte gather per position and factor
+// brings four lanes (half a 32-byte sector; the other half is the neighbouring
+// block's), the eight inverse transforms run together, the CRT uses Shoup
+// companions of its two constants and the 12-bit switch an exact 64-bit rounding
+// (v 2^13 + q < 2^64 for v < q).  LN = 1: one lane per block, for so few shards
+// and queries that the blocks do not fill the SMs.  Bound by shared memory and
+// barriers (three blocks an SM).  Against digits through global memory and a kernel
+// for their columns (256 queries of 128 shards): 2.95 + 2.03 -> 4.25 ms, and the
+// digits' buffer is not needed.
 constexpr int EPI_NT = 512;
 
 __device__ __forceinline__ uint32_t ms_encode12(uint64_t v) {
@@ -354,8 +359,8 @@ __device__ __forceinline__ uint32_t ms_encode12(uint64_t v) {
 template <int LN>
 __global__ void __launch_bounds__(EPI_NT, LN == 4 ? 3 : 0) primary_epilogue2k_kernel(
     const uint32_t* __restrict__ fin, int nshards, const uint32_t* __restrict__ a_ms,
-    const int* __restrict__ distinct_of, uint16_t* __restrict__ sec_in, int nq, int chunk,
-    const uint32_t* __restrict__ uof, NttTables T, uint32_t k1, uint32_t k1q, uint32_t k2, uint32_t k2q) {
+    const int* __restrict__ distinct_of, uint32_t* __restrict__ A, const uint32_t* __restrict__ uof, NttTables T,
+    uint32_t k1, uint32_t k1q, uint32_t k2, uint32_t k2q) {
   extern __shared__ __align__(16) uint32_t sm[];  // [q1 lanes l0 .. l0 + LN - 1][q2 lanes], padded
   using namespace n2k;
   const int s = blockIdx.x, l0 = blockIdx.y * LN, b = blockIdx.z;
@@ -374,10 +379,6 @@ __global__ void __launch_bounds__(EPI_NT, LN == 4 ? 3 : 0) primary_epilogue2k_ke
   __syncthreads();
   inv<EPI_NT>(sm, LN, LN, T);
   const int ds = distinct_of[s];
-  // the secondary input of queries [c * chunk, ...) is one [t][lanes_c][N] block
-  const int c = b / chunk, bl = b % chunk;
-  const size_t lanes_c = (size_t)CTXT_PARTS * min(chunk, nq - c * chunk);
-  uint16_t* const base = sec_in + (size_t)c * chunk * CTXT_PARTS * nshards * SIMD * N;
   for (int x = threadIdx.x; x < LN * N; x += EPI_NT) {
     const int ll = x >> 11, n = x & (N - 1);
     const uint32_t o = phys(n);
@@ -390,11 +391,41 @@ __global__ void __launch_bounds__(EPI_NT, LN == 4 ? 3 : 0) primary_epilogue2k_ke
     const uint32_t d0 = w % TPLAIN;
     w /= TPLAIN;
     const uint32_t d1 = w % TPLAIN;
-    const uint32_t d2 = w / TPLAIN;
-    uint16_t* op = base + (((size_t)s * SIMD + l0 + ll) * lanes_c + (size_t)bl * CTXT_PARTS) * N + n;
-    op[0] = (uint16_t)d0;
-    op[N] = (uint16_t)d1;
-    op[2 * N] = (uint16_t)d2;
+    const uint32_t d2 = w / TPLAIN;  // below 2^29 / 1025^2 < 2^10
+    sm[ll * PS + o] = d0 | (d1 << 11) | (d2 << 22);
+  }
+  __syncthreads();
+  uint32_t* const work = sm + LN * PS;
+  const size_t nl = (size_t)CTXT_PARTS * gridDim.z;
+#pragma unroll 1
+  for (int digit = 0; digit < CTXT_PARTS; digit++) {
+    {
+      const int po = threadIdx.x >> 8, base = (int)phys(threadIdx.x & 255);
+      for (int ll = po; ll < LN; ll += EPI_NT / 256) {
+        uint32_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = (sm[ll * PS + base + k * Geo8<1>::STR] >> (11 * digit)) & 0x7FFu;
+        fwd8_bf(v, param_tw8(T.fw7[0]), P1);
+#pragma unroll
+        for (int k = 0; k < 8; k++) work[ll * PS + base + k * Geo8<1>::STR] = v[k];
+      }
+    }
+    __syncthreads();
+    pass8<EPI_NT, 8, false>(work, LN, 0, T, (void*)nullptr);
+    pass8<EPI_NT, 64, false>(work, LN, 0, T, (void*)nullptr);
+    const int g = threadIdx.x;  // quad of transform positions
+    const Tw4 tw = load_tw4(T.fw2[0], g);
+#pragma unroll
+    for (int ll = 0; ll < LN; ll++) {
+      uint4 v = *reinterpret_cast<const uint4*>(work + ll * PS + phys(4 * g));
+      ct(v.x, v.z, tw.a, tw.aq, P1);
+      ct(v.y, v.w, tw.a, tw.aq, P1);
+      ct(v.x, v.y, tw.b0, tw.b0q, P1);
+      ct(v.z, v.w, tw.b1, tw.b1q, P1);
+      reinterpret_cast<uint4*>(A + (((size_t)s * SIMD + l0 + ll) * nl + (size_t)b * CTXT_PARTS + digit) * N)[g] =
+          make_uint4(canon(v.x, P1), canon(v.y, P1), canon(v.z, P1), canon(v.w, P1));
+    }
+    __syncthreads();
   }
 }
 
@@ -507,26 +538,29 @@ int launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, c
 void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
                              uint16_t* sec_in, int chunk, const Group& g, const SlotMaps& maps, const NttTables& T,
                              cudaStream_t st) {
-  if (g.log2n == 11) {
-    const CrtConst cc = host_crt_const();
-    const uint32_t k1q = (uint32_t)(((uint64_t)cc.q2inv1 << 32) / P1);
-    const uint32_t k2q = (uint32_t)(((uint64_t)cc.q1inv2 << 32) / P2);
-    if ((size_t)nshards * SIMD * nq <= 256) {
-      primary_epilogue2k_kernel<1><<<dim3(nshards, SIMD, nq), EPI_NT, (size_t)2 * n2k::PS * 4, st>>>(
-          fin, nshards, a_ms, distinct_of, sec_in, nq, chunk, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
-      return;
-    }
-    const size_t smem = (size_t)8 * n2k::PS * 4;
-    set_smem(primary_epilogue2k_kernel<4>, smem);
-    primary_epilogue2k_kernel<4><<<dim3(nshards, SIMD / 4, nq), EPI_NT, smem, st>>>(
-        fin, nshards, a_ms, distinct_of, sec_in, nq, chunk, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
-    return;
-  }
   const size_t smem = (size_t)4 * g.n * 4;
   dim3 grid(nshards, SIMD / 2, nq);
   set_smem(primary_epilogue_kernel, smem);
   primary_epilogue_kernel<<<grid, 256, smem, st>>>(fin, nshards, a_ms, distinct_of, sec_in, nq, chunk, g,
                                                    maps.uof, T, host_crt_const());
+}
+
+int epilogue_cols_supported(const Group& g) { return g.log2n == LOG2_N_MAX; }
+
+void launch_epilogue_cols(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
+                          uint32_t* A, const SlotMaps& maps, const NttTables& T, cudaStream_t st) {
+  const CrtConst cc = host_crt_const();
+  const uint32_t k1q = (uint32_t)(((uint64_t)cc.q2inv1 << 32) / P1);
+  const uint32_t k2q = (uint32_t)(((uint64_t)cc.q1inv2 << 32) / P2);
+  if ((size_t)nshards * SIMD * nq <= 256) {
+    primary_epilogue2k_kernel<1><<<dim3(nshards, SIMD, nq), EPI_NT, (size_t)2 * n2k::PS * 4, st>>>(
+        fin, nshards, a_ms, distinct_of, A, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
+    return;
+  }
+  const size_t smem = (size_t)8 * n2k::PS * 4;
+  set_smem(primary_epilogue2k_kernel<4>, smem);
+  primary_epilogue2k_kernel<4><<<dim3(nshards, SIMD / 4, nq), EPI_NT, smem, st>>>(
+      fin, nshards, a_ms, distinct_of, A, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
 }
 
 int preload_pir_split_kernels() {

@@ -114,7 +114,7 @@ size_t group_bytes(dnspir_fleet* f, int nb, int Bk) {
   const size_t n = f->g1.n;
   const Group& g2 = f->g2;
   size_t slot = (size_t)3 * Bk * QV_WORDS_PER_QUERY * n * 4 + (size_t)Bk * f->S * 2 * n * SIMD * 4 +
-                (size_t)g2.l * CTXT_PARTS * nb * n * 2 + (size_t)nb * (full_query_bytes(f) + dnspir_reply_bytes());
+                (size_t)nb * (full_query_bytes(f) + dnspir_reply_bytes());
   const int cmax = std::min(nb, f->sec_chunk);
   const size_t sec = (size_t)CTXT_PARTS * cmax * n * 4 * ((size_t)2 * g2.H * g2.L + (size_t)g2.H * 4);
   size_t qb = f->engine == DNSPIR_ENGINE_TENSOR ? tscan_query_bytes(f->g1, Bk) : 0;
