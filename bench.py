@@ -766,7 +766,7 @@ def extra_legs(args, dp, torch, dev, local_rank):
                                    "rule gives full shards at 2^20 (pir_wrapper.rs:188, 223-227)")
         legs["config4"] = batched_leg(dp, torch, dev, 1 << 20, "tensor", [16, 64, 256], 3)
         legs["config4"]["note"] = ("INT8 limb products on tcgen05 (u8 x u8 -> s32, 16 limb products per residue "
-                                   "product, K <= 6144 so no partial sum overflows), recombined and reduced mod each "
+                                   "product, K = 4096, so no partial sum overflows), recombined and reduced mod each "
                                    "prime; scan_tensor_pops counts int8 limb operations (2 per MAC)")
         results, prep_s = serve_mix(args, local_rank, [5000.0], 3.0)
         legs["served"] = {"offered_per_sec": 5000.0, "seconds": 3.0, "preprocess_s": prep_s,
@@ -799,9 +799,8 @@ def main():
     slab_bytes = stored_shard_bytes(dp, l1, local_rank)
     free, _ = torch.cuda.mem_get_info()
     sizes = [int(x) for x in args.batched.split(",") if x.strip()]
-    # workspaces: two buffer slots, each with the scan output and the
-    # secondary input of the largest group, the secondary phase's chunk (at
-    # most 6 GiB) and headroom
+    # workspaces: two buffer slots, each with the scan output of the largest
+    # group, the secondary phase's chunk (at most 8 GiB) and headroom
     per_query_ws = shards * 2 * dp.N * 8 * 4 + l2 * 3 * dp.N * 2
     reserve = args.reserve_gib * (1 << 30) if args.reserve_gib > 0 else \
         2 * max(sizes + [1]) * per_query_ws + (10 << 30)

@@ -1042,8 +1042,8 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
 // canonical high digits' transforms go to `digits`, the same layout.  Three
 // blocks fit an SM (67 KiB, 80 registers), so up to one wave of 444 chains runs
 // at once.  Against two-block clusters with one factor per block (radix-4
-// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (2.7 when
-// there are fewer, on two SMs each, below).
+// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (2.2 on two
+// SMs each, below).
 constexpr int PRIM2K_KC = 3;
 constexpr int PRIM2K_WORDS = 2 * n2k::PS + PRIM2K_KC * 2 * 2 * 256 * 4;
 
@@ -1129,8 +1129,9 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // step is half as long for a thread.  PAIR: the factors' threads are the two
 // blocks of a cluster, on two SMs while there are two for every chain -- a
 // chain alone on one SM keeps its heavy FMA pipe 60 % busy, so the second SM
-// is what shortens the step (2.7 us against 3.7).  Otherwise they are the two
-// halves of one 512-thread block (up to one chain per SM).  The factors send each other their inverse outputs:
+// is what shortens the step (2.06 us against 3.66).  Otherwise they are the two
+// halves of one 512-thread block (up to one chain per SM).  The factors send each
+// other their inverse outputs:
 // every thread writes its eight values into the other's inbox (double-buffered
 // by step parity, so that one may run ahead of the other's reads) before the
 // one barrier of a step that both meet.  F: the factor, so that primes and
@@ -1670,9 +1671,9 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
   a.nl = nq * CTXT_PARTS;
   a.out = out;
   // N = 2048 (1024 steps of order 2048): a part's chain on two SMs while there
-  // are two for each (2.7 ms), on one while there is one (3.8), beyond that the
-  // three parts of a query and half per block (10.2, the constants kept once).  Other lengths,
-  // or a-parts with a zero query slot: one part and factor per block in
+  // are two for each (2.1 ms), on one while there is one (3.75), beyond that the
+  // three parts of a query and half per block (10.2, the constants kept once).
+  // Other lengths, or a-parts with a zero query slot: one part and factor per block in
   // two-block clusters while the chunk needs at most one block per SM, then one
   // block per part carrying both factors.  `clustered` asks for the cluster
   // form at any chunk size (its blocks share SMs with a running scan; the

@@ -182,7 +182,7 @@ int dnspir_fleet_tune_cuda_cores(dnspir_fleet* fleet, uint32_t batch, double* ms
  * group's secondary phase, 1 it waits for all of that phase, 2 it waits until
  * that phase starts its last chunk; plus 4: its secondary chains run as
  * two-block clusters (one RNS factor per block) at every chunk size instead of
- * one block per part beyond one wave.  -1 returns to the default (0).  Either
+ * one block per chain, or per query and half, where a chain has no two SMs.  -1 returns to the default (0).  Either
  * engine.  No counterpart in the reference. */
 int dnspir_fleet_set_schedule(dnspir_fleet* fleet, uint32_t batch, int schedule);
 /* The schedule in force for groups of `batch` queries, in the encoding of
@@ -286,7 +286,8 @@ int dnspir_fleet_batch_timings(dnspir_fleet* fleet, uint32_t max, double* latenc
 /* Launch on a caller-owned cudaStream_t (NULL restores the fleet's own stream). */
 int dnspir_fleet_set_stream(dnspir_fleet* fleet, void* cuda_stream);
 /* Kernels the fleet's answer pipeline has launched so far (counted at each
- * launch: decode, query operand and scan, epilogue, and per secondary chunk the
+ * launch: decode, query vectors, query operand and scan, the epilogue -- at
+ * N = 2048 part of the encoder's first kernel -- and per secondary chunk the
  * encoder's three kernels, the chains and the replies).  No counterpart in the
  * reference. */
 int dnspir_fleet_launch_count(dnspir_fleet* fleet, uint64_t* count);
