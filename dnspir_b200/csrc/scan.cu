@@ -338,7 +338,7 @@ __global__ void primary_epilogue_kernel(const uint32_t* __restrict__ fin, int ns
 // (v 2^13 + q < 2^64 for v < q).  LN = 1: one lane per block, for so few shards
 // and queries that the blocks do not fill the SMs.  Bound by shared memory and
 // barriers (three blocks an SM).  Against digits through global memory and a kernel
-// for their columns (256 queries of 128 shards): 2.95 + 2.03 -> 4.25 ms, and the
+// for their columns (256 queries of 64 shards): 2.95 + 2.03 -> 4.25 ms, and the
 // digits' buffer is not needed.
 constexpr int EPI_NT = 512;
 
