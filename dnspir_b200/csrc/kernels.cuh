@@ -3,15 +3,33 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "ntt.cuh"
 
 namespace dnspir {
 
 // Raises a kernel's dynamic shared-memory limit when a launch needs more than
-// the default 48 KB (the attribute is per function and per device).
+// the default 48 KB.  The limit is one value per function and device and is
+// only ever raised: kernels launched with several sizes are launched from
+// several host threads (fleets, shards, the server), and a thread that set its
+// smaller size between another's call and launch would have that launch refused.
+inline void raise_smem_limit(const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limits;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& limit = limits[{dev, kernel}];
+  if (bytes > limit &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+    limit = bytes;
+}
 template <class K>
 inline void set_smem(K* kernel, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 48 * 1024) raise_smem_limit((const void*)kernel, bytes);
 }
 
 // Shape of one PIR database (IndexGroup, base_pir.rs:132-183).
