@@ -97,6 +97,8 @@ def lib():
         L.dnspir_fleet_tune_pipeline.argtypes = [_vp, c.c_uint32, _vp, _vp]
         L.dnspir_fleet_tune_cuda_cores.argtypes = [_vp, c.c_uint32, _vp, _vp]
         L.dnspir_fleet_set_wait_limit.argtypes = [_vp, c.c_uint64, c.c_int]
+        L.dnspir_fleet_withhold_chain_step.argtypes = [_vp, c.c_int]
+        L.dnspir_db_set_wait_limit.argtypes = [_vp, c.c_uint64, c.c_int]
         L.dnspir_server_create.argtypes = [c.c_int, c.c_uint32, c.POINTER(_vp)]
         L.dnspir_server_add_db.argtypes = [_vp, _vp, c.c_uint32, _u32p]
         L.dnspir_server_start.argtypes = [_vp, c.c_int]
@@ -269,6 +271,11 @@ class PIRDatabase:
         else:
             e = np.ascontiguousarray(entries, dtype=np.uint16)
             _check(lib().dnspir_db_set_db(self._h, _ptr(e), e.size, 0))
+
+    def set_wait_limit(self, wait_ns=0, withhold_step=-1):
+        """Limit of the paired preprocessing chains' waits (0: default 2 s);
+        withhold_step >= 0 is their timeout test hook."""
+        _check(lib().dnspir_db_set_wait_limit(self._h, wait_ns, withhold_step))
 
     def get_a(self):
         out = np.zeros((8, self.n), dtype=np.uint64)
@@ -443,9 +450,14 @@ class Fleet:
         return s.value
 
     def set_wait_limit(self, wait_ns=0, withhold_chunk=-1):
-        """Tensor engine: limit of the scan's pipeline waits (0: default 2 s);
-        withhold_chunk >= 0 is the timeout path's test hook."""
+        """Limit of the waits inside the tensor scan and the paired chains (0:
+        default 2 s); withhold_chunk >= 0 is the scan's timeout test hook."""
         _check(lib().dnspir_fleet_set_wait_limit(self._h, wait_ns, withhold_chunk))
+
+    def withhold_chain_step(self, step=-1):
+        """Timeout test hook of the paired chains: the second block of the
+        first chain leaves before that step (-1: off)."""
+        _check(lib().dnspir_fleet_withhold_chain_step(self._h, step))
 
     def set_engine(self, engine):
         """ENGINE_CUDA_CORES or ENGINE_TENSOR; marks every shard unprepared."""

@@ -393,7 +393,7 @@ uint32_t preprocess_batch(const Group& g) {
 
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
                       const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, uint32_t* err,
-                      cudaStream_t st, uint32_t* last) {
+                      const WaitLimits& lim, cudaStream_t st, uint32_t* last) {
   const size_t per_shard = (size_t)SIMD * g.l * g.n;
   const SlotMaps maps = slot_maps(c, g.log2n);
   const ChainConsts cc = chain_consts(c, g.log2n, used_seeds);
@@ -411,7 +411,7 @@ int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* co
       launch_encode_lift(rows, rows, g, SIMD, 1, maps, c->T, st);
     }
     uint32_t* const rows = ws.rows.as<uint32_t>();
-    launch_primary_chain_rows(rows, rows + words, stride, count, a_out, err, g, cc, c->T, st);
+    launch_primary_chain_rows(rows, rows + words, stride, count, a_out, err, lim, g, cc, c->T, st);
     launch_primary_finalize(a_out, count, a_zq, a_ms, g, c->T, st);
     if (last) {
       launch_order_rows(rows, count * stride, maps, st);
@@ -465,6 +465,7 @@ struct dnspir_db {
   uint32_t* slab = nullptr;
   DBuf a_zq, a_ms, qz, qlane, qv, sum, out;
   DBuf err;  // wait-error word of the preprocessing chains
+  WaitLimits limits;
   HBuf pin;  // host staging of perform_pir_split: query elements in, reply out
   EncodeWs ws;
   std::mutex mu;
@@ -622,6 +623,15 @@ int dnspir_db_create(int device, uint32_t log2_n, uint32_t group_order, int used
   return DNSPIR_OK;
 }
 
+int dnspir_db_set_wait_limit(dnspir_db* db, uint64_t wait_ns, int withhold_step) {
+  if (!db) return fail(DNSPIR_ERR_BAD_ARG, "null database");
+  if (withhold_step < -1) return fail(DNSPIR_ERR_BAD_ARG, "withhold_step must be -1 or a step index");
+  std::lock_guard<std::mutex> lk(db->mu);
+  db->limits.wait_ns = wait_ns;
+  db->limits.withhold_step = withhold_step;
+  return DNSPIR_OK;
+}
+
 int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int entries_on_device) {
   if (!db || !entries) return fail(DNSPIR_ERR_BAD_ARG, "null argument");
   std::lock_guard<std::mutex> lk(db->mu);
@@ -651,7 +661,7 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   }
   uint32_t* slabs[1] = {db->slab};
   CKR(preprocess_shards(db->ctx, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
-                        db->a_ms.as<uint32_t>(), db->ws, db->err.as<uint32_t>(), db->st));
+                        db->a_ms.as<uint32_t>(), db->ws, db->err.as<uint32_t>(), db->limits, db->st));
   CKR(db->pin.ensure(4));
   CK(cudaMemcpyAsync(db->pin.p, db->err.p, 4, cudaMemcpyDeviceToHost, db->st));
   CK(cudaStreamSynchronize(db->st));

@@ -243,7 +243,11 @@ struct ChainArgs {
   // primary: slabs and a-part output
   uint32_t* const* slabs;
   uint32_t* a_out;
-  uint32_t* err;  // set to 1 when a wait for the peer block gives up
+  // paired chains: error word, set to 1 when a wait for the peer block gives up;
+  // limit of that wait; step that the first chain's second block leaves before (~0u: none)
+  uint32_t* err;
+  uint64_t wait_ns;
+  uint32_t withhold;
   uint32_t c_first, cinv_first, inv5;
 };
 
@@ -1138,39 +1142,86 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // shared twiddles are constants of its code.
 // As pairs the inbox fills by st.async, which counts its bytes on the
 // receiver's mbarrier: no barrier of the cluster and no fence in a step.  A wait
-// is bounded; when it gives up the block raises the error word, stops waiting and
-// runs to its end on what it has.
+// is bounded.  When it gives up, which the threads of a block do together or not at
+// all, the block raises the error word and ends there: it arms and sends no more,
+// so the peer's next wait runs out too.  That path never comes back, which keeps
+// it out of the steps' code: one query's 1024 steps as long as without it (2.64 ms the
+// call), a shard's 0.9 % longer; with a way out of the loop, a guard around the
+// sends or a flag asked in each step they took 1 to 5 % longer.
 constexpr uint64_t PEER_WAIT_NS = 2000000000ull;
 // The states a and b^ are kept apart from the transforms' work space and
 // transposed, position 8 t + m at word 256 m + t: sigma_5 maps a warp's
 // positions of one m to 32 positions whose t differ mod 32, so its gathers have
 // no bank conflict (three-way in the padded order), and the first pass may
 // write its work space without waiting for them.
-constexpr int few_words(int kc) {  // of one factor: work space, a, b^ (secondary), inbox[2], constants, two mbarriers
-  return n2k::PS + (kc > 3 ? 4 : 3) * N_MAX + kc * 2 * 256 * 4 + 4;
+constexpr int few_words(int kc) {  // of one factor: work space, a, b^ (secondary), inbox[2], constants, two
+                                   // mbarriers, the peer's steps (12 bytes spare)
+  return n2k::PS + (kc > 3 ? 4 : 3) * N_MAX + kc * 2 * 256 * 4 + 8;
 }
 __device__ __forceinline__ uint32_t state_word(uint32_t pos) { return ((pos & 7) << 8) | (pos >> 3); }
 
-// Waits for the phase of `parity` of a barrier that the peer block's copies
-// complete; false after PEER_WAIT_NS.
-__device__ __forceinline__ bool wait_peer(uint32_t bar, uint32_t parity) {
-  auto done = [&] {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
-        "p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-  };
-  if (done()) return true;
+__device__ __forceinline__ bool peer_done(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
+      "p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same until limit_ns have passed (and one look after them: the thread may
+// have been held up between the last one and the clock).
+__device__ __forceinline__ bool peer_done_within(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
   uint64_t t0, t1;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (;;) {
-    if (done()) return true;
+  do {
+    if (peer_done(bar, parity)) return true;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-    if (t1 - t0 > PEER_WAIT_NS) return false;
+  } while (t1 - t0 <= limit_ns);
+  return peer_done(bar, parity);
+}
+// Waits, in all 256 threads of a block, for the phase of `parity` of a barrier
+// that the peer block's copies complete; false in all of them or in none.  A thread
+// whose time is up makes the phase wait for one byte more: if the phase was still
+// open then, it now stays open for the others too; if it had just completed, the
+// byte went to the next phase, which cannot have begun to complete while this
+// thread is here, and is taken back.
+__device__ __forceinline__ bool wait_peer(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
+#pragma unroll 1
+  for (int k = 0; k < 64; k++)
+    if (peer_done(bar, parity)) return true;
+  if (peer_done_within(bar, parity, limit_ns)) return true;
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+  if (!peer_done(bar, parity)) return false;
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+  return true;
+}
+// Expects the peer's values of one step (256 threads, 32 bytes each).
+__device__ __forceinline__ void arm_inbox(uint32_t bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(256 * 32) : "memory");
+}
+constexpr uint32_t PEER_SENT = 16;  // byte offset of the peer's number of steps sent from the barriers
+// End of a paired chain, for all threads of the block: neither block leaves while
+// the peer may still write into it.  `waited` steps' values have come, `sent` are
+// armed and sent (one more when a wait has given up).  Stores of st.async are not
+// ordered by the cluster barrier, so a block that leaves early waits, bounded again,
+// for those that its peer had sent besides (at most two steps': a block sends step
+// i + 2 only after the peer's step i + 1 has come).
+__device__ __noinline__ void leave_pair(uint32_t bars, uint32_t peer_bars, uint32_t waited, uint32_t sent, uint32_t L,
+                                        int t, uint64_t limit_ns) {
+  if (t == 0 && sent < L)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_bars + PEER_SENT), "r"(sent) : "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  if (t != 0) return;
+  if (sent > waited)  // the bytes of the threads' waits that gave up
+    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], 256;" ::"r"(bars + (waited & 1) * 8) : "memory");
+  uint32_t peer_sent;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(peer_sent) : "r"(bars + PEER_SENT) : "memory");
+  for (uint32_t j = waited; j < peer_sent; j++) {
+    const uint32_t bar = bars + (j & 1) * 8;
+    if (j >= sent) arm_inbox(bar);
+    peer_done_within(bar, (j >> 1) & 1, limit_ns);
   }
 }
 
@@ -1228,14 +1279,15 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   uint32_t peer = (uint32_t)__cvta_generic_to_shared(PAIR ? X : sm + (1 - F) * WORDS + XO);
   if constexpr (PAIR) asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(peer) : "r"(1 - F));
   // PAIR: one mbarrier per parity, behind the constants; its phase i / 2 ends with
-  // the peer's 8 KiB of step i
+  // the peer's 8 KiB of step i.  The steps that the peer has sent lie behind them.
   const uint32_t bars = (uint32_t)__cvta_generic_to_shared(KC + NKC * 2 * 256);
   const uint32_t peer_bars = peer + (bars - (uint32_t)__cvta_generic_to_shared(X));
-  bool alive = true;
+  const uint32_t steps = PAIR && F == 1 && blockIdx.x < 2 && blockIdx.y == 0 ? min(a.g.L, a.withhold) : a.g.L;
   if (PAIR && t == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tmbarrier.init.shared::cta.b64 [%0 + 8], 1;\n\t"
                  "fence.mbarrier_init.release.cluster;" ::"r"(bars)
                  : "memory");
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(bars + PEER_SENT), "r"(a.g.L) : "memory");
   }
   sync_both();  // both run, both inboxes are free and the barriers exist
   const size_t lanes = SEC ? (size_t)a.nl : SIMD;
@@ -1263,7 +1315,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
 #pragma unroll
     for (int k = 0; k < 8; k++) y[k * Gm::STR] = v[k];
   };
-  for (uint32_t i = 0; i < a.g.L; i++) {
+  for (uint32_t i = 0; i < steps; i++) {
     const size_t row = first + (size_t)(a.g.L - 1 - i) * lanes * N;
     uint32_t ta[8], tb[8];
 #pragma unroll
@@ -1310,11 +1362,12 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
               "r"(v[4 * h4]), "r"(v[4 * h4 + 1]), "r"(v[4 * h4 + 2]), "r"(v[4 * h4 + 3]), "r"(peer_bars + bo)
               : "memory");
         // (copies may land before this: the count may run below zero meanwhile)
-        if (t == 0)
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + bo), "r"(256 * 32) : "memory");
-        if (alive && !wait_peer(bars + bo, (i >> 1) & 1)) {
-          alive = false;
-          if (a.err) atomicOr(a.err, 1u);
+        if (t == 0) arm_inbox(bars + bo);
+        if (!wait_peer(bars + bo, (i >> 1) & 1, a.wait_ns)) {
+          if (t == 0) atomicOr(a.err, 1u);
+          leave_pair(bars, peer_bars, i, i + 1, a.g.L, t, a.wait_ns);
+          asm volatile("exit;");
+          __builtin_unreachable();
         }
       } else {
 #pragma unroll
@@ -1382,7 +1435,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
     }
     sync();
   }
-  if constexpr (PAIR) sync_both();  // neither block leaves while the peer may still write into it
+  if constexpr (PAIR) leave_pair(bars, peer_bars, steps, steps, a.g.L, t, a.wait_ns);
   constexpr uint64_t mu = barrett_mu(p);
   const uint32_t kinv = a.cp[F].kinv;
 #pragma unroll 1
@@ -1583,6 +1636,12 @@ static ChainArgs chain_args(const Group& g, const ChainConsts& cc, const NttTabl
   return a;
 }
 
+static void set_limits(ChainArgs& a, uint32_t* err, const WaitLimits& lim) {
+  a.err = err;
+  a.wait_ns = lim.wait_ns ? lim.wait_ns : PEER_WAIT_NS;
+  a.withhold = lim.withhold_step < 0 ? ~0u : (uint32_t)lim.withhold_step;
+}
+
 static size_t chain_smem(const Group& g, int secondary_parts) {
   return (size_t)(secondary_parts ? sec_smem_words(secondary_parts) : 12) * g.n * 4;
 }
@@ -1607,11 +1666,11 @@ int chain_rows_supported(const Group& g) { return g.log2n == LOG2_N_MAX && g.na 
 size_t chain_rows_words(const Group& g) { return (size_t)2 * g.H * g.L * SIMD * g.n; }
 
 void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
-                               uint32_t* err, const Group& g, const ChainConsts& cc, const NttTables& T,
-                               cudaStream_t st) {
+                               uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
+                               const NttTables& T, cudaStream_t st) {
   ChainArgs a = chain_args(g, cc, T);
   a.a_out = a_out;
-  a.err = err;
+  set_limits(a, err, lim);
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1661,10 +1720,10 @@ int secondary_chain_wave(const Group& g, int sms) {
 }
 
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            uint32_t* err, const Group& g, const ChainConsts& cc, const ScanConsts* sc,
-                            const NttTables& T, cudaStream_t st, bool clustered) {
+                            uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
+                            const ScanConsts* sc, const NttTables& T, cudaStream_t st, bool clustered) {
   ChainArgs a = chain_args(g, cc, T);
-  a.err = err;
+  set_limits(a, err, lim);
   a.E = E;
   a.qv = qv;
   a.qv_stride = qv_stride;

@@ -274,8 +274,8 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     launch_encode_rows(A, E, g2, l_in, nl, f->ctx->T, st);
     launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
-                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), f->err_word.as<uint32_t>(), g2, cc,
-                           two ? &sc : nullptr, f->ctx->T, st, clustered);
+                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), f->err_word.as<uint32_t>(), f->limits,
+                           g2, cc, two ? &sc : nullptr, f->ctx->T, st, clustered);
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);
@@ -479,7 +479,7 @@ int dnspir_fleet_tune(dnspir_fleet* f, uint32_t batch, double* ms_per_shape, int
         cudaEventRecord(e0, f->st);
         ok = launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, qv.as<uint32_t>(), nb, pad, qb.as<uint8_t>(),
                           out.as<uint32_t>(), f->err_word.as<uint32_t>(), f->last.as<uint32_t>(),
-                          f->distinct_dev.as<int>(), g1, sh[i], f->st, TScanLimits(), f->tmaps.p) == 0;
+                          f->distinct_dev.as<int>(), g1, sh[i], f->st, WaitLimits(), f->tmaps.p) == 0;
         cudaEventRecord(e1, f->st);
         if (ok && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) {
           if (r > 0) tot += t;  // the first run warms up
@@ -761,6 +761,15 @@ int dnspir_fleet_set_wait_limit(dnspir_fleet* f, uint64_t wait_ns, int withhold_
   return DNSPIR_OK;
 }
 
+int dnspir_fleet_withhold_chain_step(dnspir_fleet* f, int step) {
+  if (!f) return fail(DNSPIR_ERR_BAD_ARG, "null fleet");
+  std::lock_guard<std::mutex> lk(f->mu);
+  NOT_SERVING(f);
+  if (step < -1) return fail(DNSPIR_ERR_BAD_ARG, "step must be -1 or a step index");
+  f->limits.withhold_step = step;
+  return DNSPIR_OK;
+}
+
 int dnspir_tscan_shapes(int* nq, int* mtpc, int* stages, int* persistent, int max) {
   int count = 0;
   const TScanShape* sh = tscan_shapes(&count);
@@ -822,12 +831,13 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
       CKR(f->tmp_lane.ensure((size_t)cnt * words * 4));
       std::vector<uint32_t*> tmp(cnt);
       for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
-      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws, f->err_word.as<uint32_t>(), f->st, last));
+      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws,
+                            f->err_word.as<uint32_t>(), f->limits, f->st, last));
       for (uint32_t i = 0; i < cnt; i++)
         launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d0 + i]), f->g1, f->st);
     } else {
       CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws,
-                            f->err_word.as<uint32_t>(), f->st, last));
+                            f->err_word.as<uint32_t>(), f->limits, f->st, last));
     }
   }
   CK(cudaGetLastError());

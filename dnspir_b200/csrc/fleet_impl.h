@@ -61,7 +61,7 @@ struct dnspir_fleet {
   bool one_group = false;                     // the call in progress is one group (default tile shape)
   dnspir::DBuf qb, tmp_lane;                  // tensor engine: query operand, preprocessing scratch
   dnspir::DBuf err_word;                      // set by a kernel whose bounded wait gave up
-  dnspir::TScanLimits limits;                 // tensor engine: wait limit (and the timeout-test hook)
+  dnspir::WaitLimits limits;                  // of every bounded wait, with the timeout tests' hooks
   std::map<int, int> tuned;                   // tensor engine: group size -> tile shape index
   std::map<int, int> tuned_cc;                // CUDA-core engine: group size -> queries per block
   std::map<int, int> tuned_chain;             // group size -> 1: two-block-cluster chains at every chunk size

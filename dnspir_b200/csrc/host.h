@@ -135,7 +135,7 @@ bool reduced(const uint64_t* v, size_t n);
 // looks at err (launch_primary_chain_rows).
 int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
                       const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, uint32_t* err,
-                      cudaStream_t st, uint32_t* last = nullptr);
+                      const WaitLimits& lim, cudaStream_t st, uint32_t* last = nullptr);
 // Shards that one call of preprocess_shards may carry.
 uint32_t preprocess_batch(const Group& g);
 

@@ -93,6 +93,16 @@ __host__ __device__ __forceinline__ size_t scan_vec_off(uint32_t n, int h, int v
 void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk, int nb, int nb_pad, uint32_t* qv,
                          const Group& g, const ScanConsts& sc, const SlotMaps& maps, cudaStream_t st);
 
+// Limits of the bounded waits inside kernels, wait_ns (0: the default, 2 s), and
+// the test hooks of the paths they end in (-1: off): the tensor scan's first
+// block stops copying before chunk `withhold`, the second block of the first
+// paired chain leaves before step `withhold_step`.
+struct WaitLimits {
+  uint64_t wait_ns = 0;
+  int withhold = -1;
+  int withhold_step = -1;
+};
+
 // ---- DB encoding (set_transformed_entries, base_pir.rs:662-772)
 // in: coefficients [t < l_in][lane < nl][n < N] (< t); A: [t][lane][x] (q1, transform
 // position x = slot brv(x))
@@ -128,8 +138,8 @@ void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_o
 int chain_rows_supported(const Group& g);
 size_t chain_rows_words(const Group& g);
 void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_words, int nshards, uint32_t* a_out,
-                               uint32_t* err, const Group& g, const ChainConsts& cc, const NttTables& T,
-                               cudaStream_t st);
+                               uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
+                               const NttTables& T, cudaStream_t st);
 // Rows of `words` words in all: bit-reversed positions -> (sign, e) order, in place.
 void launch_order_rows(uint32_t* rows, size_t words, const SlotMaps& maps, cudaStream_t st);
 // One shard's rows and digits (bit-reversed positions) -> its lane-layout slab.
@@ -151,8 +161,8 @@ void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq,
 // sc: scan_consts of the secondary's a-part set, or null when one of its query
 // slots is zero.
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
-                            uint32_t* err, const Group& g, const ChainConsts& cc, const ScanConsts* sc,
-                            const NttTables& T, cudaStream_t st, bool clustered = false);
+                            uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
+                            const ScanConsts* sc, const NttTables& T, cudaStream_t st, bool clustered = false);
 // Queries whose chains fill the SMs once.
 int secondary_chain_wave(const Group& g, int sms);
 
@@ -182,13 +192,6 @@ void launch_retile_rows(const uint32_t* rows, const uint32_t* digits, uint8_t* t
                         cudaStream_t st);
 const TScanShape* tscan_shapes(int* count);
 size_t tscan_query_bytes(const Group& g, int nb_pad);
-// Limits of the tensor scan's pipeline waits: wait_ns (0: the default, 2 s)
-// and, for tests of the timeout path, a chunk that CTA 0's producer never
-// copies (withhold >= 0), so that its MMA thread's wait runs out.
-struct TScanLimits {
-  uint64_t wait_ns = 0;
-  int withhold = -1;
-};
 // nb queries (qv: launch_scan_vectors) padded to nb_pad (a multiple of
 // shape.nq / 4); qb: tscan_query_bytes of workspace; out as
 // launch_scan_batch; err: one device word set to 1 when a bounded wait gave
@@ -199,7 +202,7 @@ struct TScanLimits {
 // tensor-map pair shapes (persistent 3), which are refused (-1) without it.
 int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int nb, int nb_pad, uint8_t* qb,
                  uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
-                 const TScanShape& shape, cudaStream_t st, const TScanLimits& lim = TScanLimits(),
+                 const TScanShape& shape, cudaStream_t st, const WaitLimits& lim = WaitLimits(),
                  const void* slab_maps = nullptr);
 // A shard's chain state after its last row times 2^32, [p][u][half][lane] (na =
 // 2), from its a_out (launch_primary_chain).

@@ -1311,7 +1311,7 @@ size_t tscan_slab_map_bytes(int nshards) { return (size_t)nshards * sizeof(CUten
 
 int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int nb, int nb_pad, uint8_t* qb,
                  uint32_t* out, uint32_t* err, const uint32_t* last, const int* distinct_of, const Group& g,
-                 const TScanShape& shape, cudaStream_t st, const TScanLimits& lim, const void* slab_maps) {
+                 const TScanShape& shape, cudaStream_t st, const WaitLimits& lim, const void* slab_maps) {
   uint32_t mt, kc;
   tensor_dims(g, &mt, &kc);
   const int qpc = shape.nq / 4;

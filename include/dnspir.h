@@ -89,6 +89,11 @@ int dnspir_db_create(int device, uint32_t log2_n, uint32_t group_order, int used
 /* PIRDatabase::set_db (base_pir.rs:632): count must equal 8 * group_order * N
  * coefficients; entries_on_device != 0 if `entries` is a device pointer. */
 int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int entries_on_device);
+/* Limit of the waits between the two blocks of a paired chain in set_db
+ * (wait_ns; 0 restores the default of 2 s), which then fails with
+ * DNSPIR_ERR_TIMEOUT, and the test hook of that path: withhold_step as in
+ * dnspir_fleet_withhold_chain_step.  No counterpart in the reference. */
+int dnspir_db_set_wait_limit(dnspir_db* db, uint64_t wait_ns, int withhold_step);
 /* PIRDatabase::get_a (base_pir.rs:897): out = 8 x N coefficients */
 int dnspir_db_get_a(dnspir_db* db, uint64_t* out);
 /* PIRDatabase::perform_pir_split (base_pir.rs:958): lane k answers query k.
@@ -193,15 +198,21 @@ int dnspir_fleet_get_schedule(dnspir_fleet* fleet, uint32_t batch, int* schedule
  * groups of `batch` queries, overriding the table or a previous tune; -1
  * returns to the default.  No counterpart in the reference. */
 int dnspir_fleet_set_tile(dnspir_fleet* fleet, uint32_t batch, int shape_index);
-/* Tensor engine: limit of every wait in the scan's copy/MMA/epilogue pipeline
- * (wait_ns; 0 restores the default of 2 s).  A wait that runs out makes the
- * scan's blocks stop, wait (bounded) for their copies in flight, free their
+/* Limit of every wait between threads of a kernel that is not a hardware barrier
+ * (wait_ns; 0 restores the default of 2 s): in the tensor scan's
+ * copy/MMA/epilogue pipeline, and between the two blocks of a paired chain in
+ * the secondary phase and in set_shards.  A wait that runs out makes the
+ * blocks stop, wait (bounded) for their copies in flight, free their
  * tensor memory and return; the call then fails with DNSPIR_ERR_TIMEOUT and
  * the device stays usable.  withhold_chunk >= 0 is a test hook for that path:
  * the first block's producer stops before copying that chunk, so the block's
  * MMA thread waits for a copy that never comes (-1: off).  No counterpart in
  * the reference. */
 int dnspir_fleet_set_wait_limit(dnspir_fleet* fleet, uint64_t wait_ns, int withhold_chunk);
+/* The same test hook for the paired chains: the second block of the first chain
+ * leaves before that step, so the first waits for values that never come (-1:
+ * off).  No counterpart in the reference. */
+int dnspir_fleet_withhold_chain_step(dnspir_fleet* fleet, int step);
 /* The tensor scan's tile shapes (query-operand rows per CTA, m-tiles per CTA,
  * pipeline stages, kernel: 0 one tile per CTA, 1 persistent warp-specialised,
  * 2 CTA pair with relayed bulk copies, 3 CTA pair with tensor-map copies);
