@@ -98,6 +98,7 @@ def lib():
         L.dnspir_fleet_tune_cuda_cores.argtypes = [_vp, c.c_uint32, _vp, _vp]
         L.dnspir_fleet_set_wait_limit.argtypes = [_vp, c.c_uint64, c.c_int]
         L.dnspir_fleet_withhold_chain_step.argtypes = [_vp, c.c_int]
+        L.dnspir_fleet_withhold_group_size.argtypes = [_vp, c.c_uint32]
         L.dnspir_db_set_wait_limit.argtypes = [_vp, c.c_uint64, c.c_int]
         L.dnspir_server_create.argtypes = [c.c_int, c.c_uint32, c.POINTER(_vp)]
         L.dnspir_server_add_db.argtypes = [_vp, _vp, c.c_uint32, _u32p]
@@ -458,6 +459,10 @@ class Fleet:
         """Timeout test hook of the paired chains: the second block of the
         first chain leaves before that step (-1: off)."""
         _check(lib().dnspir_fleet_withhold_chain_step(self._h, step))
+
+    def withhold_group_size(self, queries=0):
+        """Both hooks act in groups of that many queries only (0: in all)."""
+        _check(lib().dnspir_fleet_withhold_group_size(self._h, queries))
 
     def set_engine(self, engine):
         """ENGINE_CUDA_CORES or ENGINE_TENSOR; marks every shard unprepared."""

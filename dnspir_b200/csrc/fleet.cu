@@ -35,6 +35,7 @@ namespace {
 
 const size_t SEC_BUDGET = (size_t)8 << 30;  // secondary workspace of one chunk
 const int TENSOR_MAX_BATCH = 256;
+const size_t ERR_BYTES = 2 * 4;  // error words of the two slots
 
 #define NOT_SERVING(f) \
   if ((f)->serving) return fail(DNSPIR_ERR_BAD_ARG, "the fleet is attached to a running server")
@@ -113,14 +114,14 @@ int slot_acquire(dnspir_fleet* f, QSlot& s) {
 int fleet_drain(dnspir_fleet* f) {
   for (auto& s : f->slot)
     if (s.sec_pending) CK(cudaStreamWaitEvent(f->st, s.sec_done, 0));
-  // the error word comes with the same wait
-  CKR(f->epin.ensure(4));
-  CK(cudaMemcpyAsync(f->epin.p, f->err_word.p, 4, cudaMemcpyDeviceToHost, f->st));
+  // the error words come with the same wait
+  CKR(f->epin.ensure(ERR_BYTES));
+  CK(cudaMemcpyAsync(f->epin.p, f->err_words.p, ERR_BYTES, cudaMemcpyDeviceToHost, f->st));
   CK(cudaStreamSynchronize(f->st));
   CK(cudaStreamSynchronize(f->sec));
   for (auto& s : f->slot) s.sec_pending = false;
-  if (*f->epin.as<uint32_t>()) {
-    CK(cudaMemset(f->err_word.p, 0, 4));
+  if (f->epin.as<uint32_t>()[0] | f->epin.as<uint32_t>()[1]) {
+    CK(cudaMemset(f->err_words.p, 0, ERR_BYTES));
     return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
   }
   return DNSPIR_OK;
@@ -137,8 +138,8 @@ int launch_scan(dnspir_fleet* f, QSlot& s, int nb, int Bk) {
     const TScanShape& shape = tensor_shape(f, nb, &nb_pad);
     if (nb_pad != Bk) return fail(DNSPIR_ERR_BAD_ARG, "tensor scan batch mismatch");
     if (launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, s.qv.as<uint32_t>(), nb, Bk, f->qb.as<uint8_t>(),
-                     s.fin.as<uint32_t>(), f->err_word.as<uint32_t>(), f->last.as<uint32_t>(),
-                     f->distinct_dev.as<int>(), g1, shape, f->st, f->limits, f->tmaps.p))
+                     s.fin.as<uint32_t>(), slot_err(f, s), f->last.as<uint32_t>(), f->distinct_dev.as<int>(), g1,
+                     shape, f->st, f->limits.of_group(nb), f->tmaps.p))
       return fail(DNSPIR_ERR_BAD_ARG, "tensor scan shape does not fit");
     f->launches += 2;  // query operand + scan
     return DNSPIR_OK;
@@ -274,8 +275,8 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     launch_encode_rows(A, E, g2, l_in, nl, f->ctx->T, st);
     launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
-                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), f->err_word.as<uint32_t>(), f->limits,
-                           g2, cc, two ? &sc : nullptr, f->ctx->T, st, clustered);
+                           QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), slot_err(f, s),
+                           f->limits.of_group(nb), g2, cc, two ? &sc : nullptr, f->ctx->T, st, clustered);
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);
@@ -390,8 +391,8 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   for (uint32_t s = 0; s < num_shards; s++) dist[s] = (int)(s % num_distinct);
   CKR(f->distinct_dev.ensure(num_shards * sizeof(int)));
   CK(cudaMemcpy(f->distinct_dev.p, dist.data(), num_shards * sizeof(int), cudaMemcpyHostToDevice));
-  CKR(f->err_word.ensure(4));
-  CK(cudaMemset(f->err_word.p, 0, 4));
+  CKR(f->err_words.ensure(ERR_BYTES));
+  CK(cudaMemset(f->err_words.p, 0, ERR_BYTES));
   CKR(allocate_slabs(f.get()));
   CKR(f->a_zq.ensure((size_t)num_distinct * SIMD * f->g1.n * 8));
   CKR(f->a_ms.ensure((size_t)num_distinct * SIMD * f->g1.n * 4));
@@ -478,7 +479,7 @@ int dnspir_fleet_tune(dnspir_fleet* f, uint32_t batch, double* ms_per_shape, int
       for (int r = 0; r < 3 && ok; r++) {
         cudaEventRecord(e0, f->st);
         ok = launch_tscan(f->slabs_dev.as<uint8_t*>(), f->S, qv.as<uint32_t>(), nb, pad, qb.as<uint8_t>(),
-                          out.as<uint32_t>(), f->err_word.as<uint32_t>(), f->last.as<uint32_t>(),
+                          out.as<uint32_t>(), f->err_words.as<uint32_t>(), f->last.as<uint32_t>(),
                           f->distinct_dev.as<int>(), g1, sh[i], f->st, WaitLimits(), f->tmaps.p) == 0;
         cudaEventRecord(e1, f->st);
         if (ok && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&t, e0, e1) == cudaSuccess) {
@@ -500,9 +501,9 @@ int dnspir_fleet_tune(dnspir_fleet* f, uint32_t batch, double* ms_per_shape, int
   cudaEventDestroy(e1);
   CK(cudaStreamSynchronize(f->st));
   uint32_t e = 0;
-  CK(cudaMemcpy(&e, f->err_word.p, 4, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(&e, f->err_words.p, 4, cudaMemcpyDeviceToHost));
   if (e) {
-    CK(cudaMemset(f->err_word.p, 0, 4));
+    CK(cudaMemset(f->err_words.p, 0, 4));
     return fail(DNSPIR_ERR_TIMEOUT, "tensor scan: a pipeline wait gave up");
   }
   if (best_i < 0) return fail(DNSPIR_ERR_CUDA, "no tile shape ran");
@@ -761,6 +762,14 @@ int dnspir_fleet_set_wait_limit(dnspir_fleet* f, uint64_t wait_ns, int withhold_
   return DNSPIR_OK;
 }
 
+int dnspir_fleet_withhold_group_size(dnspir_fleet* f, uint32_t queries) {
+  if (!f) return fail(DNSPIR_ERR_BAD_ARG, "null fleet");
+  std::lock_guard<std::mutex> lk(f->mu);
+  NOT_SERVING(f);
+  f->limits.only_group = (int)queries;
+  return DNSPIR_OK;
+}
+
 int dnspir_fleet_withhold_chain_step(dnspir_fleet* f, int step) {
   if (!f) return fail(DNSPIR_ERR_BAD_ARG, "null fleet");
   std::lock_guard<std::mutex> lk(f->mu);
@@ -832,12 +841,12 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
       std::vector<uint32_t*> tmp(cnt);
       for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
       CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws,
-                            f->err_word.as<uint32_t>(), f->limits, f->st, last));
+                            f->err_words.as<uint32_t>(), f->limits, f->st, last));
       for (uint32_t i = 0; i < cnt; i++)
         launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d0 + i]), f->g1, f->st);
     } else {
       CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws,
-                            f->err_word.as<uint32_t>(), f->limits, f->st, last));
+                            f->err_words.as<uint32_t>(), f->limits, f->st, last));
     }
   }
   CK(cudaGetLastError());

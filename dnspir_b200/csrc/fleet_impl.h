@@ -13,6 +13,7 @@ namespace dnspir {
 struct QSlot {
   DBuf qbytes, qdesc, qnat, qbrv, qv, fin, sec_in, reply_dev;
   HBuf qpin, dpin, rpin;  // host staging: query bytes, descriptors, reply bytes
+  HBuf epin;              // the slot's error word (served groups)
   cudaEvent_t prim_done = nullptr, sec_done = nullptr;
   cudaEvent_t sec_tail = nullptr;  // the secondary phase has reached its last chunk
   bool sec_pending = false, prim_recorded = false;
@@ -53,14 +54,14 @@ struct dnspir_fleet {
   dnspir::QSlot slot[2];
   dnspir::DBuf secE, chain_out, qzq, reply_zq;  // used by one stream at a time
   dnspir::HBuf rpin;                            // host staging of the replies of one call
-  dnspir::HBuf zpin, epin;                      // host staging of perform_double_pir's elements, of the error word
+  dnspir::HBuf zpin, epin;                      // host staging of perform_double_pir's elements, of the error words
   int batch = 1;
   int sec_chunk = 1;  // queries per secondary launch sequence
   int engine = DNSPIR_ENGINE_CUDA_CORES;
   bool serving = false;                       // attached to a running server
   bool one_group = false;                     // the call in progress is one group (default tile shape)
   dnspir::DBuf qb, tmp_lane;                  // tensor engine: query operand, preprocessing scratch
-  dnspir::DBuf err_word;                      // set by a kernel whose bounded wait gave up
+  dnspir::DBuf err_words;                     // one per slot, set by a kernel of its group whose bounded wait gave up
   dnspir::WaitLimits limits;                  // of every bounded wait, with the timeout tests' hooks
   std::map<int, int> tuned;                   // tensor engine: group size -> tile shape index
   std::map<int, int> tuned_cc;                // CUDA-core engine: group size -> queries per block
@@ -87,6 +88,9 @@ int fleet_ready(dnspir_fleet* f);
 // Workspace of a slot for groups of up to nb queries (kernel batch Bk) and
 // qbytes of query bytes.
 int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbytes);
+// The slot's error word: two groups are in flight at once, and only the one
+// whose kernel gave up has failed.
+inline uint32_t* slot_err(dnspir_fleet* f, const QSlot& s) { return f->err_words.as<uint32_t>() + (&s - f->slot); }
 // Secondary workspace for groups of up to nb queries.
 int fleet_secondary_workspace(dnspir_fleet* f, int nb);
 // Primary kernels of a group on f->st: decode (bytes and descriptors already

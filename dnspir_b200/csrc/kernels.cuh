@@ -96,11 +96,18 @@ void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk
 // Limits of the bounded waits inside kernels, wait_ns (0: the default, 2 s), and
 // the test hooks of the paths they end in (-1: off): the tensor scan's first
 // block stops copying before chunk `withhold`, the second block of the first
-// paired chain leaves before step `withhold_step`.
+// paired chain leaves before step `withhold_step`, in groups of `only_group`
+// queries (0: in all).
 struct WaitLimits {
   uint64_t wait_ns = 0;
   int withhold = -1;
   int withhold_step = -1;
+  int only_group = 0;
+  WaitLimits of_group(int nb) const {
+    WaitLimits l = *this;
+    if (only_group && only_group != nb) l.withhold = l.withhold_step = -1;
+    return l;
+  }
 };
 
 // ---- DB encoding (set_transformed_entries, base_pir.rs:662-772)

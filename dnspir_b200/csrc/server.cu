@@ -138,6 +138,7 @@ int presize(Db& db) {
     CKR(s.qpin.ensure((size_t)nb * full_query_bytes(f)));
     CKR(s.reply_dev.ensure((size_t)nb * RB));
     CKR(s.rpin.ensure((size_t)nb * RB));
+    CKR(s.epin.ensure(4));
   }
   CKR(fleet_secondary_workspace(f, nb));
   return DNSPIR_OK;
@@ -192,6 +193,7 @@ int launch_group(dnspir_server* sv, Db& db, int k, const std::vector<Request*>& 
     CK(cudaStreamWaitEvent(f->sec, s.prim_done, 0));
     CKR(fleet_secondary_kernels(f, s, nb, s.reply_dev.as<uint8_t>(), RB, nullptr, s.rpin.as<uint8_t>()));
   }
+  CK(cudaMemcpyAsync(s.epin.p, slot_err(f, s), 4, cudaMemcpyDeviceToHost, f->sec));
   CK(cudaEventRecord(s.sec_done, f->sec));
   db.groups++;
   if (sv->use_graphs && !graphs) {
@@ -264,12 +266,9 @@ void worker_main(dnspir_server* sv) {
         if (e != cudaSuccess) {
           cudaGetLastError();
           status = DNSPIR_ERR_CUDA;
-        } else {
-          uint32_t w = 0;
-          if (cudaMemcpy(&w, db.f->err_word.p, 4, cudaMemcpyDeviceToHost) != cudaSuccess || w) {
-            cudaMemset(db.f->err_word.p, 0, 4);
-            status = DNSPIR_ERR_TIMEOUT;
-          }
+        } else if (*db.f->slot[k].epin.as<uint32_t>()) {
+          status = DNSPIR_ERR_TIMEOUT;
+          cudaMemsetAsync(slot_err(db.f, db.f->slot[k]), 0, 4, db.f->st);  // before the slot's next group
         }
         finish_group(sv, db, k, status);
         progress = true;
@@ -316,6 +315,7 @@ void worker_main(dnspir_server* sv) {
         cudaGetLastError();
         cudaStreamSynchronize(db.f->st);
         cudaStreamSynchronize(db.f->sec);
+        cudaMemsetAsync(slot_err(db.f, db.f->slot[k]), 0, 4, db.f->st);
         finish_group(sv, db, k, r);
       }
       progress = true;

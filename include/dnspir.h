@@ -213,6 +213,9 @@ int dnspir_fleet_set_wait_limit(dnspir_fleet* fleet, uint64_t wait_ns, int withh
  * leaves before that step, so the first waits for values that never come (-1:
  * off).  No counterpart in the reference. */
 int dnspir_fleet_withhold_chain_step(dnspir_fleet* fleet, int step);
+/* Both hooks act in groups of that many queries only (0: in all groups).  No
+ * counterpart in the reference. */
+int dnspir_fleet_withhold_group_size(dnspir_fleet* fleet, uint32_t queries);
 /* The tensor scan's tile shapes (query-operand rows per CTA, m-tiles per CTA,
  * pipeline stages, kernel: 0 one tile per CTA, 1 persistent warp-specialised,
  * 2 CTA pair with relayed bulk copies, 3 CTA pair with tensor-map copies);
