@@ -272,42 +272,38 @@ static int build_scan_consts(const uint32_t* consts_dev, int log2n, uint32_t** o
   return DNSPIR_OK;
 }
 
-// a-parts and the sigma_5 position map for ring dimension 2^log2n
-// a-parts in NTT form for the a-parts now in effect (rebuilt after
-// dnspir_set_a_parts; earlier buffers are kept, a kernel queued before the
-// change may still read them)
-static int ctx_a_parts(DeviceCtx* c, int log2n, uint64_t* version) {
+// Constants of the a-parts now in effect for ring dimension 2^log2n (rebuilt
+// after dnspir_set_a_parts; earlier buffers are kept, shards preprocessed under
+// them still refer to them).
+static int ctx_a_parts(DeviceCtx* c, int log2n, APartConsts* ap) {
   const uint32_t n = 1u << log2n;
+  APartConsts& now = c->ap[log2n];
   uint64_t ver = a_parts_version(log2n);
-  if (version) *version = ver;
-  if (c->consts[log2n] && c->consts_ver[log2n] == ver) return DNSPIR_OK;
-  std::vector<uint64_t> ap(6 * (size_t)n);
-  a_parts_host(log2n, ap.data(), &ver);
-  if (version) *version = ver;
-  uint64_t* dz = nullptr;
-  uint32_t* dc = nullptr;
-  CK(cudaMalloc(&dz, ap.size() * 8));
-  CK(cudaMalloc(&dc, (size_t)6 * 2 * n * 4));
-  CK(cudaMemcpy(dz, ap.data(), ap.size() * 8, cudaMemcpyHostToDevice));
-  launch_ring_to_ntt(dz, 6, nullptr, dc, log2n, c->T, 0);
-  CK(cudaGetLastError());
-  CK(cudaDeviceSynchronize());
-  CK(cudaFree(dz));
-  uint32_t* ds = nullptr;
-  uint32_t na[2];
-  CKR(build_scan_consts(dc, log2n, &ds, na));
-  if (c->consts[log2n]) c->retired.push_back(c->consts[log2n]);
-  if (c->scan[log2n]) c->retired.push_back(c->scan[log2n]);
-  c->scan[log2n] = ds;
-  c->scan_na[log2n][0] = na[0], c->scan_na[log2n][1] = na[1];
-  c->consts[log2n] = dc;
-  c->consts_ver[log2n] = ver;
+  if (!now.ntt || now.version != ver) {
+    std::vector<uint64_t> parts(6 * (size_t)n);
+    a_parts_host(log2n, parts.data(), &ver);
+    uint64_t* dz = nullptr;
+    uint32_t *dc = nullptr, *ds = nullptr;
+    CK(cudaMalloc(&dz, parts.size() * 8));
+    CK(cudaMalloc(&dc, (size_t)6 * 2 * n * 4));
+    CK(cudaMemcpy(dz, parts.data(), parts.size() * 8, cudaMemcpyHostToDevice));
+    launch_ring_to_ntt(dz, 6, nullptr, dc, log2n, c->T, 0);
+    CK(cudaGetLastError());
+    CK(cudaDeviceSynchronize());
+    CK(cudaFree(dz));
+    APartConsts next;
+    CKR(build_scan_consts(dc, log2n, &ds, next.na));
+    next.version = ver, next.ntt = dc, next.scan = ds;
+    now = next;
+  }
+  *ap = now;
   return DNSPIR_OK;
 }
 
-int ctx_consts(DeviceCtx* c, int log2n, uint64_t* version) {
+// The same, with the tables of the dimension (sigma_5 and the slot orders), made once.
+int ctx_consts(DeviceCtx* c, int log2n, APartConsts* ap) {
   std::lock_guard<std::mutex> lk(c->mu);
-  if (c->galb[log2n]) return ctx_a_parts(c, log2n, version);
+  if (c->galb[log2n]) return ctx_a_parts(c, log2n, ap);
   const uint32_t n = 1u << log2n;
   uint32_t* dg = nullptr;
   CK(cudaMalloc(&dg, (size_t)n * 4));
@@ -344,7 +340,7 @@ int ctx_consts(DeviceCtx* c, int log2n, uint64_t* version) {
   device_pow5(log2n, false);
   device_pow5(log2n, true);
   c->galb[log2n] = dg;
-  return ctx_a_parts(c, log2n, version);
+  return ctx_a_parts(c, log2n, ap);
 }
 
 SlotMaps slot_maps(DeviceCtx* c, int log2n) {
@@ -354,26 +350,25 @@ SlotMaps slot_maps(DeviceCtx* c, int log2n) {
   return m;
 }
 
-ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds) {
+ChainConsts chain_consts(DeviceCtx* c, const APartConsts& ap, int log2n, int used_seeds) {
   const size_t n2 = (size_t)2 << log2n;
   ChainConsts cc;
-  cc.gka = c->consts[log2n];
-  cc.qa = c->consts[log2n] + (2 + 2 * used_seeds) * n2;
+  cc.gka = ap.ntt;
+  cc.qa = ap.ntt + (2 + 2 * used_seeds) * n2;
   cc.galb = c->galb[log2n];
   cc.maps = slot_maps(c, log2n);
   return cc;
 }
 
-ScanConsts scan_consts(DeviceCtx* c, const Group& g, int used_seeds) {
+ScanConsts scan_consts(const APartConsts& ap, const Group& g, int used_seeds) {
   const size_t n2 = (size_t)2 << g.log2n;
   ScanConsts sc;
-  sc.gka0 = c->scan[g.log2n];
-  sc.kappa = c->scan[g.log2n] + n2;
-  sc.qinv = c->scan[g.log2n] + (2 + 2 * used_seeds) * n2;
+  sc.gka0 = ap.scan;
+  sc.kappa = ap.scan + n2;
+  sc.qinv = ap.scan + (2 + 2 * used_seeds) * n2;
   for (int p = 0; p < 2; p++) chain_state_scale(g, p, &sc.xscale[p], &sc.xinv[p]);
   return sc;
 }
-uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds) { return c->scan_na[log2n][used_seeds]; }
 
 int check_group(uint32_t log2n, uint32_t l) {
   if (log2n < 3 || log2n > LOG2_N_MAX) return fail(DNSPIR_ERR_BAD_SHAPE, "log2_n must be in [3, 11]");
@@ -391,12 +386,12 @@ uint32_t preprocess_batch(const Group& g) {
   return (uint32_t)std::max<size_t>(1, ROWS_BUDGET / (2 * chain_rows_words(g) * 4));
 }
 
-int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
-                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, uint32_t* err,
-                      const WaitLimits& lim, cudaStream_t st, uint32_t* last) {
+int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int used_seeds, uint32_t* const* slabs_host,
+                      int count, const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws,
+                      uint32_t* err, const WaitLimits& lim, cudaStream_t st, uint32_t* last) {
   const size_t per_shard = (size_t)SIMD * g.l * g.n;
   const SlotMaps maps = slot_maps(c, g.log2n);
-  const ChainConsts cc = chain_consts(c, g.log2n, used_seeds);
+  const ChainConsts cc = chain_consts(c, ap, g.log2n, used_seeds);
   const size_t a_out_words = (size_t)g.H * SIMD * 2 * g.n;
   CKR(ws.a_out.ensure(count * a_out_words * 4));
   uint32_t* const a_out = ws.a_out.as<uint32_t>();
@@ -417,7 +412,7 @@ int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* co
       launch_order_rows(rows, count * stride, maps, st);
       for (int s = 0; s < count; s++) {
         launch_retile_rows(rows + s * stride, rows + s * stride + words, reinterpret_cast<uint8_t*>(slabs_host[s]), g, st);
-        launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(c, g, used_seeds), maps, st);
+        launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(ap, g, used_seeds), maps, st);
       }
     } else {
       for (int s = 0; s < count; s++)
@@ -439,7 +434,7 @@ int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* co
   launch_primary_finalize(a_out, count, a_zq, a_ms, g, c->T, st);
   if (last && g.na == 2)
     for (int s = 0; s < count; s++)
-      launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(c, g, used_seeds), maps, st);
+      launch_last_rows(a_out + s * a_out_words, last + s * last_rows_words(g), g, scan_consts(ap, g, used_seeds), maps, st);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(st));  // slabs_host is the caller's
   return DNSPIR_OK;
@@ -459,7 +454,7 @@ struct dnspir_db {
   Group g;
   int used_seeds = 0;
   bool ready = false;
-  uint64_t ap_ver = 0;  // a-parts version the slab was preprocessed under
+  APartConsts ap;  // a-parts the slab was preprocessed under
   cudaStream_t st = nullptr;
   cudaEvent_t noalloc_done = nullptr;  // recorded on the caller's stream after each no-allocation call
   uint32_t* slab = nullptr;
@@ -481,7 +476,7 @@ int noalloc_reserve(int device);  // noalloc.cu
 
 static int db_ready(const dnspir_db* db) {
   if (!db->ready) return fail(DNSPIR_ERR_NOT_READY, "database not preprocessed");
-  if (db->ap_ver != a_parts_version(db->g.log2n))
+  if (db->ap.version != a_parts_version(db->g.log2n))
     return fail(DNSPIR_ERR_NOT_READY, "the a-parts changed since the database was preprocessed: call set_db again");
   return DNSPIR_OK;
 }
@@ -502,7 +497,7 @@ int db_noalloc_begin(dnspir_db* db, DbView* out) {
   out->slab = db->slab;
   out->T = db->ctx->T;
   out->maps = slot_maps(db->ctx, db->g.log2n);
-  out->sc = scan_consts(db->ctx, db->g, db->used_seeds);
+  out->sc = scan_consts(db->ap, db->g, db->used_seeds);
   return DNSPIR_OK;
 }
 int db_noalloc_end(dnspir_db* db, cudaStream_t st) {
@@ -603,11 +598,11 @@ int dnspir_db_create(int device, uint32_t log2_n, uint32_t group_order, int used
   DeviceCtx* c = nullptr;
   CKR(get_ctx(device, &c));
   DeviceGuard dg(device);
-  CKR(ctx_consts(c, log2_n));
   std::unique_ptr<dnspir_db> d(new dnspir_db());
+  CKR(ctx_consts(c, log2_n, &d->ap));
   d->device = device;
   d->ctx = c;
-  d->g = make_group(log2_n, group_order, scan_arrays(c, log2_n, used_seeds));
+  d->g = make_group(log2_n, group_order, d->ap.na[used_seeds]);
   d->used_seeds = used_seeds;
   CK(cudaStreamCreateWithFlags(&d->st, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&d->noalloc_done, cudaEventDisableTiming));
@@ -647,9 +642,8 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   db->ready = false;
   // a no-allocation call queued on another stream may still read the slab
   CK(cudaStreamWaitEvent(db->st, db->noalloc_done, 0));
-  uint64_t ver = 0;
-  CKR(ctx_consts(db->ctx, db->g.log2n, &ver));
-  const uint32_t na = scan_arrays(db->ctx, db->g.log2n, db->used_seeds);
+  CKR(ctx_consts(db->ctx, db->g.log2n, &db->ap));
+  const uint32_t na = db->ap.na[db->used_seeds];
   if (na != db->g.na || !db->slab) {
     // a-parts installed since the shard was made need the other slab layout
     CK(cudaStreamSynchronize(db->st));
@@ -660,7 +654,7 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
     CK(cudaMalloc(&db->slab, slab_words(db->g) * 4));
   }
   uint32_t* slabs[1] = {db->slab};
-  CKR(preprocess_shards(db->ctx, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
+  CKR(preprocess_shards(db->ctx, db->ap, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
                         db->a_ms.as<uint32_t>(), db->ws, db->err.as<uint32_t>(), db->limits, db->st));
   CKR(db->pin.ensure(4));
   CK(cudaMemcpyAsync(db->pin.p, db->err.p, 4, cudaMemcpyDeviceToHost, db->st));
@@ -669,7 +663,6 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
     CK(cudaMemset(db->err.p, 0, 4));
     return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
   }
-  db->ap_ver = ver;
   db->ready = true;
   return DNSPIR_OK;
 }
@@ -714,7 +707,7 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
   launch_ring_to_ntt(db->qz.as<uint64_t>(), SIMD * 4, db->qlane.as<uint32_t>(), nullptr, g.log2n, db->ctx->T, db->st);
   const SlotMaps maps = slot_maps(db->ctx, g.log2n);
   launch_scan_vectors(db->qlane.as<uint32_t>(), 8 * n, 0, 2, SIMD, SIMD, db->qv.as<uint32_t>(), g,
-                      scan_consts(db->ctx, g, db->used_seeds), maps, db->st);
+                      scan_consts(db->ap, g, db->used_seeds), maps, db->st);
   if (launch_scan_lanes(db->slab, db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g, db->st))
     return fail(DNSPIR_ERR_CUDA, "cannot clear the scan's sums");
   launch_epilogue_zq(db->sum.as<uint32_t>(), db->out.as<uint64_t>(), g, maps, db->ctx->T, db->st);

@@ -131,7 +131,7 @@ int fleet_drain(dnspir_fleet* f) {
 int launch_scan(dnspir_fleet* f, QSlot& s, int nb, int Bk) {
   const Group& g1 = f->g1;
   launch_scan_vectors(s.qnat.as<uint32_t>(), QV_WORDS_PER_QUERY * g1.n, 2, 0, nb, Bk, s.qv.as<uint32_t>(), g1,
-                      scan_consts(f->ctx, g1, 0), slot_maps(f->ctx, g1.log2n), f->st);
+                      scan_consts(f->ap, g1, 0), slot_maps(f->ctx, g1.log2n), f->st);
   f->launches += 1;
   if (f->engine == DNSPIR_ENGINE_TENSOR) {
     int nb_pad = 0;
@@ -160,7 +160,7 @@ namespace dnspir {
 int fleet_ready(dnspir_fleet* f) {
   for (uint32_t d = 0; d < f->D; d++)
     if (!f->ready[d]) return fail(DNSPIR_ERR_NOT_READY, "fleet shard not preprocessed");
-  if (f->ap_ver != a_parts_version(f->g1.log2n))
+  if (f->ap.version != a_parts_version(f->g1.log2n))
     return fail(DNSPIR_ERR_NOT_READY, "the a-parts changed since the shards were preprocessed: set the shards again");
   return DNSPIR_OK;
 }
@@ -254,9 +254,9 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     f->launches += 1;
   }
   const SlotMaps maps = slot_maps(f->ctx, g2.log2n);
-  const ChainConsts cc = chain_consts(f->ctx, g2.log2n, 1);
-  const ScanConsts sc = scan_consts(f->ctx, g2, 1);
-  const bool two = scan_arrays(f->ctx, g2.log2n, 1) == 2;
+  const ChainConsts cc = chain_consts(f->ctx, f->ap, g2.log2n, 1);
+  const ScanConsts sc = scan_consts(f->ap, g2, 1);
+  const bool two = f->ap.na[1] == 2;
   const auto tc = f->tuned_chain.find(nb);
   const bool clustered = tc != f->tuned_chain.end() && tc->second;
   for (int c0 = 0; c0 < nb; c0 += f->sec_chunk) {
@@ -346,13 +346,11 @@ int dnspir_fleet_create_general(int device, uint32_t log2_n, uint32_t primary_or
   DeviceCtx* c = nullptr;
   CKR(get_ctx(device, &c));
   DeviceGuard dg(device);
-  uint64_t ap_ver = 0;
-  CKR(ctx_consts(c, log2_n, &ap_ver));
   std::unique_ptr<dnspir_fleet> f(new dnspir_fleet());
-  f->ap_ver = ap_ver;
+  CKR(ctx_consts(c, log2_n, &f->ap));
   f->device = device;
   f->ctx = c;
-  f->g1 = make_group(log2_n, primary_order, scan_arrays(c, log2_n, 0));
+  f->g1 = make_group(log2_n, primary_order, f->ap.na[0]);
   f->g2 = make_group(log2_n, secondary_order);
   f->S = num_shards;
   f->D = num_distinct;
@@ -800,12 +798,11 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   DeviceGuard dg(f->device);
   {
     // shards preprocessed under other a-parts cannot be mixed with these
-    uint64_t ver = 0;
-    CKR(ctx_consts(f->ctx, f->g1.log2n, &ver));
-    if (ver != f->ap_ver)
+    const uint64_t before = f->ap.version;
+    CKR(ctx_consts(f->ctx, f->g1.log2n, &f->ap));
+    if (f->ap.version != before)
       for (uint32_t d = 0; d < f->D; d++) f->ready[d] = false;
-    f->ap_ver = ver;
-    const uint32_t na = scan_arrays(f->ctx, f->g1.log2n, 0);
+    const uint32_t na = f->ap.na[0];
     if (na != f->g1.na || !f->slabs[f->D - 1]) {
       // these a-parts need the other slab layout (slab_off): new slabs
       CK(cudaStreamSynchronize(f->st));
@@ -840,12 +837,12 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
       CKR(f->tmp_lane.ensure((size_t)cnt * words * 4));
       std::vector<uint32_t*> tmp(cnt);
       for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
-      CKR(preprocess_shards(f->ctx, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws,
+      CKR(preprocess_shards(f->ctx, f->ap, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws,
                             f->err_words.as<uint32_t>(), f->limits, f->st, last));
       for (uint32_t i = 0; i < cnt; i++)
         launch_retile(tmp[i], reinterpret_cast<uint8_t*>(f->slabs[d0 + i]), f->g1, f->st);
     } else {
-      CKR(preprocess_shards(f->ctx, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws,
+      CKR(preprocess_shards(f->ctx, f->ap, f->g1, 0, &f->slabs[d0], (int)cnt, src, a_zq, a_ms, f->ws,
                             f->err_words.as<uint32_t>(), f->limits, f->st, last));
     }
   }

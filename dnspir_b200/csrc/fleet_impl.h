@@ -46,7 +46,7 @@ struct dnspir_fleet {
   cudaStream_t own = nullptr, st = nullptr, sec = nullptr;
   std::vector<uint32_t*> slabs;
   std::vector<bool> ready;
-  uint64_t ap_ver = 0;  // a-parts version every ready shard was preprocessed under
+  dnspir::APartConsts ap;  // a-parts every ready shard was preprocessed under
   dnspir::DBuf slabs_dev, distinct_dev, a_zq, a_ms;
   dnspir::DBuf last;  // tensor engine: each distinct shard's chain state after its last row (launch_last_rows)
   dnspir::DBuf tmaps;  // tensor maps of the slabs (CTA-pair tensor-map scan); empty when unavailable

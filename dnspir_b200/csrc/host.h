@@ -30,15 +30,22 @@ int fail(int code, const std::string& msg);
     if (r_ != DNSPIR_OK) return r_; \
   } while (0)
 
+// Constants of one set of a-parts on a device.  A shard or fleet keeps those that
+// it was preprocessed under: dnspir_set_a_parts and the preprocessing of another
+// shard may replace the context's at any time, in another thread as well.  The
+// buffers live as long as the context.
+struct APartConsts {
+  uint64_t version = 0;
+  const uint32_t* ntt = nullptr;   // a-parts in NTT form: [6][2][N], bit-reversed positions
+  const uint32_t* scan = nullptr;  // scan constants: gka0, kappa, then qinv of each a-part set (ScanConsts)
+  uint32_t na[2] = {};             // arrays per slab row of each a-part set: 2, or 3 when qry_a has a zero slot (slab_off)
+};
+
 struct DeviceCtx {
   int device = -1;
   uint32_t* tables = nullptr;
   NttTables T;
-  uint32_t* consts[LOG2_N_MAX + 1] = {};  // a-parts in NTT form: [6][2][N], bit-reversed positions
-  uint64_t consts_ver[LOG2_N_MAX + 1] = {};  // a-parts version they were built from
-  std::vector<uint32_t*> retired;            // a-part buffers replaced by dnspir_set_a_parts
-  uint32_t* scan[LOG2_N_MAX + 1] = {};       // scan constants: gka0, kappa, then qinv of each a-part set (ScanConsts)
-  uint32_t scan_na[LOG2_N_MAX + 1][2] = {};  // arrays per slab row of each a-part set: 2, or 3 when qry_a has a zero slot
+  APartConsts ap[LOG2_N_MAX + 1];  // of the a-parts last in effect
   uint32_t* galb[LOG2_N_MAX + 1] = {};
   uint32_t* gtab[LOG2_N_MAX + 1] = {};  // scan slot order: position -> odd residue
   uint32_t* uof[LOG2_N_MAX + 1] = {};   // natural slot -> position
@@ -113,19 +120,16 @@ struct DeviceGuard {
 };
 
 int get_ctx(int device, DeviceCtx** out);
-// Per-dimension constants of a device; also brings the a-parts in NTT form up
-// to the a-parts now in effect, whose version goes to *version.
-int ctx_consts(DeviceCtx* c, int log2n, uint64_t* version = nullptr);
+// Per-dimension constants of a device, and those of the a-parts now in effect.
+int ctx_consts(DeviceCtx* c, int log2n, APartConsts* ap);
 // The six a-parts in effect for dimension 2^log2n (6 x N coefficients in
 // [0, q): gk0, gk1, FirstSet query, its conjugate, SecondSet query, its
 // conjugate) and their version.
 void a_parts_host(int log2n, uint64_t* out, uint64_t* version);
 uint64_t a_parts_version(int log2n);
 SlotMaps slot_maps(DeviceCtx* c, int log2n);
-ChainConsts chain_consts(DeviceCtx* c, int log2n, int used_seeds);
-ScanConsts scan_consts(DeviceCtx* c, const Group& g, int used_seeds);
-// Arrays per slab row of shards preprocessed under the context's a-parts (slab_off).
-uint32_t scan_arrays(DeviceCtx* c, int log2n, int used_seeds);
+ChainConsts chain_consts(DeviceCtx* c, const APartConsts& ap, int log2n, int used_seeds);
+ScanConsts scan_consts(const APartConsts& ap, const Group& g, int used_seeds);
 int check_group(uint32_t log2n, uint32_t l);
 bool reduced(const uint64_t* v, size_t n);
 // Encodes `count` shards' entries (device u16, one shard after another), runs
@@ -133,9 +137,9 @@ bool reduced(const uint64_t* v, size_t n);
 // lane layout, or tensor layout with `last` rows when last is given (tensor
 // engine, chain_rows_supported).  Queued on st; the caller synchronises and
 // looks at err (launch_primary_chain_rows).
-int preprocess_shards(DeviceCtx* c, const Group& g, int used_seeds, uint32_t* const* slabs_host, int count,
-                      const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws, uint32_t* err,
-                      const WaitLimits& lim, cudaStream_t st, uint32_t* last = nullptr);
+int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int used_seeds, uint32_t* const* slabs_host,
+                      int count, const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws,
+                      uint32_t* err, const WaitLimits& lim, cudaStream_t st, uint32_t* last = nullptr);
 // Shards that one call of preprocess_shards may carry.
 uint32_t preprocess_batch(const Group& g);
 
