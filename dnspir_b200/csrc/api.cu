@@ -381,9 +381,15 @@ int check_group(uint32_t log2n, uint32_t l) {
 
 const size_t ROWS_BUDGET = (size_t)13 << 28;  // chain layout of the shards in flight (3.25 GiB)
 
+static size_t rows_bytes(const Group& g) { return 2 * chain_rows_words(g) * 4; }  // of one shard
+
 uint32_t preprocess_batch(const Group& g) {
   if (!chain_rows_supported(g)) return 16;
-  return (uint32_t)std::max<size_t>(1, ROWS_BUDGET / (2 * chain_rows_words(g) * 4));
+  return (uint32_t)std::max<size_t>(1, ROWS_BUDGET / rows_bytes(g));
+}
+
+int preprocess_reserve(const Group& g, uint32_t count, EncodeWs& ws) {
+  return chain_rows_supported(g) ? ws.rows.ensure(count * rows_bytes(g)) : DNSPIR_OK;
 }
 
 int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int used_seeds, uint32_t* const* slabs_host,
@@ -397,7 +403,7 @@ int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int u
   uint32_t* const a_out = ws.a_out.as<uint32_t>();
   if (chain_rows_supported(g)) {
     const size_t words = chain_rows_words(g), stride = 2 * words;
-    CKR(ws.rows.ensure(count * stride * 4));
+    CKR(preprocess_reserve(g, count, ws));
     for (int s = 0; s < count; s++) {
       // the columns' transforms use the digits' space, the orbit values factor 0's rows
       uint32_t *rows = ws.rows.as<uint32_t>() + s * stride, *digits = rows + words;

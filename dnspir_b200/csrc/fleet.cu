@@ -820,13 +820,24 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   const size_t words = slab_words(f->g1), last_words = last_rows_words(f->g1);
   // without chain rows the tensor engine preprocesses into lane-layout scratch
   // and re-tiles from there, four shards at a time
-  const uint32_t batch = tensor && !rows ? 4 : preprocess_batch(f->g1);
+  uint32_t batch = std::min(count, tensor && !rows ? 4 : preprocess_batch(f->g1));
+  auto reserve = [&] {
+    if (!entries_on_device) CKR(f->ws.in16.ensure((size_t)batch * per * 2));
+    if (tensor && !rows) CKR(f->tmp_lane.ensure((size_t)batch * words * 4));
+    return preprocess_reserve(f->g1, batch, f->ws);
+  };
+  for (;;) {
+    const int r = reserve();
+    if (r == DNSPIR_OK) break;
+    // fewer shards at a time where device memory is short
+    if (r != DNSPIR_ERR_OOM || batch <= 1) return r;
+    batch = (batch + 1) / 2;
+  }
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = false;
   for (uint32_t b0 = 0; b0 < count; b0 += batch) {
     const uint32_t cnt = std::min(count - b0, batch), d0 = first + b0;
     const uint16_t* src = entries + (size_t)b0 * per;
     if (!entries_on_device) {
-      CKR(f->ws.in16.ensure((size_t)cnt * per * 2));
       CK(cudaMemcpyAsync(f->ws.in16.p, src, (size_t)cnt * per * 2, cudaMemcpyHostToDevice, f->st));
       src = f->ws.in16.as<uint16_t>();
     }
@@ -834,7 +845,6 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
     uint32_t* const a_ms = f->a_ms.as<uint32_t>() + d0 * n8;
     uint32_t* const last = tensor && f->g1.na == 2 ? f->last.as<uint32_t>() + d0 * last_words : nullptr;
     if (tensor && !rows) {
-      CKR(f->tmp_lane.ensure((size_t)cnt * words * 4));
       std::vector<uint32_t*> tmp(cnt);
       for (uint32_t i = 0; i < cnt; i++) tmp[i] = f->tmp_lane.as<uint32_t>() + i * words;
       CKR(preprocess_shards(f->ctx, f->ap, f->g1, 0, tmp.data(), (int)cnt, src, a_zq, a_ms, f->ws,
@@ -849,9 +859,10 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   CK(cudaGetLastError());
   CKR(fleet_drain(f));
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = true;
-  // the scratch of a bulk load goes back; an update of a few shards keeps its own
+  // the scratch of a bulk load goes back; an update of a few shards (four
+  // half-size, two full) keeps its own
   f->tmp_lane.release();
-  if (count > batch) f->ws.rows.release();
+  if (f->ws.rows.bytes > EncodeWs::ROWS_KEPT) f->ws.rows.release();
   return DNSPIR_OK;
 }
 

@@ -106,6 +106,7 @@ struct HBuf {
 struct EncodeWs {
   DBuf A, Ahat, in16, a_out, slab_ptrs;
   DBuf rows;  // chain layout of the shards in flight: entries, then states | digits (chain_rows_supported)
+  static constexpr size_t ROWS_KEPT = (size_t)1 << 30;  // at most this much of it outlives a fleet's call
 };
 
 struct DeviceGuard {
@@ -140,7 +141,8 @@ bool reduced(const uint64_t* v, size_t n);
 int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int used_seeds, uint32_t* const* slabs_host,
                       int count, const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws,
                       uint32_t* err, const WaitLimits& lim, cudaStream_t st, uint32_t* last = nullptr);
-// Shards that one call of preprocess_shards may carry.
+// Shards that one call of preprocess_shards may carry, and its scratch for `count`.
 uint32_t preprocess_batch(const Group& g);
+int preprocess_reserve(const Group& g, uint32_t count, EncodeWs& ws);
 
 }  // namespace dnspir
