@@ -741,8 +741,9 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
 //     b^' = sigma_5(b^) + t (C + sigma_5(r)) + n1 V
 // (t = sigma_5(a), n1 = NTT(d1), ka1 = gk_a1 - 2^26 gk_a0, C = gk_b0 - gk_a0 r,
 // V = gk_b1 - 2^26 gk_b0 - ka1 r): five products and five constants a position
-// instead of six; b = b^ + r a once at the end.  Needs every slot of qry_a
-// invertible (launch_secondary_chain).
+// instead of six; b = b^ + r a once at the end.  Where qry_a is zero, r is taken as
+// 0 and the slot's b^' keeps its entry, E qry_b: a-parts with such slots (ZEROS) have
+// a sixth constant, qry_b there and zero elsewhere.
 //
 // The state is carried as k a, k the factor's CRT constant: a global scale that
 // the constants absorb (ka1 and qa times k, C + sigma_5(r) over k), so that the
@@ -761,8 +762,8 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
 // Shared memory: per part A[2], B[2] (padded polynomials; A is also the
 // transforms' work space), then the five constants (Montgomery form) as
 // [j][factor][quad half][thread] 16-byte vectors.
-constexpr int SEC2K_KC = 5;
-constexpr int SEC2K_WORDS = CTXT_PARTS * 4 * n2k::PS + SEC2K_KC * 2 * 2 * 256 * 4;
+constexpr int sec_consts(bool zeros) { return zeros ? 6 : 5; }
+constexpr int sec2k_words(bool zeros) { return CTXT_PARTS * 4 * n2k::PS + sec_consts(zeros) * 2 * 2 * 256 * 4; }
 
 // T R^-1 mod p, below T / 2^32 + p (T < 2^62)
 __device__ __forceinline__ uint32_t mont_lazy(uint64_t T, uint32_t p, uint32_t pinv) {
@@ -909,7 +910,9 @@ __device__ __forceinline__ void state_constants(const ChainArgs& a, int h, int f
   for (int j = 0; j < 3; j++) k[j] = mont_reduce((uint64_t)c[j] * cp.r2, cp.p, cp.pinv);
 }
 
-// the same, then (C + sigma_5(r)) / k and V; from: the position sigma_5 brings here
+// the same, then (C + sigma_5(r)) / k and V (and qry_b where qry_a is zero, for
+// ZEROS); from: the position sigma_5 brings here
+template <bool ZEROS>
 __device__ __forceinline__ void secondary_constants(const ChainArgs& a, const ScanConsts& sc, int h, int q, int f,
                                                     uint32_t pos, uint32_t from, uint32_t* k) {
   state_constants(a, h, f, pos, k);
@@ -925,11 +928,17 @@ __device__ __forceinline__ void secondary_constants(const ChainArgs& a, const Sc
   const uint32_t V = sub_mod(sub_mod(gb1, mul_mod(gb0, c26, cp.p, mu), cp.p), mul_mod(ka1, r, cp.p, mu), cp.p);
   k[3] = mont_reduce((uint64_t)mul_mod(add_mod(C, r5, cp.p), cp.kinv, cp.p, mu) * cp.r2, cp.p, cp.pinv);
   k[4] = mont_reduce((uint64_t)V * cp.r2, cp.p, cp.pinv);
+  if constexpr (ZEROS) {
+    const uint32_t qb = __ldg(qq + ((size_t)(4 + h) * 2 + f) * N_MAX + pos);
+    k[5] = __ldg(a.qa + (size_t)h * 2 * N_MAX + o) ? 0 : mont_reduce((uint64_t)qb * cp.r2, cp.p, cp.pinv);
+  }
 }
 
+template <bool ZEROS>
 __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(ChainArgs a, ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
   using namespace n2k;
+  constexpr int NKC = sec_consts(ZEROS);
   constexpr int PARTS = CTXT_PARTS, NT = 256 * PARTS;
   const int h = blockIdx.x, q = blockIdx.y;
   const int part = threadIdx.x >> 8, t = threadIdx.x & 255;
@@ -959,13 +968,13 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
       const int it = threadIdx.x + c * NT;
       if (it < 2 * N) {
         const int f = it / N, pos = it & (N - 1);
-        uint32_t k[SEC2K_KC];
+        uint32_t k[NKC];
         uint32_t src_pos = from[0];
 #pragma unroll
         for (int x = 1; x < PER; x++) src_pos = c == x ? from[x] : src_pos;
-        secondary_constants(a, sc, h, q, f, pos, src_pos, k);
+        secondary_constants<ZEROS>(a, sc, h, q, f, pos, src_pos, k);
 #pragma unroll
-        for (int j = 0; j < SEC2K_KC; j++)
+        for (int j = 0; j < NKC; j++)
           reinterpret_cast<uint32_t*>(KC)[(((j * 2 + f) * 2 + (pos >> 2 & 1)) * 256 + (pos >> 3)) * 4 + (pos & 3)] = k[j];
       }
     }
@@ -999,9 +1008,9 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
         const uint4 v = last_stages(A, f, h4, t, qb, a.T);
         const uint32_t n1[4] = {v.x, v.y, v.z, v.w};
         const uint32_t es[4] = {e[f][h4].x, e[f][h4].y, e[f][h4].z, e[f][h4].w};
-        uint32_t kc[SEC2K_KC][4], an[4], b4[4];
+        uint32_t kc[NKC][4], an[4], b4[4];
 #pragma unroll
-        for (int j = 0; j < SEC2K_KC; j++) {
+        for (int j = 0; j < NKC; j++) {
           const uint4 c = KC[((j * 2 + f) * 2 + h4) * 256 + t];
           kc[j][0] = c.x, kc[j][1] = c.y, kc[j][2] = c.z, kc[j][3] = c.w;
         }
@@ -1012,8 +1021,9 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
           an[m] = red(mont_lazy((uint64_t)tt * kc[0][m] + (uint64_t)n1[m] * kc[1][m] + (uint64_t)es[m] * kc[2][m], p,
                                 pinv),
                       p);
-          b4[m] = red(mont_lazy(((uint64_t)tb << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m], p, pinv),
-                      2 * p);
+          uint64_t bt = ((uint64_t)tb << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m];
+          if constexpr (ZEROS) bt += (uint64_t)es[m] * kc[5][m];
+          b4[m] = red(mont_lazy(bt, p, pinv), 2 * p);
         }
         *reinterpret_cast<uint4*>(A + f * PS + qb + 4 * h4) = make_uint4(an[0], an[1], an[2], an[3]);
         bn[f][h4] = make_uint4(b4[0], b4[1], b4[2], b4[3]);
@@ -1225,11 +1235,11 @@ __device__ __noinline__ void leave_pair(uint32_t bars, uint32_t peer_bars, uint3
   }
 }
 
-template <int F, bool SEC, bool PAIR>
+template <int F, bool SEC, bool PAIR, bool ZEROS>
 __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm, int h, int q,
                                            int unit, uint32_t* rows, uint32_t* digits) {
   using namespace n2k;
-  constexpr int NKC = SEC ? SEC2K_KC : PRIM2K_KC;
+  constexpr int NKC = SEC ? sec_consts(ZEROS) : PRIM2K_KC;
   constexpr uint32_t p = F ? P2 : P1;
   constexpr int WORDS = few_words(NKC), XO = PS + (SEC ? 2 : 1) * N;
   const int t = threadIdx.x & 255;
@@ -1268,7 +1278,7 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
   for (int m = 0; m < 8; m++) {
     uint32_t k[NKC];
     if constexpr (SEC)
-      secondary_constants(a, sc, h, q, F, 8 * t + m, X[8 * t + m], k);
+      secondary_constants<ZEROS>(a, sc, h, q, F, 8 * t + m, X[8 * t + m], k);
     else
       state_constants(a, h, F, 8 * t + m, k);
 #pragma unroll
@@ -1417,10 +1427,11 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
         const uint32_t tt = ta[4 * h4 + m];
         an[m] = red(mont_lazy((uint64_t)tt * kc[0][m] + (uint64_t)n1[m] * kc[1][m] + (uint64_t)es[m] * kc[2][m], p, pinv),
                     p);
-        if constexpr (SEC)
-          bn[m] = red(mont_lazy(((uint64_t)tb[4 * h4 + m] << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m],
-                                p, pinv),
-                      2 * p);
+        if constexpr (SEC) {
+          uint64_t bt = ((uint64_t)tb[4 * h4 + m] << 32) + (uint64_t)tt * kc[3][m] + (uint64_t)n1[m] * kc[4][m];
+          if constexpr (ZEROS) bt += (uint64_t)es[m] * kc[5][m];
+          bn[m] = red(mont_lazy(bt, p, pinv), 2 * p);
+        }
       }
 #pragma unroll
       for (int m = 0; m < 4; m++) {
@@ -1452,23 +1463,25 @@ __device__ __forceinline__ void few_chain(const ChainArgs& a, const ScanConsts& 
 }
 
 // grid: x = part * H + half (times 2, + factor, as pairs), y = query
-template <bool PAIR>
+template <bool PAIR, bool ZEROS>
 __device__ __forceinline__ void few_secondary(const ChainArgs& a, const ScanConsts& sc, uint32_t* sm) {
   const int c = PAIR ? blockIdx.x >> 1 : blockIdx.x, f = PAIR ? blockIdx.x & 1 : threadIdx.x >> 8;
   const int h = c % a.g.H, q = blockIdx.y, unit = q * CTXT_PARTS + c / a.g.H;
   if (f == 0)
-    few_chain<0, true, PAIR>(a, sc, sm, h, q, unit, nullptr, nullptr);
+    few_chain<0, true, PAIR, ZEROS>(a, sc, sm, h, q, unit, nullptr, nullptr);
   else
-    few_chain<1, true, PAIR>(a, sc, sm, h, q, unit, nullptr, nullptr);
+    few_chain<1, true, PAIR, ZEROS>(a, sc, sm, h, q, unit, nullptr, nullptr);
 }
+template <bool ZEROS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1) secondary_chain_pair_kernel(ChainArgs a,
                                                                                                ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
-  few_secondary<true>(a, sc, sm);
+  few_secondary<true, ZEROS>(a, sc, sm);
 }
+template <bool ZEROS>
 __global__ void __launch_bounds__(512, 1) secondary_chain_wide_kernel(ChainArgs a, ScanConsts sc) {
   extern __shared__ __align__(16) uint32_t sm[];
-  few_secondary<false>(a, sc, sm);
+  few_secondary<false, ZEROS>(a, sc, sm);
 }
 
 // grid: x = lane * H + half (times 2, + factor, as pairs), y = shard
@@ -1480,9 +1493,9 @@ __device__ __forceinline__ void few_primary(ChainArgs& a, uint32_t* rows, uint32
   rows += s * shard_words, digits += s * shard_words;
   a.a_out += (size_t)s * a.g.H * SIMD * 2 * N_MAX;
   if (f == 0)
-    few_chain<0, false, PAIR>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+    few_chain<0, false, PAIR, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
   else
-    few_chain<1, false, PAIR>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
+    few_chain<1, false, PAIR, false>(a, ScanConsts(), sm, h, 0, lane, rows, digits);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     primary_chain_pair_kernel(ChainArgs a, uint32_t* rows, uint32_t* digits, size_t shard_words) {
@@ -1657,8 +1670,13 @@ void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_o
   a.cinv_first = pow_mod2n(a.inv5, g.L - 1, mask);
   const size_t smem = chain_smem(g, 0);
   dim3 grid(2, SIMD * g.H, nshards);
-  set_smem(primary_chain_kernel<0>, smem);
-  primary_chain_kernel<0><<<grid, CT, smem, st>>>(a);
+  if (g.log2n == LOG2_N_MAX) {  // three arrays a row
+    set_smem(primary_chain_kernel<LOG2_N_MAX>, smem);
+    primary_chain_kernel<LOG2_N_MAX><<<grid, CT, smem, st>>>(a);
+  } else {
+    set_smem(primary_chain_kernel<0>, smem);
+    primary_chain_kernel<0><<<grid, CT, smem, st>>>(a);
+  }
 }
 
 int chain_rows_supported(const Group& g) { return g.log2n == LOG2_N_MAX && g.na == 2; }
@@ -1719,9 +1737,30 @@ int secondary_chain_wave(const Group& g, int sms) {
   return std::max(1, g.log2n == LOG2_N_MAX ? sms / (int)g.H : 2 * sms / (2 * CTXT_PARTS * (int)g.H));
 }
 
+template <bool ZEROS>
+static void launch_secondary_2048(const ChainArgs& a, const ScanConsts& sc, int nq, int sms, bool clustered,
+                                  cudaStream_t st) {
+  const unsigned H = a.g.H;
+  const long chains = (long)nq * CTXT_PARTS * H;
+  if (clustered || 2 * chains <= sms) {
+    // PAIR_SMEM keeps the two blocks off one SM (and fits beside a scan block)
+    const size_t smem = clustered && 2 * chains > sms ? (size_t)few_words(sec_consts(ZEROS)) * 4 : PAIR_SMEM;
+    set_smem(secondary_chain_pair_kernel<ZEROS>, smem);
+    secondary_chain_pair_kernel<ZEROS><<<dim3(2 * CTXT_PARTS * H, nq), 256, smem, st>>>(a, sc);
+  } else if (chains <= sms) {
+    const size_t smem = (size_t)2 * few_words(sec_consts(ZEROS)) * 4;
+    set_smem(secondary_chain_wide_kernel<ZEROS>, smem);
+    secondary_chain_wide_kernel<ZEROS><<<dim3(CTXT_PARTS * H, nq), 512, smem, st>>>(a, sc);
+  } else {
+    const size_t smem = (size_t)sec2k_words(ZEROS) * 4;
+    set_smem(secondary_chain2k_kernel<ZEROS>, smem);
+    secondary_chain2k_kernel<ZEROS><<<dim3(H, nq), 256 * CTXT_PARTS, smem, st>>>(a, sc);
+  }
+}
+
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
                             uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
-                            const ScanConsts* sc, const NttTables& T, cudaStream_t st, bool clustered) {
+                            const ScanConsts& sc, bool zeros, const NttTables& T, cudaStream_t st, bool clustered) {
   ChainArgs a = chain_args(g, cc, T);
   set_limits(a, err, lim);
   a.E = E;
@@ -1732,31 +1771,20 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
   // N = 2048 (1024 steps of order 2048): a part's chain on two SMs while there
   // are two for each (2.1 ms), on one while there is one (3.75), beyond that the
   // three parts of a query and half per block (10.2, the constants kept once).
-  // Other lengths, or a-parts with a zero query slot: one part and factor per block in
-  // two-block clusters while the chunk needs at most one block per SM, then one
-  // block per part carrying both factors.  `clustered` asks for the cluster
-  // form at any chunk size (its blocks share SMs with a running scan; the
-  // pipeline tuner picks it per group size when faster).
+  // Other lengths: one part and factor per block in two-block clusters while the
+  // chunk needs at most one block per SM, then one block per part carrying both
+  // factors.  `clustered` asks for the cluster form at any chunk size (its blocks
+  // share SMs with a running scan; the pipeline tuner picks it per group size when
+  // faster).
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool full = g.log2n == LOG2_N_MAX;
-  const bool reg = full && sc;
-  const long chains = (long)nq * CTXT_PARTS * g.H;
-  if (reg && (clustered || 2 * chains <= sms)) {
-    // PAIR_SMEM keeps the two blocks off one SM (and fits beside a scan block)
-    const size_t smem = clustered && 2 * chains > sms ? (size_t)few_words(SEC2K_KC) * 4 : PAIR_SMEM;
-    set_smem(secondary_chain_pair_kernel, smem);
-    secondary_chain_pair_kernel<<<dim3(2 * CTXT_PARTS * g.H, nq), 256, smem, st>>>(a, *sc);
-  } else if (reg && chains <= sms) {
-    const size_t smem = (size_t)2 * few_words(SEC2K_KC) * 4;
-    set_smem(secondary_chain_wide_kernel, smem);
-    secondary_chain_wide_kernel<<<dim3(CTXT_PARTS * g.H, nq), 512, smem, st>>>(a, *sc);
-  } else if (reg) {
-    const size_t smem = (size_t)SEC2K_WORDS * 4;
-    set_smem(secondary_chain2k_kernel, smem);
-    secondary_chain2k_kernel<<<dim3(g.H, nq), 256 * CTXT_PARTS, smem, st>>>(a, *sc);
-  } else if (clustered || 2 * chains <= sms) {
+  if (g.log2n == LOG2_N_MAX) {
+    if (zeros)
+      launch_secondary_2048<true>(a, sc, nq, sms, clustered, st);
+    else
+      launch_secondary_2048<false>(a, sc, nq, sms, clustered, st);
+  } else if (clustered || 2 * (long)nq * CTXT_PARTS * g.H <= sms) {
     const size_t smem = chain_smem(g, 1);
     set_smem(secondary_chain_kernel<1, 0>, smem);
     secondary_chain_kernel<1, 0><<<dim3(2, CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);

@@ -256,7 +256,7 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
   const SlotMaps maps = slot_maps(f->ctx, g2.log2n);
   const ChainConsts cc = chain_consts(f->ctx, f->ap, g2.log2n, 1);
   const ScanConsts sc = scan_consts(f->ap, g2, 1);
-  const bool two = f->ap.na[1] == 2;
+  const bool zeros = f->ap.na[1] != 2;
   const auto tc = f->tuned_chain.find(nb);
   const bool clustered = tc != f->tuned_chain.end() && tc->second;
   for (int c0 = 0; c0 < nb; c0 += f->sec_chunk) {
@@ -276,7 +276,7 @@ int fleet_secondary_kernels(dnspir_fleet* f, QSlot& s, int nb, uint8_t* reply_de
     launch_encode_lift(E, E, g2, nl, 1, maps, f->ctx->T, st);
     launch_secondary_chain(f->secE.as<uint32_t>(), s.qbrv.as<uint32_t>() + (size_t)c0 * QV_WORDS_PER_QUERY * n,
                            QV_WORDS_PER_QUERY * n, nc, f->chain_out.as<uint32_t>(), slot_err(f, s),
-                           f->limits.of_group(nb), g2, cc, two ? &sc : nullptr, f->ctx->T, st, clustered);
+                           f->limits.of_group(nb), g2, cc, sc, zeros, f->ctx->T, st, clustered);
     launch_reply(f->chain_out.as<uint32_t>(), nc, g2.H, reply_dev ? reply_dev + (size_t)c0 * reply_stride : nullptr,
                  reply_stride, reply_zq ? reply_zq + (size_t)c0 * CTXT_PARTS * 2 * n : nullptr, g2.log2n, f->ctx->T,
                  st);

@@ -165,11 +165,11 @@ void launch_primary_finalize(const uint32_t* a_out, int nshards, uint64_t* a_zq,
 // launch_encode_lift(frame 1) with nl = 3 * nq lanes; qv: per query decoded
 // vectors [q][slot][p][pos] (bit-reversed), slots 0 gk0, 1 gk1, 2 pq, 3 pqc, 4 sq, 5 sqc.
 // out: [q][h][part][a/b][p][pos].
-// sc: scan_consts of the secondary's a-part set, or null when one of its query
-// slots is zero.
+// sc: scan_consts of the secondary's a-part set; zeros: one of its query slots is zero.
 void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_stride, int nq, uint32_t* out,
                             uint32_t* err, const WaitLimits& lim, const Group& g, const ChainConsts& cc,
-                            const ScanConsts* sc, const NttTables& T, cudaStream_t st, bool clustered = false);
+                            const ScanConsts& sc, bool zeros, const NttTables& T, cudaStream_t st,
+                            bool clustered = false);
 // Queries whose chains fill the SMs once.
 int secondary_chain_wave(const Group& g, int sms);
 
