@@ -193,7 +193,16 @@ int fleet_kernel_batch(dnspir_fleet* f, int nb) {
   return Bk;
 }
 
-int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbytes) {
+// Workspace of the answers comes before the preprocessing scratch that the fleet keeps.
+template <class Ensure>
+static int ensure_workspace(dnspir_fleet* f, const Ensure& ensure) {
+  const int r = ensure();
+  if (r != DNSPIR_ERR_OOM || !f->ws.rows.p) return r;
+  f->ws.rows.release();
+  return ensure();
+}
+
+static int slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbytes) {
   const size_t n = f->g1.n;
   CKR(s.qnat.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
   CKR(s.qbrv.ensure((size_t)Bk * QV_WORDS_PER_QUERY * n * 4));
@@ -207,7 +216,11 @@ int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbyte
   return DNSPIR_OK;
 }
 
-int fleet_secondary_workspace(dnspir_fleet* f, int nb) {
+int fleet_slot_workspace(dnspir_fleet* f, QSlot& s, int Bk, int nb, size_t qbytes) {
+  return ensure_workspace(f, [&] { return slot_workspace(f, s, Bk, nb, qbytes); });
+}
+
+static int secondary_workspace(dnspir_fleet* f, int nb) {
   const Group& g2 = f->g2;
   const size_t n = g2.n;
   const int cmax = std::min(nb, f->sec_chunk);
@@ -218,6 +231,10 @@ int fleet_secondary_workspace(dnspir_fleet* f, int nb) {
   CKR(f->secE.ensure((size_t)2 * g2.H * g2.L * nlmax * n * 4));
   CKR(f->chain_out.ensure((size_t)cmax * g2.H * CTXT_PARTS * 2 * 2 * n * 4));
   return DNSPIR_OK;
+}
+
+int fleet_secondary_workspace(dnspir_fleet* f, int nb) {
+  return ensure_workspace(f, [&] { return secondary_workspace(f, nb); });
 }
 
 int fleet_primary_kernels(dnspir_fleet* f, QSlot& s, int nb, int Bk, const uint32_t* sess_nat,
@@ -859,8 +876,7 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   CK(cudaGetLastError());
   CKR(fleet_drain(f));
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = true;
-  // the scratch of a bulk load goes back; an update of a few shards (four
-  // half-size, two full) keeps its own
+  // the scratch of a bulk load goes back; an update of a few shards keeps its own
   f->tmp_lane.release();
   if (f->ws.rows.bytes > EncodeWs::ROWS_KEPT) f->ws.rows.release();
   return DNSPIR_OK;

@@ -37,8 +37,8 @@ def test_bulk_load_gives_its_scratch_back_and_fits_where_memory_is_short(engine)
     fleet.set_engine(engine)
     before = _free(torch)
     fleet.set_shards(0, data)
-    # one piece of 10 shards takes 2.5 GiB of rows; at most 1 GiB stays (and the
-    # last rows and a-parts of 10 shards, a few MiB)
+    # one piece of 10 shards takes 2.5 GiB of rows, more than a fleet keeps (the
+    # last rows and a-parts of 10 shards, a few MiB, stay)
     assert before - _free(torch) < GIB + (64 << 20)
     want = [fleet.process_query(q) for q, _ in queries]
     for k, ((_, seed), r) in enumerate(zip(queries, want)):
@@ -52,6 +52,25 @@ def test_bulk_load_gives_its_scratch_back_and_fits_where_memory_is_short(engine)
     del hold
     torch.cuda.empty_cache()
     assert [fleet.process_query(q) for q, _ in queries] == want
+    fleet.close()
+
+
+def test_answers_take_the_scratch_where_memory_is_short():
+    # groups of 256 over 4 shards need about 0.6 GiB of workspace; the update's 1
+    # GiB of rows is what there is
+    torch = pytest.importorskip("torch")
+    shards, l2 = 4, 32
+    data, queries = _load(torch, shards, l2)
+    fleet = dp.Fleet.general(11, 1024, l2, shards)
+    fleet.set_engine(dp.ENGINE_TENSOR)
+    fleet.set_shards(0, data)
+    want = [fleet.process_query(q) for q, _ in queries]
+    hold = torch.empty(_free(torch) - GIB // 4, dtype=torch.uint8, device="cuda")
+    assert _free(torch) < GIB // 3
+    fleet.set_batch(256)
+    assert fleet.process_queries([q for q, _ in queries] * 64) == want * 64
+    del hold
+    torch.cuda.empty_cache()
     fleet.close()
 
 
