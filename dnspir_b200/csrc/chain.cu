@@ -17,12 +17,14 @@
 // Because d0 + 2^26 d1 = v exactly and v = t in each factor, NTT(d0) =
 // t - 2^26 NTT(d1): one forward transform per factor and step instead of two.
 //
-// Layout: one 2-block cluster per chain, block rank p owning RNS factor p.
-// The blocks exchange their iNTT outputs through distributed shared memory
-// (double-buffered by step parity, one cluster barrier per step), each
-// computes the CRT lift and the high digit, and transforms it in its own
-// factor.  NTT-domain vectors hold slots in bit-reversed position order
-// (position q <-> slot brv(q)); the constants are stored the same way.
+// Forms.  N = 2048, on the register transforms of ntt2048.cuh, by the number of
+// chains: two SMs each (a cluster of two blocks, one RNS factor each, which
+// exchange their inverse transforms through mbarrier-counted inboxes), one SM each
+// (both factors in one block, inboxes in its shared memory), or several chains a
+// block or SM (each thread carries both factors).  Other lengths, and preprocessing
+// with three stored arrays: a cluster of two blocks with a cluster barrier per step,
+// or one block with both factors.  NTT-domain vectors hold slots in bit-reversed
+// position order (position q <-> slot brv(q)); the constants are stored the same way.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -68,7 +70,7 @@ struct ChainPrime {
 // 2^28) and are brought back to [0, p) when it ends.
 // Forward: natural -> bit-reversed (CT butterflies), input in [0, p).
 // Inverse: bit-reversed -> natural, NOT scaled by N^-1 (the caller folds N^-1
-// into its next constant), input in [0, p).
+// into its next constant), input in [0, p), outputs in [0, 2p).
 __device__ __forceinline__ uint32_t shoup_lazy(uint32_t x, uint32_t w, uint32_t wq, uint32_t p) {
   return x * w - __umulhi(x, wq) * p;  // in [0, 2p) for any x < 2^32
 }
@@ -88,14 +90,11 @@ __device__ __forceinline__ void gs_bf(uint32_t& x, uint32_t& y, uint32_t w, uint
   y = shoup_lazy(d, w, wq, p);
 }
 
-// LN vectors `stride` words apart, transformed together: one barrier per pass,
-// and each thread handles the same butterfly group of every vector with its
-// loads issued before the arithmetic (twiddles loaded once).
 // LOGN > 0 fixes the length at compile time (the stage loop unrolls and every
 // index shift is a constant); LOGN = 0 takes logn_rt.
-template <int LN, int LOGN>
-__device__ __forceinline__ void fwd_multi(uint32_t* x0, int stride, int logn_rt, const uint32_t* __restrict__ tw,
-                                          const uint32_t* __restrict__ twq, uint32_t p) {
+template <int LOGN>
+__device__ __forceinline__ void fwd_one(uint32_t* x, int logn_rt, const uint32_t* __restrict__ tw,
+                                        const uint32_t* __restrict__ twq, uint32_t p) {
   const int logn = LOGN ? LOGN : logn_rt;
   const int N = 1 << logn;
   int s = 0;
@@ -109,51 +108,31 @@ __device__ __forceinline__ void fwd_multi(uint32_t* x0, int stride, int logn_rt,
       const uint32_t w = tw[m + blk], wq = twq[m + blk];
       const uint32_t w1 = tw[2 * m + 2 * blk], w1q = twq[2 * m + 2 * blk];
       const uint32_t w2 = tw[2 * m + 2 * blk + 1], w2q = twq[2 * m + 2 * blk + 1];
-      uint32_t v[LN][4];
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        const uint32_t* x = x0 + l * stride;
-        v[l][0] = x[j], v[l][1] = x[j + t2], v[l][2] = x[j + t], v[l][3] = x[j + t + t2];
-      }
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        ct_bf(v[l][0], v[l][2], w, wq, p);
-        ct_bf(v[l][1], v[l][3], w, wq, p);
-        ct_bf(v[l][0], v[l][1], w1, w1q, p);
-        ct_bf(v[l][2], v[l][3], w2, w2q, p);
-      }
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        uint32_t* x = x0 + l * stride;
-        x[j] = v[l][0], x[j + t2] = v[l][1], x[j + t] = v[l][2], x[j + t + t2] = v[l][3];
-      }
+      uint32_t v[4] = {x[j], x[j + t2], x[j + t], x[j + t + t2]};
+      ct_bf(v[0], v[2], w, wq, p);
+      ct_bf(v[1], v[3], w, wq, p);
+      ct_bf(v[0], v[1], w1, w1q, p);
+      ct_bf(v[2], v[3], w2, w2q, p);
+      x[j] = v[0], x[j + t2] = v[1], x[j + t] = v[2], x[j + t + t2] = v[3];
     }
     __syncthreads();
   }
   if (s < logn) {  // last stage, t = 1
     for (int b = threadIdx.x; b < N / 2; b += CT) {
-      const uint32_t w = tw[N / 2 + b], wq = twq[N / 2 + b];
-      uint32_t u[LN], v[LN];
-#pragma unroll
-      for (int l = 0; l < LN; l++) u[l] = x0[l * stride + 2 * b], v[l] = x0[l * stride + 2 * b + 1];
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        ct_bf(u[l], v[l], w, wq, p);
-        x0[l * stride + 2 * b] = red2p(red2p(u[l], 2 * p), p);
-        x0[l * stride + 2 * b + 1] = red2p(red2p(v[l], 2 * p), p);
-      }
+      uint32_t u = x[2 * b], v = x[2 * b + 1];
+      ct_bf(u, v, tw[N / 2 + b], twq[N / 2 + b], p);
+      x[2 * b] = red2p(red2p(u, 2 * p), p);
+      x[2 * b + 1] = red2p(red2p(v, 2 * p), p);
     }
   } else {
-    for (int b = threadIdx.x; b < N; b += CT)
-#pragma unroll
-      for (int l = 0; l < LN; l++) x0[l * stride + b] = red2p(red2p(x0[l * stride + b], 2 * p), p);
+    for (int b = threadIdx.x; b < N; b += CT) x[b] = red2p(red2p(x[b], 2 * p), p);
   }
   __syncthreads();
 }
 
-template <int LN, int LOGN>
-__device__ __forceinline__ void inv_multi(uint32_t* x0, int stride, int logn_rt, const uint32_t* __restrict__ tw,
-                                          const uint32_t* __restrict__ twq, uint32_t p) {
+template <int LOGN>
+__device__ __forceinline__ void inv_one(uint32_t* x, int logn_rt, const uint32_t* __restrict__ tw,
+                                        const uint32_t* __restrict__ twq, uint32_t p) {
   const int logn = LOGN ? LOGN : logn_rt;
   const int N = 1 << logn;
   int s = 0;
@@ -167,43 +146,25 @@ __device__ __forceinline__ void inv_multi(uint32_t* x0, int stride, int logn_rt,
       const uint32_t w0 = tw[h0 + 2 * blk], w0q = twq[h0 + 2 * blk];
       const uint32_t w1 = tw[h0 + 2 * blk + 1], w1q = twq[h0 + 2 * blk + 1];
       const uint32_t w = tw[h1 + blk], wq = twq[h1 + blk];
-      uint32_t v[LN][4];
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        const uint32_t* x = x0 + l * stride;
-        v[l][0] = x[j], v[l][1] = x[j + t], v[l][2] = x[j + 2 * t], v[l][3] = x[j + 3 * t];
-      }
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        gs_bf(v[l][0], v[l][1], w0, w0q, p);
-        gs_bf(v[l][2], v[l][3], w1, w1q, p);
-        gs_bf(v[l][0], v[l][2], w, wq, p);
-        gs_bf(v[l][1], v[l][3], w, wq, p);
-      }
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        uint32_t* x = x0 + l * stride;
-        x[j] = v[l][0], x[j + t] = v[l][1], x[j + 2 * t] = v[l][2], x[j + 3 * t] = v[l][3];
-      }
+      uint32_t v[4] = {x[j], x[j + t], x[j + 2 * t], x[j + 3 * t]};
+      gs_bf(v[0], v[1], w0, w0q, p);
+      gs_bf(v[2], v[3], w1, w1q, p);
+      gs_bf(v[0], v[2], w, wq, p);
+      gs_bf(v[1], v[3], w, wq, p);
+      x[j] = v[0], x[j + t] = v[1], x[j + 2 * t] = v[2], x[j + 3 * t] = v[3];
     }
     __syncthreads();
   }
   if (s < logn) {  // last stage, t = N/2
     const uint32_t w = tw[1], wq = twq[1];
     for (int j = threadIdx.x; j < N / 2; j += CT) {
-      uint32_t u[LN], v[LN];
-#pragma unroll
-      for (int l = 0; l < LN; l++) u[l] = x0[l * stride + j], v[l] = x0[l * stride + j + N / 2];
-#pragma unroll
-      for (int l = 0; l < LN; l++) {
-        gs_bf(u[l], v[l], w, wq, p);
-        x0[l * stride + j] = u[l];
-        x0[l * stride + j + N / 2] = v[l];
-      }
+      uint32_t u = x[j], v = x[j + N / 2];
+      gs_bf(u, v, w, wq, p);
+      x[j] = u;
+      x[j + N / 2] = v;
     }
     __syncthreads();
   }
-  // outputs are in [0, 2p); the consumer (high_digit via Shoup) accepts any value < 2^32
 }
 
 // High digit of the centred CRT lift from the two factors' unscaled iNTT
@@ -324,7 +285,7 @@ __device__ __forceinline__ void primary_body(const ChainArgs& a, int h, int lane
       }
     }
     __syncthreads();
-    inv_multi<1, LOGN>(D, 0, logn, IW, IWQ, pr);
+    inv_one<LOGN>(D, logn, IW, IWQ, pr);
     uint32_t* Xc = X + (i & 1) * N;
     for (int b = threadIdx.x; b < N; b += CT) Xc[b] = D[b];
     cluster.sync();
@@ -335,7 +296,7 @@ __device__ __forceinline__ void primary_body(const ChainArgs& a, int h, int lane
       D[b] = hd < 0 ? (uint32_t)(hd + (int32_t)pr) : (uint32_t)hd;
     }
     __syncthreads();
-    fwd_multi<1, LOGN>(D, 0, logn, FW, FWQ, pr);
+    fwd_one<LOGN>(D, logn, FW, FWQ, pr);
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int pos = threadIdx.x + c * CT;
@@ -366,30 +327,25 @@ __device__ __forceinline__ void primary_body(const ChainArgs& a, int h, int lane
   cluster.sync();  // keep this block's shared memory alive until the peer's last read
 }
 
-// Secondary chain: LN of the three parts of one query's secondary ciphertext
-// at half h in one block (factor p = rank in the cluster), parts part0 ..
-// part0 + LN - 1 (the library launches LN = 1: the block then needs 88 KiB and
-// shares an SM with a scan block; the register-transform chains and
-// secondary_dual_kernel below take the other cases).  The key constants gk_a0,
-// gk_a1, qry_a, gk_b0, gk_b1, qry_b (Montgomery form) and the sigma_5
-// destinations of a thread's positions live in its registers.  Each step's
+// Secondary chain at N < 2048: one of the three parts of one query's secondary
+// ciphertext at half h in one block (factor p = rank in the cluster).  The key
+// constants gk_a0, gk_a1, qry_a, gk_b0, gk_b1, qry_b (Montgomery form) and the
+// sigma_5 destinations of a thread's positions live in its registers.  Each step's
 // pointwise stage writes the next step's sigma_5-permuted a and b straight
 // into the other buffer of a pair, and the inverse transform is published to
 // the peer from its own buffer D[i mod 2] (the peer reads it between the
 // cluster barriers of steps i and i + 1; this block rewrites it only at the end
 // of step i + 1).  Shared memory (u32 words):
-//   FW FWQ IW IWQ                    4N   twiddles of this factor
-//   per part: TC[2] D[2] B[2] H      7N   sigma_5(a) kept, sigma_5(a) transformed
-//                                         (published), sigma_5(b), high digit
-// (4 + 7 LN) N words: 200 KiB for LN = 3, 88 KiB for LN = 1 at N = 2048.
+//   FW FWQ IW IWQ             4N   twiddles of this factor
+//   TC[2] D[2] B[2] H         7N   sigma_5(a) kept, sigma_5(a) transformed
+//                                  (published), sigma_5(b), high digit
 constexpr int SEC_PART_WORDS = 7;  // x N
-__host__ __device__ constexpr int sec_smem_words(int ln) { return 4 + ln * SEC_PART_WORDS; }
+constexpr int SEC_WORDS = 4 + SEC_PART_WORDS;
 
-template <int LN, int LOGN>
-__device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q, int part0, uint32_t* sm) {
+__device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q, int part, uint32_t* sm) {
   cg::cluster_group cluster = cg::this_cluster();
   const int p = (int)cluster.block_rank();
-  const int logn = LOGN ? LOGN : a.g.log2n;
+  const int logn = a.g.log2n;
   const int N = 1 << logn;
   const ChainPrime cp = a.cp[p];
   const uint32_t pr = cp.p;
@@ -397,10 +353,10 @@ __device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q,
   uint32_t* FWQ = FW + N;
   uint32_t* IW = FWQ + N;
   uint32_t* IWQ = IW + N;
-  uint32_t* P0 = IWQ + N;  // part blocks
-  const int PS = SEC_PART_WORDS * N;
-  // per part: TC[2] at 0, N; D[2] at 2N, 3N; B[2] at 4N, 5N; H at 6N
-  const int oTC = 0, oD = 2 * N, oB = 4 * N, oH = 6 * N;
+  uint32_t* TC = IWQ + N;
+  uint32_t* D = TC + 2 * N;
+  uint32_t* B = D + 2 * N;
+  uint32_t* H = B + 2 * N;
   const uint32_t* qq = a.qv + (size_t)q * a.qv_stride;
   constexpr int PER = N_MAX / CT;  // positions per thread (N <= N_MAX)
   uint32_t kc[6][PER], dst[PER];
@@ -423,80 +379,58 @@ __device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q,
     FWQ[b] = a.T.fwq[p][b];
     IW[b] = a.T.iw[p][b];
     IWQ[b] = a.T.iwq[p][b];
-#pragma unroll
-    for (int t = 0; t < LN; t++) {  // a = b = 0, so sigma_5(a) = sigma_5(b) = 0
-      P0[t * PS + oTC + b] = 0;
-      P0[t * PS + oD + b] = 0;
-      P0[t * PS + oB + b] = 0;
-    }
+    TC[b] = D[b] = B[b] = 0;  // a = b = 0, so sigma_5(a) = sigma_5(b) = 0
   }
   cluster.sync();
-  const uint32_t* peer = cluster.map_shared_rank(P0, p ^ 1);
+  const uint32_t* peerD = cluster.map_shared_rank(D, p ^ 1);
   for (uint32_t i = 0; i < a.g.L; i++) {
     const int cur = (int)(i & 1) * N, nxt = N - cur;
-    // entries of row i (the three parts' lanes are adjacent), consumed at the end of the step
+    // entries of row i, consumed at the end of the step
     const uint32_t* Ei =
-        a.E + ((((size_t)p * a.g.H + h) * a.g.L + a.g.L - 1 - i) * a.nl + (size_t)q * CTXT_PARTS + part0) * N;
-    uint32_t e[LN][PER];
+        a.E + ((((size_t)p * a.g.H + h) * a.g.L + a.g.L - 1 - i) * a.nl + (size_t)q * CTXT_PARTS + part) * N;
+    uint32_t e[PER];
 #pragma unroll
-    for (int t = 0; t < LN; t++)
-#pragma unroll
-      for (int c = 0; c < PER; c++) {
-        const int pos = threadIdx.x + c * CT;
-        e[t][c] = pos < N ? __ldg(Ei + (size_t)t * N + pos) : 0;
-      }
-    inv_multi<LN, LOGN>(P0 + oD + cur, PS, logn, IW, IWQ, pr);
+    for (int c = 0; c < PER; c++) {
+      const int pos = threadIdx.x + c * CT;
+      e[c] = pos < N ? __ldg(Ei + pos) : 0;
+    }
+    inv_one<0>(D + cur, logn, IW, IWQ, pr);
     cluster.sync();
     for (int b = threadIdx.x; b < N; b += CT) {
-      uint32_t own[LN], other[LN];
-#pragma unroll
-      for (int t = 0; t < LN; t++) own[t] = P0[t * PS + oD + cur + b], other[t] = peer[t * PS + oD + cur + b];
-#pragma unroll
-      for (int t = 0; t < LN; t++) {
-        const int32_t hd = p == 0 ? high_digit(own[t], other[t], a.cp[0], a.cp[1])
-                                  : high_digit(other[t], own[t], a.cp[0], a.cp[1]);
-        P0[t * PS + oH + b] = hd < 0 ? (uint32_t)(hd + (int32_t)pr) : (uint32_t)hd;
-      }
+      const uint32_t own = D[cur + b], other = peerD[cur + b];
+      const int32_t hd = p == 0 ? high_digit(own, other, a.cp[0], a.cp[1]) : high_digit(other, own, a.cp[0], a.cp[1]);
+      H[b] = hd < 0 ? (uint32_t)(hd + (int32_t)pr) : (uint32_t)hd;
     }
     __syncthreads();
-    fwd_multi<LN, LOGN>(P0 + oH, PS, logn, FW, FWQ, pr);
+    fwd_one<0>(H, logn, FW, FWQ, pr);
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int pos = threadIdx.x + c * CT;
       if (pos < N) {
-        const uint32_t cg0 = kc[0][c], cg1 = kc[1][c], cqa = kc[2][c];
-        const uint32_t qg0 = kc[3][c], qg1 = kc[4][c], qqb = kc[5][c];
-#pragma unroll
-        for (int t = 0; t < LN; t++) {
-          uint32_t* P = P0 + t * PS;
-          const uint32_t n1 = P[oH + pos];
-          const uint32_t n0 = sub_mod(P[oTC + cur + pos], mont_reduce((uint64_t)n1 * cp.c26, pr, cp.pinv), pr);
-          const uint32_t an =
-              mont_reduce((uint64_t)n0 * cg0 + (uint64_t)n1 * cg1 + (uint64_t)e[t][c] * cqa, pr, cp.pinv);
-          const uint32_t bn = mont_reduce(((uint64_t)P[oB + cur + pos] << 32) + (uint64_t)n0 * qg0 +
-                                              (uint64_t)n1 * qg1 + (uint64_t)e[t][c] * qqb,
-                                          pr, cp.pinv);
-          // sigma_5 for the next step
-          P[oTC + nxt + dst[c]] = an;
-          P[oD + nxt + dst[c]] = an;
-          P[oB + nxt + dst[c]] = bn;
-        }
+        const uint32_t n1 = H[pos];
+        const uint32_t n0 = sub_mod(TC[cur + pos], mont_reduce((uint64_t)n1 * cp.c26, pr, cp.pinv), pr);
+        const uint32_t an = mont_reduce(
+            (uint64_t)n0 * kc[0][c] + (uint64_t)n1 * kc[1][c] + (uint64_t)e[c] * kc[2][c], pr, cp.pinv);
+        const uint32_t bn = mont_reduce(((uint64_t)B[cur + pos] << 32) + (uint64_t)n0 * kc[3][c] +
+                                            (uint64_t)n1 * kc[4][c] + (uint64_t)e[c] * kc[5][c],
+                                        pr, cp.pinv);
+        // sigma_5 for the next step
+        TC[nxt + dst[c]] = an;
+        D[nxt + dst[c]] = an;
+        B[nxt + dst[c]] = bn;
       }
     }
     __syncthreads();
   }
   // the state after the last step sits sigma_5-permuted in buffer L mod 2
   const int fin = (int)(a.g.L & 1) * N;
+  uint32_t* o = a.out + ((((size_t)q * a.g.H + h) * CTXT_PARTS + part) * 2) * 2 * N;
 #pragma unroll
   for (int c = 0; c < PER; c++) {
     const int pos = threadIdx.x + c * CT;
     if (pos < N) {
-#pragma unroll
-      for (int t = 0; t < LN; t++) {
-        uint32_t* o = a.out + ((((size_t)q * a.g.H + h) * CTXT_PARTS + part0 + t) * 2) * 2 * N;
-        o[(size_t)p * N + pos] = P0[t * PS + oTC + fin + dst[c]];
-        o[2 * (size_t)N + (size_t)p * N + pos] = P0[t * PS + oB + fin + dst[c]];
-      }
+      o[(size_t)p * N + pos] = TC[fin + dst[c]];
+      o[2 * (size_t)N + (size_t)p * N + pos] = B[fin + dst[c]];
     }
   }
   cluster.sync();  // keep this block's shared memory alive until the peer's last read
@@ -508,13 +442,11 @@ __device__ __forceinline__ void secondary_body(const ChainArgs& a, int h, int q,
 // transforms from this block's shared memory (no cluster barrier, no remote
 // reads), and each barrier covers twice the work of the clustered form.
 // Shared memory (u32 words): twiddles FW FWQ IW IWQ of each factor (8N), per
-// factor TC[2] D[2] B[2] H (7N): 22N = 176 KiB at N = 2048, one block per SM.
+// factor TC[2] D[2] B[2] H (7N): 22N.
 constexpr int SEC_DUAL_WORDS = 8 + 2 * SEC_PART_WORDS;  // x N
 
-template <int LOGN>
-__device__ __forceinline__ void fwd_dual(uint32_t* x0, uint32_t* x1, int logn_rt, const uint32_t* const* tw,
+__device__ __forceinline__ void fwd_dual(uint32_t* x0, uint32_t* x1, int logn, const uint32_t* const* tw,
                                          const uint32_t* const* twq, uint32_t p0, uint32_t p1) {
-  const int logn = LOGN ? LOGN : logn_rt;
   const int N = 1 << logn;
   uint32_t* xs[2] = {x0, x1};
   const uint32_t ps[2] = {p0, p1};
@@ -567,10 +499,8 @@ __device__ __forceinline__ void fwd_dual(uint32_t* x0, uint32_t* x1, int logn_rt
   __syncthreads();
 }
 
-template <int LOGN>
-__device__ __forceinline__ void inv_dual(uint32_t* x0, uint32_t* x1, int logn_rt, const uint32_t* const* tw,
+__device__ __forceinline__ void inv_dual(uint32_t* x0, uint32_t* x1, int logn, const uint32_t* const* tw,
                                          const uint32_t* const* twq, uint32_t p0, uint32_t p1) {
-  const int logn = LOGN ? LOGN : logn_rt;
   const int N = 1 << logn;
   uint32_t* xs[2] = {x0, x1};
   const uint32_t ps[2] = {p0, p1};
@@ -619,9 +549,8 @@ __device__ __forceinline__ void inv_dual(uint32_t* x0, uint32_t* x1, int logn_rt
   }
 }
 
-template <int LOGN>
 __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, int q, int part, uint32_t* sm) {
-  const int logn = LOGN ? LOGN : a.g.log2n;
+  const int logn = a.g.log2n;
   const int N = 1 << logn;
   const uint32_t pr0 = a.cp[0].p, pr1 = a.cp[1].p;
   const uint32_t* tws[2] = {sm, sm + 4 * N};
@@ -678,14 +607,14 @@ __device__ __forceinline__ void secondary_dual_body(const ChainArgs& a, int h, i
         e[p][c] = pos < N ? __ldg(Ei + pos) : 0;
       }
     }
-    inv_dual<LOGN>(F0 + oD + cur, F0 + FS + oD + cur, logn, itws, itwqs, pr0, pr1);
+    inv_dual(F0 + oD + cur, F0 + FS + oD + cur, logn, itws, itwqs, pr0, pr1);
     for (int b = threadIdx.x; b < N; b += CT) {
       const int32_t hd = high_digit(F0[oD + cur + b], F0[FS + oD + cur + b], a.cp[0], a.cp[1]);
       F0[oH + b] = hd < 0 ? (uint32_t)(hd + (int32_t)pr0) : (uint32_t)hd;
       F0[FS + oH + b] = hd < 0 ? (uint32_t)(hd + (int32_t)pr1) : (uint32_t)hd;
     }
     __syncthreads();
-    fwd_dual<LOGN>(F0 + oH, F0 + FS + oH, logn, tws, twqs, pr0, pr1);
+    fwd_dual(F0 + oH, F0 + FS + oH, logn, tws, twqs, pr0, pr1);
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int pos = threadIdx.x + c * CT;
@@ -1551,17 +1480,15 @@ __global__ void __launch_bounds__(512) lane_rows_kernel(const uint32_t* __restri
 }
 
 // grid: x = part * H + half, y = query (no cluster)
-template <int LOGN>
 __global__ void __launch_bounds__(CT, 1) secondary_dual_kernel(ChainArgs a) {
   extern __shared__ uint32_t sm[];
-  secondary_dual_body<LOGN>(a, blockIdx.x % a.g.H, blockIdx.y, blockIdx.x / a.g.H, sm);
+  secondary_dual_body(a, blockIdx.x % a.g.H, blockIdx.y, blockIdx.x / a.g.H, sm);
 }
 
-// grid: x = factor (cluster of 2), y = (part group) * H + half, z = query
-template <int LN, int LOGN>
+// grid: x = factor (cluster of 2), y = part * H + half, z = query
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CT) secondary_chain_kernel(ChainArgs a) {
   extern __shared__ uint32_t sm[];
-  secondary_body<LN, LOGN>(a, blockIdx.y % a.g.H, blockIdx.z, (blockIdx.y / a.g.H) * LN, sm);
+  secondary_body(a, blockIdx.y % a.g.H, blockIdx.z, blockIdx.y / a.g.H, sm);
 }
 
 // grid: x = factor (cluster of 2), y = lane * H + half, z = shard
@@ -1655,9 +1582,6 @@ static void set_limits(ChainArgs& a, uint32_t* err, const WaitLimits& lim) {
   a.withhold = lim.withhold_step < 0 ? ~0u : (uint32_t)lim.withhold_step;
 }
 
-static size_t chain_smem(const Group& g, int secondary_parts) {
-  return (size_t)(secondary_parts ? sec_smem_words(secondary_parts) : 12) * g.n * 4;
-}
 
 void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_out, const Group& g,
                           const ChainConsts& cc, const NttTables& T, cudaStream_t st) {
@@ -1668,7 +1592,7 @@ void launch_primary_chain(uint32_t* const* slabs_dev, int nshards, uint32_t* a_o
   a.inv5 = inv5_mod2n(2 * g.n);
   a.c_first = pow_mod2n(5, g.L - 1, mask);
   a.cinv_first = pow_mod2n(a.inv5, g.L - 1, mask);
-  const size_t smem = chain_smem(g, 0);
+  const size_t smem = (size_t)12 * g.n * 4;
   dim3 grid(2, SIMD * g.H, nshards);
   if (g.log2n == LOG2_N_MAX) {  // three arrays a row
     set_smem(primary_chain_kernel<LOG2_N_MAX>, smem);
@@ -1689,9 +1613,7 @@ void launch_primary_chain_rows(uint32_t* rows, uint32_t* digits, size_t shard_wo
   ChainArgs a = chain_args(g, cc, T);
   a.a_out = a_out;
   set_limits(a, err, lim);
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const long chains = SIMD * (long)g.H * nshards;
   if (2 * chains <= sms) {
     set_smem(primary_chain_pair_kernel, PAIR_SMEM);
@@ -1776,22 +1698,20 @@ void launch_secondary_chain(const uint32_t* E, const uint32_t* qv, size_t qv_str
   // factors.  `clustered` asks for the cluster form at any chunk size (its blocks
   // share SMs with a running scan; the pipeline tuner picks it per group size when
   // faster).
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   if (g.log2n == LOG2_N_MAX) {
     if (zeros)
       launch_secondary_2048<true>(a, sc, nq, sms, clustered, st);
     else
       launch_secondary_2048<false>(a, sc, nq, sms, clustered, st);
   } else if (clustered || 2 * (long)nq * CTXT_PARTS * g.H <= sms) {
-    const size_t smem = chain_smem(g, 1);
-    set_smem(secondary_chain_kernel<1, 0>, smem);
-    secondary_chain_kernel<1, 0><<<dim3(2, CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
+    const size_t smem = (size_t)SEC_WORDS * g.n * 4;
+    set_smem(secondary_chain_kernel, smem);
+    secondary_chain_kernel<<<dim3(2, CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
   } else {
     const size_t smem = (size_t)SEC_DUAL_WORDS * g.n * 4;
-    set_smem(secondary_dual_kernel<0>, smem);
-    secondary_dual_kernel<0><<<dim3(CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
+    set_smem(secondary_dual_kernel, smem);
+    secondary_dual_kernel<<<dim3(CTXT_PARTS * g.H, nq), CT, smem, st>>>(a);
   }
 }
 

@@ -505,7 +505,7 @@ void launch_encode_cols(const uint16_t* in, uint32_t* A, const Group& g, uint32_
   const uint32_t total = l_in * nl;
   if (!total) return;
   if (g.log2n == 11) {
-    const int ppc = total <= 592 ? 1 : 4;  // polynomials per block, as above
+    const int ppc = total <= 4 * (uint32_t)sm_count() ? 1 : 4;  // polynomials per block: one while four blocks an SM hold them all
     const size_t smem = (size_t)ppc * n2k::PS * 4;
     set_smem(encode_cols2k_kernel, smem);
     encode_cols2k_kernel<<<(total + ppc - 1) / ppc, NT2K, smem, st>>>(in, A, total, ppc, T);
@@ -564,7 +564,7 @@ void launch_encode_lift(const uint32_t* Ahat, uint32_t* out, const Group& g, int
     const uint32_t sq = (uint32_t)(((uint64_t)linv << 32) / TPLAIN);
     // lanes share a block's twiddles; one lane per block where that many
     // blocks (three fit an SM) do not fill the SMs once
-    const int lpb = (size_t)g.L * g.H * nl <= 444 ? 1 : LIFT_LANES_CHAIN;
+    const int lpb = (size_t)g.L * g.H * nl <= 3 * (size_t)sm_count() ? 1 : LIFT_LANES_CHAIN;
     const int nlg = nl < lpb ? nl : lpb;
     const size_t smem = (size_t)2 * nlg * n2k::PS * 4;
     dim3 grid(g.L, g.H, (nl + lpb - 1) / lpb);

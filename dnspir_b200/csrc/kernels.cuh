@@ -32,6 +32,14 @@ inline void set_smem(K* kernel, size_t bytes) {
   if (bytes > 48 * 1024) raise_smem_limit((const void*)kernel, bytes);
 }
 
+// Streaming multiprocessors of the current device.
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Shape of one PIR database (IndexGroup, base_pir.rs:132-183).
 struct Group {
   int log2n;    // ring dimension N = 2^log2n

@@ -130,22 +130,10 @@ struct ScaleStore {
   }
 };
 
-// Ends a pass: SYNC = 0 synchronises the block; SYNC = 1 only the 256-thread
-// group of the calling thread (named barrier 1 + threadIdx.x / 256), for
-// blocks of 512 threads whose two halves work on one polynomial each.
-template <int SYNC>
-__device__ __forceinline__ void pass_sync() {
-  if constexpr (SYNC == 0) {
-    __syncthreads();
-  } else {
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + (threadIdx.x >> 8)) : "memory");
-  }
-}
-
 // One radix-8 pass over polynomials [0, cnt0) (factor 0) and [cnt0, cnt0 +
 // cnt1) (factor 1) of x.  INV selects Gentleman-Sande with the iw tables; FIN
 // (inverse, M = 1 only) receives the finished values instead of a store.
-template <int NT, int M, bool INV, int SYNC = 0, class Fin>
+template <int NT, int M, bool INV, class Fin>
 __device__ __forceinline__ void pass8(uint32_t* x, int cnt0, int cnt1, const NttTables& T, const Fin& fin) {
   using S = Split<NT, 256>;
   using Gm = Geo8<M>;
@@ -184,7 +172,7 @@ __device__ __forceinline__ void pass8(uint32_t* x, int cnt0, int cnt1, const Ntt
       }
     }
   }
-  pass_sync<SYNC>();
+  __syncthreads();
 }
 
 // Radix-4 pass on the aligned quads 4g .. 4g + 3 (forward stages 9-10 with

@@ -111,13 +111,14 @@ __device__ __forceinline__ void ld_lanes(const uint32_t* p, uint32_t* v, int lpt
 // B queries per block, LPT lanes per thread, MINB blocks per SM (0: as many as
 // the registers give), UN rows unrolled.  One and two queries are bound by HBM
 // and take light threads with many rows in flight (64 full shards: one query 4.65
-// ms, 7.4 TB/s; two 4.8, 5.2 as eight lanes a thread); from four on the wide multiply-adds bound it (four cycles a warp on the heavy
-// FMA pipe: 7.5 ms for 8 queries of 64 full shards), and four lanes a thread
-// halve the shared-memory reads per product against two: 8 queries 9.7 ms as
-// two blocks per SM, 16 19.0 as two such groups against 21.2 as 16 with two lanes;
-// four queries 5.7 at three blocks per SM and four lanes, 8.1 at eight lanes
-// (130 registers; 0.38 / 0.56 at 4 half-size shards).  Tried: a third of the queries on the FP64 pipe, exactly, with
-// 13-bit halves (8 queries 16 ms).
+// ms, 7.4 TB/s; two 4.8, 5.2 as eight lanes a thread).  From four on the wide
+// multiply-adds bound it (four cycles a warp on the heavy FMA pipe: 7.5 ms for 8
+// queries of 64 full shards), and four lanes a thread halve the shared-memory
+// reads per product against two: 8 queries 9.7 ms as two blocks per SM, 16 19.0 as
+// two such groups against 21.2 as 16 with two lanes; four queries 5.7 at three
+// blocks per SM and four lanes, 8.1 at eight lanes (130 registers; 0.38 / 0.56 at
+// 4 half-size shards).  Tried: a third of the queries on the FP64 pipe, exactly,
+// with 13-bit halves (8 queries 16 ms).
 template <int B, int LPT, int NA, int MINB, int UN>
 __global__ void __launch_bounds__(SCAN_NT, MINB) scan_batch_kernel(ScanArgs a) {
   constexpr int LG = SIMD / LPT;     // lane groups per slot
@@ -335,8 +336,8 @@ __global__ void primary_epilogue_kernel(const uint32_t* __restrict__ fin, int ns
 // brings four lanes (half a 32-byte sector; the other half is the neighbouring
 // block's), the eight inverse transforms run together, the CRT uses Shoup
 // companions of its two constants and the 12-bit switch an exact 64-bit rounding
-// (v 2^13 + q < 2^64 for v < q).  LN = 1: one lane per block, for so few shards
-// and queries that the blocks do not fill the SMs.  Bound by shared memory and
+// (v 2^13 + q < 2^64 for v < q).  LN = 1: one lane per block, for few shards and
+// queries (launch_epilogue_cols).  Bound by shared memory and
 // barriers (three blocks an SM).  Against digits through global memory and a kernel
 // for their columns (256 queries of 64 shards): 2.95 + 2.03 -> 4.25 ms, and the
 // digits' buffer is not needed.
@@ -505,9 +506,7 @@ int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* q
       // many give it themselves (4 / 11 / 25 half-size and 64 full shards: 4 rows
       // 0.51 / 0.52 / 0.55 / 4.65 ms, 8 rows 0.37 / 0.39 / 0.48 / 4.85, 12 rows at
       // three blocks per SM 0.25 / 0.30 / 0.76 / 4.69)
-      int sms = 0, dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int sms = sm_count();
       const size_t blocks = (size_t)nshards * 4 * ((g.n / 2 + 127) / 128) * groups;
       if (blocks <= (size_t)3 * sms) launch_batch<1, 4, 3, 12>(a, st);
       else if (blocks <= (size_t)7 * sms) launch_batch<1, 4, 0, 8>(a, st);
@@ -552,7 +551,10 @@ void launch_epilogue_cols(const uint32_t* fin, int nq, int nshards, const uint32
   const CrtConst cc = host_crt_const();
   const uint32_t k1q = (uint32_t)(((uint64_t)cc.q2inv1 << 32) / P1);
   const uint32_t k2q = (uint32_t)(((uint64_t)cc.q1inv2 << 32) / P2);
-  if ((size_t)nshards * SIMD * nq <= 256) {
+  // one lane per block while three blocks an SM hold them all (one query's first
+  // kernel of the secondary phase and what follows, order 512, in us, one lane /
+  // four: 8 shards 1162 / 1182, 32 1167 / 1180, 48 1175 / 1179, 64 1185 / 1181)
+  if ((size_t)nshards * SIMD * nq <= 3 * (size_t)sm_count()) {
     primary_epilogue2k_kernel<1><<<dim3(nshards, SIMD, nq), EPI_NT, (size_t)2 * n2k::PS * 4, st>>>(
         fin, nshards, a_ms, distinct_of, A, maps.uof, T, cc.q2inv1, k1q, cc.q1inv2, k2q);
     return;

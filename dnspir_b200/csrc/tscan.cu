@@ -1136,15 +1136,13 @@ int launch_tp(const TScanArgs& a0, int stages, cudaStream_t st) {
   if (smem > 227 * 1024) return -1;
   set_smem(tscanp_kernel<NQ, MTPC>, smem);
   constexpr int COLS = tmem_cols((2 * MTPC * NQ <= 512 ? 2 : 1) * MTPC * NQ);
-  int per_sm = 0, dev = 0, sms = 0;
+  int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tscanp_kernel<NQ, MTPC>, tscanp_nt<NQ>(), smem);
   // resident CTAs must not ask for more TMEM columns than the SM has (a CTA
   // whose allocation waits would hold its SM until a neighbour finishes)
   if (per_sm < 1 || per_sm * COLS > 512) return -1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t items = (size_t)a.nshards * 4 * (a.mt_total / MTPC) * a.groups;
-  size_t grid = std::min(items, (size_t)sms * per_sm);
+  size_t grid = std::min(items, (size_t)sm_count() * per_sm);
   // a multiple of the query-group count, so that the CTAs sharing a slab
   // tile are the same in every round (as for the CTA pairs below)
   if (grid >= a.groups) grid -= grid % a.groups;
@@ -1214,10 +1212,7 @@ int launch_t2(const TScanArgs& a0, int stages, cudaStream_t st) {
     return -1;
   }
   // one CTA per SM: TMEM columns of a resident CTA never exceed the SM's 512
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  clusters = std::min(clusters, sms / 2);
+  clusters = std::min(clusters, sm_count() / 2);
   // the query groups of one slab tile are consecutive items: with a cluster
   // count that is a multiple of the group count, the same clusters share a
   // slab tile in every round and stay in step, so the tile comes from HBM
