@@ -983,10 +983,10 @@ __global__ void __launch_bounds__(256 * CTXT_PARTS, 1) secondary_chain2k_kernel(
 // half, lane) per block of 256 threads on the same step, without a b part.
 // Rows of the chain layout, E on input, take the state k a' in their place; the
 // canonical high digits' transforms go to `digits`, the same layout.  Three
-// blocks fit an SM (67 KiB, 80 registers), so up to one wave of 444 chains runs
-// at once.  Against two-block clusters with one factor per block (radix-4
-// passes, uncoalesced stores): 9.9 -> 5.0 ms for 64 chains of 1024 steps (2.2 on two
-// SMs each, below).
+// blocks fit an SM (67 KiB, 80 registers).  Taken by calls of more chains than SMs,
+// which are of order 512 or less: shards of larger orders fill a call's scratch with
+// 104 chains (preprocess_batch).  160 chains of 512 steps 4.2 ms; 144 on one SM
+// each (below) 2.05.
 constexpr int PRIM2K_KC = 3;
 constexpr int PRIM2K_WORDS = 2 * n2k::PS + PRIM2K_KC * 2 * 2 * 256 * 4;
 
