@@ -468,6 +468,7 @@ struct dnspir_db {
   DBuf err;  // wait-error word of the preprocessing chains
   WaitLimits limits;
   HBuf pin;  // host staging of perform_pir_split: query elements in, reply out
+  bool pin_busy = false;
   EncodeWs ws;
   std::mutex mu;
   ~dnspir_db() {
@@ -662,12 +663,16 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   uint32_t* slabs[1] = {db->slab};
   CKR(preprocess_shards(db->ctx, db->ap, db->g, db->used_seeds, slabs, 1, src, db->a_zq.as<uint64_t>(),
                         db->a_ms.as<uint32_t>(), db->ws, db->err.as<uint32_t>(), db->limits, db->st));
-  CKR(db->pin.ensure(4));
-  CK(cudaMemcpyAsync(db->pin.p, db->err.p, 4, cudaMemcpyDeviceToHost, db->st));
-  CK(cudaStreamSynchronize(db->st));
-  if (*db->pin.as<uint32_t>()) {
-    CK(cudaMemset(db->err.p, 0, 4));
-    return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
+  if (chain_rows_supported(db->g)) {  // other shapes' chains have no bounded waits, and have been waited for
+    CKR(db->pin.ensure(4));
+    db->pin_busy = true;
+    CK(cudaMemcpyAsync(db->pin.p, db->err.p, 4, cudaMemcpyDeviceToHost, db->st));
+    CK(cudaStreamSynchronize(db->st));
+    db->pin_busy = false;
+    if (*db->pin.as<uint32_t>()) {
+      CK(cudaMemset(db->err.p, 0, 4));
+      return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
+    }
   }
   db->ready = true;
   return DNSPIR_OK;
@@ -693,7 +698,8 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
   const size_t n = g.n;
   // [lane][v][N], v = qry, qry_conj, gk0, gk1
   DeviceGuard dg(db->device);
-  CK(cudaStreamSynchronize(db->st));  // an earlier call that failed may still copy from the staging buffer
+  // a call that failed on its way may still copy from the staging buffer
+  if (db->pin_busy) CK(cudaStreamSynchronize(db->st));
   const size_t words = (size_t)SIMD * 4 * n;
   CKR(db->pin.ensure(words * 8));
   uint64_t* const z = db->pin.as<uint64_t>();
@@ -709,17 +715,17 @@ int dnspir_db_perform_pir_split(dnspir_db* db, const uint64_t* qry_b, const uint
   CKR(db->qv.ensure((size_t)SIMD * 4 * SCAN_VECS * n * 4));
   CKR(db->sum.ensure(scan_lanes_sum_words(g) * 4));
   CKR(db->out.ensure((size_t)SIMD * n * 8));
+  db->pin_busy = true;
   CK(cudaMemcpyAsync(db->qz.p, z, words * 8, cudaMemcpyHostToDevice, db->st));
-  launch_ring_to_ntt(db->qz.as<uint64_t>(), SIMD * 4, db->qlane.as<uint32_t>(), nullptr, g.log2n, db->ctx->T, db->st);
   const SlotMaps maps = slot_maps(db->ctx, g.log2n);
-  launch_scan_vectors(db->qlane.as<uint32_t>(), 8 * n, 0, 2, SIMD, SIMD, db->qv.as<uint32_t>(), g,
-                      scan_consts(db->ap, g, db->used_seeds), maps, db->st);
-  if (launch_scan_lanes(db->slab, db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g, db->st))
-    return fail(DNSPIR_ERR_CUDA, "cannot clear the scan's sums");
+  launch_lane_vectors(db->qz.as<uint64_t>(), db->qlane.as<uint32_t>(), db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g,
+                      scan_consts(db->ap, g, db->used_seeds), maps, db->ctx->T, db->st);
+  launch_scan_lanes(db->slab, db->qv.as<uint32_t>(), db->sum.as<uint32_t>(), g, db->st);
   launch_epilogue_zq(db->sum.as<uint32_t>(), db->out.as<uint64_t>(), g, maps, db->ctx->T, db->st);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(z, db->out.p, (size_t)SIMD * n * 8, cudaMemcpyDeviceToHost, db->st));
   CK(cudaStreamSynchronize(db->st));
+  db->pin_busy = false;
   memcpy(out_b, z, (size_t)SIMD * n * 8);
   return DNSPIR_OK;
 }

@@ -229,12 +229,16 @@ void launch_last_rows(const uint32_t* a_out, uint32_t* last, const Group& g, con
 // driver cannot encode them.
 size_t tscan_slab_map_bytes(int nshards);
 int tscan_slab_maps(uint8_t* const* host_slabs, int nshards, const Group& g, void* dev_maps);
-// Per-lane queries (perform_pir_split): qv = launch_scan_vectors of 8 queries,
-// one per lane.  sum: scan_lanes_sum_words of workspace.  -1 on a CUDA error.
+// Per-lane queries (perform_pir_split).  launch_lane_vectors: ring elements zq
+// [lane][query, conjugate, gk0, gk1][N] -> the scan vectors of 8 queries, one per
+// lane, and sum (scan_lanes_sum_words) cleared; ntt: their transforms' space at N >
+// 512.  launch_scan_lanes adds the scan up in sum.
+void launch_lane_vectors(const uint64_t* zq, uint32_t* ntt, uint32_t* qv, uint32_t* sum, const Group& g,
+                         const ScanConsts& sc, const SlotMaps& maps, const NttTables& T, cudaStream_t st);
 constexpr int SCAN_MAX_CHUNKS = 16;  // row chunks per half
 size_t scan_lanes_sum_words(const Group& g);
-int launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st);
-// Loads the kernels of launch_scan_vectors, launch_scan_lanes and
+void launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st);
+// Loads the kernels of launch_lane_vectors, launch_scan_lanes and
 // launch_epilogue_zq on the current device (0, or -1 on a CUDA error).
 int preload_pir_split_kernels();
 // Primary epilogue for nq queries: scan output -> b (iNTT, CRT), mod-switch,

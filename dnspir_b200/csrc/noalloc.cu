@@ -150,9 +150,9 @@ static int noalloc_queue(const DbView& v, const uint64_t* qry_b, const uint64_t*
     if (e == cudaSuccess)
       e = cudaMemcpy2DAsync((char*)zq + 2 * row, pitch, gk_b, 2 * row, 2 * row, SIMD, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) {
-      launch_ring_to_ntt(zq, SIMD * 4, ntt, nullptr, g.log2n, v.T, st);
-      launch_scan_vectors(ntt, 8 * n, 0, 2, SIMD, SIMD, qv, g, v.sc, v.maps, st);
-      if (launch_scan_lanes(v.slab, qv, sum, g, st) == 0) launch_epilogue_zq(sum, out_b, g, v.maps, v.T, st);
+      launch_lane_vectors(zq, ntt, qv, sum, g, v.sc, v.maps, v.T, st);
+      launch_scan_lanes(v.slab, qv, sum, g, st);
+      launch_epilogue_zq(sum, out_b, g, v.maps, v.T, st);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

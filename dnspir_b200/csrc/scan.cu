@@ -40,24 +40,12 @@ constexpr int SCAN_NT = 256;
 // output is 5 j: array 0 of every row but the last meets r[j] + C[5^-1 j].
 // The last row's state has no following t, so its C term is taken back (v = 2).
 // In (sign, e) order 5^-1 is e - 1.  States stored with a scale (ScanConsts xinv)
-// meet vectors divided by it.  One thread per slot, factor and query.
-__global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_stride, int s_q, int s_gk, int nb,
-                                    uint32_t* __restrict__ qv, Group g, ScanConsts sc,
-                                    const uint32_t* __restrict__ gtab) {
+// meet vectors divided by it.  One slot u and factor p of one query; at(slot, x):
+// the decoded vector of that slot at position x.
+template <class At>
+__device__ __forceinline__ void scan_vectors(const At& at, uint32_t u, int p, int s_q, int s_gk, uint32_t* o,
+                                             const Group& g, const ScanConsts& sc) {
   const uint32_t N = g.n, half = N / 2;
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= N) return;
-  const int p = blockIdx.y, q = blockIdx.z;
-  uint32_t* o = qv + (size_t)q * 2 * SCAN_VECS * 2 * N;
-  if (q >= nb) {
-    for (int h = 0; h < (int)g.H; h++)
-      for (int v = 0; v < SCAN_VECS; v++) o[scan_vec_off(N, h, v, p) + u] = 0;
-    return;
-  }
-  src += (size_t)q * q_stride;
-  auto at = [&](int slot, uint32_t x) {
-    return __ldg(src + ((size_t)slot * 2 + p) * N + ((__ldg(gtab + x) - 1) >> 1));
-  };
   const uint32_t pr = prime_of(p);
   const uint64_t mu = barrett_mu(pr);
   const uint32_t gk0 = at(s_gk, u), gk1 = at(s_gk + 1, u);
@@ -81,6 +69,58 @@ __global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_s
     o[scan_vec_off(N, h, 0, p) + u] = mul_mod(add_mod(r, cm, pr), sc.xinv[p], pr, mu);
     o[scan_vec_off(N, h, 1, p) + u] = sub_mod(g1, mul_mod(ka, r, pr, mu), pr);
     o[scan_vec_off(N, h, 2, p) + u] = cm ? pr - mul_mod(cm, sc.xinv[p], pr, mu) : 0;
+  }
+}
+
+// One thread per slot, factor and query.  sum: cleared for scan_lanes_kernel (or null).
+__global__ void scan_vectors_kernel(const uint32_t* __restrict__ src, size_t q_stride, int s_q, int s_gk, int nb,
+                                    uint32_t* __restrict__ qv, uint32_t* __restrict__ sum, Group g, ScanConsts sc,
+                                    const uint32_t* __restrict__ gtab) {
+  const uint32_t N = g.n;
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= N) return;
+  const int p = blockIdx.y, q = blockIdx.z;
+  uint32_t* o = qv + (size_t)q * 2 * SCAN_VECS * 2 * N;
+  if (sum) sum[((size_t)p * N + u) * SIMD + q] = 0;
+  if (q >= nb) {
+    for (int h = 0; h < (int)g.H; h++)
+      for (int v = 0; v < SCAN_VECS; v++) o[scan_vec_off(N, h, v, p) + u] = 0;
+    return;
+  }
+  src += (size_t)q * q_stride;
+  auto at = [&](int slot, uint32_t x) {
+    return __ldg(src + ((size_t)slot * 2 + p) * N + ((__ldg(gtab + x) - 1) >> 1));
+  };
+  scan_vectors(at, u, p, s_q, s_gk, o, g, sc);
+}
+
+// The same from the ring elements of a per-lane query, for N <= 512: one block per
+// lane and factor transforms the lane's elements (query, conjugate if the group
+// has one, both keys) in shared memory and takes the vectors from there.  A small
+// shard's call is a row of short kernels, and this is one instead of two: 45 us the
+// call instead of 50 at N = 64, 62 / 64 at 256; at N = 1024 (90 / 88) the 64 blocks of
+// separate transforms are worth their launch.
+constexpr int LANE_VECS_NT = 512;
+__global__ void __launch_bounds__(LANE_VECS_NT) lane_vectors_kernel(const uint64_t* __restrict__ zq,
+                                                                    uint32_t* __restrict__ qv,
+                                                                    uint32_t* __restrict__ sum, Group g,
+                                                                    ScanConsts sc, const uint32_t* __restrict__ gtab,
+                                                                    NttTables T) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const int lane = blockIdx.x, p = blockIdx.y;
+  const uint32_t N = g.n, pr = prime_of(p);
+  const uint64_t* src = zq + (size_t)lane * 4 * N;
+  const uint32_t gap = g.H == 2 ? 0 : N;  // no conjugate: its element is left out
+  for (uint32_t b = threadIdx.x; b < 4 * N - gap; b += LANE_VECS_NT)
+    sm[b] = reduce64(__ldg(src + b + (b < N ? 0 : gap)), pr, barrett_mu(pr));
+  __syncthreads();
+  ntt_fwd_smem(sm, g.log2n, g.H == 2 ? 4 : 3, T, p);
+  auto at = [&](int slot, uint32_t x) {
+    return sm[slot * N - (slot < 2 ? 0 : gap) + brv((__ldg(gtab + x) - 1) >> 1, g.log2n)];
+  };
+  for (uint32_t u = threadIdx.x; u < N; u += LANE_VECS_NT) {
+    sum[((size_t)p * N + u) * SIMD + lane] = 0;
+    scan_vectors(at, u, p, 0, 2, qv + (size_t)lane * 2 * SCAN_VECS * 2 * N, g, sc);
   }
 }
 
@@ -217,7 +257,7 @@ __global__ void __launch_bounds__(SCAN_NT, MINB) scan_batch_kernel(ScanArgs a) {
 // where it added up 256 (3.0 ms of a 3.5 ms call at N = 2048; the whole
 // set_db + get_a + split call 14.9 -> 11.6 ms);
 // the chunks' residues (at most 2 SCAN_MAX_CHUNKS = 32 of them, below 2^31 in
-// all) add up in `sum` [p][u][lane], zeroed before the launch.
+// all) add up in `sum` [p][u][lane], zeroed by the kernel that makes the vectors.
 constexpr int LANES_NT = 256;
 __global__ void __launch_bounds__(LANES_NT) scan_lanes_kernel(const uint32_t* __restrict__ slab,
                                                               const uint32_t* __restrict__ qv,
@@ -481,7 +521,19 @@ CrtConst host_crt_const();
 void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk, int nb, int nb_pad, uint32_t* qv,
                          const Group& g, const ScanConsts& sc, const SlotMaps& maps, cudaStream_t st) {
   const unsigned nt = g.n < 256 ? g.n : 256;
-  scan_vectors_kernel<<<dim3(g.n / nt, 2, nb_pad), nt, 0, st>>>(src, q_stride, s_q, s_gk, nb, qv, g, sc, maps.g);
+  scan_vectors_kernel<<<dim3(g.n / nt, 2, nb_pad), nt, 0, st>>>(src, q_stride, s_q, s_gk, nb, qv, nullptr, g, sc,
+                                                                maps.g);
+}
+
+void launch_lane_vectors(const uint64_t* zq, uint32_t* ntt, uint32_t* qv, uint32_t* sum, const Group& g,
+                         const ScanConsts& sc, const SlotMaps& maps, const NttTables& T, cudaStream_t st) {
+  if (g.n <= 512) {
+    const size_t smem = (size_t)4 * g.n * 4;
+    lane_vectors_kernel<<<dim3(SIMD, 2), LANE_VECS_NT, smem, st>>>(zq, qv, sum, g, sc, maps.g, T);
+    return;
+  }
+  launch_ring_to_ntt(zq, SIMD * 4, ntt, nullptr, g.log2n, T, st);
+  scan_vectors_kernel<<<dim3(g.n / 256, 2, SIMD), 256, 0, st>>>(ntt, 8 * (size_t)g.n, 0, 2, SIMD, qv, sum, g, sc, maps.g);
 }
 
 int scan_batch_supported(int B) { return B >= 1 && B <= 256 && (B & (B - 1)) == 0; }
@@ -524,14 +576,12 @@ int launch_scan_batch(uint32_t* const* slabs_dev, int nshards, const uint32_t* q
 
 size_t scan_lanes_sum_words(const Group& g) { return (size_t)2 * g.n * SIMD; }
 
-int launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st) {
-  if (cudaMemsetAsync(sum, 0, scan_lanes_sum_words(g) * 4, st) != cudaSuccess) return -1;
+void launch_scan_lanes(const uint32_t* slab, const uint32_t* qv, uint32_t* sum, const Group& g, cudaStream_t st) {
   const int nt = g.n / 2 < (uint32_t)LANES_NT ? (int)(g.n / 2) : LANES_NT;
   const int R = (int)std::max<uint32_t>(1, std::min<uint32_t>(SCAN_MAX_CHUNKS, g.L / 8));
   const uint32_t rows = (g.L + R - 1) / R;
   const size_t smem = (size_t)g.na * SIMD * (nt + rows - 1) * 4;
   scan_lanes_kernel<<<dim3(2 * (g.n / 2 / nt), g.H * R, 2), nt, smem, st>>>(slab, qv, sum, g, R);
-  return 0;
 }
 
 void launch_primary_epilogue(const uint32_t* fin, int nq, int nshards, const uint32_t* a_ms, const int* distinct_of,
@@ -570,6 +620,7 @@ int preload_pir_split_kernels() {
   // single-shard scan kernels now (cudaFuncGetAttributes forces the load)
   cudaFuncAttributes a;
   if (cudaFuncGetAttributes(&a, (const void*)scan_vectors_kernel) != cudaSuccess ||
+      cudaFuncGetAttributes(&a, (const void*)lane_vectors_kernel) != cudaSuccess ||
       cudaFuncGetAttributes(&a, (const void*)scan_lanes_kernel) != cudaSuccess ||
       cudaFuncGetAttributes(&a, (const void*)epilogue_zq_kernel) != cudaSuccess) {
     cudaGetLastError();
