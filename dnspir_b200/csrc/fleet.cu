@@ -114,23 +114,27 @@ int slot_acquire(dnspir_fleet* f, QSlot& s) {
 int fleet_drain(dnspir_fleet* f) {
   for (auto& s : f->slot)
     if (s.sec_pending) CK(cudaStreamWaitEvent(f->st, s.sec_done, 0));
-  // the error words come with the same wait
-  CKR(f->epin.ensure(ERR_BYTES));
-  CK(cudaMemcpyAsync(f->epin.p, f->err_words.p, ERR_BYTES, cudaMemcpyDeviceToHost, f->st));
+  // the error words come with the same wait; bounded waits are in the tensor
+  // scan and in the chains at N = 2048
+  const bool words = f->engine == DNSPIR_ENGINE_TENSOR || f->g1.log2n == LOG2_N_MAX;
+  if (words) {
+    CKR(f->epin.ensure(ERR_BYTES));
+    CK(cudaMemcpyAsync(f->epin.p, f->err_words.p, ERR_BYTES, cudaMemcpyDeviceToHost, f->st));
+  }
   CK(cudaStreamSynchronize(f->st));
   CK(cudaStreamSynchronize(f->sec));
   for (auto& s : f->slot) s.sec_pending = false;
-  if (f->epin.as<uint32_t>()[0] | f->epin.as<uint32_t>()[1]) {
+  if (words && (f->epin.as<uint32_t>()[0] | f->epin.as<uint32_t>()[1])) {
     CK(cudaMemset(f->err_words.p, 0, ERR_BYTES));
     return fail(DNSPIR_ERR_TIMEOUT, "a kernel's bounded wait gave up");
   }
   return DNSPIR_OK;
 }
 
-// Scan of the decoded queries in s.qnat (kernel batch Bk) into s.fin.
-int launch_scan(dnspir_fleet* f, QSlot& s, int nb, int Bk) {
+// Scan of nb decoded queries at qnat (kernel batch Bk) into s.fin.
+int launch_scan(dnspir_fleet* f, QSlot& s, const uint32_t* qnat, int nb, int Bk) {
   const Group& g1 = f->g1;
-  launch_scan_vectors(s.qnat.as<uint32_t>(), QV_WORDS_PER_QUERY * g1.n, 2, 0, nb, Bk, s.qv.as<uint32_t>(), g1,
+  launch_scan_vectors(qnat, QV_WORDS_PER_QUERY * g1.n, 2, 0, nb, Bk, s.qv.as<uint32_t>(), g1,
                       scan_consts(f->ap, g1, 0), slot_maps(f->ctx, g1.log2n), f->st);
   f->launches += 1;
   if (f->engine == DNSPIR_ENGINE_TENSOR) {
@@ -197,8 +201,8 @@ int fleet_kernel_batch(dnspir_fleet* f, int nb) {
 template <class Ensure>
 static int ensure_workspace(dnspir_fleet* f, const Ensure& ensure) {
   const int r = ensure();
-  if (r != DNSPIR_ERR_OOM || !f->ws.rows.p) return r;
-  f->ws.rows.release();
+  if (r != DNSPIR_ERR_OOM || !f->scratch_bytes()) return r;
+  f->release_scratch();
   return ensure();
 }
 
@@ -248,7 +252,7 @@ int fleet_primary_kernels(dnspir_fleet* f, QSlot& s, int nb, int Bk, const uint3
     f->launches += 1;
   }
   if (scan0) CK(cudaEventRecord(scan0, f->st));
-  CKR(launch_scan(f, s, nb, Bk));
+  CKR(launch_scan(f, s, s.qnat.as<uint32_t>(), nb, Bk));
   if (scan1) CK(cudaEventRecord(scan1, f->st));
   CK(cudaGetLastError());
   return DNSPIR_OK;
@@ -759,8 +763,7 @@ int dnspir_fleet_scan(dnspir_fleet* f, const uint32_t* qnat_dev, uint32_t nq, ui
     const int nb = (int)std::min<uint32_t>(f->batch, nq - g0);
     const int Bk = fleet_kernel_batch(f, nb);
     CKR(fleet_slot_workspace(f, s, Bk, nb, 0));
-    CK(cudaMemcpyAsync(s.qnat.p, qnat_dev + g0 * qv, (size_t)nb * qv * 4, cudaMemcpyDeviceToDevice, f->st));
-    CKR(launch_scan(f, s, nb, Bk));
+    CKR(launch_scan(f, s, qnat_dev + g0 * qv, nb, Bk));
     CK(cudaMemcpyAsync(out_dev + g0 * per_out, s.fin.p, (size_t)nb * per_out * 4, cudaMemcpyDeviceToDevice, f->st));
   }
   CK(cudaGetLastError());
@@ -874,11 +877,10 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
     }
   }
   CK(cudaGetLastError());
-  CKR(fleet_drain(f));
+  if (rows || tensor) CKR(fleet_drain(f));  // otherwise preprocess_shards has waited
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = true;
   // the scratch of a bulk load goes back; an update of a few shards keeps its own
-  f->tmp_lane.release();
-  if (f->ws.rows.bytes > EncodeWs::ROWS_KEPT) f->ws.rows.release();
+  if (f->scratch_bytes() > EncodeWs::ROWS_KEPT) f->release_scratch();
   return DNSPIR_OK;
 }
 

@@ -73,6 +73,12 @@ struct dnspir_fleet {
   std::vector<int> q_group;                   // per query of the last call: its group, or -1
   uint64_t launches = 0;                      // kernels launched by the answer pipeline so far
   std::mutex mu;
+  // scratch of set_shards that outlives it (EncodeWs::ROWS_KEPT)
+  size_t scratch_bytes() const { return ws.rows.bytes + tmp_lane.bytes; }
+  void release_scratch() {
+    ws.rows.release();
+    tmp_lane.release();
+  }
   ~dnspir_fleet();
 };
 

@@ -402,7 +402,7 @@ int dnspir_server_start(dnspir_server* sv, int use_graphs) {
     Db& db = *dbp;
     dnspir_fleet* f = db.f;
     std::lock_guard<std::mutex> lk(f->mu);
-    f->ws.rows.release();  // no shard is prepared while the fleet is served
+    f->release_scratch();  // no shard is prepared while the fleet is served
     for (int nb = db.max_batch;; nb = nb / 2) {
       if (nb < 1) return fail(DNSPIR_ERR_OOM, "no group size fits in device memory");
       const int bk = bk_max_of(f, nb);
