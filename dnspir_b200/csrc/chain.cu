@@ -1087,7 +1087,6 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // it out of the steps' code: one query's 1024 steps as long as without it (2.64 ms the
 // call), a shard's 0.9 % longer; with a way out of the loop, a guard around the
 // sends or a flag asked in each step they took 1 to 5 % longer.
-constexpr uint64_t PEER_WAIT_NS = 2000000000ull;
 // The states a and b^ are kept apart from the transforms' work space and
 // transposed, position 8 t + m at word 256 m + t: sigma_5 maps a warp's
 // positions of one m to 32 positions whose t differ mod 32, so its gathers have
@@ -1578,7 +1577,7 @@ static ChainArgs chain_args(const Group& g, const ChainConsts& cc, const NttTabl
 
 static void set_limits(ChainArgs& a, uint32_t* err, const WaitLimits& lim) {
   a.err = err;
-  a.wait_ns = lim.wait_ns ? lim.wait_ns : PEER_WAIT_NS;
+  a.wait_ns = lim.ns();
   a.withhold = lim.withhold_step < 0 ? ~0u : (uint32_t)lim.withhold_step;
 }
 

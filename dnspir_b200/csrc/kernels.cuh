@@ -101,7 +101,9 @@ __host__ __device__ __forceinline__ size_t scan_vec_off(uint32_t n, int h, int v
 void launch_scan_vectors(const uint32_t* src, size_t q_stride, int s_q, int s_gk, int nb, int nb_pad, uint32_t* qv,
                          const Group& g, const ScanConsts& sc, const SlotMaps& maps, cudaStream_t st);
 
-// Limits of the bounded waits inside kernels, wait_ns (0: the default, 2 s), and
+// Limits of the bounded waits inside kernels, wait_ns (0: the default, 2 s; at
+// least 0.1 ms, since a block that gave up waits under the same limit for its
+// copies in flight, which take microseconds, before its memory is released), and
 // the test hooks of the paths they end in (-1: off): the tensor scan's first
 // block stops copying before chunk `withhold`, the second block of the first
 // paired chain leaves before step `withhold_step`, in groups of `only_group`
@@ -111,6 +113,7 @@ struct WaitLimits {
   int withhold = -1;
   int withhold_step = -1;
   int only_group = 0;
+  uint64_t ns() const { return wait_ns == 0 ? 2000000000ull : wait_ns < 100000 ? 100000 : wait_ns; }
   WaitLimits of_group(int nb) const {
     WaitLimits l = *this;
     if (only_group && only_group != nb) l.withhold = l.withhold_step = -1;

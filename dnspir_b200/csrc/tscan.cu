@@ -47,7 +47,6 @@ namespace {
 
 constexpr uint32_t TBLK = 16384;  // one 128 x 128-byte block
 constexpr int TSCAN_NT = 128;
-constexpr uint64_t WAIT_NS = 2000000000ull;
 
 __device__ __forceinline__ uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -1328,7 +1327,7 @@ int launch_tscan(uint8_t* const* slabs_dev, int nshards, const uint32_t* qv, int
   a.kc_total = kc;
   a.groups = nb_pad / qpc;
   a.stages = 0;
-  a.wait_ns = lim.wait_ns ? lim.wait_ns : WAIT_NS;
+  a.wait_ns = lim.ns();
   a.withhold = lim.withhold < 0 ? ~0u : (uint32_t)lim.withhold;
   a.tmaps = static_cast<const CUtensorMap*>(slab_maps);
   a.qv = qv;

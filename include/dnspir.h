@@ -199,9 +199,9 @@ int dnspir_fleet_get_schedule(dnspir_fleet* fleet, uint32_t batch, int* schedule
  * returns to the default.  No counterpart in the reference. */
 int dnspir_fleet_set_tile(dnspir_fleet* fleet, uint32_t batch, int shape_index);
 /* Limit of every wait between threads of a kernel that is not a hardware barrier
- * (wait_ns; 0 restores the default of 2 s): in the tensor scan's
- * copy/MMA/epilogue pipeline, and between the two blocks of a paired chain in
- * the secondary phase and in set_shards.  A wait that runs out makes the
+ * (wait_ns; 0 restores the default of 2 s, less than 0.1 ms counts as 0.1 ms):
+ * in the tensor scan's copy/MMA/epilogue pipeline, and between the two blocks of a
+ * paired chain in the secondary phase and in set_shards.  A wait that runs out makes the
  * blocks stop, wait (bounded) for their copies in flight, free their
  * tensor memory and return; the call then fails with DNSPIR_ERR_TIMEOUT and
  * the device stays usable.  withhold_chunk >= 0 is a test hook for that path:

@@ -65,3 +65,25 @@ def test_answers_time_out_and_recover(engine):
     assert r == orc.process_query([ref, ref], q, l2)
     assert np.array_equal(orc.process_reply(r, seed), data[0][4000].astype(np.int64))
     fleet.close()
+
+
+@pytest.mark.parametrize("engine", [dp.ENGINE_CUDA_CORES, dp.ENGINE_TENSOR])
+def test_shortest_limit_leaves_the_device_usable(engine):
+    # nothing is withheld: whether a wait of a busy device outlasts the limit or
+    # not, the call answers rightly or says that it timed out
+    l1, l2 = 1024, 16
+    data = np.random.default_rng(6).integers(0, orc.T, size=(1, 8 * l1, 2048), dtype=np.uint16)
+    fleet = dp.Fleet.general(11, l1, l2, 2, 1)
+    fleet.set_engine(engine)
+    fleet.set_shards(0, data)
+    fleet.set_batch(4)
+    queries = [dp.prepare_query(bytes([k]) + bytes(31), 900 * k, k % 2, l1, l2)[0] for k in range(8)]
+    want = fleet.process_queries(queries)
+    for ns in (1, 1, 100_000, 0):
+        fleet.set_wait_limit(ns)
+        try:
+            assert fleet.process_queries(queries) == want
+        except dp.DnspirError as e:
+            assert e.code == 5 and ns
+    assert fleet.process_queries(queries) == want
+    fleet.close()
