@@ -641,9 +641,10 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
   if (count != want) return fail(DNSPIR_ERR_BAD_SIZE, "set_db needs exactly 8 * group_order entries of N coefficients");
   DeviceGuard dg(db->device);
   const uint16_t* src = entries;
-  if (!entries_on_device) {
+  if (!entries_in_place(entries, entries_on_device)) {
     CKR(db->ws.in16.ensure(want * 2));
-    CK(cudaMemcpyAsync(db->ws.in16.p, entries, want * 2, cudaMemcpyHostToDevice, db->st));
+    CK(cudaMemcpyAsync(db->ws.in16.p, entries, want * 2,
+                       entries_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, db->st));
     src = db->ws.in16.as<uint16_t>();
   }
   db->ready = false;

@@ -841,8 +841,9 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   // without chain rows the tensor engine preprocesses into lane-layout scratch
   // and re-tiles from there, four shards at a time
   uint32_t batch = std::min(count, tensor && !rows ? 4 : preprocess_batch(f->g1));
+  const bool in_place = entries_in_place(entries, entries_on_device);
   auto reserve = [&] {
-    if (!entries_on_device) CKR(f->ws.in16.ensure((size_t)batch * per * 2));
+    if (!in_place) CKR(f->ws.in16.ensure((size_t)batch * per * 2));
     if (tensor && !rows) CKR(f->tmp_lane.ensure((size_t)batch * words * 4));
     return preprocess_reserve(f->g1, batch, f->ws);
   };
@@ -857,8 +858,9 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   for (uint32_t b0 = 0; b0 < count; b0 += batch) {
     const uint32_t cnt = std::min(count - b0, batch), d0 = first + b0;
     const uint16_t* src = entries + (size_t)b0 * per;
-    if (!entries_on_device) {
-      CK(cudaMemcpyAsync(f->ws.in16.p, src, (size_t)cnt * per * 2, cudaMemcpyHostToDevice, f->st));
+    if (!in_place) {
+      CK(cudaMemcpyAsync(f->ws.in16.p, src, (size_t)cnt * per * 2,
+                         entries_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, f->st));
       src = f->ws.in16.as<uint16_t>();
     }
     uint64_t* const a_zq = f->a_zq.as<uint64_t>() + d0 * n8;

@@ -144,6 +144,12 @@ bool reduced(const uint64_t* v, size_t n);
 int preprocess_shards(DeviceCtx* c, const APartConsts& ap, const Group& g, int used_seeds, uint32_t* const* slabs_host,
                       int count, const uint16_t* entries_dev, uint64_t* a_zq, uint32_t* a_ms, EncodeWs& ws,
                       uint32_t* err, const WaitLimits& lim, cudaStream_t st, uint32_t* last = nullptr);
+// Whether the encoder may read the caller's entries where they are: on the device
+// and on an 8-byte boundary (four coefficients a load); a view that starts on
+// another coefficient is copied.
+inline bool entries_in_place(const uint16_t* entries, int on_device) {
+  return on_device && reinterpret_cast<uintptr_t>(entries) % 8 == 0;
+}
 // Shards that one call of preprocess_shards may carry, and its scratch for `count`.
 uint32_t preprocess_batch(const Group& g);
 int preprocess_reserve(const Group& g, uint32_t count, EncodeWs& ws);
