@@ -658,6 +658,7 @@ int dnspir_db_set_db(dnspir_db* db, const uint16_t* entries, uint64_t count, int
     CK(cudaEventSynchronize(db->noalloc_done));
     if (db->slab) CK(cudaFree(db->slab));
     db->slab = nullptr;
+    db->ws.rows.release();  // three arrays a row are made without them
     db->g.na = na;
     CK(cudaMalloc(&db->slab, slab_words(db->g) * 4));
   }

@@ -826,6 +826,7 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
     if (na != f->g1.na || !f->slabs[f->D - 1]) {
       // these a-parts need the other slab layout (slab_off): new slabs
       CK(cudaStreamSynchronize(f->st));
+      f->release_scratch();
       for (uint32_t*& p : f->slabs) {
         if (p) CK(cudaFree(p));
         p = nullptr;
@@ -850,8 +851,14 @@ int dnspir_fleet_set_shards(dnspir_fleet* f, uint32_t first, uint32_t count, con
   for (;;) {
     const int r = reserve();
     if (r == DNSPIR_OK) break;
-    // fewer shards at a time where device memory is short
-    if (r != DNSPIR_ERR_OOM || batch <= 1) return r;
+    if (r != DNSPIR_ERR_OOM) return r;
+    // where device memory is short, what an earlier call left goes first, then
+    // fewer shards at a time
+    if (f->scratch_bytes()) {
+      f->release_scratch();
+      continue;
+    }
+    if (batch <= 1) return r;
     batch = (batch + 1) / 2;
   }
   for (uint32_t i = 0; i < count; i++) f->ready[first + i] = false;

@@ -74,6 +74,38 @@ def test_answers_take_the_scratch_where_memory_is_short():
     fleet.close()
 
 
+def test_updates_and_new_layouts_take_the_kept_scratch_where_memory_is_short():
+    # an update from host memory needs staging (32 MiB a shard) besides the rows,
+    # a-parts with a zero slot need slabs half as large again (1 -> 1.5 GiB)
+    torch = pytest.importorskip("torch")
+    shards, l2 = 4, 32
+    data, queries = _load(torch, shards, l2)
+    host = data.cpu().numpy()
+    fleet = dp.Fleet.general(11, 1024, l2, shards)
+    fleet.set_shards(0, data)
+    want = [fleet.process_query(q) for q, _ in queries]
+    hold = torch.empty(_free(torch) - (16 << 20), dtype=torch.uint8, device="cuda")
+    fleet.set_shards(1, host[1:2])
+    assert [fleet.process_query(q) for q, _ in queries] == want
+    del hold
+    torch.cuda.empty_cache()
+    fleet.set_shards(0, data)
+    hold = torch.empty(_free(torch) - GIB // 4, dtype=torch.uint8, device="cuda")
+    parts = dp.get_a_parts(11).copy()
+    parts[2] = 0
+    try:
+        dp.set_a_parts(11, parts)
+        fleet.set_shards(0, data)
+    finally:
+        dp.set_a_parts(11, None)
+        del hold
+        torch.cuda.empty_cache()
+    assert fleet.slab_bytes == shards * dp.required_memory_general(11, 1024) * 32
+    fleet.set_shards(0, data)
+    assert [fleet.process_query(q) for q, _ in queries] == want
+    fleet.close()
+
+
 def test_serving_starts_with_the_scratch_returned():
     torch = pytest.importorskip("torch")
     shards, l2 = 4, 32
