@@ -1085,7 +1085,7 @@ __global__ void __launch_bounds__(256, 3) primary_chain2k_kernel(ChainArgs a, ui
 // all, the block raises the error word and ends there: it arms and sends no more,
 // so the peer's next wait runs out too.  That path never comes back, which keeps
 // it out of the steps' code: one query's 1024 steps as long as without it (2.64 ms the
-// call), a shard's 0.9 % longer; with a way out of the loop, a guard around the
+// call), a shard's 0.7 % longer; with a way out of the loop, a guard around the
 // sends or a flag asked in each step they took 1 to 5 % longer.
 // The states a and b^ are kept apart from the transforms' work space and
 // transposed, position 8 t + m at word 256 m + t: sigma_5 maps a warp's
@@ -1126,9 +1126,6 @@ __device__ __forceinline__ bool peer_done_within(uint32_t bar, uint32_t parity, 
 // byte went to the next phase, which cannot have begun to complete while this
 // thread is here, and is taken back.
 __device__ __forceinline__ bool wait_peer(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-#pragma unroll 1
-  for (int k = 0; k < 64; k++)
-    if (peer_done(bar, parity)) return true;
   if (peer_done_within(bar, parity, limit_ns)) return true;
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
   if (!peer_done(bar, parity)) return false;
